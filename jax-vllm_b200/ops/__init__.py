@@ -1312,7 +1312,7 @@ def gate_heads(o: torch.Tensor, gate: torch.Tensor | None) -> torch.Tensor:
 def bmm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """One product per head: out[h] = a[h] @ w[h].T, a [heads, n, k] (any strides with unit inner stride),
     w [heads, m, k] contiguous, out [heads, n, m] (made contiguous if not given; given, any strides with unit
-    inner stride).  float32 operands: the CUDA-core product of this package, k ascending (csrc/gemm_simt.cu);
+    inner stride).  float32 operands: the CUDA-core product of this package (csrc/gemm_simt.cu);
     bfloat16: the library's batched product (as the prompt products of this package are the library's)."""
     _cuda(a, "a", contiguous=False); _cuda(w, "w", a.dtype)
     heads, n, k = a.shape

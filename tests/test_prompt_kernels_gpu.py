@@ -1,0 +1,57 @@
+"""Kernels that take over from a general one over part of its range, at the sizes where they can go wrong: edges of tiles,
+remainders, the smallest and the largest they take.  Compared with 64-bit arithmetic; the tolerances are bounds on 32-bit sums
+unless a test says otherwise."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+EPS32 = 2.0 ** -24
+
+
+def _ops():
+    from jax_vllm_b200 import ops
+    return ops
+
+
+def _rand(*shape, seed, dtype=torch.float32, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(shape, generator=g, device="cuda") * scale).to(dtype)
+
+
+def _entries(lengths):
+    cu = torch.tensor([0] + lengths, device="cuda").cumsum(0).to(torch.int32)
+    slots = torch.tensor([len(lengths) - i for i in range(len(lengths))], dtype=torch.int32, device="cuda")
+    return cu, slots, len(lengths) + 2
+
+
+# ------------------------------------------------------------------------------- the 32-bit product
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 16, 17, 64, 65, 200])
+@pytest.mark.parametrize("n,k", [(1, 1), (31, 5), (33, 127), (64, 128), (65, 129), (100, 260), (700, 1000), (64, 2304)])
+def test_product_32bit(m, n, k):
+    ops = _ops()
+    for xd, wd, od in ((torch.float32, torch.float32, torch.float32), (torch.bfloat16, torch.float32, torch.bfloat16),
+                       (torch.float32, torch.bfloat16, torch.float32)):
+        x, w = _rand(m, k + 3, seed=m, dtype=xd)[:, :k], _rand(n, k, seed=n + k, dtype=wd)
+        for a in (x, x.contiguous()):                   # rows off and on 16-byte boundaries
+            y = ops.gemm_simt(a, w, od)
+            want = x.double() @ w.double().T
+            bound = (k + 2) * EPS32 * (x.double().abs() @ w.double().abs().T) + 1e-30
+            if od == torch.bfloat16:
+                bound = bound + want.abs() * 2.0 ** -8
+            assert ((y.double() - want).abs() <= bound).all()
+        # the sum of a row does not depend on the other rows of the batch
+        for rows in (1, 5, 16, 40):
+            if rows < m:
+                assert torch.equal(ops.gemm_simt(x[:rows], w, od), y[:rows])
+
+
+@pytest.mark.parametrize("heads,n,k,m", [(3, 1, 36, 20), (5, 70, 64, 130), (16, 20, 128, 512)])
+def test_product_32bit_batched(heads, n, k, m):
+    ops = _ops()
+    a, w = _rand(n, heads, k + 5, seed=1)[:, :, :k].transpose(0, 1), _rand(heads, m, k, seed=2)
+    out = torch.full((n, heads, m + 3), 7.0, device="cuda")
+    ops.bmm_heads(a, w, out=out[:, :, :m].transpose(0, 1))
+    want = torch.einsum("hnk,hmk->nhm", a.double(), w.double())
+    bound = (k + 2) * EPS32 * torch.einsum("hnk,hmk->nhm", a.double().abs(), w.double().abs())
+    assert ((out[:, :, :m].double() - want).abs() <= bound).all() and (out[:, :, m:] == 7.0).all()
