@@ -34,7 +34,7 @@
 //
 // jv_head_norm_gate finishes all: each head's output divided by its root mean square, times a weight per element (of all
 // heads, or one vector that the heads share), times sigmoid(gate) or silu(gate), rounded for the output product.
-#include "common.cuh"
+#include "scan.cuh"
 #include <math.h>
 
 namespace {
@@ -220,19 +220,6 @@ struct ScanParams {
   int* status;
 };
 
-// Which entry and which of its segments the segment number g is; false if there is no such segment.
-__device__ __forceinline__ bool find_segment(const int* __restrict__ cu_seqlens, int n_entries, int seg_len, int g,
-                                             int& entry, int& seg, int& n_seg) {
-  int acc = 0;
-  for (int e = 0; e < n_entries; ++e) {
-    const int len = cu_seqlens[e + 1] - cu_seqlens[e];
-    const int ns = max(1, (len + seg_len - 1) / seg_len);
-    if (g < acc + ns) { entry = e; seg = g - acc; n_seg = ns; return true; }
-    acc += ns;
-  }
-  return false;
-}
-
 constexpr int SCAN_THREADS = 128;    // with the removal term: 4 warps of 8 columns x 4 key lanes
 constexpr int SCAN_COLS = 32;
 
@@ -240,17 +227,6 @@ template <int KPT> struct ScanShape {
   static constexpr int ROW = 4 * (KPT + 4);          // floats of one vector in shared memory: a lane's KPT channels, 4 of padding
   static constexpr int CHUNK = KPT >= 64 ? 4 : 8;    // tokens per stage
 };
-
-__device__ __forceinline__ void cp_async_4(float* dst, const float* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_16(float* dst, const float* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <int KPT, typename T>
 __global__ void __launch_bounds__(SCAN_THREADS) state_scan_kernel(const ScanParams p) {

@@ -50,6 +50,8 @@ class _StateMixer(Part):
 
 
 class DeltaRule(_StateMixer):
+    kernels = _StateMixer.kernels + ("delta_scan",)
+
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx
         self.prefix = f"{prefix}.{spec.prefix}" if spec.prefix else prefix
@@ -93,8 +95,12 @@ class DeltaRule(_StateMixer):
         hd, dt = self.hd, self.ctx.dtype
         low = ops.unary_act(row[:, 5 * hd:5 * hd + self.rank], "tanh")
         zw = ops.linear(low, self.w_up, dt)
-        packed = ops.delta_prepare(row, 0, hd, 4 * hd, zw, self.a_bias, self.w_bias, self.h, self.d)
-        o = ops.state_scan(packed, row, 2 * hd, cache.state, step.cu_seqlens, step.state_slots, step.n_entries, self.d)
+        if step.n_tokens >= ops.DELTA_GROUP_MIN_TOKENS * step.n_entries:
+            o = ops.delta_scan(row, 0, hd, 4 * hd, 2 * hd, zw, self.a_bias, self.w_bias, cache.state, step.cu_seqlens,
+                               step.state_slots, step.n_entries, self.h, self.d, self.d)
+        else:
+            packed = ops.delta_prepare(row, 0, hd, 4 * hd, zw, self.a_bias, self.w_bias, self.h, self.d)
+            o = ops.state_scan(packed, row, 2 * hd, cache.state, step.cu_seqlens, step.state_slots, step.n_entries, self.d)
         return ops.head_norm_gate(o, self.norm, row[:, 3 * hd:4 * hd], out, self.h, self.d, self.spec.norm_eps)
 
 

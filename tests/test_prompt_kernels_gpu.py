@@ -55,3 +55,44 @@ def test_product_32bit_batched(heads, n, k, m):
     want = torch.einsum("hnk,hmk->nhm", a.double(), w.double())
     bound = (k + 2) * EPS32 * torch.einsum("hnk,hmk->nhm", a.double().abs(), w.double().abs())
     assert ((out[:, :, :m].double() - want).abs() <= bound).all() and (out[:, :, m:] == 7.0).all()
+
+
+# ------------------------------------------------------------------- the delta rule, four tokens at a time
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dim,columns", [(1, 1), (7, 7), (32, 16), (33, 17), (64, 64), (65, 33), (128, 128), (200, 40), (256, 18)])
+def test_delta_four_tokens_at_a_time(dim, columns, dtype):
+    from tests.plain.nufapel_plain import delta_decay, delta_scan
+    ops, heads, lengths = _ops(), 2, [1, 4, 70, 3, 5, 2, 17, 64]
+    cu, slots, n_slots = _entries(lengths)
+    n, hd, hv = sum(lengths), heads * dim, heads * columns
+    proj = _rand(n, 3 * hd + hv + 1, seed=dim, dtype=dtype)[:, 1:]
+    zw, ab, wb = _rand(n, hd, seed=3, dtype=dtype), _rand(hd, seed=4), _rand(hd, seed=5)
+    state = _rand(n_slots, hd * columns + 3, seed=6)
+    before = state.clone()
+    out = ops.delta_scan(proj, 0, hd, 2 * hd, 3 * hd, zw, ab, wb, state, cu, slots, len(lengths), heads, dim, columns)
+    p = proj.double().cpu()
+    r, k, za = (p[:, i * hd:(i + 1) * hd].view(n, heads, dim) for i in range(3))
+    v = p[:, 3 * hd:].view(n, heads, columns)
+    w = delta_decay(zw.double().cpu() + wb.double().cpu()).view(n, heads, dim)
+    a = torch.sigmoid(za + ab.double().cpu().view(heads, dim))
+    at = 0
+    for e, length in enumerate(lengths):
+        s = int(slots[e])
+        o, S = delta_scan(*(t[at:at + length] for t in (r, k, v, w, a)), before[s, :hd * columns].double().cpu().view(heads, dim, columns))
+        # sums of up to 256 terms, carried over up to 70 tokens by decays below one
+        for got, want in ((out[at:at + length].cpu().view(length, heads, columns), o), (state[s, :hd * columns].cpu().view_as(S), S)):
+            assert (got.double() - want).norm() <= 4e-6 * want.norm()
+        assert torch.equal(state[s, hd * columns:], before[s, hd * columns:])
+        at += length
+    for s in set(range(n_slots)) - set(slots.tolist()):
+        assert torch.equal(state[s], before[s])
+
+
+def test_delta_later_infinity_stays_out_of_earlier_outputs():
+    ops, heads, dim, n = _ops(), 1, 16, 8
+    cu, slots, n_slots = _entries([n])
+    proj = _rand(n, 4 * dim, seed=1)
+    proj[6, 3 * dim + 2] = float("inf")                  # a value of the third token of the second group
+    zw, b = _rand(n, dim, seed=2), _rand(dim, seed=3)
+    out = ops.delta_scan(proj, 0, dim, 2 * dim, 3 * dim, zw, b, b, _rand(n_slots, dim * dim, seed=4), cu, slots, 1, heads, dim, dim)
+    assert torch.isfinite(out[:6]).all() and not torch.isfinite(out[6, 2]) and torch.isfinite(out[:, :2]).all()
