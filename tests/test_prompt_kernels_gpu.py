@@ -96,3 +96,25 @@ def test_delta_later_infinity_stays_out_of_earlier_outputs():
     zw, b = _rand(n, dim, seed=2), _rand(dim, seed=3)
     out = ops.delta_scan(proj, 0, dim, 2 * dim, 3 * dim, zw, b, b, _rand(n_slots, dim * dim, seed=4), cu, slots, 1, heads, dim, dim)
     assert torch.isfinite(out[:6]).all() and not torch.isfinite(out[6, 2]) and torch.isfinite(out[:, :2]).all()
+
+
+# ------------------------------------------------------------------------- heads normed and gated
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("columns,off", [(2, 0), (63, 0), (64, 0), (64, 1), (66, 0), (128, 4), (130, 0), (256, 0), (500, 4), (512, 0), (516, 0)])
+def test_head_norm_gate_widths(columns, off, dtype):
+    ops, n, heads = _ops(), 5, 3
+    o, gates = _rand(n, heads * columns, seed=1), _rand(n, heads, 4, seed=2)
+    wide = _rand(n, heads * columns + 8, seed=3, dtype=dtype)
+    gate = wide[:, off:off + heads * columns]
+    for shared, act, mem in ((False, "sigmoid", None), (True, "silu", None), (False, "sigmoid", gates)):
+        weight = _rand(columns if shared else heads * columns, seed=4)
+        out = torch.full((n, heads * columns + 8), 9.0, device="cuda", dtype=dtype)
+        got = ops.head_norm_gate(o, weight, gate, out[:, off:off + heads * columns], heads, columns, 1e-5, gates=mem, gate_act=act)
+        y = o.double().view(n, heads, columns)
+        if mem is not None:
+            y = y / (torch.maximum(mem[:, :, 3].double().abs(), torch.exp(-mem[:, :, 2].double())) + 1e-6)[:, :, None]
+        y = y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5) * weight.double().view(-1, columns)
+        z = gate.double().reshape(n, heads, columns)
+        y = y * torch.sigmoid(z) * (z if act == "silu" else 1.0)
+        assert ((got.double().reshape(y.shape) - y).abs() <= (2e-6 if dtype == torch.float32 else 2.0 ** -8) * y.abs() + 1e-7).all()
+        assert (out[:, :off] == 9.0).all() and (out[:, off + heads * columns:] == 9.0).all()
