@@ -1784,6 +1784,14 @@ def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
             raise KernelError("state_scan: the normaliser does not fit")
         nq = gates.data_ptr() + 3 * 4
     out = torch.empty((n, heads * value_dim), dtype=torch.float32, device=packed.device)
+    if segment is None and n == n_entries:         # single tokens: the state is read and written once (csrc/state_step.cu)
+        f = _fn("state_step", "jv_state_step", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p, c_longlong,
+                                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
+                                                c_void_p, c_void_p])
+        _check(f(packed.data_ptr(), 1 if nv == 5 else 0, v.data_ptr(), _code(v, "v"), v.stride(0), v_off, out.data_ptr(),
+                 state.data_ptr(), state.stride(0), cu_seqlens.data_ptr(), slots.data_ptr(), state.shape[0], n_entries, heads, dim,
+                 value_dim, _ptr(state_n), nq, 4, _status_ptr(packed.device), _stream()), "state_step")
+        return out
     if segment is None:
         # with the removal term a segment carries `dim` more columns and the chain is a matrix product a segment: at
         # the sizes measured (32 heads of 64, 2,048 tokens) the three launches take longer than the one

@@ -23,7 +23,7 @@ from .registry import register_mixer
 
 
 class StateSpace(Part):
-    kernels = ("short_conv", "mamba2", "recurrent", "gemm_simt")
+    kernels = ("short_conv", "mamba2", "recurrent", "state_step", "gemm_simt")
 
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx

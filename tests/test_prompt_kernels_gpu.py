@@ -118,3 +118,23 @@ def test_head_norm_gate_widths(columns, off, dtype):
         y = y * torch.sigmoid(z) * (z if act == "silu" else 1.0)
         assert ((got.double().reshape(y.shape) - y).abs() <= (2e-6 if dtype == torch.float32 else 2.0 ** -8) * y.abs() + 1e-7).all()
         assert (out[:, :off] == 9.0).all() and (out[:, off + heads * columns:] == 9.0).all()
+
+
+# ------------------------------------------------------------------------------ states, one token each
+@pytest.mark.parametrize("dim,columns", [(1, 1), (7, 5), (64, 64), (65, 130), (128, 256), (129, 12), (256, 96)])
+@pytest.mark.parametrize("removal", [True, False])
+def test_state_single_tokens(dim, columns, removal):
+    ops, heads, entries = _ops(), 3, 5
+    for dtype, extra in ((torch.bfloat16, 0), (torch.float32, 3)):       # state rows on and off 16-byte boundaries
+        packed = _rand(entries, heads, 5 if removal else 3, dim, seed=dim)
+        v = _rand(entries, heads * columns + 2, seed=2, dtype=dtype)
+        cu, slots, n_slots = _entries([1] * entries)
+        rows = _rand(n_slots, heads * dim * (columns + 1) + extra, seed=3)
+        runs = []
+        for segment in (None, 0):                        # the kernel for single tokens, the scan of whole entries
+            st, gates = rows.clone(), torch.zeros(entries, heads, 4, device="cuda")
+            more = {} if removal else dict(state_n=st[:, heads * dim * columns:heads * dim * (columns + 1)], gates=gates)
+            o = ops.state_scan(packed, v, 2, st, cu, slots, entries, columns, segment=segment, **more)
+            runs.append((o, st, gates[:, :, 3]))
+        for got, want in zip(*runs):                     # sums of up to 256 terms in two orders
+            assert (got.double() - want.double()).norm() <= 2e-6 * want.double().norm() + 1e-30
