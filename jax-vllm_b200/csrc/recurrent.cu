@@ -29,8 +29,8 @@
 // computed.  With the removal term (state_scan_kernel) a warp holds 8 columns x 4 lanes that share the key channels, and
 // the two dot products of a token are two shuffles each.  Without it (column_scan_kernel) a thread holds a block of the
 // state, a part of the key channels x 4 columns, so that what it reads of the vectors serves four columns, in packed
-// pairs of channels; 8 or 16 lanes share the channels and sum the four outputs in four or five shuffles.  A step of single tokens is the
-// same kernel with one token an entry: it then reads and writes the state once, which is all its traffic.
+// pairs of channels; 8 or 16 lanes share the channels and sum the four outputs in four or five shuffles.  Steps of single tokens run on
+// state_step.cu, long portions with one decay a head on chunk_scan.cu, and portions of the delta rule on delta_scan.cu.
 //
 // jv_head_norm_gate finishes all: each head's output divided by its root mean square, times a weight per element (of all
 // heads, or one vector that the heads share), times sigmoid(gate) or silu(gate), rounded for the output product.
@@ -934,7 +934,7 @@ JV_EXPORT int jv_gla_prepare(const void* proj, int dtype, long long stride, int 
 
 // proj as above with q, k (heads * D each) and the two gates' pre-activations (heads each) at the given columns;
 // gates: [n, heads, 4] float (keep, take, running maximum; the fourth place is left for the scan's n . q); packed:
-// [n, heads, 3, D] float; state_m: the running maximum of slot 0, rows `slot_stride` floats apart.
+// [n, heads, 3, D] float (null: the gates alone); state_m: the running maximum of slot 0, rows `slot_stride` floats apart.
 JV_EXPORT int jv_memory_gates(const void* proj, int dtype, long long stride, int q_off, int k_off, int i_off, int f_off,
                               const void* i_bias, const void* f_bias, int w_dtype, float cap, float q_scale, float* gates,
                               float* packed, float* state_m, long long slot_stride, const int* cu_seqlens,
@@ -945,7 +945,7 @@ JV_EXPORT int jv_memory_gates(const void* proj, int dtype, long long stride, int
     const int rc = jv_launch(gate_scan_kernel<T, W>, dim3(entries, heads), dim3(32), 0, stream, (const T*)proj, stride,
                              i_off, f_off, (const W*)i_bias, (const W*)f_bias, cap, gates, state_m, slot_stride,
                              cu_seqlens, slots, n_slots, heads, status);
-    if (rc != JV_OK) return rc;
+    if (rc != JV_OK || packed == nullptr) return rc;
     return jv_launch(memory_prepare_kernel<T>, dim3(n, heads), dim3(D > 64 ? 128 : 64), 0, stream, (const T*)proj, stride,
                      q_off, k_off, q_scale, (const float*)gates, packed, heads, D);
   }));

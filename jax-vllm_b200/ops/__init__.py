@@ -1710,11 +1710,12 @@ def gla_prepare(proj: torch.Tensor, q_off: int, k_off: int, low_off: int, w_up: 
 
 def memory_gates(proj: torch.Tensor, q_off: int, k_off: int, i_off: int, f_off: int, i_bias: torch.Tensor,
                  f_bias: torch.Tensor, cap: float, q_scale: float, state_m: torch.Tensor, cu_seqlens: torch.Tensor,
-                 slots: torch.Tensor, n_entries: int, heads: int, dim: int):
+                 slots: torch.Tensor, n_entries: int, heads: int, dim: int, gates_only: bool = False):
     """The gates of a matrix memory with exponential gating: the running maximum `state_m` [slots, heads] (a view of
     the state rows) is scanned over every entry's tokens, then all tokens at once are prepared.  Returns (packed
     float32 [n, heads, 3, dim]: the scaled query, the key times its input gate, the decay; gates float32 [n, heads,
-    4]: decay, input gate, running maximum, and a place that `state_scan` fills with n . q)."""
+    4]: decay, input gate, running maximum, and a place that the scan fills with n . q).  With `gates_only` (for `chunk_scan`) the
+    packed vectors are not made and None stands in their place."""
     _cuda(proj, "proj", contiguous=False); _cuda(i_bias, "i_bias"); _cuda(f_bias, "f_bias", i_bias.dtype)
     _cuda(state_m, "state_m", torch.float32, contiguous=False)
     _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
@@ -1722,15 +1723,15 @@ def memory_gates(proj: torch.Tensor, q_off: int, k_off: int, i_off: int, f_off: 
     if proj.stride(1) != 1 or state_m.stride(1) != 1 or state_m.shape[1] != heads or dim > SCAN_MAX_KEY or \
             max(q_off, k_off) + heads * dim > proj.shape[1] or max(i_off, f_off) + heads > proj.shape[1]:
         raise KernelError("memory_gates: shapes do not fit")
-    packed = torch.empty((n, heads, 3, dim), dtype=torch.float32, device=proj.device)
+    packed = None if gates_only else torch.empty((n, heads, 3, dim), dtype=torch.float32, device=proj.device)
     gates = torch.empty((n, heads, 4), dtype=torch.float32, device=proj.device)
     f = _fn("recurrent", "jv_memory_gates", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                              c_int, c_float, c_float, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
                                              c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(f(proj.data_ptr(), _code(proj, "proj"), proj.stride(0), q_off, k_off, i_off, f_off, i_bias.data_ptr(),
-             f_bias.data_ptr(), _code(i_bias, "i_bias"), float(cap), float(q_scale), gates.data_ptr(), packed.data_ptr(),
+             f_bias.data_ptr(), _code(i_bias, "i_bias"), float(cap), float(q_scale), gates.data_ptr(), _ptr(packed),
              state_m.data_ptr(), state_m.stride(0), cu_seqlens.data_ptr(), slots.data_ptr(), state_m.shape[0], n_entries,
-             n, heads, dim, _status_ptr(proj.device), _stream()), "memory_gates", launches=2)
+             n, heads, dim, _status_ptr(proj.device), _stream()), "memory_gates", launches=1 if gates_only else 2)
     return packed, gates
 
 
@@ -1811,6 +1812,67 @@ def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
              state.data_ptr(), state.stride(0), cu_seqlens.data_ptr(), slots.data_ptr(), state.shape[0], n_entries, heads,
              dim, value_dim, _ptr(state_n), nq, 4, int(segment), max_segments, _ptr(seg_local), _ptr(seg_start),
              _status_ptr(packed.device), _stream()), "state_scan", launches=3 if segment > 0 else 1)
+    return out
+
+
+# `chunk_scan` goes through an entry's tokens in order, so it is taken where entries are long and where two-warp blocks, one per
+# entry, head and 32 value columns, give the device 120 or more: fewer leave multiprocessors idle for all of the launch, and the
+# scan in segments is faster (2,048 tokens of 8 heads of 128 x 256: 352 against 333 us with the preparation; of 64 heads of 128 x 64, 128
+# blocks: 329 against 510).
+CHUNK_SCAN_MIN_TOKENS, CHUNK_SCAN_MIN_BLOCKS = 64, 120
+CHUNK_SCAN_MAX_KEY = 128
+
+
+def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, dim: int, columns: int) -> bool:
+    """Whether `chunk_scan` takes these sizes and is the better choice: 16-bit rows whose heads start on 16-byte boundaries, keys of
+    up to 128 in steps of 8, values in steps of 8, enough tokens an entry and enough blocks."""
+    return (row.dtype == torch.bfloat16 and row.shape[0] >= CHUNK_SCAN_MIN_TOKENS * n_entries and 8 <= dim <= CHUNK_SCAN_MAX_KEY
+            and n_entries * heads * -(-columns // 32) >= CHUNK_SCAN_MIN_BLOCKS
+            and dim % 8 == 0 and columns % 8 == 0 and row.stride(1) == 1 and row.stride(0) % 8 == 0
+            and all((row.data_ptr() + 2 * o) % 16 == 0 for o in offsets))
+
+
+def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor, cu_seqlens: torch.Tensor,
+               slots: torch.Tensor, n_entries: int, heads: int, groups: int, dim: int, columns: int, scale: float = 1.0,
+               gates: torch.Tensor | None = None, state_n: torch.Tensor | None = None, dt_raw: torch.Tensor | None = None,
+               dt_bias: torch.Tensor | None = None, a_log: torch.Tensor | None = None) -> torch.Tensor:
+    """S <- a S + g k v^T and o = scale * S^T q with one decay a and one step g a head and token, 32 tokens at a time
+    (csrc/chunk_scan.cu): the mixers' scan (`mamba_prepare` or the second half of `memory_gates`, then `state_scan`) for portions
+    of many tokens.  `row` [n, ..] bfloat16 holds q and k (`groups` of `dim`, shared by heads // groups heads each) and v (`heads` of
+    `columns`).  Either `gates` [n, heads, 4] (keep, take, ..) with `state_n` as for `state_scan`, or the raw step sizes `dt_raw`
+    [n, heads] with `dt_bias` and `a_log`.  Returns o [n, heads * columns] float32; states are carried on in place."""
+    _cuda(row, "row", torch.bfloat16, contiguous=False); _cuda(state, "state", torch.float32, contiguous=False)
+    _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
+    n, width = row.shape
+    if min(q_off, k_off, v_off) < 0 or max(max(q_off, k_off) + groups * dim, v_off + heads * columns) > width or heads % groups or \
+            row.stride(1) != 1 or state.stride(1) != 1 or state.shape[1] < heads * dim * columns:
+        raise KernelError("chunk_scan: shapes do not fit")
+    if cu_seqlens.numel() < n_entries + 1 or slots.numel() < n_entries:
+        raise KernelError("chunk_scan: an offset and a slot per entry")
+    w_code = 0
+    if gates is not None:
+        _cuda(gates, "gates", torch.float32)
+        if tuple(gates.shape) != (n, heads, 4):
+            raise KernelError("chunk_scan: gates are [n, heads, 4]")
+        if state_n is not None:
+            _cuda(state_n, "state_n", torch.float32, contiguous=False)
+            if state_n.stride(0) != state.stride(0) or state_n.stride(1) != 1 or state_n.shape != (state.shape[0], heads * dim):
+                raise KernelError("chunk_scan: the normaliser does not fit")
+    else:
+        _cuda(dt_raw, "dt_raw", torch.bfloat16, contiguous=False); _cuda(dt_bias, "dt_bias"); _cuda(a_log, "a_log", dt_bias.dtype)
+        if state_n is not None or tuple(dt_raw.shape) != (n, heads) or dt_raw.stride(1) != 1 or dt_bias.numel() != heads or \
+                a_log.numel() != heads:
+            raise KernelError("chunk_scan: the step sizes do not fit")
+        w_code = _code(dt_bias, "dt_bias")
+    out = torch.empty((n, heads * columns), dtype=torch.float32, device=row.device)
+    f = _fn("chunk_scan", "jv_chunk_scan", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_float, c_void_p,
+                                            c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
+                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    base = row.data_ptr()
+    _check(f(base + 2 * q_off, row.stride(0), base + 2 * k_off, row.stride(0), base + 2 * v_off, row.stride(0), heads // groups,
+             float(scale), _ptr(gates), _ptr(dt_raw), 0 if dt_raw is None else dt_raw.stride(0), _ptr(dt_bias), _ptr(a_log), w_code,
+             out.data_ptr(), state.data_ptr(), state.stride(0), _ptr(state_n), cu_seqlens.data_ptr(), slots.data_ptr(),
+             state.shape[0], n_entries, heads, dim, columns, _status_ptr(row.device), _stream()), "chunk_scan")
     return out
 
 

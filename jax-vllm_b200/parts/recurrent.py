@@ -108,6 +108,8 @@ register_mixer("delta_rule", DeltaRule)
 
 
 class MatrixMemory(_StateMixer):
+    kernels = _StateMixer.kernels + ("chunk_scan",)
+
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx
         self.prefix = f"{prefix}.{spec.prefix}" if spec.prefix else prefix
@@ -146,11 +148,15 @@ class MatrixMemory(_StateMixer):
         hd, hv, h = self.hd, self.hv, self.h
         state = cache.state
         mats = hd * self.dv
+        chunks = ops.chunk_scan_supports(row, (0, hd, 2 * hd), step.n_entries, h, self.d, self.dv)
         packed, gates = ops.memory_gates(row, 0, hd, 2 * hd + 2 * hv, 2 * hd + 2 * hv + h, self.i_bias, self.f_bias,
                                          self.spec.gate_cap, self.d ** -0.5, state[:, mats + hd:], step.cu_seqlens,
-                                         step.state_slots, step.n_entries, h, self.d)
-        o = ops.state_scan(packed, row, 2 * hd, state, step.cu_seqlens, step.state_slots, step.n_entries, self.dv,
-                           state_n=state[:, mats:mats + hd], gates=gates)
+                                         step.state_slots, step.n_entries, h, self.d, gates_only=chunks)
+        where, state_n = (state, step.cu_seqlens, step.state_slots, step.n_entries), state[:, mats:mats + hd]
+        if chunks:
+            o = ops.chunk_scan(row, 0, hd, 2 * hd, *where, h, h, self.d, self.dv, scale=self.d ** -0.5, gates=gates, state_n=state_n)
+        else:
+            o = ops.state_scan(packed, row, 2 * hd, *where, self.dv, state_n=state_n, gates=gates)
         return ops.head_norm_gate(o, self.norm, row[:, 2 * hd + hv:2 * hd + 2 * hv], out, h, self.dv, self.spec.norm_eps,
                                   gates=gates)
 

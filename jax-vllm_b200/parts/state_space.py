@@ -5,7 +5,8 @@
     dt   = softplus(dt + dt_bias);  a = exp(-exp(A_log) * dt)                             csrc/mamba2.cu, 32-bit
     S   <- a S + dt B x^T,  y = S^T C + D x    per head, S [N, E]; head h reads B, C of group h // (H / G)
                                                csrc/recurrent.cu: the scan of a matrix state with key dt * B, query C
-                                               and the decay a in every key channel
+                                               and the decay a in every key channel; long portions in 16-bit mode:
+                                               csrc/chunk_scan.cu
     out  = (norm_groups x RMSNorm)(y * silu(z)) * weight @ W_o^T        the gate comes before the norm
 
 State per request (`FixedStateNeed`, in a state slot, zeroed at admission): the last taps - 1 inputs of the
@@ -23,7 +24,7 @@ from .registry import register_mixer
 
 
 class StateSpace(Part):
-    kernels = ("short_conv", "mamba2", "recurrent", "state_step", "gemm_simt")
+    kernels = ("short_conv", "mamba2", "recurrent", "state_step", "chunk_scan", "gemm_simt")
 
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx
@@ -90,9 +91,14 @@ class StateSpace(Part):
         conv_state = state[:, mats:] if self.taps > 1 else None
         xbc = ops.short_conv(row[:, inner:inner + self.conv_channels], self.conv_w, conv_state, step.cu_seqlens,
                              step.state_slots, step.n_entries, dt, bias=self.conv_b, act="silu")
-        packed = ops.mamba_prepare(xbc, inner, inner + gn, row[:, 2 * inner + 2 * gn:2 * inner + 2 * gn + self.h],
-                                   self.dt_bias, self.a_log, self.h, self.g, self.n)
-        o = ops.state_scan(packed, xbc, 0, state, step.cu_seqlens, step.state_slots, step.n_entries, self.e)
+        dt_raw = row[:, 2 * inner + 2 * gn:2 * inner + 2 * gn + self.h]
+        where = (state, step.cu_seqlens, step.state_slots, step.n_entries)
+        if ops.chunk_scan_supports(xbc, (0, inner, inner + gn), step.n_entries, self.h, self.n, self.e):
+            o = ops.chunk_scan(xbc, inner + gn, inner, 0, *where, self.h, self.g, self.n, self.e, dt_raw=dt_raw,
+                               dt_bias=self.dt_bias, a_log=self.a_log)
+        else:
+            packed = ops.mamba_prepare(xbc, inner, inner + gn, dt_raw, self.dt_bias, self.a_log, self.h, self.g, self.n)
+            o = ops.state_scan(packed, xbc, 0, *where, self.e)
         return ops.mamba_finish(o, xbc[:, :inner], row[:, :inner], self.skip, self.norm, out, self.h, self.e, self.ng,
                                 self.spec.norm_eps)
 

@@ -138,3 +138,83 @@ def test_state_single_tokens(dim, columns, removal):
             runs.append((o, st, gates[:, :, 3]))
         for got, want in zip(*runs):                     # sums of up to 256 terms in two orders
             assert (got.double() - want.double()).norm() <= 2e-6 * want.double().norm() + 1e-30
+
+
+# --------------------------------------------------------------- one decay a head, 32 tokens at a time
+@pytest.mark.parametrize("heads,groups,dim,columns", [(4, 1, 8, 8), (2, 2, 16, 24), (3, 3, 32, 16), (4, 2, 64, 64), (2, 1, 72, 40),
+                                                      (80, 8, 64, 72), (2, 1, 128, 64), (150, 1, 128, 64), (2, 2, 128, 256)])
+def test_chunked_states_with_step_sizes(heads, groups, dim, columns):
+    ops, lengths = _ops(), [1, 33, 150, 31, 32, 64, 7]
+    cu, slots, n_slots = _entries(lengths)
+    n, gn, hv = sum(lengths), groups * dim, heads * columns
+    row = _rand(n, hv + 2 * gn, seed=dim, dtype=torch.bfloat16)
+    dt_raw, dt_bias = _rand(n, heads, seed=3, dtype=torch.bfloat16, scale=2.0), _rand(heads, seed=4)
+    a_log = _rand(heads, seed=5, scale=2.0)              # decays from nearly one to zero
+    state = _rand(n_slots, heads * dim * columns + 4, seed=6)
+    before = state.clone()
+    out = ops.chunk_scan(row, hv + gn, hv, 0, state, cu, slots, len(lengths), heads, groups, dim, columns, dt_raw=dt_raw,
+                         dt_bias=dt_bias, a_log=a_log)
+    old = before.clone()
+    packed = ops.mamba_prepare(row, hv, hv + gn, dt_raw, dt_bias, a_log, heads, groups, dim)
+    general = ops.state_scan(packed, row, 0, old, cu, slots, len(lengths), columns, segment=0)
+    B, C = (row[:, hv + i * gn:hv + (i + 1) * gn].double().view(n, groups, dim).repeat_interleave(heads // groups, 1) for i in range(2))
+    x, dt = row[:, :hv].double().view(n, heads, columns), torch.nn.functional.softplus(dt_raw.double() + dt_bias.double())
+    a = torch.exp(-torch.exp(a_log.double()) * dt)
+    at = 0
+    for e, length in enumerate(lengths):
+        s = int(slots[e])
+        S = before[s, :hv * dim].double().view(heads, dim, columns)
+        want = torch.empty(length, heads, columns, dtype=torch.float64, device="cuda")
+        for t in range(length):
+            i = at + t
+            S = a[i][:, None, None] * S + dt[i][:, None, None] * B[i][:, :, None] * x[i][:, None, :]
+            want[t] = torch.einsum("hdv,hd->hv", S, C[i])
+        # no further from 64-bit arithmetic than the general scan (both err by about 1e-7)
+        for got, base, true in ((out[at:at + length], general[at:at + length], want), (state[s, :hv * dim], old[s, :hv * dim], S)):
+            err, err_general = (got.double().reshape(true.shape) - true).norm(), (base.double().reshape(true.shape) - true).norm()
+            assert err <= 1.5 * err_general + 2e-7 * true.norm(), (err / true.norm(), err_general / true.norm())
+        assert torch.equal(state[s, hv * dim:], before[s, hv * dim:])
+        at += length
+    for s in set(range(n_slots)) - set(slots.tolist()):
+        assert torch.equal(state[s], before[s])
+
+
+@pytest.mark.parametrize("heads,dim,columns", [(2, 8, 8), (4, 64, 128), (2, 128, 256), (8, 128, 264)])
+def test_chunked_states_with_gates_and_normaliser(heads, dim, columns):
+    ops, lengths = _ops(), [40, 1, 200, 32]
+    cu, slots, n_slots = _entries(lengths)
+    n, hd, hv = sum(lengths), heads * dim, heads * columns
+    row = _rand(n, 2 * hd + hv, seed=1, dtype=torch.bfloat16)
+    gates = torch.rand(n, heads, 4, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    gates[5] = 0.0                                       # a decay of zero forgets what was before
+    rows = _rand(n_slots, hd * columns + hd + heads, seed=3)
+    runs = []
+    for chunked in (True, False):
+        st, g = rows.clone(), gates.clone()
+        state_n = st[:, hd * columns:hd * columns + hd]
+        if chunked:
+            o = ops.chunk_scan(row, 0, hd, 2 * hd, st, cu, slots, len(lengths), heads, heads, dim, columns, scale=dim ** -0.5, gates=g,
+                               state_n=state_n)
+        else:
+            q, k = (row[:, i * hd:(i + 1) * hd].float().view(n, heads, dim) for i in range(2))
+            packed = torch.stack([q * dim ** -0.5, g[:, :, 1:2] * k, g[:, :, :1].expand(n, heads, dim)], 2).contiguous()
+            o = ops.state_scan(packed, row, 2 * hd, st, cu, slots, len(lengths), columns, state_n=state_n, gates=g, segment=0)
+        runs.append((o, st, g[:, :, 3]))
+    for got, want in zip(*runs):                         # two 32-bit sums of up to 200 + 128 terms
+        assert (got.double() - want.double()).norm() <= 3e-6 * want.double().norm()
+
+
+def test_chunked_states_later_infinity_stays_out_of_earlier_outputs():
+    ops, dim, columns, n = _ops(), 16, 16, 70
+    cu, slots, n_slots = _entries([n])
+    row = _rand(n, columns + 2 * dim, seed=1, dtype=torch.bfloat16)
+    row[40, 3], row[41, 6] = float("inf"), float("nan")
+    zero = torch.zeros(1, device="cuda")
+    state = _rand(n_slots, dim * columns, seed=2)
+    out = ops.chunk_scan(row, columns + dim, columns, 0, state, cu, slots, 1, 1, 1, dim, columns,
+                         dt_raw=_rand(n, 1, seed=3, dtype=torch.bfloat16), dt_bias=zero, a_log=zero)
+    bad = ~torch.isfinite(out)
+    assert not bad[:40].any() and bad[40:, 3].all() and not bad[40].logical_xor(torch.arange(columns, device="cuda") == 3).any()
+    assert bad[41:, 6].all() and bad[41:].sum() == 2 * (n - 41)
+    left = ~torch.isfinite(state[int(slots[0])].view(dim, columns))
+    assert left[:, [3, 6]].all() and left.sum() == 2 * dim
