@@ -89,6 +89,71 @@ __global__ void __launch_bounds__(1024) mamba_finish_kernel(const float* __restr
     for (int i = threadIdx.x; i < group_size; i += blockDim.x) dst[i] = from_f32<T>(gated(i) * inv * to_f32(w[first + i]));
   }
 }
+
+// The same for groups in whole vectors: eight neighbouring elements a thread (all of one head), read once.
+template <typename T> __device__ __forceinline__ void load_eight(float (&v)[8], const T* p) {
+  if constexpr (sizeof(T) == 4) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+    const uint4 a = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  }
+}
+template <typename T> __device__ __forceinline__ void store_eight(T* p, const float (&v)[8]) {
+  if constexpr (sizeof(T) == 4) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  } else {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+template <typename T, typename TW>
+__global__ void __launch_bounds__(1024) mamba_finish_vec_kernel(const float* __restrict__ o, const T* __restrict__ x,
+                                                                long long x_stride, const T* __restrict__ z, long long z_stride,
+                                                                const TW* __restrict__ skip, const TW* __restrict__ w,
+                                                                T* __restrict__ out, long long out_stride, float eps,
+                                                                int value_dim, int group_size, int inner) {
+  __shared__ float scratch[33];
+  pdl_trigger();
+  pdl_wait();
+  const int t = blockIdx.x, i = threadIdx.x * 8, at = blockIdx.y * group_size + i;
+  const bool live = i < group_size;
+  float y[8] = {};
+  float ss = 0.f;
+  if (live) {
+    float xv[8], zv[8];
+    load_eight<float>(y, o + (size_t)t * inner + at);
+    load_eight<T>(xv, x + (size_t)t * x_stride + at);
+    load_eight<T>(zv, z + (size_t)t * z_stride + at);
+    const float D = to_f32(skip[at / value_dim]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      y[e] = (y[e] + D * xv[e]) * (zv[e] / (1.f + expf(-zv[e])));
+      ss = fmaf(y[e], y[e], ss);
+    }
+  }
+  const float inv = rsqrtf(block_sum(ss, scratch) / (float)group_size + eps);
+  if (!live) return;
+  float wv[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) wv[e] = to_f32(w[at + e]);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) y[e] *= inv * wv[e];
+  store_eight<T>(out + (size_t)t * out_stride + at, y);
+}
 }  // namespace
 
 // xbc: rows of `dtype`, B at b_off and C at c_off ([groups][state] each); dt_raw: rows of `dtype`, [heads] used;
@@ -115,6 +180,19 @@ JV_EXPORT int jv_mamba_finish(const float* o, const void* x, long long x_stride,
   if (n == 0) return JV_OK;
   const int inner = heads * value_dim;
   if (heads < 1 || value_dim < 1 || norm_groups < 1 || inner % norm_groups) return JV_ERR_UNSUPPORTED;
+  // Eight elements a thread where vectors fit (heads and groups in steps of 8, rows on 16-byte boundaries) and there are tokens
+  // enough to fill the device with so few threads: 4,096 tokens of 8 groups of 1,024 in 62 us against 222, 200 of 4,096 in 4.2
+  // against 6.8.
+  const int group_size = inner / norm_groups, size = dtype == 0 ? 4 : 2;
+  auto eights = [&](const void* q, long long stride, int bytes) { return ((uintptr_t)q & 15) == 0 && stride * bytes % 16 == 0; };
+  if (n >= 64 && value_dim % 8 == 0 && group_size % 8 == 0 && group_size <= 8192 && eights(o, inner, 4) && eights(x, x_stride, size) &&
+      eights(z, z_stride, size) && eights(out, out_stride, size)) {
+    const int threads = (group_size / 8 + 31) / 32 * 32;
+    JV_DISPATCH_DTYPE(dtype, T, JV_DISPATCH_DTYPE(w_dtype, TW,
+        return jv_launch(mamba_finish_vec_kernel<T, TW>, dim3(n, norm_groups), dim3(threads), 0, stream, o, (const T*)x, x_stride,
+                         (const T*)z, z_stride, (const TW*)skip, (const TW*)w, (T*)out, out_stride, eps, value_dim, group_size,
+                         inner)));
+  }
   // two elements a thread where the group allows: many warps hide the loads' latency when there are few tokens
   int threads = ((inner / norm_groups + 1) / 2 + 31) / 32 * 32;
   threads = threads < 32 ? 32 : threads > 1024 ? 1024 : threads;

@@ -106,8 +106,133 @@ __global__ void __launch_bounds__(THREADS) short_conv_kernel(const ConvParams p)
   }
 }
 
+// The same with VEC neighbouring channels a thread: 8 bytes (16 in 32-bit) a load where one channel has 2, which is what a portion
+// of many tokens is bound by.
+constexpr int VEC = 4;
+
+template <typename T> __device__ __forceinline__ void load_raw(uint32_t (&r)[VEC * sizeof(T) / 4], const T* p) {
+  if constexpr (sizeof(T) == 4) {
+    const uint4 a = *reinterpret_cast<const uint4*>(p);
+    r[0] = a.x; r[1] = a.y; r[2] = a.z; r[3] = a.w;
+  } else {
+    const uint2 a = *reinterpret_cast<const uint2*>(p);
+    r[0] = a.x; r[1] = a.y;
+  }
+}
+template <typename T> __device__ __forceinline__ float raw_at(const uint32_t (&r)[VEC * sizeof(T) / 4], int v) {
+  if constexpr (sizeof(T) == 4) return __uint_as_float(r[v]);
+  else return __uint_as_float((v & 1) ? r[v / 2] & 0xffff0000u : r[v / 2] << 16);
+}
+template <typename T> __device__ __forceinline__ void store_four(T* p, const float (&y)[VEC]) {
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(p) = make_float4(y[0], y[1], y[2], y[3]);
+  } else {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(y[0], y[1]), b = __floats2bfloat162_rn(y[2], y[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+  }
+}
+
+template <typename TI, typename TO, typename TW, int TAPS>
+__global__ void __launch_bounds__(THREADS) short_conv_vec_kernel(const ConvParams p) {
+  constexpr int K = TAPS - 1, RAW = VEC * sizeof(TI) / 4;
+  static_assert(K > 0, "one tap keeps no state");
+  pdl_trigger();
+  pdl_wait();
+  int entry = -1, seg = 0, before = 0;
+  for (int e = 0; e < p.n_entries; ++e) {
+    const int q = p.cu_seqlens[e + 1] - p.cu_seqlens[e];
+    const int segs = (q + SEG - 1) / SEG;
+    if ((int)blockIdx.x < before + segs) { entry = e; seg = blockIdx.x - before; break; }
+    before += segs;
+  }
+  if (entry < 0) return;
+  const int c = (blockIdx.y * THREADS + threadIdx.x) * VEC;
+  if (c >= p.channels) return;
+  const int t_begin = p.cu_seqlens[entry], q = p.cu_seqlens[entry + 1] - t_begin;
+  const int i0 = seg * SEG, i1 = min(q, i0 + SEG);
+  const int slot = p.slots[entry];
+  if (slot < 0 || slot >= p.n_slots) {
+    if (threadIdx.x == 0) atomicOr(p.status, JV_STATUS_BAD_ROW);
+    return;
+  }
+  const TI* in = (const TI*)p.in + (size_t)t_begin * p.in_stride + c;
+  TO* out = (TO*)p.out + (size_t)t_begin * p.out_stride + c;
+  float* st = p.state + (size_t)slot * p.state_stride + c;
+  uint32_t ahead[BATCH][RAW];
+  auto fetch = [&](int i) {
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u) load_raw<TI>(ahead[u], in + (size_t)min(i + u, i1 - 1) * p.in_stride);
+  };
+  fetch(i0);
+  float wt[TAPS][VEC], bias[VEC], win[K][VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) {
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) wt[j][v] = to_f32(((const TW*)p.w)[(size_t)(c + v) * TAPS + j]);
+    bias[v] = p.bias != nullptr ? to_f32(((const TW*)p.bias)[c + v]) : 0.f;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int i = i0 - K + k;
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) win[k][v] = i >= 0 ? to_f32(in[(size_t)i * p.in_stride + v]) : st[(size_t)(K + i) * p.channels + v];
+  }
+  if (seg == 0) {
+    // the state after this step: the last K inputs of (old state, this entry's tokens)
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const int i = q - K + j;
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        float x = 0.f;
+        if (i >= 0) {
+          x = to_f32(in[(size_t)i * p.in_stride + v]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < K; ++k) if (k == K + i) x = win[k][v];
+        }
+        st[(size_t)j * p.channels + v] = x;
+      }
+    }
+  }
+  for (int i = i0; i < i1; i += BATCH) {
+    uint32_t now[BATCH][RAW];
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u)
+#pragma unroll
+      for (int r = 0; r < RAW; ++r) now[u][r] = ahead[u][r];
+    if (i + BATCH < i1) fetch(i + BATCH);
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u) {
+      if (i + u >= i1) break;
+      float y[VEC];
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        const float x = raw_at<TI>(now[u], v);
+        float acc = wt[K][v] * x;
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc = fmaf(wt[k][v], win[k][v], acc);
+#pragma unroll
+        for (int k = 0; k + 1 < K; ++k) win[k][v] = win[k + 1][v];
+        win[K - 1][v] = x;
+        y[v] = p.residual ? x + acc : acc + bias[v];
+        if (p.act == 1) y[v] = y[v] / (1.f + expf(-y[v]));
+      }
+      store_four<TO>(out + (size_t)(i + u) * p.out_stride, y);
+    }
+  }
+}
+
 template <typename TI, typename TO, typename TW>
-int launch_taps(const ConvParams& p, int taps, dim3 grid, cudaStream_t stream) {
+int launch_taps(const ConvParams& p, int taps, bool vec, dim3 grid, cudaStream_t stream) {
+  if (vec) {
+    const dim3 wide(grid.x, (p.channels + THREADS * VEC - 1) / (THREADS * VEC));
+    switch (taps) {
+      case 2: return jv_launch(short_conv_vec_kernel<TI, TO, TW, 2>, wide, dim3(THREADS), 0, stream, p);
+      case 3: return jv_launch(short_conv_vec_kernel<TI, TO, TW, 3>, wide, dim3(THREADS), 0, stream, p);
+      default: return jv_launch(short_conv_vec_kernel<TI, TO, TW, 4>, wide, dim3(THREADS), 0, stream, p);
+    }
+  }
   switch (taps) {
     case 1: return jv_launch(short_conv_kernel<TI, TO, TW, 1>, grid, dim3(THREADS), 0, stream, p);
     case 2: return jv_launch(short_conv_kernel<TI, TO, TW, 2>, grid, dim3(THREADS), 0, stream, p);
@@ -140,7 +265,15 @@ JV_EXPORT int jv_short_conv(const void* in, int in_dtype, long long in_stride, v
   p.state = state; p.state_stride = state_stride; p.cu_seqlens = cu_seqlens; p.slots = slots; p.n_entries = n_entries;
   p.n_slots = n_slots; p.channels = channels; p.act = act; p.residual = residual ? 1 : 0; p.status = status;
   const dim3 grid(n_tokens / SEG + n_entries, (channels + THREADS - 1) / THREADS);
+  // Four channels a thread from 8 M elements on, for two to four taps and rows on four-element boundaries: 4,096 tokens of 10,240
+  // channels in 84 us against 108 one by one, 2,048 of 4,352 in 20 against 24; with fewer tokens or channels the threads of one
+  // channel each are needed to fill the device (2,048 of 2,304 channels: 16.3 against 15.1).
+  auto fours = [](const void* q, long long stride, int dtype) {
+    return ((uintptr_t)q & (dtype == 0 ? 15 : 7)) == 0 && stride % VEC == 0;
+  };
+  const bool vec = (long long)n_tokens * channels >= (8LL << 20) && taps >= 2 && taps <= 4 && channels % VEC == 0 &&
+                   fours(in, in_stride, in_dtype) && fours(out, out_stride, out_dtype);
   JV_DISPATCH_DTYPE(in_dtype, TI, JV_DISPATCH_DTYPE(out_dtype, TO, JV_DISPATCH_DTYPE(w_dtype, TW,
-      return launch_taps<TI, TO, TW>(p, taps, grid, stream))));
+      return launch_taps<TI, TO, TW>(p, taps, vec, grid, stream))));
   return JV_ERR_UNSUPPORTED;
 }

@@ -1653,9 +1653,9 @@ def delta_prepare(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, zw: to
     return packed
 
 
-# Average new tokens of an entry from which `delta_scan` is taken (parts/recurrent.py).  32 heads of 64, prepare and scan: eight entries of
-# 8 tokens 17.2 us, of 4 tokens on the kernels that go token by token 13.0 us, which grow by 0.4 us a token where `delta_scan` grows by 0.13.
-DELTA_GROUP_MIN_TOKENS = 8
+# Average new tokens of an entry from which `delta_scan` is taken (parts/recurrent.py).  32 heads of 64, preparation and scan: eight entries
+# of 8 tokens 19.8 against 17.3 us on the kernels that go token by token; those grow by 0.4 us a token, `delta_scan` by 0.13.
+DELTA_GROUP_MIN_TOKENS = 16
 
 
 def delta_scan(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, v_off: int, zw: torch.Tensor, a_bias: torch.Tensor,

@@ -218,3 +218,46 @@ def test_chunked_states_later_infinity_stays_out_of_earlier_outputs():
     assert bad[41:, 6].all() and bad[41:].sum() == 2 * (n - 41)
     left = ~torch.isfinite(state[int(slots[0])].view(dim, columns))
     assert left[:, [3, 6]].all() and left.sum() == 2 * dim
+
+
+# ------------------------------------------------------- convolution and finish of the state-space mixer
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("channels,off", [(8192, 0), (8196, 4), (8192, 2), (512, 0)])
+def test_short_conv_many_tokens(taps, channels, off):
+    ops, lengths = _ops(), [1000, 1, 33, 2, 64]
+    cu, slots, n_slots = _entries(lengths)
+    n = sum(lengths)
+    for dtype, out_dtype in ((torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16), (torch.float32, torch.float32)):
+        x = _rand(n, channels + 8, seed=1, dtype=dtype)[:, off:off + channels]
+        w, b = _rand(channels, taps, seed=2), _rand(channels, seed=3)
+        state = _rand(n_slots, (taps - 1) * channels, seed=4)
+        before = state.clone()
+        got = ops.short_conv(x, w, state, cu, slots, len(lengths), out_dtype, bias=b, act="silu")
+        at = 0
+        for e, length in enumerate(lengths):
+            s = int(slots[e])
+            rows = torch.cat([before[s].double().view(taps - 1, channels), x[at:at + length].double()])
+            y = sum(rows[j:j + length] * w[:, j].double() for j in range(taps)) + b.double()
+            # a few roundings of a sum of this size, and silu's own (its slope is at most 1.1)
+            size = sum(rows[j:j + length].abs() * w[:, j].double().abs() for j in range(taps)) + b.double().abs()
+            y = y * torch.sigmoid(y)
+            tol = 2.0 ** -8 if out_dtype == torch.bfloat16 else 8 * EPS32
+            assert ((got[at:at + length].double() - y).abs() <= tol * y.abs() + 8 * EPS32 * size).all()
+            assert torch.equal(state[s].view(taps - 1, channels), rows[-(taps - 1):].float())
+            at += length
+
+
+@pytest.mark.parametrize("n", [63, 64])
+@pytest.mark.parametrize("heads,value_dim,groups,off", [(2, 8, 2, 0), (3, 24, 1, 0), (16, 64, 8, 8), (16, 64, 1, 1), (5, 7, 1, 0), (96, 128, 1, 0)])
+def test_mamba_finish_vectors(n, heads, value_dim, groups, off):
+    ops, inner = _ops(), heads * value_dim
+    for dtype in (torch.float32, torch.bfloat16):
+        o = _rand(n, inner, seed=1)
+        x, z = (_rand(n, inner + 8, seed=s, dtype=dtype)[:, off:off + inner] for s in (2, 3))
+        skip, w = _rand(heads, seed=4), _rand(inner, seed=5)
+        out = torch.empty(n, inner, dtype=dtype, device="cuda")
+        ops.mamba_finish(o, x, z, skip, w, out, heads, value_dim, groups, 1e-5)
+        y = (o.double().view(n, heads, value_dim) + skip.double()[:, None] * x.double().reshape(n, heads, value_dim)).reshape(n, inner)
+        y = (y * z.double() * torch.sigmoid(z.double())).reshape(n, groups, -1)
+        y = (y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5)).reshape(n, inner) * w.double()
+        assert ((out.double() - y).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 4e-6) * y.abs() + 1e-6).all()
