@@ -170,6 +170,52 @@ __global__ void pick_rows_sum_kernel(const TD* __restrict__ y, const int* __rest
   }
 }
 
+// The same in vectors of four elements: a block takes four times its threads of a row's columns, and the loads of up to
+// eight picked rows are under way together (one after the other they cost a memory latency each).
+template <typename TD>
+__global__ void __launch_bounds__(128) pick_rows_sum_vec_kernel(const TD* __restrict__ y, const int* __restrict__ pick,
+                                                                const float* __restrict__ coef, int parts, int y_rows,
+                                                                const TD* __restrict__ own, const float* __restrict__ own_coef,
+                                                                float* __restrict__ out, int hidden, int* __restrict__ status) {
+  constexpr int AT_ONCE = 8;
+  pdl_trigger();
+  pdl_wait();
+  const int r = blockIdx.x, c = (blockIdx.y * 128 + threadIdx.x) * 4;
+  if (c >= hidden) return;
+  auto load = [](const TD* p) -> float4 {
+    if constexpr (sizeof(TD) == 4) {
+      return *reinterpret_cast<const float4*>(p);
+    } else {
+      const uint2 a = *reinterpret_cast<const uint2*>(p);
+      return make_float4(__uint_as_float(a.x << 16), __uint_as_float(a.x & 0xffff0000u), __uint_as_float(a.y << 16),
+                         __uint_as_float(a.y & 0xffff0000u));
+    }
+  };
+  auto fma4 = [](float f, const float4& x, float4& v) {
+    v.x = fmaf(f, x.x, v.x); v.y = fmaf(f, x.y, v.y); v.z = fmaf(f, x.z, v.z); v.w = fmaf(f, x.w, v.w);
+  };
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f), mine = v;
+  if (own != nullptr) mine = load(own + (size_t)r * hidden + c);
+  for (int s0 = 0; s0 < parts; s0 += AT_ONCE) {
+    int src[AT_ONCE];
+    float4 x[AT_ONCE];
+#pragma unroll
+    for (int s = 0; s < AT_ONCE; ++s) src[s] = s0 + s < parts ? pick[(size_t)r * parts + s0 + s] : -1;
+#pragma unroll
+    for (int s = 0; s < AT_ONCE; ++s) {
+      const bool there = src[s] >= 0 && src[s] < y_rows;
+      if (!there && s0 + s < parts && c == 0 && (src[s] != -1 || own == nullptr)) atomicOr(status, JV_STATUS_BAD_ROW);
+      if (there) x[s] = load(y + (size_t)src[s] * hidden + c);
+      else src[s] = -1;
+    }
+#pragma unroll
+    for (int s = 0; s < AT_ONCE; ++s)
+      if (src[s] >= 0) fma4(coef[(size_t)r * parts + s0 + s], x[s], v);
+  }
+  if (own != nullptr) fma4(own_coef[r], mine, v);
+  *reinterpret_cast<float4*>(out + (size_t)r * hidden + c) = v;
+}
+
 template <typename TX>
 __global__ void cast_rows_kernel(const float* __restrict__ h, TX* __restrict__ x, size_t n) {
   pdl_trigger();
@@ -222,6 +268,14 @@ JV_EXPORT int jv_pick_rows_sum(const void* y, int y_dtype, const int* pick, cons
                                const void* own, const float* own_coef, float* out, int n, int hidden, int* status,
                                cudaStream_t stream) {
   if (n == 0) return JV_OK;
+  // vectors where rows consist of them: 8 rows of 2,048, 4 picks each, 3.0 us against 15.9; 777 rows
+  // 10.3 against 21.6
+  const int mask = y_dtype == 0 ? 15 : 7;
+  if (hidden % 4 == 0 && ((uintptr_t)y & mask) == 0 && ((uintptr_t)own & mask) == 0 && ((uintptr_t)out & 15) == 0 && hidden <= 512 * 65535) {
+    JV_DISPATCH_DTYPE(y_dtype, TD, return jv_launch(pick_rows_sum_vec_kernel<TD>, dim3(n, (hidden + 511) / 512), dim3(128), 0, stream,
+                                                    (const TD*)y, pick, coef, parts, y_rows, (const TD*)own, own_coef, out, hidden,
+                                                    status));
+  }
   JV_DISPATCH_DTYPE(y_dtype, TD, return jv_launch(pick_rows_sum_kernel<TD>, dim3(n), dim3(256), 0, stream, (const TD*)y,
                                                   pick, coef, parts, y_rows, (const TD*)own, own_coef, out, hidden, status));
   return JV_ERR_UNSUPPORTED;

@@ -16,7 +16,12 @@
 // parts[s] ([splits, M, N], 32-bit) and the kernel that reads the result adds the parts in the order of s:
 // nobody waits and no block sums up after another.  The partition depends on N, K and the number of
 // multiprocessors only, never on the batch, and the sum over a part's k runs in ascending order.
-// Weights are asked for before the wait on the kernel that produces x (nobody writes them).  Every wait on an
+// The grouped form (routed experts, few tokens) takes a stack of weights and x in row tiles of one expert each: a unit is a strip of
+// the expert's weight with the rows of one tile, which leaves the strips of experts that nobody chose unread; it writes bfloat16, after
+// the exact gelu if asked.  8 tokens of 4 choices among 32 experts, up and down products of
+// 3 x 2,048 x 1,024 (252 MB of the 20 experts chosen): 52 us, 74 on 128-row tiles of x (gemm_tcgen05.cu); 64 tokens 79 against 90.
+// Weights are asked for before the wait on the kernel that produces x (nobody writes them; in the grouped form which ones is known
+// only after it).  Every wait on an
 // mbarrier is bounded by a clock deadline; a wait that runs out sets a bit in the status word and the block
 // goes to its tear-down (tensor memory is freed) instead of spinning.
 #include "common.cuh"
@@ -75,8 +80,11 @@ struct Params {
   int M, N, K, rows16;               // rows16: rows of x rounded up to a multiple of 16 (N of the instruction)
   int n_strips, splits, chunks, chunks_per_part, stages, stage_bytes, tmem_cols;
   int* status;
+  // grouped: the expert of every row tile (of rows16 rows) of x, how many leading tiles there are, 1: gelu
+  const int* tile_expert; const int* used_tiles; int max_tiles, gelu;
 };
 
+template <bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_constant__ CUtensorMap w_map,
                                                                    const __grid_constant__ CUtensorMap x_map,
                                                                    const Params p) {
@@ -84,7 +92,6 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
   unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   Shared* sh = reinterpret_cast<Shared*>(tiles + p.stages * p.stage_bytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_units = p.n_strips * p.splits;
   pdl_trigger();
 
   if (threadIdx.x == 0) {
@@ -102,13 +109,26 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  int n_units = p.n_strips * p.splits;
+  if (GROUPED) {
+    pdl_wait();                       // which experts were chosen is what the kernels before this one found out
+    n_units = p.n_strips * min(*p.used_tiles, p.max_tiles);
+  }
   const uint32_t tmem_base = sh->tmem_base;
   const int acc_cols = p.tmem_cols / 2;
 
-  // the chunks of this block, unit after unit: (unit, chunk index, end, first row of the strip)
-  struct Cursor { int u, c, c1, n0; };
+  // the chunks of this block, unit after unit: (unit, chunk index, end, first row of the strip, first row of x)
+  struct Cursor { int u, c, c1, n0, m0; };
   auto open_unit = [&](Cursor& it) {
-    if (it.u < n_units) {
+    if (GROUPED) {
+      if (it.u < n_units) {
+        const int tile = it.u / p.n_strips;
+        it.n0 = p.tile_expert[tile] * p.N + (it.u % p.n_strips) * BM;
+        it.m0 = tile * p.rows16;
+        it.c = 0;
+        it.c1 = p.chunks;
+      }
+    } else if (it.u < n_units) {
       const int part = it.u % p.splits;
       it.n0 = (it.u / p.splits) * BM;
       it.c = part * p.chunks_per_part;
@@ -128,14 +148,14 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
         for (int b = 0; b < BOXES; ++b)
           tma_load_2d(tiles + s * p.stage_bytes + b * W_BOX_BYTES, &w_map, c * BK + b * BOX_K, n0, &sh->full[s]);
       };
-      auto load_x = [&](int s, int c) {
+      auto load_x = [&](int s, int c, int m0) {
 #pragma unroll
         for (int b = 0; b < BOXES; ++b)
-          tma_load_2d(tiles + s * p.stage_bytes + W_BYTES + b * x_box, &x_map, c * BK + b * BOX_K, 0, &sh->full[s]);
+          tma_load_2d(tiles + s * p.stage_bytes + W_BYTES + b * x_box, &x_map, c * BK + b * BOX_K, m0, &sh->full[s]);
       };
-      Cursor it{(int)blockIdx.x, 0, 0, 0};
+      Cursor it{(int)blockIdx.x, 0, 0, 0, 0};
       open_unit(it);
-      // the weights of the first chunks are asked for before the kernel that makes x has finished
+      // the weights of the first chunks are asked for before the kernel that makes x has finished (unless grouped)
       Cursor ahead = it;
       int n_ahead = 0;
       for (; n_ahead < p.stages && ahead.u < n_units; ++n_ahead, advance(ahead)) {
@@ -143,9 +163,9 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
         mbar_expect_tx(&sh->full[n_ahead], W_BYTES + x_bytes);
         load_w(n_ahead, ahead.c, ahead.n0);
       }
-      pdl_wait();
+      if (!GROUPED) pdl_wait();
       for (int s = 0; s < n_ahead; ++s, advance(it))
-        load_x(s, it.c);
+        load_x(s, it.c, it.m0);
       int s = n_ahead == p.stages ? 0 : n_ahead, phase = n_ahead == p.stages ? 1 : 0;
       bool ok = true;
       for (; it.u < n_units && ok; advance(it)) {
@@ -153,7 +173,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
         sh->armed[s] = phase;
         mbar_expect_tx(&sh->full[s], W_BYTES + x_bytes);
         load_w(s, it.c, it.n0);
-        load_x(s, it.c);
+        load_x(s, it.c, it.m0);
         if (++s == p.stages) { s = 0; phase ^= 1; }
       }
       if (!ok) { atomicOr(p.status, JV_STATUS_WAIT_EXPIRED); sh->failed = 1; }
@@ -167,8 +187,8 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
       bool ok = true;
       for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++n) {
         const int acc = n & 1, acc_phase = (n >> 1) & 1;
-        const int part = u % p.splits;
-        const int c0 = part * p.chunks_per_part, c1 = min(p.chunks, c0 + p.chunks_per_part);
+        const int part = GROUPED ? 0 : u % p.splits;
+        const int c0 = part * p.chunks_per_part, c1 = GROUPED ? p.chunks : min(p.chunks, c0 + p.chunks_per_part);
         if (!mbar_wait(&sh->acc_empty[acc], acc_phase ^ 1)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t tmem_d = tmem_base + acc * acc_cols;
@@ -195,11 +215,12 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
     const int quad = warp & 3;                     // the 32 TMEM lanes this warp may read
     int n = 0;
     bool ok = true;
-    pdl_wait();                                    // nothing is written before the kernels before this one are done
+    if (!GROUPED) pdl_wait();                      // nothing is written before the kernels before this one are done
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++n) {
       const int acc = n & 1, acc_phase = (n >> 1) & 1;
-      const int part = u % p.splits;
-      const int col = (u / p.splits) * BM + quad * 32 + lane;      // column of y = row of W
+      const int part = GROUPED ? 0 : u % p.splits;
+      const int col = (GROUPED ? u % p.n_strips : u / p.splits) * BM + quad * 32 + lane;      // column of y = row of W
+      const int first = GROUPED ? u / p.n_strips * p.rows16 : 0;   // the unit's first row of y
       if (!mbar_wait(&sh->acc_full[acc], acc_phase)) { ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * acc_cols;
@@ -208,7 +229,14 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
         float v[16];
         tmem_ld16(taddr + m0, v);
         if (col < p.N) {
-          if (p.splits > 1) {
+          if (GROUPED) {
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.y) + (size_t)(first + m0) * p.ldy + col;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const float y = p.gelu ? 0.5f * v[i] * (1.f + erff(v[i] * 0.70710678118654752f)) : v[i];
+              dst[(size_t)i * p.ldy] = __float2bfloat16_rn(y);
+            }
+          } else if (p.splits > 1) {
             float* dst = p.parts + ((size_t)part * p.M + m0) * p.N + col;
 #pragma unroll
             for (int i = 0; i < 16; ++i)
@@ -309,6 +337,23 @@ int choose_splits(int n_strips, int K, int sms) {
   if (best_cost > cost(1) * 0.95) best = 1;
   return best;
 }
+
+// The sizes that follow from rows16, and the launch on at most `units` blocks.
+template <bool GROUPED>
+int launch(const CUtensorMap& w_map, const CUtensorMap& x_map, Params p, long long units, cudaStream_t stream) {
+  p.stage_bytes = W_BYTES + BOXES * p.rows16 * 128;          // a multiple of 1 KB: rows16 is a multiple of 16
+  p.stages = SMEM_TILES / p.stage_bytes < MAX_STAGES ? SMEM_TILES / p.stage_bytes : MAX_STAGES;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < 2 * p.rows16) p.tmem_cols *= 2;
+  constexpr size_t smem = SMEM_TILES + sizeof(Shared) + 1024;
+  static bool ready[JV_MAX_DEVICES];
+  if (!jv_once_per_device(ready, [&] {
+        return cudaFuncSetAttribute(linear_stream_kernel<GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+      }))
+    return JV_ERR_UNSUPPORTED;
+  const int sms = multiprocessors();
+  return jv_launch(linear_stream_kernel<GROUPED>, dim3((unsigned)(units < sms ? units : sms)), dim3(THREADS), smem, stream, w_map, x_map, p);
+}
 }  // namespace
 
 // Largest number of rows of x the kernel takes.
@@ -331,25 +376,32 @@ JV_EXPORT int jv_linear_stream(const void* X, int ldx, const void* W, int ldw, v
   if (splits < 1 || splits > 8 || (splits > 1 && parts == nullptr)) return JV_ERR_UNSUPPORTED;
   const int cpp = (chunks + splits - 1) / splits;
   if ((long long)(splits - 1) * cpp >= chunks) return JV_ERR_UNSUPPORTED;
-  Params p;
+  Params p = {};
   p.y = Y; p.ldy = ldy; p.out_bf16 = out_dtype == 1; p.parts = parts;
   p.M = M; p.N = N; p.K = K; p.rows16 = (M + 15) / 16 * 16;
   p.n_strips = (N + BM - 1) / BM; p.splits = splits; p.chunks = chunks; p.chunks_per_part = cpp;
-  p.stage_bytes = W_BYTES + BOXES * p.rows16 * 128;          // a multiple of 1 KB: rows16 is a multiple of 16
-  p.stages = SMEM_TILES / p.stage_bytes < MAX_STAGES ? SMEM_TILES / p.stage_bytes : MAX_STAGES;
-  p.tmem_cols = 32;
-  while (p.tmem_cols < 2 * p.rows16) p.tmem_cols *= 2;
   p.status = status;
   CUtensorMap w_map, x_map;
   if (!make_map(&w_map, W, N, K, ldw, BM) || !make_map(&x_map, X, M, K, ldx, p.rows16)) return JV_ERR_UNSUPPORTED;
-  constexpr size_t smem = SMEM_TILES + sizeof(Shared) + 1024;
-  static bool ready[JV_MAX_DEVICES];
-  if (!jv_once_per_device(ready, [&] {
-        return cudaFuncSetAttribute(linear_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
-      }))
+  return launch<false>(w_map, x_map, p, (long long)p.n_strips * splits, stream);
+}
+
+// Grouped: X: [max_tiles * tile, K] rows of ldx in tiles of `tile` rows (a multiple of 16, up to 128), tile t all of expert
+// tile_expert[t]; used_tiles: one int on the device, how many leading tiles there are; W: [experts, N, K] contiguous; Y: [max_tiles *
+// tile, N] bfloat16 rows of ldy, of which the tiles there are get written.  gelu: the exact gelu of the result.
+JV_EXPORT int jv_moe_linear_stream(const void* X, int ldx, int tile, int max_tiles, const int* tile_expert, const int* used_tiles,
+                                   const void* W, int experts, void* Y, int ldy, int N, int K, int gelu, int* status,
+                                   cudaStream_t stream) {
+  if (max_tiles == 0 || N == 0) return JV_OK;
+  if (tile < 16 || tile % 16 || tile > MAX_ROWS || K < 8 || (K % 8) || (ldx % 8) || ((uintptr_t)X % 16) || ((uintptr_t)W % 16) ||
+      tile_expert == nullptr || used_tiles == nullptr || experts < 1 || (long long)experts * N > 0x7fffffff ||
+      (long long)max_tiles * tile > 0x7fffffff)
     return JV_ERR_UNSUPPORTED;
-  const long long units = (long long)p.n_strips * splits;
-  const int sms = multiprocessors();
-  const int blocks = units < sms ? (int)units : sms;
-  return jv_launch(linear_stream_kernel, dim3(blocks), dim3(THREADS), smem, stream, w_map, x_map, p);
+  Params p = {};
+  p.y = Y; p.ldy = ldy; p.out_bf16 = 1; p.M = tile; p.N = N; p.K = K; p.rows16 = tile;
+  p.n_strips = (N + BM - 1) / BM; p.splits = 1; p.chunks = (K + BK - 1) / BK; p.chunks_per_part = p.chunks;
+  p.status = status; p.tile_expert = tile_expert; p.used_tiles = used_tiles; p.max_tiles = max_tiles; p.gelu = gelu;
+  CUtensorMap w_map, x_map;
+  if (!make_map(&w_map, W, experts * N, K, K, BM) || !make_map(&x_map, X, max_tiles * tile, K, ldx, tile)) return JV_ERR_UNSUPPORTED;
+  return launch<true>(w_map, x_map, p, (long long)max_tiles * p.n_strips, stream);
 }

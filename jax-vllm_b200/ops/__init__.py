@@ -1484,6 +1484,27 @@ def moe_gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, tile_expert: torch.Tensor
 
 
 # ---------------------------------------------------------------- per-layer token input
+MOE_STREAM_MAX_TOKENS = 64      # tokens up to which the experts' weights are streamed past them (parts/routed_experts.py)
+
+
+def moe_linear_stream(a: torch.Tensor, tile: int, w: torch.Tensor, tile_expert: torch.Tensor, used_tiles: torch.Tensor,
+                      act: str | None = None) -> torch.Tensor:
+    """`moe_gemm_tcgen05` for few rows an expert: row tiles of `tile` rows (a multiple of 16), the weight as the 128-row
+    operand of the tensor cores and a tile as the narrow one (csrc/linear_stream.cu)."""
+    _cuda(a, "a", torch.bfloat16); _cuda(w, "w", torch.bfloat16); _cuda(tile_expert, "tile_expert", torch.int32)
+    _cuda(used_tiles, "used_tiles", torch.int32)
+    max_tiles = tile_expert.numel()
+    experts, n_out, k = w.shape
+    if tuple(a.shape) != (max_tiles * tile, k):
+        raise KernelError("grouped product: rows do not fit the tiles")
+    out = torch.empty((max_tiles * tile, n_out), dtype=torch.bfloat16, device=a.device)
+    f = _fn("linear_stream", "jv_moe_linear_stream", [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
+                                                      c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(a.data_ptr(), a.stride(0), tile, max_tiles, tile_expert.data_ptr(), used_tiles.data_ptr(), w.data_ptr(), experts,
+             out.data_ptr(), out.stride(0), n_out, k, MOE_ACTS[act], _status_ptr(a.device), _stream()), "moe_linear_stream")
+    return out
+
+
 def token_gate(z: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, offset: int,
                out_dtype: torch.dtype | None = None) -> torch.Tensor:
     """g[t, j] = gelu_tanh(z[t, j]) * table[tokens[t], offset + j] in `out_dtype` (z's by default)

@@ -99,7 +99,7 @@ class RoutedExperts(Part):
         self.w_up = torch.stack(ups).contiguous()
         self.w_down = torch.stack(downs).contiguous()
         if self._tensor_cores():
-            self.kernels = ("moe_route", "gemm_tcgen05", "gemm_simt") + (("activation",) if self.gated else ())
+            self.kernels = ("moe_route", "gemm_tcgen05", "linear_stream", "gemm_simt") + (("activation",) if self.gated else ())
         if self.shared is not None:
             self.shared.bind(tensors)
             self.kernels += tuple(k for k in self.shared.kernels if k not in self.kernels)
@@ -146,12 +146,22 @@ class RoutedExperts(Part):
         own = (x, own[0]) if own else (None, None)
         first = None if self.gated else "gelu"
         if self._tensor_cores():
-            _, pos_of, tile_expert, used = ops.moe_align(ids, s.num_experts, ops.MOE_TCGEN05_TILE, s.identity)
-            rows = ops.moe_gather_rows(x, pos_of, tile_expert.numel() * ops.MOE_TCGEN05_TILE)
-            act = ops.moe_gemm_tcgen05(rows, self.w_up, tile_expert, act=first, used_tiles=used)
+            # Few tokens: an expert has at most one row a token, so a tile as high as the tokens holds all of its rows; the product is
+            # bound by the weights of the experts that were chosen, and everything around it by the rows, padding included.
+            few = x.shape[0] <= ops.MOE_STREAM_MAX_TOKENS
+            tile = -(-x.shape[0] // 16) * 16 if few else ops.MOE_TCGEN05_TILE
+            _, pos_of, tile_expert, used = ops.moe_align(ids, s.num_experts, tile, s.identity)
+            rows = ops.moe_gather_rows(x, pos_of, tile_expert.numel() * tile)
+
+            def product(a, w, act=None):
+                if few:
+                    return ops.moe_linear_stream(a, tile, w, tile_expert, used, act)
+                return ops.moe_gemm_tcgen05(a, w, tile_expert, act=act, used_tiles=used)
+
+            act = product(rows, self.w_up, first)
             if self.gated:
                 act = self._gate(act)
-            return ops.PickedRows(ops.moe_gemm_tcgen05(act, self.w_down, tile_expert, used_tiles=used), pos_of, weights, *own)
+            return ops.PickedRows(product(act, self.w_down), pos_of, weights, *own)
         sorted_token, pos_of, tile_expert, _ = ops.moe_align(ids, s.num_experts, ops.moe_gemm_simt_tile(), s.identity)
         act = ops.moe_gemm_simt(x, sorted_token, self.w_up, tile_expert, dt, act=first)
         if self.gated:

@@ -261,3 +261,51 @@ def test_mamba_finish_vectors(n, heads, value_dim, groups, off):
         y = (y * z.double() * torch.sigmoid(z.double())).reshape(n, groups, -1)
         y = (y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5)).reshape(n, inner) * w.double()
         assert ((out.double() - y).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 4e-6) * y.abs() + 1e-6).all()
+
+
+# --------------------------------------------------------------------- experts of few tokens, picked rows
+@pytest.mark.parametrize("tokens,top,experts,n,k", [(1, 1, 1, 128, 128), (3, 2, 5, 136, 200), (16, 4, 8, 256, 1024), (17, 6, 64, 384, 128),
+                                                    (64, 8, 8, 2048, 136)])
+@pytest.mark.parametrize("act", [None, "gelu"])
+def test_experts_streamed_past_few_tokens(tokens, top, experts, n, k, act):
+    ops = _ops()
+    x, w = _rand(tokens, k, seed=1, dtype=torch.bfloat16), _rand(experts, n, k, seed=2, dtype=torch.bfloat16, scale=k ** -0.5)
+    ids = torch.rand(tokens, experts + 1, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda").argsort(1)[:, :top]
+    ids = ids.to(torch.int32).contiguous()               # choice `experts` is an identity expert: no row
+    tile = -(-tokens // 16) * 16
+    _, pos_of, tile_expert, used = ops.moe_align(ids, experts, tile, identity=1)
+    rows = ops.moe_gather_rows(x, pos_of, tile_expert.numel() * tile)
+    y = ops.moe_linear_stream(rows, tile, w, tile_expert, used, act)
+    for t in range(tokens):
+        for j in range(top):
+            e = int(ids[t, j])
+            if e == experts:
+                assert int(pos_of[t, j]) == -1
+                continue
+            want = w[e].double() @ x[t].double()
+            want = torch.nn.functional.gelu(want) if act else want
+            assert ((y[int(pos_of[t, j])].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+    ops.check_status()
+
+
+@pytest.mark.parametrize("hidden", [4, 512, 516, 33])
+@pytest.mark.parametrize("parts", [1, 8, 9])
+def test_picked_rows_in_vectors(hidden, parts):
+    ops, n, rows = _ops(), 5, 40
+    for dtype in (torch.float32, torch.bfloat16):
+        y, own = _rand(rows, hidden, seed=1, dtype=dtype), _rand(n, hidden, seed=2, dtype=dtype)
+        pick = torch.randint(0, rows, (n, parts), generator=torch.Generator(device="cuda").manual_seed(3), device="cuda").to(torch.int32)
+        coef, own_coef = _rand(n, parts, seed=4), _rand(n, seed=5)
+        for with_own in (False, True):
+            p = pick.clone()
+            if with_own:
+                p[2, 0] = -1                             # an identity expert: no row
+            got = ops.PickedRows(y, p, coef, *((own, own_coef) if with_own else ())).tensor()
+            want = ((coef * (p >= 0)).double()[:, :, None] * y.double()[p.clamp(min=0).long()]).sum(1)
+            if with_own:
+                want = want + own_coef.double()[:, None] * own.double()
+            assert ((got.double() - want).abs() <= 1e-5).all()
+    ops.check_status()
+    ops.PickedRows(_rand(4, hidden, seed=1), torch.full((1, 1), 4, dtype=torch.int32, device="cuda"), _rand(1, 1, seed=2)).tensor()
+    with pytest.raises(ops.KernelError):
+        ops.check_status()
