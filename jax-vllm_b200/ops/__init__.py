@@ -1322,6 +1322,8 @@ def bmm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None)
     if a.dtype != torch.float32:
         if out is None:
             return torch.bmm(a, w.transpose(1, 2))
+        if out.shape == (heads, n, m) and out.dtype == a.dtype and n:
+            return torch.bmm(a, w.transpose(1, 2), out=out)      # written in place, a row of any stride
         out.copy_(torch.bmm(a, w.transpose(1, 2)))
         return out
     if out is None:

@@ -158,20 +158,22 @@ class LatentAttention(Part):
             row = ops.linear(ops.rms_rows(row[:, :self.dq], self.q_norm, self.spec.latent_norm_eps), self.w_uq, dt)
         q_plain = row[:, :H * (self.dp + self.dr)].view(n, H, self.dp + self.dr)[:, :, :self.dp].transpose(0, 1)
         q = torch.empty((n, H * self.dk), dtype=dt, device=x.device)
-        if dt == torch.float32:
-            # the batched product writes the latent part of every query head in place
-            ops.bmm_heads(q_plain, self.w_uk, out=q.view(n, H, self.dk)[:, :, :self.dc].transpose(0, 1))
-            q_lat = None
-        else:
-            q_lat = ops.bmm_heads(q_plain, self.w_uk.to(dt) if wide else self.w_uk)
-        ops.latent_prepare(row, 0, self.kv_off, q_lat, q, step.positions, step.token_entry, table,
+        # the batched product writes the latent part of every query head in place
+        ops.bmm_heads(q_plain, self.w_uk.to(dt) if wide else self.w_uk,
+                      out=q.view(n, H, self.dk)[:, :, :self.dc].transpose(0, 1))
+        ops.latent_prepare(row, 0, self.kv_off, None, q, step.positions, step.token_entry, table,
                            self.position.table() if self.position is not None else None,
                            self.latent_norm, self.spec.latent_norm_eps, cache.k if writes else None,
                            H, self.dp, self.dr, self.dc, kv_row=kv_row, interleaved=self.interleaved)
         o_lat = self.attend(q, step, cache, table)                      # [n, H, >= latent_dim], the latent part leads
-        o = ops.bmm_heads(o_lat[:, :, :self.dc].transpose(0, 1), self.w_uv.to(dt) if wide else self.w_uv)
-        gate = (row if kv_row is None else kv_row)[:, self.g_off:self.g_off + H * self.dv] if self.g_off >= 0 else None
-        return ops.linear(ops.gate_heads(o, gate), self.w_o, dt, parts_ok=True)
+        w_uv = self.w_uv.to(dt) if wide else self.w_uv
+        if self.g_off < 0:                                              # no gate: the product writes the rows in place
+            o = torch.empty((n, H * self.dv), dtype=o_lat.dtype, device=x.device)
+            ops.bmm_heads(o_lat[:, :, :self.dc].transpose(0, 1), w_uv, out=o.view(n, H, self.dv).transpose(0, 1))
+        else:
+            o = ops.bmm_heads(o_lat[:, :, :self.dc].transpose(0, 1), w_uv)
+            o = ops.gate_heads(o, (row if kv_row is None else kv_row)[:, self.g_off:self.g_off + H * self.dv])
+        return ops.linear(o, self.w_o, dt, parts_ok=True)
 
     def attend(self, q, step, cache, table):
         """One key/value head: the cache row is the key, its leading latent part the value."""
@@ -188,7 +190,9 @@ class LatentAttention(Part):
             if n_dec:
                 # keys in splits of 32 to decode_split_size positions, so short that the blocks about fill the device
                 # (one block a multiprocessor); the merge adds a request's splits in ascending order
-                want = -(-step.max_seq_len * n_dec // ops.multiprocessors(q.device))
+                # under a window no more than its keys are looked at
+                seen = min(step.max_seq_len, self.spec.window) if self.spec.window else step.max_seq_len
+                want = -(-seen * n_dec // ops.multiprocessors(q.device))
                 split = min(self.ctx.decode_split_size, max(32, -(-want // 32) * 32))
                 split = max(split, -(-step.max_seq_len // (32 * 1024)) * 32)        # the merge takes up to 1,024 splits
                 ops.attn_latent_mma(q, q.stride(0), out, *args, dwork, n_dec, H, dk, self.dc, self.spec.scale,

@@ -309,3 +309,87 @@ def test_picked_rows_in_vectors(hidden, parts):
     ops.PickedRows(_rand(4, hidden, seed=1), torch.full((1, 1), 4, dtype=torch.int32, device="cuda"), _rand(1, 1, seed=2)).tensor()
     with pytest.raises(ops.KernelError):
         ops.check_status()
+
+
+# ------------------------------------------------------------------------------- latent rows
+@pytest.mark.parametrize("heads,dk,dv", [(1, 48, 40), (8, 288, 256), (16, 576, 512), (16, 104, 99), (17, 576, 512), (32, 88, 80), (33, 160, 128), (16, 640, 512)])
+@pytest.mark.parametrize("split,window,sink", [(32, 0, False), (64, 70, True), (160, 0, True), (96, 1, False)])
+def test_latent_rows_single_tokens(heads, dk, dv, split, window, sink):
+    """A token's heads fill 16, 32 or 64 rows of the tile: chunks of keys shared out among four groups, two, or one.  Contexts
+    at the edges of chunks and splits; unowned places of the pages hold NaN."""
+    ops = _ops()
+    ctx, page = [0, 15, 16, 31, 64, 95, 200, 333], 16
+    n, widest = len(ctx), max(ctx) // page + 1
+    cache = torch.full((n * widest, page, 1, dk), float("nan"), device="cuda", dtype=torch.bfloat16)
+    table = torch.randperm(n * widest, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(n, widest).cuda()
+    keys = []
+    for e, c in enumerate(ctx):
+        rows = _rand(c + 1, dk, seed=e, dtype=torch.bfloat16)
+        keys.append(rows.double())
+        at = torch.arange(c + 1, device="cuda")
+        cache[table[e, at // page].long(), at % page, 0] = rows
+    q = _rand(n, heads * dk, seed=9, dtype=torch.bfloat16)
+    sinks = _rand(heads, seed=3) if sink else None
+    out = torch.full((n, heads * dv), float("nan"), device="cuda", dtype=torch.bfloat16)
+    cu = torch.arange(n + 1, device="cuda", dtype=torch.int32)
+    work = torch.tensor([(e, 0) for e in range(n)], dtype=torch.int32, device="cuda")
+    scale = dk ** -0.5
+    ops.attn_latent_mma(q, q.stride(0), out, cache, table, cu, torch.tensor(ctx, dtype=torch.int32, device="cuda"), work, n, heads,
+                        dk, dv, scale, split_size=split, n_splits=-(-(max(ctx) + 1) // split), window=window, sink=sinks)
+    ops.check_status()
+    for e, c in enumerate(ctx):
+        seen = keys[e][max(0, c + 1 - window):] if window else keys[e]
+        score = q[e].view(heads, dk).double() @ seen.T * scale
+        if sink:
+            score = torch.cat([score, sinks.double()[:, None]], 1)
+        p = score.softmax(1)[:, :seen.shape[0]]
+        want, weight = p @ seen[:, :dv], p @ seen[:, :dv].abs()
+        # the weights and the result are rounded to 16 bits (2^-9 each); scores of dk products in 32 bits
+        bound = 2.0 ** -8 * weight + 2.0 ** -8 * want.abs() + 1e-5
+        assert bool(((out[e].view(heads, dv).double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("width,off", [(8, 0), (256, 8), (1536, 0), (1536, 4), (2056, 0), (8192, 0), (8200, 0), (77, 0)])
+@pytest.mark.parametrize("weight", [None, torch.float32, torch.bfloat16])
+def test_normed_rows_in_vectors(width, off, weight):
+    ops = _ops()
+    x = _rand(5, width + off + 8, seed=width, dtype=torch.bfloat16)[:, off:off + width]
+    w = None if weight is None else _rand(width, seed=2, dtype=weight)
+    y = ops.rms_rows(x, w, 1e-5).double()
+    want = x.double() * (x.double().square().mean(1, keepdim=True) + 1e-5).rsqrt() * (1.0 if w is None else w.double())
+    assert bool(((y - want).abs() <= (2.0 ** -8 + (width + 8) * EPS32) * want.abs()).all())
+
+
+@pytest.mark.parametrize("heads,rot,latent", [(3, 12, 20), (16, 64, 512), (5, 256, 1024), (2, 258, 1032), (130, 2, 8)])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_latent_rows_prepared(heads, rot, latent, interleaved):
+    """Cos and sin kept over a thread's pairs where their place in the head repeats; a latent kept in registers, and longer."""
+    ops = _ops()
+    n, plain, dk = 3, 8, latent + rot
+    row = _rand(n, heads * (plain + rot) + dk, seed=rot, dtype=torch.bfloat16)
+    pos = torch.tensor([0, 3, 700], dtype=torch.int32, device="cuda")
+    table = torch.zeros((n, 176), dtype=torch.int32, device="cuda")
+    table[1], table[2] = 1, 2
+    freq = 100.0 ** (-torch.arange(0, rot, 2, device="cuda", dtype=torch.float32) / rot)
+    w = _rand(latent, seed=1)
+    cache = torch.zeros((3, 4, 1, dk), device="cuda", dtype=torch.bfloat16)
+    q_latent = _rand(heads, n, latent, seed=2, dtype=torch.bfloat16)
+    q = torch.zeros((n, heads * dk), device="cuda", dtype=torch.bfloat16)
+    ops.latent_prepare(row, 0, heads * (plain + rot), q_latent, q, pos, torch.arange(n, dtype=torch.int32, device="cuda"), table,
+                       freq, w, 1e-5, cache, heads, plain, rot, latent, interleaved=interleaved)
+    ops.check_status()
+
+    def turned(x):                                          # [..., n at dim 0, rot]
+        a = (pos.float()[:, None] * freq).double().view(n, *[1] * (x.dim() - 2), rot // 2)
+        u, v = (x[..., 0::2], x[..., 1::2]) if interleaved else (x[..., :rot // 2], x[..., rot // 2:])
+        y = (u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin())
+        return torch.stack(y, -1).flatten(-2) if interleaved else torch.cat(y, -1)
+    got = q.view(n, heads, dk).double()
+    assert torch.equal(q.view(n, heads, dk)[..., :latent], q_latent.transpose(0, 1))
+    kv = row[:, heads * (plain + rot):].double()
+    c = kv[:, :latent] * (kv[:, :latent].square().mean(1, keepdim=True) + 1e-5).rsqrt() * w.double()
+    rows = torch.stack([cache[0, 0, 0], cache[1, 3, 0], cache[2, 0, 0]]).double()
+    want_q = turned(row[:, :heads * (plain + rot)].view(n, heads, plain + rot)[..., plain:].double())
+    # results rounded to 16 bits, of numbers up to 6; cos and sin of 32-bit angles good to a few 2^-24
+    for a, b in ((got[..., latent:], want_q), (rows[:, :latent], c), (rows[:, latent:], turned(kv[:, latent:]))):
+        assert bool(((a - b).abs() <= 2.0 ** -8 * b.abs() + 1e-5).all())
