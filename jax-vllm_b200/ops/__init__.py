@@ -748,6 +748,39 @@ def attn_latent_mma(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache: to
              int(split_size), int(n_splits), _status_ptr(q.device), _stream()), "attn_latent_mma", launches=2 if n_splits > 0 else 1)
 
 
+def attn_latent_tcgen05_supports(dtype: torch.dtype, n_heads: int, dk: int, dv: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel over latent rows takes the case (csrc/attn_latent_tcgen05.cu); restated here for callers
+    without the library."""
+    return (dtype == torch.bfloat16 and 1 <= n_heads <= 128 and dk % 8 == 0 and 8 <= dk <= 576 and dv % 8 == 0
+            and 8 <= dv <= min(dk, 512) and page_size in (8, 16, 32, 64, 128))
+
+
+def attn_latent_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
+                        cu_seqlens: torch.Tensor, start_pos: torch.Tensor, work: torch.Tensor, n_work: int, n_heads: int,
+                        dk: int, dv: int, scale: float, window: int = 0, sink: torch.Tensor | None = None) -> None:
+    """`attn_latent_mma` for prompt portions on the tcgen05 tensor cores (csrc/attn_latent_tcgen05.cu): `work` holds tiles of
+    128 // n_heads tokens."""
+    if sink is not None:
+        _cuda(sink, "sink", torch.float32)
+        if sink.numel() != n_heads:
+            raise KernelError("attn_latent_tcgen05: a sink per head")
+    for t, nm in ((q, "q"), (out, "out"), (cache, "cache")):
+        _cuda(t, nm, torch.bfloat16, contiguous=(nm != "q"))
+    for t, nm in ((block_table, "block_table"), (cu_seqlens, "cu_seqlens"), (start_pos, "start_pos"), (work, "work")):
+        _cuda(t, nm, torch.int32)
+    if n_work == 0:
+        return
+    if cache.shape[2:] != (1, dk) or q.stride(1) != 1 or q.shape[1] < n_heads * dk or out.shape[1] < n_heads * dv:
+        raise KernelError(f"attn_latent_tcgen05: cache {tuple(cache.shape)}, queries or output do not fit rows of {dk}")
+    f = _fn("attn_latent_tcgen05", "jv_attn_latent_tcgen05",
+            [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int,
+             c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p])
+    _check(f(q.data_ptr(), q_stride, q.shape[0], out.data_ptr(), out.stride(0), cache.data_ptr(), block_table.data_ptr(),
+             block_table.shape[1], cu_seqlens.data_ptr(), start_pos.data_ptr(), work.data_ptr(), n_work, n_heads, dk, dv,
+             cache.shape[1], cache.shape[0], float(scale), int(window), _ptr(sink), _status_ptr(q.device), _stream()),
+           "attn_latent_tcgen05")
+
+
 _counters: dict[int, torch.Tensor] = {}
 _counters_outgrown: list = []     # smaller buffers that a captured graph may still point at: never freed
 

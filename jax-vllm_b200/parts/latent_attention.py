@@ -56,10 +56,10 @@ class LatentAttention(Part):
         # bfloat16 with a row size the tensor-core kernels are built for; else the CUDA-core kernel
         # (the kernels built for fixed head sizes have no sink)
         self.use_mma = ops.attn_mma_supports(ctx.dtype, self.dk) and spec.sink is None
-        # other row sizes in bfloat16: the tensor-core kernel written for latent rows (key = the row, value = its start)
+        # other row sizes in bfloat16: the tensor-core kernels written for latent rows (key = the row, value = its start)
         self.use_latent_mma = not self.use_mma and ops.attn_latent_mma_supports(ctx.dtype, self.dk, self.dc)
         if self.use_latent_mma:
-            self.kernels = ("latent_prepare", "attn_latent_mma", "gemm_simt", "linear_skinny")
+            self.kernels = ("latent_prepare", "attn_latent_mma", "attn_latent_tcgen05", "gemm_simt", "linear_skinny")
         if self.use_mma:
             self.kernels = ("latent_prepare", "attn_mma", "gemm_simt", "linear_skinny")
             if self.dk == 128:
@@ -126,6 +126,11 @@ class LatentAttention(Part):
         return PagedKVNeed(1, self.dk, self.spec.window or None, shared_kv=True)
 
     FOREVER = 1 << 30
+    # Of portions of two tokens or more the tcgen05 kernel takes all whose sizes it takes (16 heads, rows of 576: 2 tokens behind
+    # 1,500 121 -> 69 us, 64 behind none 28.7 -> 21.5, 2,048 in a window of 1,024 371 -> 179), but for short rows where no request
+    # has more keys than one chunk of the other kernel's holds (8 heads, rows of 288: 2 tokens alone 14.3 against 16.4 us, behind
+    # 1,500 76.8 against 51.2; rows of 576 18.5 against 18.4).
+    SHORT_ROWS, SHORT_KEYS = 512, 32
 
     def _head_group(self) -> int:
         """The tcgen05 kernels take up to 16 query heads on one key/value head: more heads go through them in
@@ -134,7 +139,11 @@ class LatentAttention(Part):
 
     def tile_classes(self, page_size: int):
         if self.use_latent_mma:
-            return [(ops.attn_latent_mma_tokens_per_tile(self.h), 2, self.FOREVER)]
+            small = (ops.attn_latent_mma_tokens_per_tile(self.h), 2, self.FOREVER)
+            if not ops.attn_latent_tcgen05_supports(self.ctx.dtype, self.h, self.dk, self.dc, page_size):
+                return [small]
+            big = (128 // self.h, 2, self.FOREVER)
+            return [big] if self.dk > self.SHORT_ROWS or big == small else [big, small]
         small = (ops.attn_mma_tokens_per_tile if self.use_mma else ops.attn_simt_tokens_per_tile)(self.h, 1)
         g = self._head_group()
         if self.use_mma and ops.attn_tcgen05_supports(self.ctx.dtype, self.dk, g, 1, page_size, self.mask):
@@ -182,10 +191,13 @@ class LatentAttention(Part):
         if self.use_latent_mma:
             out = torch.empty((n, H * self.dc), dtype=q.dtype, device=q.device)
             args = (cache.k, table, step.cu_seqlens, step.start_pos)
-            for cls in self.tile_classes(cache.k.shape[1]):
-                work, n_work = step.tile_work[cls]
-                ops.attn_latent_mma(q, q.stride(0), out, *args, work, n_work, H, dk, self.dc, self.spec.scale,
-                                    window=self.mask, sink=self.sink)
+            page = cache.k.shape[1]
+            kernel, classes = ops.attn_latent_mma, self.tile_classes(page)
+            if ops.attn_latent_tcgen05_supports(q.dtype, H, dk, self.dc, page) and \
+                    (dk > self.SHORT_ROWS or step.max_seq_len > self.SHORT_KEYS):
+                kernel = ops.attn_latent_tcgen05
+            work, n_work = step.tile_work[classes[0] if kernel is ops.attn_latent_tcgen05 else classes[-1]]
+            kernel(q, q.stride(0), out, *args, work, n_work, H, dk, self.dc, self.spec.scale, window=self.mask, sink=self.sink)
             dwork, n_dec = step.decode_work
             if n_dec:
                 # keys in splits of 32 to decode_split_size positions, so short that the blocks about fill the device

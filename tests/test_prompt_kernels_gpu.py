@@ -393,3 +393,52 @@ def test_latent_rows_prepared(heads, rot, latent, interleaved):
     # results rounded to 16 bits, of numbers up to 6; cos and sin of 32-bit angles good to a few 2^-24
     for a, b in ((got[..., latent:], want_q), (rows[:, :latent], c), (rows[:, latent:], turned(kv[:, latent:]))):
         assert bool(((a - b).abs() <= 2.0 ** -8 * b.abs() + 1e-5).all())
+
+
+@pytest.mark.parametrize("heads,dk,dv,page", [(16, 576, 512, 16), (8, 288, 256, 64), (1, 64, 64, 8), (3, 40, 24, 128), (24, 328, 264, 32),
+                                              (128, 576, 512, 16), (5, 72, 72, 16)])
+@pytest.mark.parametrize("mask,sink", [(0, False), (130, True), (-192, True), (1, False)])
+def test_latent_rows_of_prompts(heads, dk, dv, page, mask, sink):
+    """Tiles of 128 rows that heads fill or leave rows of, pieces of 64 and part of one, one half of the columns or two; contexts
+    and lengths at the edges of key tiles; places and pages that no query sees hold NaN or are missing."""
+    ops = _ops()
+
+    def first_visible_key(pos, mask):
+        return max(0, pos - mask + 1) if mask > 0 else pos - pos % -mask if mask < 0 else 0
+    ctx, new = [0, 127, 300, 5], [1, 130, 129, 40]
+    n, widest = len(ctx), -(-max(c + m for c, m in zip(ctx, new)) // page)
+    cache = torch.full((n * widest, page, 1, dk), float("nan"), device="cuda", dtype=torch.bfloat16)
+    table = torch.randperm(n * widest, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(n, widest).cuda()
+    keys = []
+    for e, (c, m) in enumerate(zip(ctx, new)):
+        rows, low = _rand(c + m, dk, seed=e, dtype=torch.bfloat16), first_visible_key(c, mask)
+        keys.append(rows.double())
+        at = torch.arange(low, c + m, device="cuda")
+        cache[table[e, at // page].long(), at % page, 0] = rows[low:]
+        table[e, :low // page] = -1
+    tokens, per = sum(new), 128 // heads
+    q = _rand(tokens, heads * dk + 8, seed=9, dtype=torch.bfloat16)
+    sinks = _rand(heads, seed=3) if sink else None
+    out = torch.full((tokens, heads * dv), float("nan"), device="cuda", dtype=torch.bfloat16)
+    cu = torch.tensor([0] + new, device="cuda").cumsum(0).to(torch.int32)
+    work = torch.tensor([(e, i) for e in range(n) for i in range(0, new[e], per)], dtype=torch.int32, device="cuda")
+    assert ops.attn_latent_tcgen05_supports(torch.bfloat16, heads, dk, dv, page)
+    ops.attn_latent_tcgen05(q, q.stride(0), out, cache, table, cu, torch.tensor(ctx, dtype=torch.int32, device="cuda"), work,
+                            work.shape[0], heads, dk, dv, dk ** -0.5, window=mask, sink=sinks)
+    ops.check_status()
+    row = 0
+    for e, (c, m) in enumerate(zip(ctx, new)):
+        pos, at = c + torch.arange(m, device="cuda"), torch.arange(c + m, device="cuda")
+        low = torch.tensor([first_visible_key(int(x), mask) for x in pos], device="cuda")
+        hidden = (at[None] > pos[:, None]) | (at[None] < low[:, None])
+        score = torch.einsum("thd,jd->htj", q[row:row + m, :heads * dk].view(m, heads, dk).double(), keys[e]) * dk ** -0.5
+        score = score.masked_fill(hidden[None], float("-inf"))
+        if sink:
+            score = torch.cat([score, sinks.double()[:, None, None].expand(-1, m, 1)], 2)
+        p = score.softmax(2)[:, :, :c + m]
+        want = torch.einsum("htj,jd->thd", p, keys[e][:, :dv])
+        weight = torch.einsum("htj,jd->thd", p, keys[e][:, :dv].abs())
+        # the weights and the result are rounded to 16 bits (2^-9 each); scores of dk products in 32 bits
+        bound = 2.0 ** -8 * weight + 2.0 ** -8 * want.abs() + 1e-5
+        assert bool(((out[row:row + m].view(m, heads, dv).double() - want).abs() <= bound).all())
+        row += m
