@@ -442,3 +442,60 @@ def test_latent_rows_of_prompts(heads, dk, dv, page, mask, sink):
         bound = 2.0 ** -8 * weight + 2.0 ** -8 * want.abs() + 1e-5
         assert bool(((out[row:row + m].view(m, heads, dv).double() - want).abs() <= bound).all())
         row += m
+
+
+# ------------------------------------------------------------------------------- heads before and after attention
+@pytest.mark.parametrize("n", [1, 3, 700])
+@pytest.mark.parametrize("dim,rot,v_rot", [(8, 8, 0), (64, 64, 0), (64, 32, 64), (128, 96, 32), (256, 256, 0), (16, 0, 16), (64, 6, 0)])
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("norms", ["none", "weights", "unit"])
+def test_heads_prepared_in_vectors(n, dim, rot, v_rot, interleaved, norms):
+    """Whole vectors against the general kernel, which takes the same heads two bytes off the 16-byte boundary; one head a
+    thread and four, a page that is missing, rotations of part of a head, values rotated by a table of their own."""
+    ops = _ops()
+    hq, hk, hv, page = 16, 4, 3, 16
+    width = (hq + hk + hv) * dim
+    data = _rand(n, width, seed=n + dim, dtype=torch.bfloat16)
+    pos = torch.arange(n, dtype=torch.int32, device="cuda") + 5
+    table = torch.randperm(n // page + 2, generator=torch.Generator().manual_seed(2)).to(torch.int32).cuda()[None]
+    freq = None if not rot else 1e3 ** (-torch.arange(0, rot, 2, device="cuda", dtype=torch.float32) / rot)
+    v_freq = None if not v_rot else 1e2 ** (-torch.arange(0, v_rot, 2, device="cuda", dtype=torch.float32) / v_rot)
+    weight = _rand(dim, seed=4) if norms == "weights" else None
+    results = []
+    for off in (0, 1):
+        buf = torch.zeros((n, width + 8), device="cuda", dtype=torch.bfloat16)
+        buf[:, off:off + width] = data
+        q = torch.zeros((n, hq * dim), device="cuda", dtype=torch.bfloat16)
+        k = torch.zeros((table.shape[1], page, hk, dim), device="cuda", dtype=torch.bfloat16)
+        v = torch.zeros((table.shape[1], page, hv, dim), device="cuda", dtype=torch.bfloat16)
+        ops.head_prepare(buf, off, off + hq * dim, off + (hq + hk) * dim, q, pos, torch.zeros(n, dtype=torch.int32, device="cuda"),
+                         table, freq, interleaved, weight, weight, 1e-5, norms == "unit", v_freq, k, v, hq, hk, hv, dim, dim,
+                         unit_heads=norms == "unit", gain=1.5)
+        ops.check_status()
+        results.append((q, k, v))
+    assert bool(results[0][0].any()) and bool(results[0][1].any()) and bool(results[0][2].any())
+    for a, b in zip(*results):
+        a, b = a.double(), b.double()
+        # the same 32-bit arithmetic, sums of squares in another order: results of up to 6 differ by rounding to 16 bits at most
+        assert bool(((a - b).abs() <= 2.0 ** -7 * b.abs() + 1e-5).all())
+        assert float((a != b).double().mean()) < 0.01
+
+
+@pytest.mark.parametrize("maps", [1, 2])
+@pytest.mark.parametrize("gate", [0, 1, 2])
+@pytest.mark.parametrize("dv,dtype", [(8, torch.float32), (64, torch.bfloat16), (72, torch.bfloat16), (256, torch.float32)])
+def test_heads_finished_in_vectors(maps, gate, dv, dtype):
+    ops = _ops()
+    n, heads = 37, 5
+    a = _rand(n, maps * heads * dv, seed=dv, dtype=dtype)
+    g = None if not gate else _rand(n, 8 + heads * dv, seed=3, dtype=torch.bfloat16)[:, 8:8 + (heads if gate == 1 else heads * dv)]
+    out = torch.empty((n, heads * dv), device="cuda", dtype=torch.bfloat16)
+    ops.attn_finish(a, out, heads, dv, maps=maps, lam=0.7, post=1.25, gate=g)
+    x = a.double().view(n, maps, heads, dv)
+    want, size = x[:, 0], x[:, 0].abs()
+    if maps == 2:
+        want, size = want - 0.7 * x[:, 1], size + 0.7 * x[:, 1].abs()
+    scale = 1.25 if not gate else 1.25 * torch.sigmoid(g.double()).view(n, heads, -1)
+    want, size = want * scale, size * scale
+    # rounded to 16 bits; a few 32-bit operations before
+    assert bool(((out.view(n, heads, dv).double() - want).abs() <= 2.0 ** -8 * want.abs() + 16 * EPS32 * size).all())
