@@ -4,8 +4,8 @@
 //   dt  = softplus(dt_raw + dt_bias)                 a = exp(-exp(A_log) * dt)
 //   S  <- a S + dt * B x^T                           y = S^T C + D x
 //
-// which is the update of csrc/recurrent.cu's state scan with the key dt * B, the query C and the decay a in every
-// key channel.  B and C are shared by the heads of a group (head h uses group h / (heads / groups)).
+// which is the update of csrc/recurrent.cu's state scan (long portions: csrc/chunk_scan.cu) with the key dt * B, the
+// query C and the decay a in every key channel.  B and C are shared by the heads of a group (head h uses group h / (heads / groups)).
 //
 // jv_mamba_prepare, one warp per (token, head): packed[t, h] = (C_g, dt * B_g, a) as float32 [3][N], from the
 //   convolved rows xbc = [x | B | C] and the raw step sizes; softplus, both exponentials and the product with B in 32-bit.

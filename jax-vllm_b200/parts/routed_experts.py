@@ -8,6 +8,7 @@ activation is a kernel of its own).
                or, with `scoring` "table", no router: a table names each token id's experts, all weights 1 / top_k
     order    = pairs sorted by expert   every expert's rows padded to a row tile (csrc/moe_route.cu, jv_moe_align)
     a        = act(x[token] @ W_up_e^T) grouped product, rows gathered as they are read, activation in its epilogue
+                                        (few tokens: the weights stream past them, csrc/linear_stream.cu)
     y        = a @ W_down_e^T           grouped product
     out[t]   = sum_k w[t, k] * y[pos(t, k)]     added up in 32-bit, k ascending, by the reader of the result
 
