@@ -459,11 +459,11 @@ template <int DVW, int WD, bool SPLIT, int KG>
 int launch_one(const LatentParams& p, dim3 grid, cudaStream_t stream) {
   auto kern = attn_latent_mma_kernel<DVW, WD, SPLIT, KG>;
   const size_t smem = smem_bytes(KG, p.qstride_s, p.kstride_s, WD);
-  static size_t allowed = 0;       // set once per size: the attribute call is kept out of stream captures
-  if (smem > allowed) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return JV_ERR_UNSUPPORTED;
-    allowed = smem;
-  }
+  static bool ready[JV_MAX_DEVICES];       // for the largest size that is taken
+  if (!jv_once_per_device(ready, [&] {
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM) == cudaSuccess;
+      }))
+    return JV_ERR_UNSUPPORTED;
   return jv_launch(kern, grid, dim3(128 * WD), smem, stream, p);
 }
 

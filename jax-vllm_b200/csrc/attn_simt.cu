@@ -289,6 +289,8 @@ __global__ void attn_combine_kernel(const AttnParams p) {
   }
 }
 
+constexpr size_t MAX_SMEM = 227 * 1024;      // the largest size that is taken
+
 size_t smem_bytes(int D, int DV) {
   return sizeof(float) * ((size_t)BLOCK_M * D + (size_t)BLOCK_N * (D + 1) + (size_t)BLOCK_N * DV +
                           BLOCK_M * BLOCK_N + 3 * BLOCK_M) + sizeof(int) * BLOCK_M;
@@ -332,7 +334,7 @@ JV_EXPORT int jv_attn_simt_ex(const void* q, int q_stride, void* out, int out_st
   if (n_k_heads <= 0) n_k_heads = n_kv_heads;
   // whole key rows where they fit in shared memory beside the values, else pieces of 256 elements
   const int d_chunk = smem_bytes(head_dim, v_dim) <= 200 * 1024 ? head_dim : 256;
-  if (head_dim < 1 || v_dim > v_row || v_dim > 512 || smem_bytes(d_chunk, v_dim) > 227 * 1024 || n_kv_heads < 1 ||
+  if (head_dim < 1 || v_dim > v_row || v_dim > 512 || smem_bytes(d_chunk, v_dim) > MAX_SMEM || n_kv_heads < 1 ||
       n_q_heads % n_kv_heads != 0)
     return JV_ERR_UNSUPPORTED;
   AttnParams p;
@@ -358,12 +360,11 @@ JV_EXPORT int jv_attn_simt_ex(const void* q, int q_stride, void* out, int out_st
   JV_DISPATCH_DTYPE(dtype, T, {
     if (n_splits > 0) {
       auto kern = attn_simt_kernel<T, true>;
-      static size_t allowed = 0;   // set once per size: the attribute call is kept out of stream captures
-      if (smem > allowed) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-          return JV_ERR_UNSUPPORTED;
-        allowed = smem;
-      }
+      static bool ready[JV_MAX_DEVICES];
+      if (!jv_once_per_device(ready, [&] {
+            return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM) == cudaSuccess;
+          }))
+        return JV_ERR_UNSUPPORTED;
       kern<<<grid, THREADS, smem, stream>>>(p);
       rc = jv_check_launch();
       if (rc == JV_OK) {
@@ -372,12 +373,11 @@ JV_EXPORT int jv_attn_simt_ex(const void* q, int q_stride, void* out, int out_st
       }
     } else {
       auto kern = attn_simt_kernel<T, false>;
-      static size_t allowed = 0;
-      if (smem > allowed) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-          return JV_ERR_UNSUPPORTED;
-        allowed = smem;
-      }
+      static bool ready[JV_MAX_DEVICES];
+      if (!jv_once_per_device(ready, [&] {
+            return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM) == cudaSuccess;
+          }))
+        return JV_ERR_UNSUPPORTED;
       kern<<<grid, THREADS, smem, stream>>>(p);
       rc = jv_check_launch();
     }

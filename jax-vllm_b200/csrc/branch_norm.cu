@@ -13,6 +13,7 @@
 
 namespace {
 constexpr int MAX_PICKS = 64;     // rows that one row of a branch may be the weighted sum of
+constexpr size_t MAX_SMEM = 200 * 1024;     // of a row in 32-bit
 
 template <typename TD, typename TW, typename TX>
 __global__ void branch_norm_add_kernel(float* __restrict__ h, const TD* __restrict__ y, size_t part_stride, int parts,
@@ -234,7 +235,7 @@ JV_EXPORT int jv_branch_norm_add(float* h, const void* y, int y_dtype, long long
                                  int weight_dtype, void* x_out, int x_dtype, int n, int hidden, float eps, float mult,
                                  int* status, cudaStream_t stream) {
   if (n == 0) return JV_OK;
-  if (parts < 1 || (pick != nullptr && parts > MAX_PICKS) || (size_t)hidden * sizeof(float) > 200 * 1024) return JV_ERR_UNSUPPORTED;
+  if (parts < 1 || (pick != nullptr && parts > MAX_PICKS) || (size_t)hidden * sizeof(float) > MAX_SMEM) return JV_ERR_UNSUPPORTED;
   int threads = 64;
   while (threads < 512 && threads * 4 < hidden) threads *= 2;
   const size_t smem = (size_t)hidden * sizeof(float);
@@ -247,13 +248,12 @@ JV_EXPORT int jv_branch_norm_add(float* h, const void* y, int y_dtype, long long
   JV_DISPATCH_DTYPE(y_dtype, TD, JV_DISPATCH_DTYPE(weight_dtype, TW, JV_DISPATCH_DTYPE(x_dtype, TX, {
     auto kern = vec ? branch_norm_add_vec_kernel<TD, TW, TX> : branch_norm_add_kernel<TD, TW, TX>;
     if (smem > 48 * 1024) {       // rows beyond 12,288 elements: both forms are allowed the larger size once
-      static size_t allowed = 0;
-      if (smem > allowed) {
-        if (cudaFuncSetAttribute(branch_norm_add_vec_kernel<TD, TW, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaFuncSetAttribute(branch_norm_add_kernel<TD, TW, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-          return JV_ERR_UNSUPPORTED;
-        allowed = smem;
-      }
+      static bool ready[JV_MAX_DEVICES];
+      if (!jv_once_per_device(ready, [&] {
+            return cudaFuncSetAttribute(branch_norm_add_vec_kernel<TD, TW, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM) == cudaSuccess &&
+                   cudaFuncSetAttribute(branch_norm_add_kernel<TD, TW, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM) == cudaSuccess;
+          }))
+        return JV_ERR_UNSUPPORTED;
     }
     return jv_launch(kern, dim3(n), dim3(threads), smem, stream, h, (const TD*)y, (size_t)part_stride, parts, pick,
                      coef, y_rows, (const TW*)weight, (TX*)x_out, hidden, eps, mult, status);
