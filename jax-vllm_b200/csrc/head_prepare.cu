@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(256) rms_rows_vec_kernel(const __nv_bfloat16* 
   pdl_wait();
   const __nv_bfloat16* src = in + (size_t)blockIdx.x * in_stride;
   __nv_bfloat16* dst = out + (size_t)blockIdx.x * out_stride;
-  uint4 raw[ROW_VECS];
-  TW weight[ROW_VECS][8];
+  constexpr int W_VECS = sizeof(TW) / 2;                // vectors of sixteen bytes that eight weights fill
+  uint4 raw[ROW_VECS], weight[ROW_VECS][W_VECS];
 #pragma unroll
   for (int k = 0; k < ROW_VECS; ++k) {
     const int d = (threadIdx.x + k * blockDim.x) * 8;
@@ -276,8 +276,7 @@ __global__ void __launch_bounds__(256) rms_rows_vec_kernel(const __nv_bfloat16* 
     raw[k] = *reinterpret_cast<const uint4*>(src + d);
     if (w != nullptr) {
 #pragma unroll
-      for (int j = 0; j < (int)sizeof(TW) / 2; ++j)
-        reinterpret_cast<uint4*>(weight[k])[j] = reinterpret_cast<const uint4*>(w + d)[j];
+      for (int j = 0; j < W_VECS; ++j) weight[k][j] = reinterpret_cast<const uint4*>(w + d)[j];
     }
   }
   float ss = 0.f;
@@ -297,7 +296,7 @@ __global__ void __launch_bounds__(256) rms_rows_vec_kernel(const __nv_bfloat16* 
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       float v = to_f32(e[j]) * inv;
-      if (w != nullptr) v *= to_f32(weight[k][j]);
+      if (w != nullptr) v *= to_f32(reinterpret_cast<const TW*>(weight[k])[j]);
       e[j] = from_f32<__nv_bfloat16>(v);
     }
     *reinterpret_cast<uint4*>(dst + d) = raw[k];
