@@ -11,9 +11,10 @@
 // in chunks of 32 rows (64 with groups, below) by cp.async, two buffers; the chunk in shared memory is the B operand of S = Q K^T as it lies (k contiguous) and, read through ldmatrix.trans, of
 // O += P V: the row is loaded once for both.  Softmax is the running (max, sum) form in registers.
 //
-// SPLIT: work items are single tokens; split s covers key positions [s*split_size, (s+1)*split_size); it writes its
+// SPLIT: work items are single tokens; the keys are cut at multiples of split_size, split 0 is the first that holds a key
+// which the token sees (a window asks for as many splits as it can touch, wherever it lies); a split writes its
 // unnormalised sums and (max, sum) to part_o / part_ml, and `latent_combine_kernel` merges the splits of a row in
-// ascending order, so a result does not depend on what else is in the batch.  Bound by latency: a block has a few chunks.
+// ascending order.  Where the cuts fall hangs on split_size alone.  Bound by latency: a block has a few chunks.
 // 8 tokens of 16 heads, rows of 576, 1,024 visible keys:
 // 22.4 us where one pair of warps took all keys (and half of the blocks held none), 15.7 with groups.
 #include "common.cuh"
@@ -95,8 +96,9 @@ __global__ void __launch_bounds__(128 * WD, 1) attn_latent_mma_kernel(const Late
   if (tokens_here <= 0) return;
   int j_lo = first_visible(ctx + q_off, p.window), j_hi = ctx + q_off + tokens_here;      // keys [j_lo, j_hi)
   if (SPLIT) {
-    j_lo = max(j_lo, (int)blockIdx.z * p.split_size);
-    j_hi = min(j_hi, (blockIdx.z + 1) * p.split_size);
+    const int split = j_lo / p.split_size + blockIdx.z;      // numbered from the first that holds a visible key
+    j_lo = max(j_lo, split * p.split_size);
+    j_hi = min(j_hi, (split + 1) * p.split_size);
     if (j_lo >= j_hi) return;
   }
   const int dk = p.dk, qs = p.qstride_s, ks = p.kstride_s;
@@ -393,13 +395,13 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const LatentParams 
   const int entry = p.work[2 * x];
   const int pos = p.start_pos[entry];
   const size_t token = (size_t)p.cu_seqlens[entry];
-  int s_last = pos / p.split_size;
-  if (s_last >= p.n_splits) {
-    if (threadIdx.x == 0) atomicOr(p.status, JV_STATUS_BAD_ROW);
-    s_last = p.n_splits - 1;
-  }
-  const size_t base = ((size_t)x * p.n_heads + head) * p.n_splits;
   const int s_first = first_visible(pos, p.window) / p.split_size;      // splits before it hold no visible key
+  int s_last = pos / p.split_size;
+  if (s_last - s_first >= p.n_splits) {
+    if (threadIdx.x == 0) atomicOr(p.status, JV_STATUS_BAD_ROW);
+    s_last = s_first + p.n_splits - 1;
+  }
+  const size_t base = ((size_t)x * p.n_heads + head) * p.n_splits - s_first;      // split s_first was written first
   const int d = threadIdx.x * 4;                                         // VEC: the thread's columns
   float4 part[COMBINE_AHEAD];
   auto fetch = [&](int s0) {
@@ -417,7 +419,7 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const LatentParams 
     float l = 0.f;
     for (int s = s_first + lane; s <= s_last; s += 32) {
       const float w = exp2f(p.part_ml[(base + s) * 2] - m_all);
-      w_s[s] = w;
+      w_s[s - s_first] = w;
       l += w * p.part_ml[(base + s) * 2 + 1];
     }
     l = warp_sum(l);
@@ -435,7 +437,7 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const LatentParams 
 #pragma unroll
       for (int k = 0; k < COMBINE_AHEAD; ++k)
         if (s0 + k <= s_last) {
-          const float w = w_s[s0 + k];
+          const float w = w_s[s0 + k - s_first];
           o.x = fmaf(w, part[k].x, o.x); o.y = fmaf(w, part[k].y, o.y);
           o.z = fmaf(w, part[k].z, o.z); o.w = fmaf(w, part[k].w, o.w);
         }
@@ -445,7 +447,7 @@ __global__ void __launch_bounds__(128) latent_combine_kernel(const LatentParams 
   }
   for (int c = threadIdx.x; c < p.dv; c += blockDim.x) {
     float o = 0.f;
-    for (int s = s_first; s <= s_last; ++s) o = fmaf(w_s[s], p.part_o[(base + s) * p.dv + c], o);
+    for (int s = s_first; s <= s_last; ++s) o = fmaf(w_s[s - s_first], p.part_o[(base + s) * p.dv + c], o);
     dst[c] = __float2bfloat16_rn(o * inv);
   }
 }
@@ -501,7 +503,8 @@ JV_EXPORT int jv_attn_latent_mma_supports(int dk, int dv) {
 // q: bfloat16 rows of q_stride elements (head h of token n at q[n*q_stride + h*dk]); out: [n, out_stride], head h at
 // h*dv; cache: [num_pages, page_size, dk] bfloat16; block_table, cu_seqlens, start_pos, work as for the other paged
 // attention kernels; window: the mask (0: causal only); sink: [n_heads] floats or null.  n_splits == 0: every work item attends to all its keys and writes `out`.  n_splits > 0: work
-// items are single tokens; part_o [n_work*heads*n_splits*dv] and part_ml [n_work*heads*n_splits*2] floats are scratch.
+// items are single tokens; part_o [n_work*heads*n_splits*dv] and part_ml [n_work*heads*n_splits*2] floats are scratch, n_splits
+// at least the splits of split_size that the keys of one token touch.
 JV_EXPORT int jv_attn_latent_mma(const void* q, int q_stride, void* out, int out_stride, float* part_o, float* part_ml,
                                  const void* cache, const int* block_table, int table_width, const int* cu_seqlens,
                                  const int* start_pos, const int* work, int n_work, int n_heads, int dk, int dv,

@@ -715,6 +715,21 @@ def attn_latent_mma_tokens_per_tile(n_heads: int) -> int:
     return 64 // min(n_heads, 64)
 
 
+LATENT_MAX_SPLITS = 1024         # of one token that the merge of csrc/attn_latent_mma.cu takes
+
+
+def latent_splits(max_seq_len: int, window: int, n_tokens: int, blocks: int, most: int) -> tuple[int, int]:
+    """(split size, number of splits) for `attn_latent_mma` on `n_tokens` single tokens behind up to `max_seq_len` positions, of
+    which a window of `window` (0: none) lets so many through: 32 to `most` positions, so short that the splits about fill `blocks`
+    blocks.  The number is that of the splits which one token's keys can touch: the engine's captured steps pass the longest
+    sequence that there may ever be, and blocks and scratch for keys before the window would grow with it."""
+    seen = min(max_seq_len, window) if window else max_seq_len
+    split = min(most, max(32, -(-seen * n_tokens // (32 * blocks)) * 32))
+    split = max(split, -(-seen // (32 * (LATENT_MAX_SPLITS - 1 if window else LATENT_MAX_SPLITS))) * 32)
+    n_splits = max(1, -(-max_seq_len // split))
+    return split, min(n_splits, -(-(window - 1) // split) + 1) if window else n_splits
+
+
 def attn_latent_mma(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
                     cu_seqlens: torch.Tensor, start_pos: torch.Tensor, work: torch.Tensor, n_work: int, n_heads: int,
                     dk: int, dv: int, scale: float, split_size: int = 0, n_splits: int = 0, window: int = 0,
@@ -722,7 +737,8 @@ def attn_latent_mma(q: torch.Tensor, q_stride: int, out: torch.Tensor, cache: to
     """Paged causal attention with one key/value head whose key is the cache row [dk] and whose value is the row's
     first dv elements, on the tensor cores (csrc/attn_latent_mma.cu); `work` and the split arguments as for
     `attn_simt`, with `attn_latent_mma_tokens_per_tile` tokens per prompt tile; out has dv elements per head.
-    `window`: the mask as one number (`mask_code`); `sink` [n_heads] float32: exp(sink) counts once in the denominator."""
+    `window`: the mask as one number (`mask_code`); `sink` [n_heads] float32: exp(sink) counts once in the denominator.
+    `n_splits`: at least the splits that one token's visible keys touch (`latent_splits`)."""
     if sink is not None:
         _cuda(sink, "sink", torch.float32)
         if sink.numel() != n_heads:

@@ -200,16 +200,11 @@ class LatentAttention(Part):
             kernel(q, q.stride(0), out, *args, work, n_work, H, dk, self.dc, self.spec.scale, window=self.mask, sink=self.sink)
             dwork, n_dec = step.decode_work
             if n_dec:
-                # keys in splits of 32 to decode_split_size positions, so short that the blocks about fill the device
-                # (one block a multiprocessor); the merge adds a request's splits in ascending order
-                # under a window no more than its keys are looked at
-                seen = min(step.max_seq_len, self.spec.window) if self.spec.window else step.max_seq_len
-                want = -(-seen * n_dec // ops.multiprocessors(q.device))
-                split = min(self.ctx.decode_split_size, max(32, -(-want // 32) * 32))
-                split = max(split, -(-step.max_seq_len // (32 * 1024)) * 32)        # the merge takes up to 1,024 splits
+                # one block a multiprocessor; the merge adds a request's splits in ascending order
+                split, n_splits = ops.latent_splits(step.max_seq_len, self.spec.window or 0, n_dec, ops.multiprocessors(q.device),
+                                                    self.ctx.decode_split_size)
                 ops.attn_latent_mma(q, q.stride(0), out, *args, dwork, n_dec, H, dk, self.dc, self.spec.scale,
-                                    split_size=split, n_splits=max(1, -(-step.max_seq_len // split)),
-                                    window=self.mask, sink=self.sink)
+                                    split_size=split, n_splits=n_splits, window=self.mask, sink=self.sink)
             return out.view(n, H, self.dc)
         if self.use_mma:
             # the tensor-core kernels take keys and values of one size: they return whole rows, the latent part leads

@@ -349,6 +349,38 @@ def test_latent_rows_single_tokens(heads, dk, dv, split, window, sink):
         assert bool(((out[e].view(heads, dv).double() - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("heads,dk,dv", [(16, 576, 512), (17, 104, 99)])
+@pytest.mark.parametrize("split,window", [(32, 1), (32, 33), (64, 200), (96, 97)])
+def test_latent_rows_single_tokens_far_behind_a_window(heads, dk, dv, split, window):
+    """Splits are numbered from the first that the window touches: as many as it can touch are enough for tokens anywhere."""
+    ops = _ops()
+    ctx, page = [0, 63, 1000, 3071, 3072, 3200], 16
+    n, widest = len(ctx), max(ctx) // page + 1
+    cache = torch.full((n * 16, page, 1, dk), float("nan"), device="cuda", dtype=torch.bfloat16)
+    table = torch.full((n, widest), -1, dtype=torch.int32)
+    keys = []
+    for e, c in enumerate(ctx):
+        low = max(0, c + 1 - window)
+        rows = _rand(c + 1 - low, dk, seed=e, dtype=torch.bfloat16)
+        keys.append(rows.double())
+        for j, p in enumerate(range(low // page, c // page + 1)):        # pages before the window were given back
+            table[e, p] = e * 16 + j
+        at = torch.arange(low, c + 1)
+        cache[table[e, at // page].long().cuda(), (at % page).cuda(), 0] = rows
+    q = _rand(n, heads * dk, seed=9, dtype=torch.bfloat16)
+    out = torch.full((n, heads * dv), float("nan"), device="cuda", dtype=torch.bfloat16)
+    work = torch.tensor([(e, 0) for e in range(n)], dtype=torch.int32, device="cuda")
+    ops.attn_latent_mma(q, q.stride(0), out, cache, table.cuda(), torch.arange(n + 1, device="cuda", dtype=torch.int32),
+                        torch.tensor(ctx, dtype=torch.int32, device="cuda"), work, n, heads, dk, dv, dk ** -0.5, split_size=split,
+                        n_splits=-(-(window - 1) // split) + 1, window=window)
+    ops.check_status()
+    for e in range(n):
+        p = (q[e].view(heads, dk).double() @ keys[e].T * dk ** -0.5).softmax(1)
+        want, weight = p @ keys[e][:, :dv], p @ keys[e][:, :dv].abs()
+        # as above: weights and result rounded to 16 bits
+        assert bool(((out[e].view(heads, dv).double() - want).abs() <= 2.0 ** -8 * weight + 2.0 ** -8 * want.abs() + 1e-5).all())
+
+
 @pytest.mark.parametrize("width,off", [(8, 0), (256, 8), (1536, 0), (1536, 4), (2056, 0), (8192, 0), (8200, 0), (77, 0)])
 @pytest.mark.parametrize("weight", [None, torch.float32, torch.bfloat16])
 def test_normed_rows_in_vectors(width, off, weight):
