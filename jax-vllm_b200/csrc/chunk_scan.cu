@@ -51,6 +51,7 @@ struct ChunkParams {
   float* nq;                               // its outputs, every fourth float (the gates' last place)
   const int *cu_seqlens, *slots;
   int n_slots, heads, D, V;
+  int portions, n_entries;                 // portions > 0: entries of one token are passed by, so many others taken
   int* status;
 };
 
@@ -122,7 +123,9 @@ __global__ void __launch_bounds__(32 * WARPS + 32) chunk_scan_kernel(const Chunk
   __shared__ uint64_t rows_full[NBUF], weights_full[NBUF], empty[NBUF];
   pdl_trigger();
   pdl_wait();
-  const int entry = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int entry = entry_of(blockIdx.x, p.portions, p.cu_seqlens, p.n_entries);
+  if (entry < 0) return;
+  const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gr = lane >> 2, gq = lane & 3;             // row and column pair of a fragment
   const int e0 = blockIdx.z * ET;
   const int t0 = p.cu_seqlens[entry], len = p.cu_seqlens[entry + 1] - t0;
@@ -491,13 +494,14 @@ bool rows_of_16_bytes(const void* p, long long stride) { return ((uintptr_t)p & 
 
 // q, k, v: the first head's columns in rows of `.._stride` 16-bit elements (head h reads q and k at (h / per_group) * D, v at h * V);
 // gates [n, heads, 4] float with nq = gates + 3 and state_n, or null with dt_raw (rows of dt_stride elements, [heads] used),
-// dt_bias, a_log [heads] of w_dtype; out [n, heads * V]; state as for jv_state_scan.  Taken for D up to 128 and V, both in steps of
+// dt_bias, a_log [heads] of w_dtype; out [n, heads * V]; state as for jv_state_scan; portions > 0: entries of one token
+// are passed by, which leaves this many.  Taken for D up to 128 and V, both in steps of
 // 8, with rows on 16-byte boundaries.
 JV_EXPORT int jv_chunk_scan(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
                             int per_group, float scale, float* gates, const void* dt_raw, long long dt_stride, const void* dt_bias,
                             const void* a_log, int w_dtype, float* out, float* state, long long slot_stride, float* state_n,
-                            const int* cu_seqlens, const int* slots, int n_slots, int entries, int heads, int D, int V, int* status,
-                            cudaStream_t stream) {
+                            const int* cu_seqlens, const int* slots, int n_slots, int entries, int heads, int D, int V, int portions,
+                            int* status, cudaStream_t stream) {
   if (entries == 0) return JV_OK;
   if (D < 8 || D > 128 || D % 8 || V < 8 || V % 8 || per_group < 1 || heads % per_group || heads > 65535 || entries < 0 ||
       !rows_of_16_bytes(q, q_stride) || !rows_of_16_bytes(k, k_stride) || !rows_of_16_bytes(v, v_stride) || w_dtype < 0 || w_dtype > 1 ||
@@ -505,7 +509,8 @@ JV_EXPORT int jv_chunk_scan(const void* q, long long q_stride, const void* k, lo
     return JV_ERR_UNSUPPORTED;
   ChunkParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, per_group, scale, gates,
                 (const bf16*)dt_raw, dt_stride, dt_bias, a_log, w_dtype, out, state, slot_stride, state_n,
-                gates == nullptr ? nullptr : gates + 3, cu_seqlens, slots, n_slots, heads, D, V, status};
+                gates == nullptr ? nullptr : gates + 3, cu_seqlens, slots, n_slots, heads, D, V, portions, entries, status};
+  if (portions > 0) entries = portions;
   // four warps share a block's scores; two where that alone leaves multiprocessors without a block
   const long long blocks = (long long)entries * heads * ((V + 63) / 64);
   if (blocks >= 148) {

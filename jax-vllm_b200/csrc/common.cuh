@@ -163,6 +163,15 @@ static inline bool jv_once_per_device(bool (&done)[JV_MAX_DEVICES], F&& setup) {
   return true;
 }
 
+// Multiprocessors of the current device.
+static inline int jv_multiprocessors() {
+  static int count[JV_MAX_DEVICES] = {};
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= JV_MAX_DEVICES) return 148;
+  if (count[dev] == 0 && cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  return count[dev];
+}
+
 static inline int jv_check_launch() {
   return cudaGetLastError() == cudaSuccess ? JV_OK : JV_ERR_LAUNCH;
 }

@@ -1,5 +1,5 @@
-// The generalized delta rule over portions of several tokens, four tokens at a time (single tokens, short portions, and states in
-// segments run on the kernels of recurrent.cu).  Per head, with S [key channel, value channel] in 32-bit:
+// The generalized delta rule over portions of several tokens, four tokens at a time (entries of one token run on state_step.cu, a
+// scan token by token or in segments is in recurrent.cu).  Per head, with S [key channel, value channel] in 32-bit:
 //
 //     S <- diag(w_t) S - b_t (u_t^T S) + k_t v_t^T,   o_t = S^T r_t        (both terms of the first read the old S)
 //
@@ -46,14 +46,14 @@ template <int NCH, typename T, typename W>
 __global__ void __launch_bounds__(128) group_prepare_kernel(const T* __restrict__ proj, long long stride, int r_off, int k_off,
                                                             int a_off, const T* __restrict__ zw, long long zw_stride,
                                                             const W* __restrict__ a_bias, const W* __restrict__ w_bias,
-                                                            const int* __restrict__ cu_seqlens, int n_entries,
+                                                            const int* __restrict__ cu_seqlens, int n_entries, int portions,
                                                             float* __restrict__ packed, int heads, int D, int DP) {
   __shared__ float norms[4][T4], sums[4][32];
   __shared__ __align__(16) float coef[COEF];
   pdl_trigger();
   pdl_wait();
   int entry, group, n_groups;
-  if (!find_segment(cu_seqlens, n_entries, T4, blockIdx.x, entry, group, n_groups)) return;
+  if (!find_segment(cu_seqlens, n_entries, T4, portions, blockIdx.x, entry, group, n_groups)) return;
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
   const int first = cu_seqlens[entry] + group * T4, tokens = min(T4, cu_seqlens[entry + 1] - first);
   if (tokens <= 0) return;
@@ -165,25 +165,29 @@ struct GroupScanParams {
   float* state; long long slot_stride;     // S of (slot, head) at state + slot * slot_stride + head * D * V
   const int* cu_seqlens; const int* slots;
   int n_slots, heads, D, V;
+  int portions, n_entries, max_groups;     // portions > 0: entries of one token are passed by, so many others taken
   int* status;
 };
 
 // A block takes 16 value columns of one (entry, head), a warp eight of them; eight lanes share a pair of columns, lane kl the
 // channels 32 i + 4 kl .. + 3 (i < KPT / 4), so that a 16-byte read of eight lanes is a run of 128 bytes.  Two columns a thread:
 // shared memory hands out 128 bytes a clock and each number read should serve more than one multiply-add.
-template <int KPT> struct GroupScanShape {
+// RING_: the stages of the ring.  Six (about 100 KB, two blocks a multiprocessor) carry a block through the latency of its copies;
+// where there are more blocks than two a multiprocessor, others do that, and two stages leave room for more of them (32 heads of 64:
+// 2,048 tokens in one entry 430 us a layer with six, 598 with two; five entries of 400 313 and 281, eight of 8 tokens 51 and 45).
+template <int KPT, int RING_> struct GroupScanShape {
   static constexpr int DP = 8 * KPT;
   static constexpr int FLOATS = VECS * DP + COEF;                       // of a group
   static constexpr int GROUPS = KPT <= 8 ? 4 : KPT <= 16 ? 2 : 1;       // groups of a stage
-  static constexpr int RING = 6, COLS = 16, THREADS = 64;               // about 100 KB: two blocks a multiprocessor
+  static constexpr int RING = RING_, COLS = 16, THREADS = 64;
   static constexpr int VLD = GROUPS * T4 + 4;                           // values of a column in a stage, padded
   static constexpr int STAGE = GROUPS * FLOATS;
   static constexpr int SMEM = (int)sizeof(float) * (RING * STAGE + 2 * COLS * VLD);
 };
 
-template <int KPT, typename T>
+template <int KPT, int RING_, typename T>
 __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p) {
-  using Shape = GroupScanShape<KPT>;
+  using Shape = GroupScanShape<KPT, RING_>;
   constexpr int DP = Shape::DP, FLOATS = Shape::FLOATS, GROUPS = Shape::GROUPS, RING = Shape::RING, COLS = Shape::COLS;
   constexpr int VLD = Shape::VLD, TOK = GROUPS * T4, Q = KPT / 4, THREADS = Shape::THREADS;
   // keys of up to 64: a group's vectors are asked for before the group before is finished (there are registers for it)
@@ -193,7 +197,9 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
   __shared__ uint64_t full[RING];
   pdl_trigger();
   pdl_wait();
-  const int entry = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int entry = entry_of(blockIdx.x, p.portions, p.cu_seqlens, p.n_entries);
+  if (entry < 0) return;
+  const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int kl = lane & 7, lcol = warp * 8 + (lane >> 3) * 2, base = blockIdx.z * COLS, col = base + lcol;
   const int D = p.D, V = p.V;
   const int t0 = p.cu_seqlens[entry], t1 = p.cu_seqlens[entry + 1];
@@ -204,8 +210,12 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
   }
   if (t0 >= t1) return;
   int g0 = 0;                                          // the number of the entry's first group
-  for (int e = 0; e < entry; ++e) g0 += max(1, (p.cu_seqlens[e + 1] - p.cu_seqlens[e] + T4 - 1) / T4);
+  for (int e = 0; e < entry; ++e) g0 += segments_of(p.cu_seqlens[e + 1] - p.cu_seqlens[e], T4, p.portions);
   const int n_groups = (t1 - t0 + T4 - 1) / T4, n_stages = (n_groups + GROUPS - 1) / GROUPS;
+  if (g0 + n_groups > p.max_groups) {                  // more portions than were said to be there
+    if (tid == 0) atomicOr(p.status, JV_STATUS_BAD_ROW);
+    return;
+  }
   float* S_g = p.state + (size_t)slot * p.slot_stride + (size_t)h * D * V;
   auto channel = [&](int i) { return (i / 4) * 32 + kl * 4 + (i & 3); };
   const size_t group_stride = (size_t)p.heads * FLOATS;
@@ -423,16 +433,23 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
     }
 }
 
-template <int KPT, typename T>
-int launch_scan(const GroupScanParams& p, int entries, cudaStream_t stream) {
-  using Shape = GroupScanShape<KPT>;
-  auto kern = group_scan_kernel<KPT, T>;
+template <int KPT, int RING, typename T>
+int launch_ring(const GroupScanParams& p, int entries, cudaStream_t stream) {
+  using Shape = GroupScanShape<KPT, RING>;
+  auto kern = group_scan_kernel<KPT, RING, T>;
   static bool done[JV_MAX_DEVICES] = {};
   if (!jv_once_per_device(done, [&] {
         return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM) == cudaSuccess;
       }))
     return JV_ERR_UNSUPPORTED;
   return jv_launch(kern, dim3(entries, p.heads, (p.V + Shape::COLS - 1) / Shape::COLS), dim3(Shape::THREADS), Shape::SMEM, stream, p);
+}
+
+template <int KPT, typename T>
+int launch_scan(const GroupScanParams& p, int entries, cudaStream_t stream) {
+  constexpr int COLS = GroupScanShape<KPT, 6>::COLS;
+  const long long blocks = (long long)entries * p.heads * ((p.V + COLS - 1) / COLS);
+  return blocks > 2 * jv_multiprocessors() ? launch_ring<KPT, 2, T>(p, entries, stream) : launch_ring<KPT, 6, T>(p, entries, stream);
 }
 
 int padded(int D) { return D <= 32 ? 32 : D <= 64 ? 64 : D <= 128 ? 128 : 256; }
@@ -444,22 +461,25 @@ JV_EXPORT int jv_delta_group_floats(int D) { return VECS * padded(D) + COEF; }
 // Both kernels.  proj: [n] rows of `stride` elements of dtype `dtype` holding r, k, the removal gate's pre-activation
 // (heads * D each) and the values (heads * V) at the given columns; zw, a_bias, w_bias as for jv_delta_prepare; packed: at least
 // (n / 4 + entries) * heads * jv_delta_group_floats(D) floats, 16-byte aligned; state [n_slots] rows of `slot_stride` floats;
-// out [n, heads * V].
+// out [n, heads * V].  portions > 0: entries of one token are passed by, which leaves this many, with n tokens.
 JV_EXPORT int jv_delta_scan(const void* proj, int dtype, long long stride, int r_off, int k_off, int a_off, int v_off,
                             const void* zw, long long zw_stride, const void* a_bias, const void* w_bias, int w_dtype,
                             float* packed, float* state, long long slot_stride, const int* cu_seqlens, const int* slots,
-                            int n_slots, int entries, float* out, int n, int heads, int D, int V, int* status, cudaStream_t stream) {
+                            int n_slots, int entries, float* out, int n, int heads, int D, int V, int portions, int* status,
+                            cudaStream_t stream) {
   if (entries == 0 || n == 0) return JV_OK;
   if (D < 1 || D > 256 || V < 1 || heads > 65535) return JV_ERR_UNSUPPORTED;
   const int DP = padded(D);
-  const dim3 grid(n / T4 + entries, heads);
+  const dim3 grid(n / T4 + (portions > 0 ? portions : entries), heads);
   int rc = JV_ERR_UNSUPPORTED;
   JV_DISPATCH_DTYPE(dtype, T, JV_DISPATCH_DTYPE(w_dtype, W, rc = jv_launch(
       DP == 256 ? group_prepare_kernel<2, T, W> : group_prepare_kernel<1, T, W>, grid, dim3(DP == 256 ? 128 : DP), 0, stream,
       (const T*)proj, stride, r_off, k_off, a_off, (const T*)zw, zw_stride, (const W*)a_bias, (const W*)w_bias, cu_seqlens, entries,
-      packed, heads, D, DP)));
+      portions, packed, heads, D, DP)));
   if (rc != JV_OK) return rc;
-  GroupScanParams p{packed, proj, stride, v_off, out, state, slot_stride, cu_seqlens, slots, n_slots, heads, D, V, status};
+  GroupScanParams p{packed, proj, stride, v_off, out, state, slot_stride, cu_seqlens, slots, n_slots, heads, D, V, portions, entries,
+                    (int)grid.x, status};
+  if (portions > 0) entries = portions;
   JV_DISPATCH_DTYPE(dtype, T, {
     switch (DP) {
       case 32: return launch_scan<4, T>(p, entries, stream);

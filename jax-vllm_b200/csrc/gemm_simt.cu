@@ -321,14 +321,6 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) rows_kernel(const GemmParams 
   }
 }
 
-int multiprocessors() {
-  static int count[JV_MAX_DEVICES] = {};
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= JV_MAX_DEVICES) return 148;
-  if (count[dev] == 0 && cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
-  return count[dev];
-}
-
 template <int MR, typename TA, typename TW, typename TC>
 int launch_rows(const GemmParams& p, int batch, cudaStream_t stream) {
   auto kern = rows_kernel<MR, TA, TW, TC>;
@@ -362,7 +354,7 @@ int dispatch(const GemmParams& p, int batch, cudaStream_t stream) {
   if (p.M <= 8) return launch_rows<8, TA, TW, TC>(p, batch, stream);
   if (p.M <= 16) return launch_rows<16, TA, TW, TC>(p, batch, stream);
   const long long tiles = (long long)((p.N + BN - 1) / BN) * ((p.M + BM - 1) / BM) * batch;
-  const int sms = multiprocessors(), n_seg = (p.K + SEG - 1) / SEG;
+  const int sms = jv_multiprocessors(), n_seg = (p.K + SEG - 1) / SEG;
   if (n_seg >= 4 && tiles <= sms) return launch_tiles<4, TA, TW, TC>(p, batch, stream);
   if (n_seg >= 2 && tiles <= 3 * sms) return launch_tiles<2, TA, TW, TC>(p, batch, stream);
   return launch_tiles<1, TA, TW, TC>(p, batch, stream);

@@ -11,7 +11,7 @@
 //   convolved rows xbc = [x | B | C] and the raw step sizes; softplus, both exponentials and the product with B in 32-bit.
 // jv_mamba_finish, one block per (token, norm group): y = (o + D_h x) * silu(z), divided by the root mean square of its
 //   norm group (inner / norm_groups elements), times the norm weight; 32-bit, written in the compute type.
-#include "common.cuh"
+#include "scan.cuh"
 #include <math.h>
 
 namespace {
@@ -22,13 +22,15 @@ __global__ void __launch_bounds__(32 * WARPS) mamba_prepare_kernel(const T* __re
                                                                   int c_off, const T* __restrict__ dt_raw,
                                                                   long long dt_stride, const TW* __restrict__ dt_bias,
                                                                   const TW* __restrict__ a_log, float* __restrict__ packed,
-                                                                  int n, int heads, int groups, int state) {
+                                                                  int n, int heads, int groups, int state,
+                                                                  const int* __restrict__ work,
+                                                                  const int* __restrict__ cu_seqlens) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long item = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5);
   if (item >= (long long)n * heads) return;
-  const int t = (int)(item / heads), h = (int)(item - (long long)t * heads);
+  const int row = (int)(item / heads), h = (int)(item - (long long)row * heads), t = token_of(row, work, cu_seqlens);
   const int g = h / (heads / groups);
   const float z = to_f32(dt_raw[(size_t)t * dt_stride + h]) + to_f32(dt_bias[h]);
   const float dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));             // softplus, no clamp
@@ -157,10 +159,12 @@ __global__ void __launch_bounds__(1024) mamba_finish_vec_kernel(const float* __r
 }  // namespace
 
 // xbc: rows of `dtype`, B at b_off and C at c_off ([groups][state] each); dt_raw: rows of `dtype`, [heads] used;
-// dt_bias, a_log: [heads] of w_dtype; packed: float [n, heads, 3, state].
+// dt_bias, a_log: [heads] of w_dtype; packed: float [n, heads, 3, state].  work, cu_seqlens: n entries of one token whose tokens
+// alone are prepared, or null (all of the n rows).
 JV_EXPORT int jv_mamba_prepare(const void* xbc, int dtype, long long xbc_stride, int b_off, int c_off, const void* dt_raw,
                                long long dt_stride, const void* dt_bias, const void* a_log, int w_dtype, float* packed,
-                               int n, int heads, int groups, int state, cudaStream_t stream) {
+                               int n, int heads, int groups, int state, const int* work, const int* cu_seqlens,
+                               cudaStream_t stream) {
   if (n == 0) return JV_OK;
   if (heads < 1 || groups < 1 || heads % groups || state < 1) return JV_ERR_UNSUPPORTED;
   const long long items = (long long)n * heads;
@@ -168,7 +172,7 @@ JV_EXPORT int jv_mamba_prepare(const void* xbc, int dtype, long long xbc_stride,
   JV_DISPATCH_DTYPE(dtype, T, JV_DISPATCH_DTYPE(w_dtype, TW,
       return jv_launch(mamba_prepare_kernel<T, TW>, grid, dim3(32 * WARPS), 0, stream, (const T*)xbc, xbc_stride, b_off,
                        c_off, (const T*)dt_raw, dt_stride, (const TW*)dt_bias, (const TW*)a_log, packed, n, heads, groups,
-                       state)));
+                       state, work, cu_seqlens)));
   return JV_ERR_UNSUPPORTED;
 }
 
@@ -180,12 +184,11 @@ JV_EXPORT int jv_mamba_finish(const float* o, const void* x, long long x_stride,
   if (n == 0) return JV_OK;
   const int inner = heads * value_dim;
   if (heads < 1 || value_dim < 1 || norm_groups < 1 || inner % norm_groups) return JV_ERR_UNSUPPORTED;
-  // Eight elements a thread where vectors fit (heads and groups in steps of 8, rows on 16-byte boundaries) and there are tokens
-  // enough to fill the device with so few threads: 4,096 tokens of 8 groups of 1,024 in 62 us against 222, 200 of 4,096 in 4.2
-  // against 6.8.
+  // Eight elements a thread where vectors fit (heads and groups in steps of 8, rows on 16-byte boundaries), whatever the number of
+  // tokens: 4,096 tokens of 8 groups of 1,024 in 62 us against 222, 200 of 4,096 in 4.2 against 6.8, one of 4,096 in 2.8 against 4.0.
   const int group_size = inner / norm_groups, size = dtype == 0 ? 4 : 2;
   auto eights = [&](const void* q, long long stride, int bytes) { return ((uintptr_t)q & 15) == 0 && stride * bytes % 16 == 0; };
-  if (n >= 64 && value_dim % 8 == 0 && group_size % 8 == 0 && group_size <= 8192 && eights(o, inner, 4) && eights(x, x_stride, size) &&
+  if (value_dim % 8 == 0 && group_size % 8 == 0 && group_size <= 8192 && eights(o, inner, 4) && eights(x, x_stride, size) &&
       eights(z, z_stride, size) && eights(out, out_stride, size)) {
     const int threads = (group_size / 8 + 31) / 32 * 32;
     JV_DISPATCH_DTYPE(dtype, T, JV_DISPATCH_DTYPE(w_dtype, TW,

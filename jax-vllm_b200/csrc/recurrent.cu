@@ -40,17 +40,19 @@
 namespace {
 
 // ---------------------------------------------------------------------------------------------------- prepare
-// packed: [n, heads, NV, D] float, vectors in the order r, k, w, u, b.
+// packed: [n, heads, NV, D] float, vectors in the order r, k, w, u, b.  With `work`, a list of pairs (entry, -) of entries of one
+// token, only these tokens are prepared, a row of `packed` for each in the list's order.
 template <typename T, typename W>
 __global__ void __launch_bounds__(128) delta_prepare_kernel(const T* __restrict__ proj, long long stride, int r_off,
                                                             int k_off, int a_off, const T* __restrict__ zw,
                                                             long long zw_stride, const W* __restrict__ a_bias,
                                                             const W* __restrict__ w_bias, float* __restrict__ packed,
-                                                            int heads, int D) {
+                                                            int heads, int D, const int* __restrict__ work,
+                                                            const int* __restrict__ cu_seqlens) {
   __shared__ float scratch[33];
   pdl_trigger();
   pdl_wait();
-  const int n = blockIdx.x, h = blockIdx.y;
+  const int n = token_of(blockIdx.x, work, cu_seqlens), h = blockIdx.y;
   const T* row = proj + (size_t)n * stride;
   float ss = 0.f;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const T* __restrict_
   ss = block_sum(ss, scratch);
   const float inv = 1.f / sqrtf(ss + 1e-6f);
   const float c = 0.60653065971263342f;      // e^(-1/2)
-  float* out = packed + ((size_t)n * heads + h) * 5 * D;
+  float* out = packed + ((size_t)blockIdx.x * heads + h) * 5 * D;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     const int e = h * D + d;
     const float k = to_f32(row[k_off + e]);
@@ -179,13 +181,14 @@ __global__ void __launch_bounds__(32) gate_scan_kernel(const T* __restrict__ pro
 template <typename T>
 __global__ void __launch_bounds__(128) memory_prepare_kernel(const T* __restrict__ proj, long long stride, int q_off,
                                                              int k_off, float q_scale, const float* __restrict__ gates,
-                                                             float* __restrict__ packed, int heads, int D) {
+                                                             float* __restrict__ packed, int heads, int D,
+                                                             const int* __restrict__ work, const int* __restrict__ cu_seqlens) {
   pdl_trigger();
   pdl_wait();
-  const int n = blockIdx.x, h = blockIdx.y;
+  const int n = token_of(blockIdx.x, work, cu_seqlens), h = blockIdx.y;
   const T* row = proj + (size_t)n * stride;
   const float keep = gates[((size_t)n * heads + h) * 4], take = gates[((size_t)n * heads + h) * 4 + 1];
-  float* out = packed + ((size_t)n * heads + h) * 3 * D;
+  float* out = packed + ((size_t)blockIdx.x * heads + h) * 3 * D;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     out[d] = to_f32(row[q_off + h * D + d]) * q_scale;
     out[D + d] = take * to_f32(row[k_off + h * D + d]);
@@ -216,6 +219,7 @@ struct ScanParams {
   //   mode 2  every segment runs from seg_start (an entry's first: from the state) and writes the outputs; an entry's
   //           last segment writes the state
   int mode, seg_len, n_entries, v_tot;
+  int portions, max_segments;                        // > 0: entries of one token are passed by, so many others taken; buffers there are
   float* seg_local; float* seg_start;
   int* status;
 };
@@ -240,8 +244,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) state_scan_kernel(const ScanPara
   const int kl = lane >> 3;                            // which quarter of the key channels
   const int col = blockIdx.z * SCAN_COLS + warp * 8 + (lane & 7);
   const int D = p.D, V = p.V;
-  int entry = blockIdx.x, seg = 0, n_seg = 1;
-  if (p.mode != 0 && !find_segment(p.cu_seqlens, p.n_entries, p.seg_len, blockIdx.x, entry, seg, n_seg)) return;
+  int entry = entry_of(blockIdx.x, p.mode == 0 ? p.portions : 0, p.cu_seqlens, p.n_entries), seg = 0, n_seg = 1;
+  if (entry < 0) return;
+  if (p.mode != 0 && !find_segment(p.cu_seqlens, p.n_entries, p.seg_len, p.portions, blockIdx.x, entry, seg, n_seg)) return;
   if (p.mode == 1 && seg == n_seg - 1) return;         // nothing follows an entry's last segment
   int t0 = p.cu_seqlens[entry], t1 = p.cu_seqlens[entry + 1];
   if (p.mode != 0) {
@@ -394,8 +399,9 @@ __global__ void __launch_bounds__(SCAN_THREADS, KPT >= 16 ? 3 : 4) column_scan_k
   const int kl = lane % LANES, k0 = kl * KPT;          // this lane's key channels
   const int base = blockIdx.z * COLS, lcol = warp * Shape::WARP_COLS + lane / LANES * 4, col = base + lcol;   // its first column
   const int D = p.D, V = p.V;
-  int entry = blockIdx.x, seg = 0, n_seg = 1;
-  if (p.mode != 0 && !find_segment(p.cu_seqlens, p.n_entries, p.seg_len, blockIdx.x, entry, seg, n_seg)) return;
+  int entry = entry_of(blockIdx.x, p.mode == 0 ? p.portions : 0, p.cu_seqlens, p.n_entries), seg = 0, n_seg = 1;
+  if (entry < 0) return;
+  if (p.mode != 0 && !find_segment(p.cu_seqlens, p.n_entries, p.seg_len, p.portions, blockIdx.x, entry, seg, n_seg)) return;
   if (p.mode == 1 && seg == n_seg - 1) return;         // nothing follows an entry's last segment
   int t0 = p.cu_seqlens[entry], t1 = p.cu_seqlens[entry + 1];
   if (p.mode != 0) {
@@ -582,19 +588,24 @@ __global__ void __launch_bounds__(SCAN_THREADS, KPT >= 16 ? 3 : 4) column_scan_k
 __global__ void __launch_bounds__(128) scan_combine_diag_kernel(const ScanParams p) {
   pdl_trigger();
   pdl_wait();
-  const int entry = blockIdx.x, h = blockIdx.y;
+  const int entry = entry_of(blockIdx.x, p.portions, p.cu_seqlens, p.n_entries), h = blockIdx.y;
+  if (entry < 0) return;
   const int D = p.D, V = p.V;
   const int v_n = V + (p.state_n != nullptr ? 1 : 0);
   const int idx = blockIdx.z * 128 + threadIdx.x;
   if (idx >= D * v_n) return;
   const int kk = idx / v_n, col = idx - kk * v_n;
   const int len = p.cu_seqlens[entry + 1] - p.cu_seqlens[entry];
-  const int n_seg = max(1, (len + p.seg_len - 1) / p.seg_len);
+  const int n_seg = segments_of(len, p.seg_len, p.portions);
   if (n_seg < 2) return;
   const int slot = p.slots[entry];
   if (slot < 0 || slot >= p.n_slots) return;             // the scan reports it
   int g0 = 0;                                            // the number of the entry's first segment
-  for (int e = 0; e < entry; ++e) g0 += max(1, (p.cu_seqlens[e + 1] - p.cu_seqlens[e] + p.seg_len - 1) / p.seg_len);
+  for (int e = 0; e < entry; ++e) g0 += segments_of(p.cu_seqlens[e + 1] - p.cu_seqlens[e], p.seg_len, p.portions);
+  if (g0 + n_seg > p.max_segments) {                     // more portions than were said to be there
+    if (threadIdx.x == 0) atomicOr(p.status, JV_STATUS_BAD_ROW);
+    return;
+  }
   float S = (col == V) ? p.state_n[(size_t)slot * p.slot_stride + (size_t)h * D + kk]
                        : p.state[(size_t)slot * p.slot_stride + (size_t)h * D * V + (size_t)kk * V + col];
   const size_t seg_floats = (size_t)p.heads * D * p.v_tot;
@@ -620,7 +631,8 @@ __global__ void __launch_bounds__(128) scan_combine_kernel(const ScanParams p) {
   extern __shared__ __align__(16) float csm[];           // cols [D][32], local [D][32], T [D][DP], DP = D rounded up to 4, plus 4
   pdl_trigger();
   pdl_wait();
-  const int entry = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+  const int entry = entry_of(blockIdx.x, p.portions, p.cu_seqlens, p.n_entries), h = blockIdx.y, tid = threadIdx.x;
+  if (entry < 0) return;
   const int lane = tid & 31, col = blockIdx.z * 32 + lane, r0 = tid >> 5;
   const int D = p.D, V = p.V;
   const int DP = ((D + 3) & ~3) + 4;
@@ -628,12 +640,16 @@ __global__ void __launch_bounds__(128) scan_combine_kernel(const ScanParams p) {
   float* Ls = csm + (size_t)D * 32;
   float* Ts = csm + (size_t)D * 64;
   const int len = p.cu_seqlens[entry + 1] - p.cu_seqlens[entry];
-  const int n_seg = max(1, (len + p.seg_len - 1) / p.seg_len);
+  const int n_seg = segments_of(len, p.seg_len, p.portions);
   if (n_seg < 2) return;
   const int slot = p.slots[entry];
   if (slot < 0 || slot >= p.n_slots) return;             // the scan reports it
   int g0 = 0;
-  for (int e = 0; e < entry; ++e) g0 += max(1, (p.cu_seqlens[e + 1] - p.cu_seqlens[e] + p.seg_len - 1) / p.seg_len);
+  for (int e = 0; e < entry; ++e) g0 += segments_of(p.cu_seqlens[e + 1] - p.cu_seqlens[e], p.seg_len, p.portions);
+  if (g0 + n_seg > p.max_segments) {
+    if (tid == 0) atomicOr(p.status, JV_STATUS_BAD_ROW);
+    return;
+  }
   const bool live = col < V;
   const float* S_g = p.state + (size_t)slot * p.slot_stride + (size_t)h * D * V + col;
   float S[COMBINE_ROWS];
@@ -722,7 +738,7 @@ int launch_removal_scan(const ScanParams& p, int entries, cudaStream_t stream) {
           return cudaFuncSetAttribute(scan_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess;
         }))
       return (int)JV_ERR_UNSUPPORTED;
-    return jv_launch(scan_combine_kernel, dim3(p.n_entries, p.heads, (p.V + 31) / 32), dim3(128), csmem, stream, q);
+    return jv_launch(scan_combine_kernel, dim3(p.portions > 0 ? p.portions : p.n_entries, p.heads, (p.V + 31) / 32), dim3(128), csmem, stream, q);
   });
 }
 
@@ -738,7 +754,8 @@ int launch_column_scan(const ScanParams& p, int entries, cudaStream_t stream) {
     return JV_ERR_UNSUPPORTED;
   const int cols = p.V + (p.state_n != nullptr ? 1 : 0);
   return launch_scan(kern, smem, Shape::COLS, cols, cols + 1, p, entries, stream, [&](const ScanParams& q) {
-    return jv_launch(scan_combine_diag_kernel, dim3(p.n_entries, p.heads, (p.D * cols + 127) / 128), dim3(128), 0, stream, q);
+    return jv_launch(scan_combine_diag_kernel, dim3(p.portions > 0 ? p.portions : p.n_entries, p.heads, (p.D * cols + 127) / 128),
+                     dim3(128), 0, stream, q);
   });
 }
 
@@ -904,14 +921,16 @@ bool vec_aligned(const void* p, long long stride, int vec, int size) {
 
 // proj: [n] rows of `stride` elements of dtype `dtype` holding r, k and the removal gate's pre-activation at the given
 // columns (heads * D each); zw: [n] rows of the decay's pre-activation; a_bias, w_bias: [heads * D] of dtype `w_dtype`;
-// packed: [n, heads, 5, D] float.
+// packed: [n, heads, 5, D] float.  work, cu_seqlens: n entries of one token whose tokens alone are prepared, or null (all of the
+// n rows).
 JV_EXPORT int jv_delta_prepare(const void* proj, int dtype, long long stride, int r_off, int k_off, int a_off,
                                const void* zw, long long zw_stride, const void* a_bias, const void* w_bias, int w_dtype,
-                               float* packed, int n, int heads, int D, cudaStream_t stream) {
+                               float* packed, int n, int heads, int D, const int* work, const int* cu_seqlens,
+                               cudaStream_t stream) {
   if (n == 0) return JV_OK;
   JV_DISPATCH_DTYPE(dtype, T, JV_DISPATCH_DTYPE(w_dtype, W, return jv_launch(
       delta_prepare_kernel<T, W>, dim3(n, heads), dim3(D > 64 ? 128 : 64), 0, stream, (const T*)proj, stride, r_off, k_off,
-      a_off, (const T*)zw, zw_stride, (const W*)a_bias, (const W*)w_bias, packed, heads, D)));
+      a_off, (const T*)zw, zw_stride, (const W*)a_bias, (const W*)w_bias, packed, heads, D, work, cu_seqlens)));
   return JV_ERR_UNSUPPORTED;
 }
 
@@ -934,20 +953,21 @@ JV_EXPORT int jv_gla_prepare(const void* proj, int dtype, long long stride, int 
 
 // proj as above with q, k (heads * D each) and the two gates' pre-activations (heads each) at the given columns;
 // gates: [n, heads, 4] float (keep, take, running maximum; the fourth place is left for the scan's n . q); packed:
-// [n, heads, 3, D] float (null: the gates alone); state_m: the running maximum of slot 0, rows `slot_stride` floats apart.
+// [n, heads, 3, D] float (null: the gates alone; with `work`, n_work entries of one token, a row for each of these); state_m: the
+// running maximum of slot 0, rows `slot_stride` floats apart.
 JV_EXPORT int jv_memory_gates(const void* proj, int dtype, long long stride, int q_off, int k_off, int i_off, int f_off,
                               const void* i_bias, const void* f_bias, int w_dtype, float cap, float q_scale, float* gates,
                               float* packed, float* state_m, long long slot_stride, const int* cu_seqlens,
-                              const int* slots, int n_slots, int entries, int n, int heads, int D, int* status,
-                              cudaStream_t stream) {
+                              const int* slots, int n_slots, int entries, int n, int heads, int D, const int* work, int n_work,
+                              int* status, cudaStream_t stream) {
   if (entries == 0 || n == 0) return JV_OK;
   JV_DISPATCH_DTYPE(dtype, T, JV_DISPATCH_DTYPE(w_dtype, W, {
     const int rc = jv_launch(gate_scan_kernel<T, W>, dim3(entries, heads), dim3(32), 0, stream, (const T*)proj, stride,
                              i_off, f_off, (const W*)i_bias, (const W*)f_bias, cap, gates, state_m, slot_stride,
                              cu_seqlens, slots, n_slots, heads, status);
-    if (rc != JV_OK || packed == nullptr) return rc;
-    return jv_launch(memory_prepare_kernel<T>, dim3(n, heads), dim3(D > 64 ? 128 : 64), 0, stream, (const T*)proj, stride,
-                     q_off, k_off, q_scale, (const float*)gates, packed, heads, D);
+    if (rc != JV_OK || packed == nullptr || (work != nullptr && n_work == 0)) return rc;
+    return jv_launch(memory_prepare_kernel<T>, dim3(work != nullptr ? n_work : n, heads), dim3(D > 64 ? 128 : 64), 0, stream,
+                     (const T*)proj, stride, q_off, k_off, q_scale, (const float*)gates, packed, heads, D, work, cu_seqlens);
   }));
   return JV_ERR_UNSUPPORTED;
 }
@@ -956,21 +976,26 @@ JV_EXPORT int jv_memory_gates(const void* proj, int dtype, long long stride, int
 // state_n (or null; without removal only): [slots][heads * D], rows `slot_stride` apart, the state of one more column
 // whose value is 1 at every token; its outputs go to nq[(token * heads + head) * nq_stride].
 // seg_len > 0: entries longer than seg_len tokens run in segments of that many, side by side (see ScanParams): three
-// launches; seg_local and seg_start hold max_segments * heads * D * v_tot floats each (16-byte aligned), v_tot = V + D with
-// removal, else V + (state_n ? 1 : 0) + 1 rounded up to a multiple of 4, and max_segments is at least the number of segments of all entries together.
+// launches; portions > 0: entries of one token are passed by, which leaves this many; seg_local and seg_start hold max_segments *
+// heads * D * v_tot floats each (16-byte aligned), v_tot = V + D with
+// removal, else V + (state_n ? 1 : 0) + 1 rounded up to a multiple of 4, and max_segments is at least
+// the number of segments of all entries that are taken.
 JV_EXPORT int jv_state_scan(const float* packed, int removal, const void* v, int dtype, long long v_stride, int v_off,
                             float* out, float* state, long long slot_stride, const int* cu_seqlens, const int* slots,
                             int n_slots, int entries, int heads, int D, int V, float* state_n, float* nq, int nq_stride,
-                            int seg_len, int max_segments, float* seg_local, float* seg_start, int* status,
+                            int seg_len, int max_segments, float* seg_local, float* seg_start, int portions, int* status,
                             cudaStream_t stream) {
   if (entries == 0) return JV_OK;
   if (state_n != nullptr && (removal || nq == nullptr)) return JV_ERR_UNSUPPORTED;
-  if (seg_len > 0 && (seg_local == nullptr || seg_start == nullptr || max_segments < entries || D > 4 * COMBINE_ROWS))
+  if (seg_len > 0 && (seg_local == nullptr || seg_start == nullptr || max_segments < (portions > 0 ? portions : entries) ||
+                      D > 4 * COMBINE_ROWS))
     return JV_ERR_UNSUPPORTED;
   ScanParams p;
   p.mode = seg_len > 0 ? 1 : 0; p.seg_len = seg_len; p.n_entries = entries; p.seg_local = seg_local; p.seg_start = seg_start;
+  p.portions = portions; p.max_segments = max_segments;
   p.v_tot = removal ? V + D : (V + (state_n != nullptr ? 1 : 0) + 1 + 3) / 4 * 4;
   if (seg_len > 0) entries = max_segments;
+  else if (portions > 0) entries = portions;
   p.state_n = state_n; p.nq = nq; p.nq_stride = nq_stride;
   p.packed = packed; p.v = v; p.v_stride = v_stride; p.v_off = v_off; p.out = out; p.state = state;
   p.slot_stride = slot_stride; p.cu_seqlens = cu_seqlens; p.slots = slots; p.n_slots = n_slots; p.heads = heads;

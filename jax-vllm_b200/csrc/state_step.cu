@@ -5,7 +5,8 @@
 // It reads and writes every state once, which is all it costs, so a block is laid out for that and nothing else: 256 threads
 // hold the whole key range of COLS columns of one (entry, head), eight rows of VEC neighbouring columns a thread, all eight loads
 // under way at once; rows of a block are 128 to 512 bytes of memory in one piece.  The sums over the key channels go through
-// shared memory.  An entry of several tokens is gone through in a loop with the state in registers.
+// shared memory.  An entry of several tokens is gone through in a loop with the state in registers.  Beside portions of prompts the
+// entries of one token come in a list (`work`), and the rows of `packed` may be theirs alone.
 //
 // 48 requests of 8 heads of 128 x 256 (50 MB of states, read and written): 17.9 us (5.6 TB/s), 38.8 us on the scan for whole entries
 // (which stages vectors and values for many tokens and keeps 16 channels x 4 columns a thread).
@@ -22,6 +23,7 @@ struct StepParams {
   float* state_n; float* nq; int nq_stride;  // the normaliser's column (value 1) and where its outputs go, or null
   const int* cu_seqlens; const int* slots;
   int n_slots, heads, D, V;
+  const int* work; int compact;            // pairs (entry, -), or null: every entry; a row of packed for every pair, not every token
   int* status;
 };
 
@@ -34,7 +36,8 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p)
   __shared__ float scratch[33];
   pdl_trigger();
   pdl_wait();
-  const int entry = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, rg = tid / CQ, cq = tid % CQ;
+  const int entry = p.work != nullptr ? p.work[2 * blockIdx.x] : blockIdx.x;
+  const int h = blockIdx.y, tid = threadIdx.x, rg = tid / CQ, cq = tid % CQ;
   const int base = blockIdx.z * COLS, col = base + cq * VEC, D = p.D, V = p.V;
   const int t0 = p.cu_seqlens[entry], t1 = p.cu_seqlens[entry + 1];
   const int slot = p.slots[entry];
@@ -64,7 +67,7 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p)
   float* n_g = norm && tid < D ? p.state_n + (size_t)slot * p.slot_stride + (size_t)h * D + tid : nullptr;
   float n_state = n_g != nullptr ? *n_g : 0.f;
   for (int t = t0; t < t1; ++t) {
-    const float* src = p.packed + ((size_t)t * p.heads + h) * NV * D;
+    const float* src = p.packed + ((size_t)(p.compact ? blockIdx.x : t) * p.heads + h) * NV * D;
     float vv[VEC];
     const T* vsrc = (const T*)p.v + (size_t)t * p.v_stride + p.v_off + (size_t)h * V + (live ? col : 0);
 #pragma unroll
@@ -154,14 +157,16 @@ int dispatch(const StepParams& p, bool removal, bool vec, int entries, cudaStrea
 }
 }  // namespace
 
-// Arguments as for jv_state_scan, without segments.
+// Arguments as for jv_state_scan, without segments.  work: `entries` pairs (entry, -), or null (all entries); compact (with work,
+// entries of one token): packed has a row for every pair, in their order.
 JV_EXPORT int jv_state_step(const float* packed, int removal, const void* v, int v_dtype, long long v_stride, int v_off, float* out,
                             float* state, long long slot_stride, const int* cu_seqlens, const int* slots, int n_slots, int entries,
-                            int heads, int D, int V, float* state_n, float* nq, int nq_stride, int* status, cudaStream_t stream) {
+                            int heads, int D, int V, float* state_n, float* nq, int nq_stride, const int* work, int compact,
+                            int* status, cudaStream_t stream) {
   if (entries == 0) return JV_OK;
-  if (heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || (removal && state_n != nullptr)) return JV_ERR_UNSUPPORTED;
+  if ((compact && work == nullptr) || heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || (removal && state_n != nullptr)) return JV_ERR_UNSUPPORTED;
   StepParams p{packed, v, v_stride, v_off, out, state, slot_stride, state_n, nq, nq_stride, cu_seqlens, slots, n_slots, heads, D, V,
-               status};
+               work, compact, status};
   const bool vec = V % 4 == 0 && ((uintptr_t)state & 15) == 0 && slot_stride % 4 == 0;
   JV_DISPATCH_DTYPE(v_dtype, T, {
     if (D <= 64) return dispatch<8, T>(p, removal != 0, vec, entries, stream);

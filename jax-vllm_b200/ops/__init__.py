@@ -1705,10 +1705,66 @@ def norm_mean2(a: torch.Tensor, b: torch.Tensor, wa: torch.Tensor, wb: torch.Ten
 SCAN_MAX_KEY = 256
 
 
+def _single_entries(singles: tuple | None, n: int):
+    """(pointer to the list, rows, pointer to the offsets) of a `singles` argument (work [k, 2], k, cu_seqlens); all `n` rows
+    without one."""
+    if singles is None:
+        return None, n, None
+    work, k, cu_seqlens = singles
+    _cuda(work, "singles", torch.int32); _cuda(cu_seqlens, "cu_seqlens", torch.int32)
+    if work.shape[0] < k or work.shape[1] != 2 or k > n:
+        raise KernelError("a list of the entries of one token is [k, 2]")
+    return work.data_ptr(), k, cu_seqlens.data_ptr()
+
+
+def _scan_out(out: torch.Tensor | None, n: int, width: int, device) -> torch.Tensor:
+    if out is None:
+        return torch.empty((n, width), dtype=torch.float32, device=device)
+    _cuda(out, "out", torch.float32)
+    if out.shape != (n, width):
+        raise KernelError(f"the scan's output is [{n}, {width}]")
+    return out
+
+
+def state_step(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.Tensor, cu_seqlens: torch.Tensor,
+               slots: torch.Tensor, work: torch.Tensor | None, n_work: int, value_dim: int, out: torch.Tensor,
+               state_n: torch.Tensor | None = None, gates: torch.Tensor | None = None) -> torch.Tensor:
+    """`state_scan` for entries of one token: each state is read and written once (csrc/state_step.cu).  `work` [n_work, 2] lists
+    the entries (None: the first n_work entries, all of them); `packed` has a row for every token or, with `work`, may have one
+    for every listed entry.  Writes the entries' rows of `out` [n, heads * value_dim] (and of `gates`)."""
+    _cuda(packed, "packed", torch.float32); _cuda(v, "v", contiguous=False)
+    _cuda(state, "state", torch.float32, contiguous=False); _cuda(out, "out", torch.float32)
+    _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
+    n, (rows, heads, nv, dim) = v.shape[0], packed.shape
+    if nv not in (3, 5) or rows not in (n, n_work) or (rows != n and work is None) or v.stride(1) != 1 or \
+            v_off + heads * value_dim > v.shape[1] or state.stride(1) != 1 or state.shape[1] < heads * dim * value_dim or \
+            dim > SCAN_MAX_KEY or out.shape != (n, heads * value_dim):
+        raise KernelError("state_step: shapes do not fit")
+    if work is not None:
+        _cuda(work, "work", torch.int32)
+        if work.shape[0] < n_work or work.shape[1] != 2:
+            raise KernelError("state_step: a list of entries is [n_work, 2]")
+    nq = None
+    if state_n is not None:
+        _cuda(state_n, "state_n", torch.float32, contiguous=False); _cuda(gates, "gates", torch.float32)
+        if nv != 3 or state_n.stride(0) != state.stride(0) or state_n.stride(1) != 1 or state_n.shape[1] != heads * dim or \
+                state_n.shape[0] != state.shape[0] or tuple(gates.shape) != (n, heads, 4):
+            raise KernelError("state_step: the normaliser does not fit")
+        nq = gates.data_ptr() + 3 * 4
+    f = _fn("state_step", "jv_state_step", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p, c_longlong,
+                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
+                                            c_void_p, c_int, c_void_p, c_void_p])
+    _check(f(packed.data_ptr(), 1 if nv == 5 else 0, v.data_ptr(), _code(v, "v"), v.stride(0), v_off, out.data_ptr(),
+             state.data_ptr(), state.stride(0), cu_seqlens.data_ptr(), slots.data_ptr(), state.shape[0], n_work, heads, dim,
+             value_dim, _ptr(state_n), nq, 4, _ptr(work), int(rows != n), _status_ptr(packed.device), _stream()), "state_step")
+    return out
+
+
 def delta_prepare(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, zw: torch.Tensor, a_bias: torch.Tensor,
-                  w_bias: torch.Tensor, heads: int, dim: int) -> torch.Tensor:
+                  w_bias: torch.Tensor, heads: int, dim: int, singles: tuple | None = None) -> torch.Tensor:
     """Per token and head the vectors (r, k, w, u, b) of the generalized delta rule as float32 [n, heads, 5, dim]:
-    w = exp(-e^(-1/2) sigmoid(zw + w_bias)), u = k / sqrt(|k|^2 + 1e-6), b = sigmoid(z_a + a_bias) * u."""
+    w = exp(-e^(-1/2) sigmoid(zw + w_bias)), u = k / sqrt(|k|^2 + 1e-6), b = sigmoid(z_a + a_bias) * u.
+    `singles` (work [k, 2], k, cu_seqlens): the tokens of these k entries of one token alone, as [k, heads, 5, dim]."""
     _cuda(proj, "proj", contiguous=False); _cuda(zw, "zw", proj.dtype, contiguous=False)
     _cuda(a_bias, "a_bias"); _cuda(w_bias, "w_bias", a_bias.dtype)
     n = proj.shape[0]
@@ -1716,26 +1772,24 @@ def delta_prepare(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, zw: to
             max(r_off, k_off, a_off) + heads * dim > proj.shape[1] or a_bias.numel() != heads * dim or \
             w_bias.numel() != heads * dim:
         raise KernelError("delta_prepare: shapes do not fit")
+    work, n, cu = _single_entries(singles, n)
     packed = torch.empty((n, heads, 5, dim), dtype=torch.float32, device=proj.device)
     f = _fn("recurrent", "jv_delta_prepare", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_void_p, c_longlong,
-                                              c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p])
+                                              c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
+                                              c_void_p])
     _check(f(proj.data_ptr(), _code(proj, "proj"), proj.stride(0), r_off, k_off, a_off, zw.data_ptr(), zw.stride(0),
-             a_bias.data_ptr(), w_bias.data_ptr(), _code(a_bias, "a_bias"), packed.data_ptr(), n, heads, dim, _stream()),
+             a_bias.data_ptr(), w_bias.data_ptr(), _code(a_bias, "a_bias"), packed.data_ptr(), n, heads, dim, work, cu, _stream()),
            "delta_prepare")
     return packed
 
 
-# Average new tokens of an entry from which `delta_scan` is taken (parts/recurrent.py).  32 heads of 64, preparation and scan: eight entries
-# of 8 tokens 19.8 against 17.3 us on the kernels that go token by token; those grow by 0.4 us a token, `delta_scan` by 0.13.
-DELTA_GROUP_MIN_TOKENS = 16
-
-
 def delta_scan(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, v_off: int, zw: torch.Tensor, a_bias: torch.Tensor,
                w_bias: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, n_entries: int,
-               heads: int, dim: int, columns: int) -> torch.Tensor:
+               heads: int, dim: int, columns: int, out: torch.Tensor | None = None, portions: int = 0) -> torch.Tensor:
     """`delta_prepare` and `state_scan` in one, four tokens at a time (csrc/delta_scan.cu): the delta rule over the new tokens
     of every entry, whose states (rows of `state`, `heads * dim * columns` floats) are carried on in place.  Returns the
-    outputs [n, heads * columns] float32."""
+    outputs [n, heads * columns] float32 (`out` if given).  `portions` > 0: entries of one token are passed by (`state_step` takes
+    them), their outputs and states stay as they are; the others are this many."""
     _cuda(proj, "proj", contiguous=False); _cuda(zw, "zw", proj.dtype, contiguous=False)
     _cuda(a_bias, "a_bias"); _cuda(w_bias, "w_bias", a_bias.dtype); _cuda(state, "state", torch.float32, contiguous=False)
     _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
@@ -1749,16 +1803,18 @@ def delta_scan(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, v_off: in
         raise KernelError("delta_scan: the state does not fit")
     if cu_seqlens.numel() < n_entries + 1 or slots.numel() < n_entries:
         raise KernelError("delta_scan: an offset and a slot per entry")
-    out = torch.empty((n, heads * columns), dtype=torch.float32, device=proj.device)
+    out = _scan_out(out, n, heads * columns, proj.device)
+    taken = portions or n_entries
+    n -= n_entries - taken                          # one token for every entry that is passed by
     size = _fn("delta_scan", "jv_delta_group_floats", [c_int])(dim)
-    packed = torch.empty((n // 4 + n_entries) * heads * size, dtype=torch.float32, device=proj.device)
+    packed = torch.empty((n // 4 + taken) * heads * size, dtype=torch.float32, device=proj.device)
     f = _fn("delta_scan", "jv_delta_scan", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p,
                                             c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int,
-                                            c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+                                            c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(f(proj.data_ptr(), _code(proj, "proj"), proj.stride(0), r_off, k_off, a_off, v_off, zw.data_ptr(), zw.stride(0),
              a_bias.data_ptr(), w_bias.data_ptr(), _code(a_bias, "a_bias"), packed.data_ptr(), state.data_ptr(), state.stride(0),
              cu_seqlens.data_ptr(), slots.data_ptr(), state.shape[0], n_entries, out.data_ptr(), n, heads, dim, columns,
-             _status_ptr(proj.device), _stream()), "delta_scan", launches=2)
+             portions, _status_ptr(proj.device), _stream()), "delta_scan", launches=2)
     return out
 
 
@@ -1782,12 +1838,14 @@ def gla_prepare(proj: torch.Tensor, q_off: int, k_off: int, low_off: int, w_up: 
 
 def memory_gates(proj: torch.Tensor, q_off: int, k_off: int, i_off: int, f_off: int, i_bias: torch.Tensor,
                  f_bias: torch.Tensor, cap: float, q_scale: float, state_m: torch.Tensor, cu_seqlens: torch.Tensor,
-                 slots: torch.Tensor, n_entries: int, heads: int, dim: int, gates_only: bool = False):
+                 slots: torch.Tensor, n_entries: int, heads: int, dim: int, gates_only: bool = False,
+                 singles: tuple | None = None):
     """The gates of a matrix memory with exponential gating: the running maximum `state_m` [slots, heads] (a view of
     the state rows) is scanned over every entry's tokens, then all tokens at once are prepared.  Returns (packed
     float32 [n, heads, 3, dim]: the scaled query, the key times its input gate, the decay; gates float32 [n, heads,
     4]: decay, input gate, running maximum, and a place that the scan fills with n . q).  With `gates_only` (for `chunk_scan`) the
-    packed vectors are not made and None stands in their place."""
+    packed vectors are not made and None stands in their place.  `singles` (work [k, 2], k, cu_seqlens): the vectors of these
+    k entries of one token alone, as [k, heads, 3, dim]; the gates are those of all tokens."""
     _cuda(proj, "proj", contiguous=False); _cuda(i_bias, "i_bias"); _cuda(f_bias, "f_bias", i_bias.dtype)
     _cuda(state_m, "state_m", torch.float32, contiguous=False)
     _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
@@ -1795,15 +1853,16 @@ def memory_gates(proj: torch.Tensor, q_off: int, k_off: int, i_off: int, f_off: 
     if proj.stride(1) != 1 or state_m.stride(1) != 1 or state_m.shape[1] != heads or dim > SCAN_MAX_KEY or \
             max(q_off, k_off) + heads * dim > proj.shape[1] or max(i_off, f_off) + heads > proj.shape[1]:
         raise KernelError("memory_gates: shapes do not fit")
-    packed = None if gates_only else torch.empty((n, heads, 3, dim), dtype=torch.float32, device=proj.device)
+    work, rows, _ = _single_entries(singles, n)
+    packed = None if gates_only else torch.empty((rows, heads, 3, dim), dtype=torch.float32, device=proj.device)
     gates = torch.empty((n, heads, 4), dtype=torch.float32, device=proj.device)
     f = _fn("recurrent", "jv_memory_gates", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                              c_int, c_float, c_float, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
-                                             c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+                                             c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p])
     _check(f(proj.data_ptr(), _code(proj, "proj"), proj.stride(0), q_off, k_off, i_off, f_off, i_bias.data_ptr(),
              f_bias.data_ptr(), _code(i_bias, "i_bias"), float(cap), float(q_scale), gates.data_ptr(), _ptr(packed),
              state_m.data_ptr(), state_m.stride(0), cu_seqlens.data_ptr(), slots.data_ptr(), state_m.shape[0], n_entries,
-             n, heads, dim, _status_ptr(proj.device), _stream()), "memory_gates", launches=1 if gates_only else 2)
+             n, heads, dim, work, rows, _status_ptr(proj.device), _stream()), "memory_gates", launches=1 if gates_only else 2)
     return packed, gates
 
 
@@ -1829,7 +1888,7 @@ def scan_segment(n: int, n_entries: int, heads: int, dim: int, columns: int) -> 
 
 def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.Tensor, cu_seqlens: torch.Tensor,
                slots: torch.Tensor, n_entries: int, value_dim: int, state_n: torch.Tensor | None = None,
-               gates: torch.Tensor | None = None, segment: int | None = None) -> torch.Tensor:
+               gates: torch.Tensor | None = None, segment: int | None = None, singles: tuple | None = None) -> torch.Tensor:
     """S <- diag(w) S - b (u^T S) + k v^T and o = S^T r, token after token of every entry, for the per-head states
     `state` [slots, >= heads * dim * value_dim] float32 (a view of the state rows); `packed` [n, heads, 5 or 3, dim]
     holds (r, k, w, u, b) or, without the removal term, (r, k, w); the values are columns `v_off`.. of the rows of
@@ -1841,7 +1900,10 @@ def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
     the removal term, never with it; 0: never): every segment first runs from
     a zero state and records what it does to a state that comes in, the segments of an entry are chained, and every
     segment runs again from its true start for the outputs.  The result differs from the token-by-token order by
-    32-bit rounding only."""
+    32-bit rounding only.
+
+    `singles` (work [k, 2], k): the step's list of entries of one token.  They run on `state_step` whatever stands beside them, and
+    the rest as a step of their own would (segments and all), so neither hangs on the other."""
     _cuda(packed, "packed", torch.float32); _cuda(v, "v", contiguous=False)
     _cuda(state, "state", torch.float32, contiguous=False)
     _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
@@ -1857,32 +1919,32 @@ def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
             raise KernelError("state_scan: the normaliser does not fit")
         nq = gates.data_ptr() + 3 * 4
     out = torch.empty((n, heads * value_dim), dtype=torch.float32, device=packed.device)
-    if segment is None and n == n_entries:         # single tokens: the state is read and written once (csrc/state_step.cu)
-        f = _fn("state_step", "jv_state_step", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p, c_longlong,
-                                                c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
-                                                c_void_p, c_void_p])
-        _check(f(packed.data_ptr(), 1 if nv == 5 else 0, v.data_ptr(), _code(v, "v"), v.stride(0), v_off, out.data_ptr(),
-                 state.data_ptr(), state.stride(0), cu_seqlens.data_ptr(), slots.data_ptr(), state.shape[0], n_entries, heads, dim,
-                 value_dim, _ptr(state_n), nq, 4, _status_ptr(packed.device), _stream()), "state_step")
-        return out
+    if segment is None and n == n_entries:
+        return state_step(packed, v, v_off, state, cu_seqlens, slots, None, n_entries, value_dim, out, state_n, gates)
+    work, n_single = singles if singles is not None else (None, 0)
+    portions, n_own = 0, n                  # the entries that are scanned: how many if not all, and their tokens
+    if 0 < n_single < n_entries:
+        portions, n_own = n_entries - n_single, n - n_single
+        state_step(packed, v, v_off, state, cu_seqlens, slots, work, n_single, value_dim, out, state_n, gates)
+    own = portions or n_entries
     if segment is None:
         # with the removal term a segment carries `dim` more columns and the chain is a matrix product a segment: at
         # the sizes measured (32 heads of 64, 2,048 tokens) the three launches take longer than the one
-        segment = scan_segment(n, n_entries, heads, dim, value_dim + (state_n is not None)) if nv == 3 else 0
+        segment = scan_segment(n_own, own, heads, dim, value_dim + (state_n is not None)) if nv == 3 else 0
     if nv == 5 and 4 * dim * (64 + (dim + 3) // 4 * 4 + 4) > 200 * 1024:
         segment = 0          # the kernel that chains segments keeps a [dim][dim] transition in shared memory
     max_segments, seg_local, seg_start = 0, None, None
     if segment > 0:
-        max_segments = n // segment + n_entries
+        max_segments = n_own // segment + own
         v_tot = value_dim + dim if nv == 5 else -(-(value_dim + (1 if state_n is not None else 0) + 1) // 4) * 4
         seg_local = torch.empty((2, max_segments, heads, dim, v_tot), dtype=torch.float32, device=packed.device)
         seg_start = seg_local[1]
     f = _fn("recurrent", "jv_state_scan", [c_void_p, c_int, c_void_p, c_int, c_longlong, c_int, c_void_p, c_void_p,
                                            c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                                           c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p])
+                                           c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p])
     _check(f(packed.data_ptr(), 1 if nv == 5 else 0, v.data_ptr(), _code(v, "v"), v.stride(0), v_off, out.data_ptr(),
              state.data_ptr(), state.stride(0), cu_seqlens.data_ptr(), slots.data_ptr(), state.shape[0], n_entries, heads,
-             dim, value_dim, _ptr(state_n), nq, 4, int(segment), max_segments, _ptr(seg_local), _ptr(seg_start),
+             dim, value_dim, _ptr(state_n), nq, 4, int(segment), max_segments, _ptr(seg_local), _ptr(seg_start), portions,
              _status_ptr(packed.device), _stream()), "state_scan", launches=3 if segment > 0 else 1)
     return out
 
@@ -1895,10 +1957,13 @@ CHUNK_SCAN_MIN_TOKENS, CHUNK_SCAN_MIN_BLOCKS = 64, 120
 CHUNK_SCAN_MAX_KEY = 128
 
 
-def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, dim: int, columns: int) -> bool:
-    """Whether `chunk_scan` takes these sizes and is the better choice: 16-bit rows whose heads start on 16-byte boundaries, keys of
-    up to 128 in steps of 8, values in steps of 8, enough tokens an entry and enough blocks."""
-    return (row.dtype == torch.bfloat16 and row.shape[0] >= CHUNK_SCAN_MIN_TOKENS * n_entries and 8 <= dim <= CHUNK_SCAN_MAX_KEY
+def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, dim: int, columns: int,
+                        n_tokens: int | None = None) -> bool:
+    """Whether `chunk_scan` takes these sizes and is the better choice for `n_entries` portions of `n_tokens` tokens (all rows if
+    not given): 16-bit rows whose heads start on 16-byte boundaries, keys of up to 128 in steps of 8, values in steps of 8, enough
+    tokens a portion and enough blocks."""
+    tokens = row.shape[0] if n_tokens is None else n_tokens
+    return (row.dtype == torch.bfloat16 and tokens >= CHUNK_SCAN_MIN_TOKENS * n_entries and 8 <= dim <= CHUNK_SCAN_MAX_KEY
             and n_entries * heads * -(-columns // 32) >= CHUNK_SCAN_MIN_BLOCKS
             and dim % 8 == 0 and columns % 8 == 0 and row.stride(1) == 1 and row.stride(0) % 8 == 0
             and all((row.data_ptr() + 2 * o) % 16 == 0 for o in offsets))
@@ -1907,12 +1972,14 @@ def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, 
 def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor, cu_seqlens: torch.Tensor,
                slots: torch.Tensor, n_entries: int, heads: int, groups: int, dim: int, columns: int, scale: float = 1.0,
                gates: torch.Tensor | None = None, state_n: torch.Tensor | None = None, dt_raw: torch.Tensor | None = None,
-               dt_bias: torch.Tensor | None = None, a_log: torch.Tensor | None = None) -> torch.Tensor:
+               dt_bias: torch.Tensor | None = None, a_log: torch.Tensor | None = None, portions: int = 0) -> torch.Tensor:
     """S <- a S + g k v^T and o = scale * S^T q with one decay a and one step g a head and token, 32 tokens at a time
     (csrc/chunk_scan.cu): the mixers' scan (`mamba_prepare` or the second half of `memory_gates`, then `state_scan`) for portions
     of many tokens.  `row` [n, ..] bfloat16 holds q and k (`groups` of `dim`, shared by heads // groups heads each) and v (`heads` of
     `columns`).  Either `gates` [n, heads, 4] (keep, take, ..) with `state_n` as for `state_scan`, or the raw step sizes `dt_raw`
-    [n, heads] with `dt_bias` and `a_log`.  Returns o [n, heads * columns] float32; states are carried on in place."""
+    [n, heads] with `dt_bias` and `a_log`.  Returns o [n, heads * columns] float32; states are carried on in place.  `portions` > 0:
+    entries of one token are passed by (`state_step` takes them), their outputs stay unwritten and their states as they are; the
+    others are this many."""
     _cuda(row, "row", torch.bfloat16, contiguous=False); _cuda(state, "state", torch.float32, contiguous=False)
     _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
     n, width = row.shape
@@ -1939,12 +2006,12 @@ def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: tor
     out = torch.empty((n, heads * columns), dtype=torch.float32, device=row.device)
     f = _fn("chunk_scan", "jv_chunk_scan", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_float, c_void_p,
                                             c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
-                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     base = row.data_ptr()
     _check(f(base + 2 * q_off, row.stride(0), base + 2 * k_off, row.stride(0), base + 2 * v_off, row.stride(0), heads // groups,
              float(scale), _ptr(gates), _ptr(dt_raw), 0 if dt_raw is None else dt_raw.stride(0), _ptr(dt_bias), _ptr(a_log), w_code,
              out.data_ptr(), state.data_ptr(), state.stride(0), _ptr(state_n), cu_seqlens.data_ptr(), slots.data_ptr(),
-             state.shape[0], n_entries, heads, dim, columns, _status_ptr(row.device), _stream()), "chunk_scan")
+             state.shape[0], n_entries, heads, dim, columns, portions, _status_ptr(row.device), _stream()), "chunk_scan")
     return out
 
 
@@ -2214,21 +2281,24 @@ def poly_norm(z, coef: torch.Tensor, eps: float, out: torch.Tensor | None = None
 
 # ------------------------------------------------ state-space mixer: around the state scan (csrc/mamba2.cu)
 def mamba_prepare(xbc: torch.Tensor, b_off: int, c_off: int, dt_raw: torch.Tensor, dt_bias: torch.Tensor,
-                  a_log: torch.Tensor, heads: int, groups: int, state: int) -> torch.Tensor:
+                  a_log: torch.Tensor, heads: int, groups: int, state: int, singles: tuple | None = None) -> torch.Tensor:
     """Per token and head (C_g, softplus(dt + dt_bias) * B_g, exp(-exp(A_log) * dt)) as float32 [n, heads, 3, state]:
-    query, key and decay of `state_scan`.  B and C are [groups, state] column ranges of the rows `xbc`."""
+    query, key and decay of `state_scan`.  B and C are [groups, state] column ranges of the rows `xbc`.  `singles` (work [k, 2], k,
+    cu_seqlens): the tokens of these k entries of one token alone, as [k, heads, 3, state]."""
     _cuda(xbc, "xbc", contiguous=False); _cuda(dt_raw, "dt", xbc.dtype, contiguous=False)
     _cuda(dt_bias, "dt_bias"); _cuda(a_log, "A_log", dt_bias.dtype)
     n = xbc.shape[0]
     if xbc.stride(1) != 1 or dt_raw.stride(1) != 1 or dt_raw.shape != (n, heads) or heads % groups or \
             max(b_off, c_off) + groups * state > xbc.shape[1] or dt_bias.numel() != heads or a_log.numel() != heads:
         raise KernelError("mamba_prepare: shapes do not fit")
+    work, n, cu = _single_entries(singles, n)
     packed = torch.empty((n, heads, 3, state), dtype=torch.float32, device=xbc.device)
     f = _fn("mamba2", "jv_mamba_prepare", [c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_longlong, c_void_p,
-                                           c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+                                           c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                           c_void_p])
     _check(f(xbc.data_ptr(), _code(xbc, "xbc"), xbc.stride(0), b_off, c_off, dt_raw.data_ptr(), dt_raw.stride(0),
              dt_bias.data_ptr(), a_log.data_ptr(), _code(dt_bias, "dt_bias"), packed.data_ptr(), n, heads, groups, state,
-             _stream()), "mamba_prepare")
+             work, cu, _stream()), "mamba_prepare")
     return packed
 
 

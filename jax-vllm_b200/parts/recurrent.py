@@ -10,7 +10,9 @@
 All then divide each head's o by its root mean square, multiply by a weight and by a gate (sigmoid(W_g x), or silu for
 the linear attention), and project.
 The state is float32 and lives in the request's state slot (`FixedStateNeed`): a portion of a prompt starts from what
-the portion before left, a decoded token is a portion of one.  Everything that enters the recurrence besides the
+the portion before left, a decoded token is a portion of one.  In a step that holds both, the entries of one token (the
+step's `decode_work`) and the portions run on kernels of their own: neither kind's sums hang on the other's being there.
+Everything that enters the recurrence besides the
 projections is formed in 32-bit by the prepare kernels.  The parts offer their products to an arrangement that packs
 them (`in_weight`, `from_projection`, `out_weight`).
 """
@@ -95,12 +97,16 @@ class DeltaRule(_StateMixer):
         hd, dt = self.hd, self.ctx.dtype
         low = ops.unary_act(row[:, 5 * hd:5 * hd + self.rank], "tanh")
         zw = ops.linear(low, self.w_up, dt)
-        if step.n_tokens >= ops.DELTA_GROUP_MIN_TOKENS * step.n_entries:
-            o = ops.delta_scan(row, 0, hd, 4 * hd, 2 * hd, zw, self.a_bias, self.w_bias, cache.state, step.cu_seqlens,
-                               step.state_slots, step.n_entries, self.h, self.d, self.d)
-        else:
-            packed = ops.delta_prepare(row, 0, hd, 4 * hd, zw, self.a_bias, self.w_bias, self.h, self.d)
-            o = ops.state_scan(packed, row, 2 * hd, cache.state, step.cu_seqlens, step.state_slots, step.n_entries, self.d)
+        o = torch.empty((step.n_tokens, hd), dtype=torch.float32, device=row.device)
+        where, (work, singles) = (cache.state, step.cu_seqlens, step.state_slots), step.decode_work
+        mixed = 0 < singles < step.n_entries
+        if singles:                         # decoded tokens
+            packed = ops.delta_prepare(row, 0, hd, 4 * hd, zw, self.a_bias, self.w_bias, self.h, self.d,
+                                       singles=(work, singles, step.cu_seqlens) if mixed else None)
+            ops.state_step(packed, row, 2 * hd, *where, work if mixed else None, singles, self.d, o)
+        if singles < step.n_entries:        # portions
+            ops.delta_scan(row, 0, hd, 4 * hd, 2 * hd, zw, self.a_bias, self.w_bias, *where, step.n_entries, self.h, self.d,
+                           self.d, out=o, portions=step.n_entries - singles if mixed else 0)
         return ops.head_norm_gate(o, self.norm, row[:, 3 * hd:4 * hd], out, self.h, self.d, self.spec.norm_eps)
 
 
@@ -148,15 +154,22 @@ class MatrixMemory(_StateMixer):
         hd, hv, h = self.hd, self.hv, self.h
         state = cache.state
         mats = hd * self.dv
-        chunks = ops.chunk_scan_supports(row, (0, hd, 2 * hd), step.n_entries, h, self.d, self.dv)
+        where, state_n = (state, step.cu_seqlens, step.state_slots), state[:, mats:mats + hd]
+        work, singles = step.decode_work
+        chunks = ops.chunk_scan_supports(row, (0, hd, 2 * hd), step.n_entries - singles, h, self.d, self.dv,
+                                         n_tokens=step.n_tokens - singles)
         packed, gates = ops.memory_gates(row, 0, hd, 2 * hd + 2 * hv, 2 * hd + 2 * hv + h, self.i_bias, self.f_bias,
                                          self.spec.gate_cap, self.d ** -0.5, state[:, mats + hd:], step.cu_seqlens,
-                                         step.state_slots, step.n_entries, h, self.d, gates_only=chunks)
-        where, state_n = (state, step.cu_seqlens, step.state_slots, step.n_entries), state[:, mats:mats + hd]
+                                         step.state_slots, step.n_entries, h, self.d, gates_only=chunks and not singles,
+                                         singles=(work, singles, step.cu_seqlens) if chunks and singles else None)
         if chunks:
-            o = ops.chunk_scan(row, 0, hd, 2 * hd, *where, h, h, self.d, self.dv, scale=self.d ** -0.5, gates=gates, state_n=state_n)
+            o = ops.chunk_scan(row, 0, hd, 2 * hd, *where, step.n_entries, h, h, self.d, self.dv, scale=self.d ** -0.5, gates=gates,
+                               state_n=state_n, portions=step.n_entries - singles if singles else 0)
+            if singles:
+                ops.state_step(packed, row, 2 * hd, *where, work, singles, self.dv, o, state_n=state_n, gates=gates)
         else:
-            o = ops.state_scan(packed, row, 2 * hd, *where, self.dv, state_n=state_n, gates=gates)
+            o = ops.state_scan(packed, row, 2 * hd, *where, step.n_entries, self.dv, state_n=state_n, gates=gates,
+                               singles=step.decode_work)
         return ops.head_norm_gate(o, self.norm, row[:, 2 * hd + hv:2 * hd + 2 * hv], out, h, self.dv, self.spec.norm_eps,
                                   gates=gates)
 
@@ -207,7 +220,8 @@ class GatedLinearAttention(_StateMixer):
         hd, hv = self.hd, self.hv
         packed = ops.gla_prepare(row, 0, hd, 2 * hd + 2 * hv, self.w_up, self.bias, self.spec.tau, self.spec.q_scale, self.h,
                                  self.d)
-        o = ops.state_scan(packed, row, 2 * hd, cache.state, step.cu_seqlens, step.state_slots, step.n_entries, self.dv)
+        o = ops.state_scan(packed, row, 2 * hd, cache.state, step.cu_seqlens, step.state_slots, step.n_entries, self.dv,
+                           singles=step.decode_work)
         return ops.head_norm_gate(o, self.norm, row[:, 2 * hd + hv:2 * hd + 2 * hv], out, self.h, self.dv, self.spec.norm_eps,
                                   gate_act="silu")
 

@@ -92,13 +92,17 @@ class StateSpace(Part):
         xbc = ops.short_conv(row[:, inner:inner + self.conv_channels], self.conv_w, conv_state, step.cu_seqlens,
                              step.state_slots, step.n_entries, dt, bias=self.conv_b, act="silu")
         dt_raw = row[:, 2 * inner + 2 * gn:2 * inner + 2 * gn + self.h]
-        where = (state, step.cu_seqlens, step.state_slots, step.n_entries)
-        if ops.chunk_scan_supports(xbc, (0, inner, inner + gn), step.n_entries, self.h, self.n, self.e):
-            o = ops.chunk_scan(xbc, inner + gn, inner, 0, *where, self.h, self.g, self.n, self.e, dt_raw=dt_raw,
-                               dt_bias=self.dt_bias, a_log=self.a_log)
+        where, (work, singles) = (state, step.cu_seqlens, step.state_slots), step.decode_work
+        prepare = (xbc, inner, inner + gn, dt_raw, self.dt_bias, self.a_log, self.h, self.g, self.n)
+        if ops.chunk_scan_supports(xbc, (0, inner, inner + gn), step.n_entries - singles, self.h, self.n, self.e,
+                                   n_tokens=step.n_tokens - singles):
+            o = ops.chunk_scan(xbc, inner + gn, inner, 0, *where, step.n_entries, self.h, self.g, self.n, self.e, dt_raw=dt_raw,
+                               dt_bias=self.dt_bias, a_log=self.a_log, portions=step.n_entries - singles if singles else 0)
+            if singles:                     # decoded tokens beside the portions
+                packed = ops.mamba_prepare(*prepare, singles=(work, singles, step.cu_seqlens))
+                ops.state_step(packed, xbc, 0, *where, work, singles, self.e, o)
         else:
-            packed = ops.mamba_prepare(xbc, inner, inner + gn, dt_raw, self.dt_bias, self.a_log, self.h, self.g, self.n)
-            o = ops.state_scan(packed, xbc, 0, *where, self.e)
+            o = ops.state_scan(ops.mamba_prepare(*prepare), xbc, 0, *where, step.n_entries, self.e, singles=step.decode_work)
         return ops.mamba_finish(o, xbc[:, :inner], row[:, :inner], self.skip, self.norm, out, self.h, self.e, self.ng,
                                 self.spec.norm_eps)
 
