@@ -1949,22 +1949,35 @@ def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
     return out
 
 
-# `chunk_scan` goes through an entry's tokens in order, so it is taken where entries are long and where two-warp blocks, one per
-# entry, head and 32 value columns, give the device 120 or more: fewer leave multiprocessors idle for all of the launch, and the
-# scan in segments is faster (2,048 tokens of 8 heads of 128 x 256: 352 against 333 us with the preparation; of 64 heads of 128 x 64, 128
-# blocks: 329 against 510).
-CHUNK_SCAN_MIN_TOKENS, CHUNK_SCAN_MIN_BLOCKS = 64, 120
+# `chunk_scan` goes through a portion's tokens in order, so it is taken where portions are long and where its two-warp blocks, one
+# per portion, head and 32 value columns, keep the device busy for as long as the longest portion takes: tokens * heads * strips /
+# longest of them are at work on average.  With fewer the scan in segments is faster, the more so the fewer key channels a state has
+# (chunks take the same time for up to 64).  A layer, chunks / segments in us, by keys and blocks at work:
+#   up to 32   2,048 tokens 128 blocks 379 / 330; 300 tokens 86 / 88
+#   64         2,000 and 5 tokens 64 blocks 342 / 252; 1,500 and 600 90 blocks 272 / 234; 2,048 100 blocks 469 / 430; 1,200 and 600
+#              96 blocks 227 / 231; 900, 600 and 200 121 blocks 184 / 213; 400, 680 and 960 136 blocks 195 / 252
+#   128        2,000 and 5 64 blocks 432 / 395; 1,500 and 600 90 blocks 346 / 395; 2,048 92 blocks 463 / 582
+CHUNK_SCAN_MIN_TOKENS = 64
+
+
+def chunk_scan_min_blocks(dim: int) -> int:
+    return 160 if dim <= 32 else 105 if dim <= 64 else 80
+
+
 CHUNK_SCAN_MAX_KEY = 128
 
 
 def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, dim: int, columns: int,
-                        n_tokens: int | None = None) -> bool:
+                        n_tokens: int | None = None, longest: int = 0) -> bool:
     """Whether `chunk_scan` takes these sizes and is the better choice for `n_entries` portions of `n_tokens` tokens (all rows if
-    not given): 16-bit rows whose heads start on 16-byte boundaries, keys of up to 128 in steps of 8, values in steps of 8, enough
-    tokens a portion and enough blocks."""
+    not given), the longest of `longest` (0: all alike): 16-bit rows whose heads start on 16-byte boundaries, keys of up to 128 in
+    steps of 8, values in steps of 8, enough tokens a portion and enough blocks at work."""
+    if n_entries < 1:
+        return False
     tokens = row.shape[0] if n_tokens is None else n_tokens
+    longest = longest or -(-tokens // n_entries)
     return (row.dtype == torch.bfloat16 and tokens >= CHUNK_SCAN_MIN_TOKENS * n_entries and 8 <= dim <= CHUNK_SCAN_MAX_KEY
-            and n_entries * heads * -(-columns // 32) >= CHUNK_SCAN_MIN_BLOCKS
+            and tokens * heads * -(-columns // 32) >= chunk_scan_min_blocks(dim) * longest
             and dim % 8 == 0 and columns % 8 == 0 and row.stride(1) == 1 and row.stride(0) % 8 == 0
             and all((row.data_ptr() + 2 * o) % 16 == 0 for o in offsets))
 

@@ -138,7 +138,7 @@ class StepContext:
     decode_work: tuple            # (work [n, 2], n) for entries of exactly one token
     max_seq_len: int              # longest start_pos + new tokens in the batch (or the engine's bound, in a graph)
     # the same lengths, positions and slots as host lists, for parts that loop over entries on the host; a part
-    # that reads them must say `capturable = False`
+    # that reads them must say `capturable = False` (unless only to choose between kernels that take any lengths)
     host_q_lens: list = field(default_factory=list)
     host_start_pos: list = field(default_factory=list)
     host_slots: list = field(default_factory=list)

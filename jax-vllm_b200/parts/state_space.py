@@ -95,7 +95,7 @@ class StateSpace(Part):
         where, (work, singles) = (state, step.cu_seqlens, step.state_slots), step.decode_work
         prepare = (xbc, inner, inner + gn, dt_raw, self.dt_bias, self.a_log, self.h, self.g, self.n)
         if ops.chunk_scan_supports(xbc, (0, inner, inner + gn), step.n_entries - singles, self.h, self.n, self.e,
-                                   n_tokens=step.n_tokens - singles):
+                                   n_tokens=step.n_tokens - singles, longest=max(step.host_q_lens, default=0)):
             o = ops.chunk_scan(xbc, inner + gn, inner, 0, *where, step.n_entries, self.h, self.g, self.n, self.e, dt_raw=dt_raw,
                                dt_bias=self.dt_bias, a_log=self.a_log, portions=step.n_entries - singles if singles else 0)
             if singles:                     # decoded tokens beside the portions
