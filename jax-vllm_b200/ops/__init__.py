@@ -1534,8 +1534,10 @@ def moe_gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, tile_expert: torch.Tensor
     return out
 
 
-# ---------------------------------------------------------------- per-layer token input
-MOE_STREAM_MAX_TOKENS = 64      # tokens up to which the experts' weights are streamed past them (parts/routed_experts.py)
+# Tokens up to which the experts' weights are streamed past them (parts/routed_experts.py).  A layer of 32 experts, streamed / row
+# tiles of 128, in us: width 2,048 with 16 tokens 117 / 145, 64 145 / 162, 65 152 / 158, 128 158 / 160; width 4,096 with 64
+# 334 / 385, 128 375 / 394: beyond 64 there is less to gain, and the limit could lie higher.
+MOE_STREAM_MAX_TOKENS = 64
 
 
 def moe_linear_stream(a: torch.Tensor, tile: int, w: torch.Tensor, tile_expert: torch.Tensor, used_tiles: torch.Tensor,
@@ -1556,6 +1558,7 @@ def moe_linear_stream(a: torch.Tensor, tile: int, w: torch.Tensor, tile_expert: 
     return out
 
 
+# ---------------------------------------------------------------- per-layer token input
 def token_gate(z: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, offset: int,
                out_dtype: torch.dtype | None = None) -> torch.Tensor:
     """g[t, j] = gelu_tanh(z[t, j]) * table[tokens[t], offset + j] in `out_dtype` (z's by default)
@@ -1954,14 +1957,14 @@ def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
 # longest of them are at work on average.  With fewer the scan in segments is faster, the more so the fewer key channels a state has
 # (chunks take the same time for up to 64).  A layer, chunks / segments in us, by keys and blocks at work:
 #   up to 32   2,048 tokens 128 blocks 379 / 330; 300 tokens 86 / 88
-#   64         2,000 and 5 tokens 64 blocks 342 / 252; 1,500 and 600 90 blocks 272 / 234; 2,048 100 blocks 469 / 430; 1,200 and 600
-#              96 blocks 227 / 231; 900, 600 and 200 121 blocks 184 / 213; 400, 680 and 960 136 blocks 195 / 252
+#   64         2,000 and 5 tokens 64 blocks 342 / 252; 1,500 and 600 90 blocks 272 / 234; 2,048 100 blocks 469 / 430; 48 and 82 102
+#              blocks 49 / 84, 555 and 945 186 / 193, 1,517 and 2,579 461 / 412; 803, 1,365 and 1,928 136 blocks 373 / 414
 #   128        2,000 and 5 64 blocks 432 / 395; 1,500 and 600 90 blocks 346 / 395; 2,048 92 blocks 463 / 582
 CHUNK_SCAN_MIN_TOKENS = 64
 
 
 def chunk_scan_min_blocks(dim: int) -> int:
-    return 160 if dim <= 32 else 105 if dim <= 64 else 80
+    return 160 if dim <= 32 else 101 if dim <= 64 else 80
 
 
 CHUNK_SCAN_MAX_KEY = 128
