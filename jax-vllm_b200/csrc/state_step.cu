@@ -8,7 +8,7 @@
 // shared memory.  An entry of several tokens is gone through in a loop with the state in registers.  Beside portions of prompts the
 // entries of one token come in a list (`work`), and the rows of `packed` may be theirs alone.
 //
-// 48 requests of 8 heads of 128 x 256 (50 MB of states, read and written): 17.9 us (5.6 TB/s), 38.8 us on the scan for whole entries
+// 48 requests of 8 heads of 128 x 256 (50 MB of states, read and written): 16.0 us (6.3 TB/s), 38.8 us on the scan for whole entries
 // (which stages vectors and values for many tokens and keeps 16 channels x 4 columns a thread).
 #include "common.cuh"
 

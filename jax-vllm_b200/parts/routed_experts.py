@@ -147,8 +147,9 @@ class RoutedExperts(Part):
         own = (x, own[0]) if own else (None, None)
         first = None if self.gated else "gelu"
         if self._tensor_cores():
-            # Few tokens: an expert has at most one row a token, so a tile as high as the tokens holds all of its rows; the product is
-            # bound by the weights of the experts that were chosen, and everything around it by the rows, padding included.
+            # Few tokens: an expert has one row a token (a table that names it twice for one gives it a second tile), so a tile as
+            # high as the tokens holds all of its rows; the product is bound by the weights of the experts that were chosen, and
+            # everything around it by the rows, padding included.
             few = x.shape[0] <= ops.MOE_STREAM_MAX_TOKENS
             tile = -(-x.shape[0] // 16) * 16 if few else ops.MOE_TCGEN05_TILE
             _, pos_of, tile_expert, used = ops.moe_align(ids, s.num_experts, tile, s.identity)
