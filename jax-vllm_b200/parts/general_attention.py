@@ -385,9 +385,13 @@ class GeneralAttention(Part):
                                  sink=self.sink, out_scale=self.out_scale)
         elif n_dec:
             # the splits share what a query sees: at most its window with the kept tokens, or its chunk
-            split = self.ctx.decode_split_size
-            most = s.window + self.keep if s.window else s.chunk or step.max_seq_len
-            kernel(dwork, n_dec, split_size=split, n_splits=max(1, -(-min(step.max_seq_len, most) // split)))
+            most = min(step.max_seq_len, s.window + self.keep if s.window else s.chunk or step.max_seq_len)
+            if self.general is not None:
+                kernel(dwork, n_dec, split_size=0,
+                       n_splits=ops.attn_general_mma_splits(n_dec, self.hq, self.hk, self.dk, self.dv, most))
+            else:
+                split = self.ctx.decode_split_size
+                kernel(dwork, n_dec, split_size=split, n_splits=max(1, -(-most // split)))
 
 
 register_mixer("general_attention", GeneralAttention)

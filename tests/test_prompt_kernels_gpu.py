@@ -531,3 +531,28 @@ def test_heads_finished_in_vectors(maps, gate, dv, dtype):
     want, size = want * scale, size * scale
     # rounded to 16 bits; a few 32-bit operations before
     assert bool(((out.view(n, heads, dv).double() - want).abs() <= 2.0 ** -8 * want.abs() + 16 * EPS32 * size).all())
+
+
+# ------------------------------------------------------------------------------- keys of decoded tokens cut evenly
+@pytest.mark.parametrize("hq,hk,splits", [(4, 1, 1), (4, 1, 3), (40, 2, 7), (3, 3, 64)])
+@pytest.mark.parametrize("mask,keep,sigmoid", [(0, 0, False), (100, 5, False), (-128, 0, True)])
+def test_even_splits_of_decoded_tokens(hq, hk, splits, mask, keep, sigmoid):
+    """Fewer keys than splits have places for, one split, lengths on and off the edges of tiles: the same as splits of 64 keys."""
+    ops = _ops()
+    d, page, lengths = 64, 16, [1, 63, 64, 65, 448, 449, 1000]
+    n, widest = len(lengths), 64
+    k, v = (_rand(n * widest, page, hk, d, seed=i, dtype=torch.bfloat16) for i in (1, 2))
+    table = torch.randperm(n * widest, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(n, widest).cuda()
+    cu, start = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (list(range(n + 1)), [m - 1 for m in lengths]))
+    work = torch.tensor([(e, 0) for e in range(n)], dtype=torch.int32, device="cuda")
+    q = _rand(n, hq * d, seed=3, dtype=torch.bfloat16)
+    got = []
+    for size, count in ((0, splits), (64, 16)):
+        out = torch.full((n, hq * d), float("nan"), device="cuda")
+        ops.attn_general_mma(q, q.stride(0), out, k, v, table, cu, start, work, n, hq, hk, 0.2, split_size=size, n_splits=count,
+                             window=mask, keep=keep, sigmoid=sigmoid)
+        ops.check_status()
+        got.append(out.double())
+    # the weights of a split are rounded to 16 bits against its own maximum
+    assert float((got[0] - got[1]).abs().max()) <= 2.0 ** -7 * float(got[1].abs().max())
+    assert 1 <= ops.attn_general_mma_splits(n, hq, hk, d, d, 1000) <= 64
