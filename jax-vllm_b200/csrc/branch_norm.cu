@@ -149,10 +149,24 @@ __global__ void branch_norm_add_vec_kernel(float* __restrict__ h, const TD* __re
   }
 }
 
+// What is added behind the picked rows: `parts` tensors [n, hidden], `stride` elements apart, of floats or of 16-bit numbers; p null: nothing.
+struct Plus {
+  const void* p; int is_float, parts; size_t stride;
+  __device__ __forceinline__ float at(size_t i) const {
+    return is_float ? reinterpret_cast<const float*>(p)[i] : to_f32(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
+  }
+  __device__ __forceinline__ float4 four(size_t i) const {
+    if (is_float) return *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p) + i);
+    const uint2 a = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p) + i);
+    return make_float4(__uint_as_float(a.x << 16), __uint_as_float(a.x & 0xffff0000u), __uint_as_float(a.y << 16),
+                       __uint_as_float(a.y & 0xffff0000u));
+  }
+};
+
 template <typename TD>
 __global__ void pick_rows_sum_kernel(const TD* __restrict__ y, const int* __restrict__ pick, const float* __restrict__ coef,
                                      int parts, int y_rows, const TD* __restrict__ own, const float* __restrict__ own_coef,
-                                     float* __restrict__ out, int hidden, int* __restrict__ status) {
+                                     const Plus plus, float* __restrict__ out, int hidden, int* __restrict__ status) {
   pdl_trigger();
   pdl_wait();
   const int r = blockIdx.x;
@@ -167,6 +181,11 @@ __global__ void pick_rows_sum_kernel(const TD* __restrict__ y, const int* __rest
       v = fmaf(coef[(size_t)r * parts + s], to_f32(y[(size_t)src * hidden + c]), v);
     }
     if (own != nullptr) v = fmaf(own_coef[r], to_f32(own[(size_t)r * hidden + c]), v);
+    if (plus.p != nullptr) {
+      float d = plus.at((size_t)r * hidden + c);
+      for (int s = 1; s < plus.parts; ++s) d += plus.at(s * plus.stride + (size_t)r * hidden + c);
+      v += d;
+    }
     out[(size_t)r * hidden + c] = v;
   }
 }
@@ -177,7 +196,7 @@ template <typename TD>
 __global__ void __launch_bounds__(128) pick_rows_sum_vec_kernel(const TD* __restrict__ y, const int* __restrict__ pick,
                                                                 const float* __restrict__ coef, int parts, int y_rows,
                                                                 const TD* __restrict__ own, const float* __restrict__ own_coef,
-                                                                float* __restrict__ out, int hidden, int* __restrict__ status) {
+                                                                const Plus plus, float* __restrict__ out, int hidden, int* __restrict__ status) {
   constexpr int AT_ONCE = 8;
   pdl_trigger();
   pdl_wait();
@@ -195,8 +214,15 @@ __global__ void __launch_bounds__(128) pick_rows_sum_vec_kernel(const TD* __rest
   auto fma4 = [](float f, const float4& x, float4& v) {
     v.x = fmaf(f, x.x, v.x); v.y = fmaf(f, x.y, v.y); v.z = fmaf(f, x.z, v.z); v.w = fmaf(f, x.w, v.w);
   };
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f), mine = v;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f), mine = v, d = v;
   if (own != nullptr) mine = load(own + (size_t)r * hidden + c);
+  if (plus.p != nullptr) {
+    d = plus.four((size_t)r * hidden + c);
+    for (int s = 1; s < plus.parts; ++s) {
+      const float4 e = plus.four(s * plus.stride + (size_t)r * hidden + c);
+      d.x += e.x; d.y += e.y; d.z += e.z; d.w += e.w;
+    }
+  }
   for (int s0 = 0; s0 < parts; s0 += AT_ONCE) {
     int src[AT_ONCE];
     float4 x[AT_ONCE];
@@ -214,6 +240,7 @@ __global__ void __launch_bounds__(128) pick_rows_sum_vec_kernel(const TD* __rest
       if (src[s] >= 0) fma4(coef[(size_t)r * parts + s0 + s], x[s], v);
   }
   if (own != nullptr) fma4(own_coef[r], mine, v);
+  if (plus.p != nullptr) { v.x += d.x; v.y += d.y; v.z += d.z; v.w += d.w; }
   *reinterpret_cast<float4*>(out + (size_t)r * hidden + c) = v;
 }
 
@@ -263,21 +290,26 @@ JV_EXPORT int jv_branch_norm_add(float* h, const void* y, int y_dtype, long long
 
 // out[r, :] = sum_s coef[r, s] * y[pick[r, s], :] in 32-bit, s ascending: the weighted rows added up for a reader
 // that does not add them itself.  own [n, hidden] of the same type with own_coef [n], or null: out[r, :] += own_coef[r] *
-// own[r, :], and a pick of -1 is then no row (without it, it is reported).
+// own[r, :], and a pick of -1 is then no row (without it, it is reported).  plus: `plus_parts` tensors [n, hidden] of plus_dtype,
+// plus_stride elements apart, whose sum is added last, or null.
 JV_EXPORT int jv_pick_rows_sum(const void* y, int y_dtype, const int* pick, const float* coef, int parts, int y_rows,
-                               const void* own, const float* own_coef, float* out, int n, int hidden, int* status,
-                               cudaStream_t stream) {
+                               const void* own, const float* own_coef, const void* plus, int plus_dtype, int plus_parts,
+                               long long plus_stride, float* out, int n, int hidden, int* status, cudaStream_t stream) {
   if (n == 0) return JV_OK;
+  if (plus != nullptr && (plus_parts < 1 || plus_dtype < 0 || plus_dtype > 1)) return JV_ERR_UNSUPPORTED;
+  const Plus more{plus, plus_dtype == 0, plus_parts, (size_t)plus_stride};
+  const int plus_mask = plus_dtype == 0 ? 15 : 7;
   // vectors where rows consist of them: 8 rows of 2,048, 4 picks each, 3.0 us against 15.9; 777 rows
   // 10.3 against 21.6
   const int mask = y_dtype == 0 ? 15 : 7;
-  if (hidden % 4 == 0 && ((uintptr_t)y & mask) == 0 && ((uintptr_t)own & mask) == 0 && ((uintptr_t)out & 15) == 0 && hidden <= 512 * 65535) {
+  if (hidden % 4 == 0 && ((uintptr_t)y & mask) == 0 && ((uintptr_t)own & mask) == 0 && ((uintptr_t)out & 15) == 0 && hidden <= 512 * 65535 &&
+      ((uintptr_t)plus & plus_mask) == 0 && (plus == nullptr || plus_parts == 1 || plus_stride % 4 == 0)) {
     JV_DISPATCH_DTYPE(y_dtype, TD, return jv_launch(pick_rows_sum_vec_kernel<TD>, dim3(n, (hidden + 511) / 512), dim3(128), 0, stream,
-                                                    (const TD*)y, pick, coef, parts, y_rows, (const TD*)own, own_coef, out, hidden,
+                                                    (const TD*)y, pick, coef, parts, y_rows, (const TD*)own, own_coef, more, out, hidden,
                                                     status));
   }
   JV_DISPATCH_DTYPE(y_dtype, TD, return jv_launch(pick_rows_sum_kernel<TD>, dim3(n), dim3(256), 0, stream, (const TD*)y,
-                                                  pick, coef, parts, y_rows, (const TD*)own, own_coef, out, hidden, status));
+                                                  pick, coef, parts, y_rows, (const TD*)own, own_coef, more, out, hidden, status));
   return JV_ERR_UNSUPPORTED;
 }
 

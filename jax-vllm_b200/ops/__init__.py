@@ -47,8 +47,10 @@ class PartialSum:
         return self.parts.device
 
     def tensor(self, dtype: torch.dtype = torch.float32) -> torch.Tensor:
-        out = torch.zeros(tuple(self.shape), dtype=torch.float32, device=self.device)
-        residual_add(out, self)
+        out = torch.empty(tuple(self.shape), dtype=torch.float32, device=self.device)
+        parts = _cuda(self.parts, "parts", torch.float32)
+        f = _fn("norm", "jv_sum_parts", [c_void_p, c_void_p, c_longlong, c_int, c_longlong, c_void_p])
+        _check(f(out.data_ptr(), parts.data_ptr(), out.numel(), parts.shape[0], parts.stride(0), _stream()), "sum_parts")
         return out if dtype == torch.float32 else out.to(dtype)
 
 
@@ -81,14 +83,17 @@ class PickedRows:
     def device(self):
         return self.rows.device
 
-    def tensor(self, dtype: torch.dtype = torch.float32) -> torch.Tensor:
+    def tensor(self, dtype: torch.dtype = torch.float32, plus=None) -> torch.Tensor:
+        """`plus` (a tensor or a PartialSum) is added behind the rows."""
         self.check()
         n, width = self.shape
         out = torch.empty((n, width), dtype=torch.float32, device=self.device)
+        delta, n_parts, part_stride = _delta_parts(plus, out)
         f = _fn("branch_norm", "jv_pick_rows_sum", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
-                                                    c_void_p, c_int, c_int, c_void_p, c_void_p])
+                                                    c_void_p, c_int, c_int, c_longlong, c_void_p, c_int, c_int, c_void_p, c_void_p])
         _check(f(self.rows.data_ptr(), _code(self.rows, "rows"), self.pick.data_ptr(), self.coef.data_ptr(),
-                 self.pick.shape[1], self.rows.shape[0], _ptr(self.own), _ptr(self.own_coef), out.data_ptr(), n, width,
+                 self.pick.shape[1], self.rows.shape[0], _ptr(self.own), _ptr(self.own_coef), _ptr(delta),
+                 0 if delta is None else _code(delta, "delta"), n_parts, part_stride, out.data_ptr(), n, width,
                  _status_ptr(self.device), _stream()), "pick_rows_sum")
         return out if dtype == torch.float32 else out.to(dtype)
 
@@ -109,7 +114,7 @@ class BranchSum:
         return self.picked.device
 
     def tensor(self, dtype: torch.dtype = torch.float32) -> torch.Tensor:
-        out = residual_add(self.picked.tensor(), self.delta)
+        out = self.picked.tensor(plus=self.delta)
         return out if dtype == torch.float32 else out.to(dtype)
 
 

@@ -533,6 +533,24 @@ def test_heads_finished_in_vectors(maps, gate, dv, dtype):
     assert bool(((out.view(n, heads, dv).double() - want).abs() <= 2.0 ** -8 * want.abs() + 16 * EPS32 * size).all())
 
 
+# ------------------------------------------------------------------------------- sums of parts
+@pytest.mark.parametrize("shape", [(1, 4), (3, 33), (5, 2048)])
+@pytest.mark.parametrize("parts", [1, 2, 8, 9])
+def test_parts_added_up(shape, parts):
+    ops = _ops()
+    size = parts * shape[0] * shape[1]
+    for off in (0, 1):                                   # on and off 16-byte boundaries
+        p = _rand(size + 1, seed=parts)[off:off + size].view(parts, *shape)
+        want = p[0].clone()
+        for s in range(1, parts):
+            want = want + p[s]
+        assert torch.equal(ops.PartialSum(p).tensor(), want)
+        pick, coef = torch.zeros((shape[0], 1), dtype=torch.int32, device="cuda"), _rand(shape[0], 1, seed=1)
+        rows = _rand(1, shape[1], seed=2, dtype=torch.bfloat16)
+        for plus, d in ((ops.PartialSum(p), want), (p[0].bfloat16(), p[0].bfloat16().float()), (p[0], p[0])):
+            assert torch.equal(ops.BranchSum(plus, ops.PickedRows(rows, pick, coef)).tensor(), coef * rows.float() + d)
+
+
 # ------------------------------------------------------------------------------- keys of decoded tokens cut evenly
 @pytest.mark.parametrize("hq,hk,splits", [(4, 1, 1), (4, 1, 3), (40, 2, 7), (3, 3, 64)])
 @pytest.mark.parametrize("mask,keep,sigmoid", [(0, 0, False), (100, 5, False), (-128, 0, True)])
