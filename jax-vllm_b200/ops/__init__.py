@@ -553,6 +553,12 @@ def attn_general_mma_tokens_per_tile(n_q_heads: int, n_kv_heads: int) -> int:
     return 64 // min(n_q_heads // n_kv_heads, 16)
 
 
+def attn_general_mma_splits(n_work: int, n_q_heads: int, n_kv_heads: int, key_dim: int, value_dim: int, most: int) -> int:
+    """Into how many even splits `attn_general_mma` best cuts the keys, up to `most`, of each of `n_work` single tokens."""
+    f = _fn(attn_general_mma_library(key_dim, value_dim), "jv_attn_general_even_splits", [c_int] * 4)
+    return f(n_work, n_q_heads, n_kv_heads, most)
+
+
 def attn_general_mma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                      block_table: torch.Tensor, cu_seqlens: torch.Tensor, start_pos: torch.Tensor, work: torch.Tensor,
                      n_work: int, n_q_heads: int, n_kv_heads: int, scale: float, split_size: int = 0, n_splits: int = 0,
@@ -561,12 +567,6 @@ def attn_general_mma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache:
                      sink: torch.Tensor | None = None, window: int = 0, out_scale: float = 1.0, keep: int = 0) -> None:
     """Paged causal attention on the tensor cores with the options of `attn_simt`: the key size and the key heads are the
     key cache's, the value size and the value heads the value cache's; bfloat16 in, bfloat16 or float32 out.
-def attn_general_mma_splits(n_work: int, n_q_heads: int, n_kv_heads: int, key_dim: int, value_dim: int, most: int) -> int:
-    """Into how many even splits `attn_general_mma` best cuts the keys, up to `most`, of each of `n_work` single tokens."""
-    f = _fn(attn_general_mma_library(key_dim, value_dim), "jv_attn_general_even_splits", [c_int] * 4)
-    return f(n_work, n_q_heads, n_kv_heads, most)
-
-
     `window`: the mask as one number (`mask_code`).  Single tokens (`n_splits` > 0): splits of `split_size` keys, or with
     `split_size` 0 every token's keys cut evenly into up to `n_splits` (`attn_general_mma_splits`)."""
     n_dist = _score_extras("attn_general_mma", n_q_heads, head_scale, dist_bias, sink)
