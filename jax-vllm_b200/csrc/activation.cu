@@ -24,7 +24,8 @@ __global__ void swiglu_kernel(const T* __restrict__ gu, T* __restrict__ act, siz
 
 // Same, 16 bytes per access (block a multiple of the vector length, rows 16-byte aligned).
 template <typename T>
-__global__ void swiglu_vec_kernel(const T* __restrict__ gu, T* __restrict__ act, size_t act_stride, int inter, int block, size_t total_vec) {
+__global__ void swiglu_vec_kernel(const T* __restrict__ gu, T* __restrict__ act, size_t act_stride, int inter, int block, size_t total_vec,
+                                  const int* __restrict__ row_token) {
   pdl_trigger();
   pdl_wait();
   constexpr int V = 16 / sizeof(T);
@@ -33,6 +34,7 @@ __global__ void swiglu_vec_kernel(const T* __restrict__ gu, T* __restrict__ act,
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (; idx < total_vec; idx += stride) {
     const size_t n = idx / vec_per_row;
+    if (row_token != nullptr && row_token[n] < 0) continue;
     const int i = (int)(idx - n * vec_per_row) * V;
     const size_t col = (size_t)(i / block) * 2 * block + (i % block);
     const uint4 g4 = *reinterpret_cast<const uint4*>(gu + n * 2 * inter + col);
@@ -97,8 +99,9 @@ __global__ void swiglu_parts_kernel(const float* __restrict__ gu, T* __restrict_
 // gu: [n, 2*inter]; act: n rows of inter elements, act_stride apart; both of dtype `dtype`; block: see above (a divisor of inter).
 // parts > 1: gu is `parts` float tensors [n, 2*inter], part_stride elements apart, and act is of dtype `dtype`
 // (block and part_stride multiples of 4, gu 16-byte aligned).
+// row_token: [n] ints or null: rows with a -1 may be passed by (rows of padding between the experts').
 JV_EXPORT int jv_swiglu(const void* gu, void* act, long long act_stride, int dtype, int n, int inter, int block, int parts, long long part_stride,
-                        cudaStream_t stream) {
+                        const int* row_token, cudaStream_t stream) {
   const size_t total = (size_t)n * inter;
   if (total == 0) return JV_OK;
   if (block < 1 || inter % block || parts < 1) return JV_ERR_UNSUPPORTED;
@@ -117,7 +120,7 @@ JV_EXPORT int jv_swiglu(const void* gu, void* act, long long act_stride, int dty
     size_t blocks = (total_vec + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     JV_DISPATCH_DTYPE(dtype, T, return jv_launch(swiglu_vec_kernel<T>, dim3((int)blocks), dim3(256), 0, stream,
-                                                  (const T*)gu, (T*)act, (size_t)act_stride, inter, block, total_vec));
+                                                  (const T*)gu, (T*)act, (size_t)act_stride, inter, block, total_vec, row_token));
     return JV_ERR_UNSUPPORTED;
   }
   size_t blocks = (total + 255) / 256;

@@ -82,7 +82,8 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(
       __syncwarp();
     }
   }
-  float chosen_sum = 0.f;
+  float chosen_sum = 0.f, my_weight = 0.f;             // lane l keeps choice l (the 32 and later ones go through memory)
+  int my_id = 0;
   for (int it = 0; it < top; ++it) {
     float bv = -INFINITY; int bi = 0x7fffffff;
     for (int e = lane; e < experts; e += 32) {
@@ -100,12 +101,32 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(
     const float sv = bi == 0x7fffffff ? 0.f : s[bi];
     if (bi == 0x7fffffff) bi = 0;
     if (lane == 0) {
-      ids[(size_t)t * top + it] = bi;
-      weights[(size_t)t * top + it] = sv;
+      if (top > 32) {
+        ids[(size_t)t * top + it] = bi;
+        weights[(size_t)t * top + it] = sv;
+      }
       c[bi] = -INFINITY;                               // taken
     }
+    if (lane == it) { my_id = bi; my_weight = sv; }
     chosen_sum += sv;
     __syncwarp();
+  }
+  if (top <= 32) {
+    if (renorm) my_weight /= (chosen_sum + renorm_eps);
+    my_weight *= weight_scale;
+    if (lane < top) {
+      ids[(size_t)t * top + lane] = my_id;
+      weights[(size_t)t * top + lane] = my_weight;
+    }
+    if (own != nullptr) {                              // in the order of the choices
+      float mine = 0.f;
+      for (int it = 0; it < top; ++it) {
+        const float w = __shfl_sync(0xffffffffu, my_weight, it);
+        if (__shfl_sync(0xffffffffu, my_id, it) >= experts - identity) mine += w;
+      }
+      if (lane == 0) own[t] = mine;
+    }
+    return;
   }
   if (lane == 0) {
     float mine = 0.f;
@@ -136,43 +157,83 @@ __global__ void __launch_bounds__(128) moe_route_table_kernel(const int* __restr
   weights[i] = 1.f / (float)top;
 }
 
+// A pair takes its place among its expert's rows as it is counted, a warp's pairs of one expert by one addition; the experts' first rows
+// are then one warp's running sum.  (A count and a cursor, each moved by every pair, and one thread that went through the experts:
+// 8 tokens of 4 choices among 36 experts 6.8 us, 777 tokens 11.7; so 3.0 and 7.2.)
 __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__ ids, int pairs, int top, int experts,
                                                          int identity, int tile, int max_tiles, int* __restrict__ sorted_token,
                                                          int* __restrict__ pos_of, int* __restrict__ tile_expert,
                                                          int* __restrict__ status) {
-  extern __shared__ int sh[];                    // [experts] counts, [experts] first row, [experts] cursor
+  extern __shared__ int sh[];                    // [experts] counts, [experts] first row
   int* count = sh;
   int* first = sh + experts;
-  int* cursor = first + experts;
+  __shared__ int used;
+  constexpr int KEEP = 4;                        // pairs whose expert and place a thread keeps; those of later ones lie in pos_of
   pdl_trigger();
+  for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
   pdl_wait();
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) { count[e] = 0; cursor[e] = 0; }
+  const int lane = threadIdx.x & 31, rounds = (pairs + blockDim.x - 1) / blockDim.x;
+  int kept_e[KEEP], kept_at[KEEP];
+#pragma unroll
+  for (int r = 0; r < KEEP; ++r) {
+    const int i = r * blockDim.x + threadIdx.x;
+    kept_e[r] = i < pairs ? ids[i] : experts;
+  }
   for (int i = threadIdx.x; i < max_tiles * tile; i += blockDim.x) sorted_token[i] = -1;
-  for (int i = threadIdx.x; i < max_tiles; i += blockDim.x) tile_expert[i] = -1;
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = ids[i];
-    if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
-    else if (e < 0 || e >= experts + identity) atomicOr(status, JV_STATUS_BAD_ROW);
+  auto place = [&](int e, bool there) -> int {   // by whole warps: the pair's number among those of its expert
+    if (there && (e < 0 || e >= experts + identity)) atomicOr(status, JV_STATUS_BAD_ROW);
+    const bool has_rows = there && e >= 0 && e < experts;
+    const unsigned same = __match_any_sync(0xffffffffu, has_rows ? e : -1);
+    const int leader = __ffs(same) - 1;
+    int base = 0;
+    if (has_rows && lane == leader) base = atomicAdd(&count[e], __popc(same));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    return has_rows ? base + __popc(same & ((1u << lane) - 1)) : -1;
+  };
+#pragma unroll
+  for (int r = 0; r < KEEP; ++r)
+    if (r < rounds) kept_at[r] = place(kept_e[r], r * blockDim.x + threadIdx.x < pairs);
+  for (int r = KEEP; r < rounds; ++r) {
+    const int i = r * blockDim.x + threadIdx.x, at = place(i < pairs ? ids[i] : experts, i < pairs);
+    if (i < pairs) pos_of[i] = at;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     int row = 0;
-    for (int e = 0; e < experts; ++e) {
-      first[e] = row;
-      const int tiles = (count[e] + tile - 1) / tile;
-      for (int k = 0; k < tiles; ++k) tile_expert[row / tile + k] = e;
-      row += tiles * tile;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int mine = e0 + lane < experts ? (count[e0 + lane] + tile - 1) / tile * tile : 0;
+      int sum = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int before = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += before;
+      }
+      if (e0 + lane < experts) first[e0 + lane] = row + sum - mine;
+      row += __shfl_sync(0xffffffffu, sum, 31);
     }
-    tile_expert[max_tiles] = row / tile;          // the row tiles in use are the first this many
+    if (lane == 0) {
+      used = row / tile;
+      tile_expert[max_tiles] = used;             // the row tiles in use are the first this many
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = ids[i];
-    if (e < 0 || e >= experts) { pos_of[i] = -1; continue; }
-    const int pos = first[e] + atomicAdd(&cursor[e], 1);
-    sorted_token[pos] = i / top;
+  for (int e = threadIdx.x; e < experts; e += blockDim.x)
+    for (int k = 0; k < (count[e] + tile - 1) / tile; ++k) tile_expert[first[e] / tile + k] = e;
+  for (int i = used + threadIdx.x; i < max_tiles; i += blockDim.x) tile_expert[i] = -1;
+  auto put = [&](int i, int e, int at) {
+    const int pos = at < 0 ? -1 : first[e] + at;
+    if (pos >= 0) sorted_token[pos] = i / top;
     pos_of[i] = pos;
+  };
+#pragma unroll
+  for (int r = 0; r < KEEP; ++r) {
+    const int i = r * blockDim.x + threadIdx.x;
+    if (i < pairs) put(i, kept_e[r], kept_at[r]);
+  }
+  for (int r = KEEP; r < rounds; ++r) {
+    const int i = r * blockDim.x + threadIdx.x;
+    if (i < pairs) put(i, ids[i], pos_of[i]);
   }
 }
 
@@ -239,6 +300,6 @@ JV_EXPORT int jv_moe_align(const int* ids, int pairs, int top, int experts, int 
   if (tile < 1 || (long long)max_tiles * tile < (long long)pairs + (long long)experts * (tile - 1) ||
       experts * 3 * sizeof(int) > 48 * 1024)
     return JV_ERR_UNSUPPORTED;
-  return jv_launch(moe_align_kernel, dim3(1), dim3(1024), (size_t)experts * 3 * sizeof(int), stream, ids, pairs, top,
+  return jv_launch(moe_align_kernel, dim3(1), dim3(1024), (size_t)experts * 2 * sizeof(int), stream, ids, pairs, top,
                    experts, identity, tile, max_tiles, sorted_token, pos_of, tile_expert, status);
 }

@@ -372,10 +372,11 @@ def residual_add(h: torch.Tensor, delta) -> torch.Tensor:
 
 # ----------------------------------------------------------------------- activation
 def swiglu(gate_up, block: int | None = None, out_dtype: torch.dtype | None = None,
-           out: torch.Tensor | None = None) -> torch.Tensor:
+           out: torch.Tensor | None = None, row_token: torch.Tensor | None = None) -> torch.Tensor:
     """silu(gate) * up for a packed [n, 2*inter] tensor: blocks of `block` gate columns, each followed
     by the up columns of the same indices (default: all gate columns first).  The input may be a
-    PartialSum; the result then has `out_dtype`.  `out` [n, inter]: where to write, possibly a column range of wider rows."""
+    PartialSum; the result then has `out_dtype`.  `out` [n, inter]: where to write, possibly a column range of wider rows.
+    `row_token` [n] int32: rows with a -1 (padding between the experts' rows) need no result."""
     n_parts, part_stride = 1, 0
     if isinstance(gate_up, PartialSum):
         if out_dtype is None:
@@ -397,10 +398,12 @@ def swiglu(gate_up, block: int | None = None, out_dtype: torch.dtype | None = No
         _cuda(out, "out", act_dtype, contiguous=False)
     if act.shape != (n, two_i // 2) or act.stride(1) != 1:
         raise KernelError("swiglu: out is [n, columns / 2] with unit column stride")
+    if row_token is not None and _cuda(row_token, "row_token", torch.int32).numel() != n:
+        raise KernelError("swiglu: a token (or -1) per row")
     f = _fn("activation", "jv_swiglu", [c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_longlong,
-                                        c_void_p])
-    _check(f(gate_up.data_ptr(), act.data_ptr(), act.stride(0), _code(act, "act"), n, two_i // 2, block, n_parts, part_stride, _stream()),
-           "swiglu")
+                                        c_void_p, c_void_p])
+    _check(f(gate_up.data_ptr(), act.data_ptr(), act.stride(0), _code(act, "act"), n, two_i // 2, block, n_parts, part_stride,
+             _ptr(row_token), _stream()), "swiglu")
     return act
 
 

@@ -124,9 +124,9 @@ class RoutedExperts(Part):
         return ops.moe_route(logits, s.top_k, s.n_groups, s.keep_groups, s.renormalize, s.scoring, s.group_score,
                              s.renorm_eps, s.weight_scale, correction=self.correction, identity=s.identity)
 
-    def _gate(self, gu):
-        """The activation of experts with a gate matrix, from rows [gate | up]."""
-        return ops.swiglu(gu) if self.spec.activation == "swiglu" else ops.glu_clamped(gu, self.spec.limit)
+    def _gate(self, gu, row_token=None):
+        """The activation of experts with a gate matrix, from rows [gate | up]; rows whose token is -1 are nobody's."""
+        return ops.swiglu(gu, row_token=row_token) if self.spec.activation == "swiglu" else ops.glu_clamped(gu, self.spec.limit)
 
     def out_weight(self):
         return None if self.shared is None else self.shared.out_weight()
@@ -152,7 +152,7 @@ class RoutedExperts(Part):
             # everything around it by the rows, padding included.
             few = x.shape[0] <= ops.MOE_STREAM_MAX_TOKENS
             tile = -(-x.shape[0] // 16) * 16 if few else ops.MOE_TCGEN05_TILE
-            _, pos_of, tile_expert, used = ops.moe_align(ids, s.num_experts, tile, s.identity)
+            row_token, pos_of, tile_expert, used = ops.moe_align(ids, s.num_experts, tile, s.identity)
             rows = ops.moe_gather_rows(x, pos_of, tile_expert.numel() * tile)
 
             def product(a, w, act=None):
@@ -162,7 +162,7 @@ class RoutedExperts(Part):
 
             act = product(rows, self.w_up, first)
             if self.gated:
-                act = self._gate(act)
+                act = self._gate(act, row_token)
             return ops.PickedRows(product(act, self.w_down), pos_of, weights, *own)
         sorted_token, pos_of, tile_expert, _ = ops.moe_align(ids, s.num_experts, ops.moe_gemm_simt_tile(), s.identity)
         act = ops.moe_gemm_simt(x, sorted_token, self.w_up, tile_expert, dt, act=first)

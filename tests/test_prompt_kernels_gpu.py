@@ -288,6 +288,29 @@ def test_experts_streamed_past_few_tokens(tokens, top, experts, n, k, act):
     ops.check_status()
 
 
+@pytest.mark.parametrize("tokens,top,experts,identity,tile", [(1, 1, 1, 0, 16), (8, 4, 32, 4, 16), (777, 4, 32, 4, 128), (2000, 6, 100, 0, 128),
+                                                             (37, 33, 40, 3, 48)])
+def test_pairs_in_the_order_of_their_experts(tokens, top, experts, identity, tile):
+    """More pairs than threads keep, more experts than a warp, identity experts' pairs without a row; ids that are no expert's are reported."""
+    ops = _ops()
+    ids = torch.rand(tokens, experts + identity, generator=torch.Generator(device="cuda").manual_seed(1), device="cuda").argsort(1)[:, :top]
+    ids = ids.to(torch.int32).contiguous()
+    sorted_token, pos_of, tile_expert, used = ops.moe_align(ids, experts, tile, identity)
+    ops.check_status()
+    rows = torch.full_like(sorted_token, -1)
+    real = ids < experts
+    assert (pos_of[~real] == -1).all() and pos_of[real].unique().numel() == int(real.sum())
+    token = torch.arange(tokens, device="cuda", dtype=torch.int32)[:, None].expand_as(ids)
+    rows[pos_of[real].long()] = token[real]
+    assert torch.equal(rows, sorted_token)
+    assert torch.equal(tile_expert[(pos_of[real] // tile).long()], ids[real])
+    want = sum(-(-int((ids == e).sum()) // tile) for e in range(experts))
+    assert int(used) == want and (tile_expert[want:] == -1).all() and (tile_expert[:want] >= 0).all()
+    ops.moe_align(torch.full((2, 1), experts + identity, dtype=torch.int32, device="cuda"), experts, tile, identity)
+    with pytest.raises(ops.KernelError):
+        ops.check_status()
+
+
 @pytest.mark.parametrize("hidden", [4, 512, 516, 33])
 @pytest.mark.parametrize("parts", [1, 8, 9])
 def test_picked_rows_in_vectors(hidden, parts):
