@@ -1,4 +1,4 @@
-// Paged causal attention of prompt portions on the 5th-generation tensor cores, for head size 128:
+// Paged causal attention of prompt portions on the 5th-generation tensor cores, for heads of 128 and of 64:
 // scores and output accumulate in tensor memory (TMEM), queries, keys and values come in by TMA in the
 // 128-byte-swizzle layout that tcgen05.mma reads.
 //
@@ -27,21 +27,29 @@
 // Masks: causal, a window, chunks; under a window the first `keep` positions of a sequence may stay visible: an item's
 // tiles are then those of the kept positions (as far as they lie before the window's) followed by the window's.
 //
-// Restrictions (the caller falls back to the mma.sync kernel otherwise): bfloat16, head size 128, HPT up to 16, page size a power of two from 8 to 128.
+// Heads of 64 (a tile of keys is 16 KB then, and twice as many are in flight) were the mma.sync kernel's before: 2,999 tokens in three
+// entries behind 77, 16 heads on 4, a window of 512 that keeps 4, capped scores: 67.6 us there, 47.3 here.
+//
+// Restrictions (the caller falls back to the mma.sync kernel otherwise): bfloat16, head size 128 or 64, HPT up to 16, page size a power of two from 8 to 128.
 #include "tcgen05.cuh"
 
 #include <math.h>
 
 namespace {
 
-constexpr int D = 128, ROWS = 128, BN = 128;
-constexpr int TILE_BYTES = 128 * 128 * 2;       // a 128 x 128 bfloat16 tile: two halves of [128 rows][128 bytes]
-constexpr int HALF_BYTES = 128 * 128;            // one half: 128 rows of 128 bytes
-constexpr int K_STAGES = 2, V_STAGES = 3, Q_BUFFERS = 2;   // 7 tiles of 32 KB
+constexpr int ROWS = 128, BN = 128;
+constexpr int HALF_BYTES = 128 * 128;            // 64 elements of 128 rows: 128 rows of 128 bytes
+constexpr int Q_BUFFERS = 2;
+// D: the head size.  A tile of queries, keys or values is one [128 rows][64 elements] or two, one behind the other.
+template <int D> struct Shape {
+  static constexpr int HALVES = D / 64, TILE_BYTES = HALVES * HALF_BYTES;
+  static constexpr int K_STAGES = D == 128 ? 2 : 4, V_STAGES = D == 128 ? 3 : 6;    // 7 tiles of 32 KB, 12 of 16 KB
+  static constexpr uint32_t PV = (IDESC_PV & ~(0x3Fu << 17)) | ((uint32_t)(D >> 3) << 17);
+};
 constexpr int THREADS = 352;                     // key producer warp, mma warp, 8 softmax warps, value producer warp
 constexpr int SOFTMAX_THREADS = 256;
 constexpr int TMEM_COLS = 512;                   // S0: [0,128)  S1: [128,256)  O: [256,384)  P0: [384,448)  P1: [448,512)
-constexpr int TMEM_O = 256, TMEM_P = 384;        // a column of P holds two bfloat16: keys 2c and 2c+1
+constexpr int TMEM_O = 256, TMEM_P = 384;        // O has D columns; a column of P holds two bfloat16: keys 2c and 2c+1
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct Params {
@@ -62,6 +70,7 @@ struct Params {
   int* status;
 };
 
+template <int K_STAGES, int V_STAGES>
 struct Shared {
   uint64_t q_full[Q_BUFFERS], q_free[Q_BUFFERS], k_full[K_STAGES], k_empty[K_STAGES], v_full[V_STAGES], v_empty[V_STAGES];
   uint64_t s_full[2], p_full[2], o_done[2];
@@ -118,11 +127,14 @@ struct Item {
   __device__ __forceinline__ int tile(int j) const { return j < kept ? j : j - kept + tile0; }    // among all key tiles of the request
 };
 
+template <int D>
 __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map,
                                                                   const __grid_constant__ CUtensorMap k_map,
                                                                   const __grid_constant__ CUtensorMap v_map,
                                                                   const __grid_constant__ CUtensorMap out_map,
                                                                   const Params p) {
+  constexpr int HALVES = Shape<D>::HALVES, TILE_BYTES = Shape<D>::TILE_BYTES, K_STAGES = Shape<D>::K_STAGES, V_STAGES = Shape<D>::V_STAGES;
+  using Shared = ::Shared<K_STAGES, V_STAGES>;
   pdl_trigger();      // a kernel launched behind this one (decode attention of the same step) may take the multiprocessors that the first blocks to end leave free
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -212,9 +224,9 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
         ok = mbar_wait(&sh->q_free[qb], ph ^ 1);                 // the item two before this one has left through this buffer
         if (ok) {
           sh->armed_q[qb] = ph;
-          mbar_expect_tx(&sh->q_full[qb], 2 * 128 * G * p.tokens_per_tile);      // two boxes of 64 d x G heads x tokens
+          mbar_expect_tx(&sh->q_full[qb], HALVES * 128 * G * p.tokens_per_tile);      // boxes of 64 d x G heads x tokens
           tma_load_3d(q_s + qb * TILE_BYTES, &q_map, 0, it.kv_head * G, it.q_first, &sh->q_full[qb]);
-          tma_load_3d(q_s + qb * TILE_BYTES + HALF_BYTES, &q_map, 64, it.kv_head * G, it.q_first, &sh->q_full[qb]);
+          if (HALVES == 2) tma_load_3d(q_s + qb * TILE_BYTES + HALF_BYTES, &q_map, 64, it.kv_head * G, it.q_first, &sh->q_full[qb]);
         }
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -238,13 +250,13 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
         const int n_pages = __popc(__ballot_sync(0xffffffffu, pages >= 0));
         if (lane == 0) {
           ok = mbar_wait(&empty_bars[s], ph ^ 1);
-          if (ok) { armed[s] = ph; mbar_expect_tx(&full_bars[s], n_pages * P * 128 * 2); }
+          if (ok) { armed[s] = ph; mbar_expect_tx(&full_bars[s], n_pages * P * 128 * HALVES); }
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);      // also orders the announcement before the copies
-        // lane i issues the two boxes of page i
+        // lane i issues the boxes of page i
         if (ok && pages >= 0) {
           tma_load_4d(dst + lane * P * 128, map, 0, it.kv_head, 0, pages, &full_bars[s]);
-          tma_load_4d(dst + HALF_BYTES + lane * P * 128, map, 64, it.kv_head, 0, pages, &full_bars[s]);
+          if (HALVES == 2) tma_load_4d(dst + HALF_BYTES + lane * P * 128, map, 64, it.kv_head, 0, pages, &full_bars[s]);
         }
         pages = pages_next;
       }
@@ -258,12 +270,12 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
 #pragma unroll
       for (int b = 0; b < Q_BUFFERS; ++b) {
         q_desc[b][0] = desc_k_major(smem_u32(q_s + b * TILE_BYTES));
-        q_desc[b][1] = desc_k_major(smem_u32(q_s + b * TILE_BYTES + HALF_BYTES));
+        q_desc[b][1] = desc_k_major(smem_u32(q_s + b * TILE_BYTES + (HALVES - 1) * HALF_BYTES));
       }
 #pragma unroll
       for (int st = 0; st < K_STAGES; ++st) {
         k_desc[st][0] = desc_k_major(smem_u32(k_s + st * TILE_BYTES));
-        k_desc[st][1] = desc_k_major(smem_u32(k_s + st * TILE_BYTES + HALF_BYTES));
+        k_desc[st][1] = desc_k_major(smem_u32(k_s + st * TILE_BYTES + (HALVES - 1) * HALF_BYTES));
       }
 #pragma unroll
       for (int st = 0; st < V_STAGES; ++st) v_desc[st] = desc_mn_major(smem_u32(v_s + st * TILE_BYTES), HALF_BYTES);
@@ -299,8 +311,10 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
         const uint32_t tmem_s = tmem + (gt & 1) * 128;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) umma(tmem_s, q0 + 2 * kk, k0 + 2 * kk, IDESC_QK, kk != 0);
+        if (HALVES == 2) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) umma(tmem_s, q1 + 2 * kk, k1 + 2 * kk, IDESC_QK, 1);
+          for (int kk = 0; kk < 4; ++kk) umma(tmem_s, q1 + 2 * kk, k1 + 2 * kk, IDESC_QK, 1);
+        }
         umma_commit(&sh->k_empty[s]);
         umma_commit(&sh->s_full[gt & 1]);
         return true;
@@ -320,7 +334,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
         const uint32_t tmem_p = tmem + TMEM_P + (gt & 1) * 64;
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)   // 16 keys further: 8 columns of P, 16 rows (2048 bytes) down V
-          umma_a_tmem(tmem_o, tmem_p + kk * 8, v_desc[s] + kk * (16 * 128 / 16), IDESC_PV, (cur.j | kk) != 0);
+          umma_a_tmem(tmem_o, tmem_p + kk * 8, v_desc[s] + kk * (16 * 128 / 16), Shape<D>::PV, (cur.j | kk) != 0);
         umma_commit(&sh->v_empty[s]);
         umma_commit(&sh->o_done[gt & 1]);
         cur = nxt;
@@ -329,7 +343,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
     }
   } else {
     // ----------------------------------------------------------------- softmax
-    // Two threads per row: warps 2..5 take the first 64 keys of a tile (and the first 64 columns of O),
+    // Two threads per row: warps 2..5 take the first 64 keys of a tile (and the first half of the columns of O),
     // warps 6..9 the other 64.  A warp reads the 32 TMEM lanes of its number modulo 4.
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
@@ -461,12 +475,12 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
           if (ok) {
             TC_FENCE_AFTER();
 #pragma unroll 1
-            for (int c = 0; c < 2; ++c) {
+            for (int c = 0; c < HALVES; ++c) {
               float v[32];
-              tmem_ld32(tmem_o + lane_addr + half * 64 + c * 32, v);
+              tmem_ld32(tmem_o + lane_addr + half * (D / 2) + c * 32, v);
 #pragma unroll
               for (int i = 0; i < 32; ++i) v[i] *= alpha;
-              tmem_st32(tmem_o + lane_addr + half * 64 + c * 32, v);
+              tmem_st32(tmem_o + lane_addr + half * (D / 2) + c * 32, v);
             }
           }
         }
@@ -521,8 +535,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
           ok = __all_sync(0xffffffffu, mbar_wait(&sh->v_full[s], (gt / V_STAGES) & 1));
           if (ok) {
             const int n_zero = rows_before + (BN - rows_upto);
-            for (int i = (threadIdx.x - 64); i < n_zero * 16; i += SOFTMAX_THREADS) {
-              const int z = i / 16, part = i % 16;                // 16 chunks of 16 bytes per row (both halves)
+            for (int i = (threadIdx.x - 64); i < n_zero * 8 * HALVES; i += SOFTMAX_THREADS) {
+              const int z = i / (8 * HALVES), part = i % (8 * HALVES);      // chunks of 16 bytes of a row
               const int key_row = z < rows_before ? zero_from + z : rows_upto + (z - rows_before);
               *reinterpret_cast<uint4*>(v_s + s * TILE_BYTES + (part >> 3) * HALF_BYTES + key_row * 128 + (part & 7) * 16) =
                   make_uint4(0, 0, 0, 0);
@@ -541,7 +555,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
           stored = -1;
         }
       }
-      // ---- the item's output: O / sum, each thread its 64 columns; the row's sum is the two threads' together
+      // ---- the item's output: O / sum, each thread half of the columns; the row's sum is the two threads' together
       const int g_last = gt - 1, qb = n % Q_BUFFERS;
       sh->xch[half][row] = l_run;
       pair_barrier(quad);
@@ -560,21 +574,22 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
       // A whole tile leaves through shared memory (where the item's queries were: every product with them has
       // completed) and one TMA store per half of the head; threads that write their 128 bytes to rows 8 KB apart in
       // memory take five times as long.
-      unsigned char* row_base = q_s + qb * TILE_BYTES + half * HALF_BYTES + row * 128;
-      __nv_bfloat16* dst = p.out + (size_t)(it.q_first + t) * p.out_stride + (size_t)(it.kv_head * G + hh) * D + half * 64;
+      unsigned char* row_base = q_s + qb * TILE_BYTES + (HALVES - 1) * half * HALF_BYTES + row * 128;
+      const int first_chunk = HALVES == 2 ? 0 : half * 4;      // of this thread's in the row's 128 bytes
+      __nv_bfloat16* dst = p.out + (size_t)(it.q_first + t) * p.out_stride + (size_t)(it.kv_head * G + hh) * D + half * (D / 2);
       if (got) {
         TC_FENCE_AFTER();
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < HALVES; ++c) {
           float v[32];
-          tmem_ld32(tmem_o + lane_addr + half * 64 + c * 32, v);
+          tmem_ld32(tmem_o + lane_addr + half * (D / 2) + c * 32, v);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             uint4 pk;
             __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
             for (int e = 0; e < 4; ++e) h2[e] = __floats2bfloat162_rn(v[q * 8 + 2 * e] * inv, v[q * 8 + 2 * e + 1] * inv);
-            const int chunk = c * 4 + q;                       // 16-byte chunk within the 128-byte row
+            const int chunk = first_chunk + c * 4 + q;         // 16-byte chunk within the 128-byte row
             if (whole) *reinterpret_cast<uint4*>(row_base + ((chunk ^ (row & 7)) << 4)) = pk;
             else if (row_ok) *reinterpret_cast<uint4*>(dst + c * 32 + q * 8) = pk;
           }
@@ -589,7 +604,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
           if (got) {
             // started here, waited for after the next item's first tile (or at the end): this thread's warp is not held up
             tma_store_3d(&out_map, q_s + qb * TILE_BYTES, 0, it.kv_head * G, it.q_first);
-            tma_store_3d(&out_map, q_s + qb * TILE_BYTES + HALF_BYTES, 64, it.kv_head * G, it.q_first);
+            if (HALVES == 2) tma_store_3d(&out_map, q_s + qb * TILE_BYTES + HALF_BYTES, 64, it.kv_head * G, it.q_first);
             asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
             stored = qb;
           } else {
@@ -632,12 +647,29 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
   }
 }
 
+template <int D>
+int launch(const CUtensorMap& q_map, const CUtensorMap& k_map, const CUtensorMap& v_map, const CUtensorMap& out_map, const Params& p,
+           cudaStream_t stream) {
+  constexpr size_t smem = Shape<D>::TILE_BYTES * (Q_BUFFERS + Shape<D>::K_STAGES + Shape<D>::V_STAGES) +
+                          sizeof(Shared<Shape<D>::K_STAGES, Shape<D>::V_STAGES>) + 1024;
+  static bool ready[JV_MAX_DEVICES];
+  if (!jv_once_per_device(ready, [&] {
+        return cudaFuncSetAttribute(attn_tcgen05_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+      }))
+    return JV_ERR_UNSUPPORTED;
+  // persistent blocks: one per multiprocessor (or per item, if there are fewer)
+  const int sms = jv_multiprocessors();
+  const long long items = (long long)p.n_work * p.n_kv_heads;
+  return jv_launch(attn_tcgen05_kernel<D>, dim3((unsigned)(items < sms ? items : sms)), dim3(THREADS), smem, stream, q_map, k_map, v_map,
+                   out_map, p);
+}
+
 }  // namespace
 
 // 1 if this kernel takes the case (else the caller uses the mma.sync kernel).
 JV_EXPORT int jv_attn_tcgen05_supports(int head_dim, int n_q_heads, int n_kv_heads, int page_size, int window) {
   (void)window;                 // every mask of common.cuh's first_visible is taken
-  if (head_dim != 128 || n_kv_heads < 1 || n_q_heads % n_kv_heads) return 0;
+  if ((head_dim != 128 && head_dim != 64) || n_kv_heads < 1 || n_q_heads % n_kv_heads) return 0;
   const int G = n_q_heads / n_kv_heads;
   if (G > 16) return 0;
   return page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128;
@@ -646,8 +678,8 @@ JV_EXPORT int jv_attn_tcgen05_supports(int head_dim, int n_q_heads, int n_kv_hea
 // Tokens per 128-row tile.
 JV_EXPORT int jv_attn_tcgen05_tokens_per_tile(int n_q_heads, int n_kv_heads) { return ROWS / (n_q_heads / n_kv_heads); }
 
-// q: [n_tokens, q_stride] bfloat16 with head h of a token at column h*128; out: [n_tokens, out_stride];
-// k_cache/v_cache: [num_pages, page_size, n_kv_heads, 128]; work: [n_work, 2] (entry, first token of the tile),
+// q: [n_tokens, q_stride] bfloat16 with head h of a token at column h*head_dim; out: [n_tokens, out_stride];
+// k_cache/v_cache: [num_pages, page_size, n_kv_heads, head_dim]; work: [n_work, 2] (entry, first token of the tile),
 // tiles of jv_attn_tcgen05_tokens_per_tile tokens, in ascending order of work.
 // sigmoid != 0: the weights are sigmoid(q.k * scale + bias[query head]) instead of a softmax (bias: [n_q_heads] floats or null).
 // head_scale [n_q_heads], dist_bias [n_q_heads][n_dist], sink [n_q_heads] (floats, each may be null; softmax only): see Params.
@@ -670,7 +702,7 @@ JV_EXPORT int jv_attn_tcgen05_ex(const void* q, int q_stride, int n_tokens, void
     return JV_ERR_UNSUPPORTED;
   auto fn = encode_fn();
   if (fn == nullptr) return JV_ERR_UNSUPPORTED;
-  const int G = n_q_heads / n_kv_heads;
+  const int G = n_q_heads / n_kv_heads, D = head_dim;
   CUtensorMap q_map, k_map, v_map, out_map;
   for (int which = 0; which < 2; ++which) {
     // queries and output: (d, head, token); a box is 64 d x G heads x (128 / G) tokens = 128 rows, head fastest
@@ -701,22 +733,7 @@ JV_EXPORT int jv_attn_tcgen05_ex(const void* q, int q_stride, int n_tokens, void
   p.scale_log2 = scale * LOG2E; p.status = status; p.sigmoid = sigmoid ? 1 : 0; p.bias = bias;
   p.head_scale = head_scale; p.dist_bias = dist_bias; p.n_dist = n_dist; p.sink = sink; p.window = window;
   p.out_scale = out_scale; p.keep = window > 0 ? keep : 0; p.score_cap_log2 = score_cap > 0.f ? score_cap * LOG2E : 0.f;
-  constexpr size_t smem = TILE_BYTES * (Q_BUFFERS + K_STAGES + V_STAGES) + sizeof(Shared) + 1024;
-  static bool ready[JV_MAX_DEVICES];
-  if (!jv_once_per_device(ready, [&] {
-        return cudaFuncSetAttribute(attn_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
-      }))
-    return JV_ERR_UNSUPPORTED;
-  // persistent blocks: one per multiprocessor (or per item, if there are fewer)
-  static int sm_count[JV_MAX_DEVICES];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= JV_MAX_DEVICES) return JV_ERR_UNSUPPORTED;
-  if (sm_count[dev] == 0 &&
-      (cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count[dev] <= 0))
-    sm_count[dev] = 148;
-  const long long items = (long long)n_work * n_kv_heads;
-  const int blocks = items < sm_count[dev] ? (int)items : sm_count[dev];
-  return jv_launch(attn_tcgen05_kernel, dim3(blocks), dim3(THREADS), smem, stream, q_map, k_map, v_map, out_map, p);
+  return D == 128 ? launch<128>(q_map, k_map, v_map, out_map, p, stream) : launch<64>(q_map, k_map, v_map, out_map, p, stream);
 }
 
 JV_EXPORT int jv_attn_tcgen05(const void* q, int q_stride, int n_tokens, void* out, int out_stride, const void* k_cache,

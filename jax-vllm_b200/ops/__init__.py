@@ -863,7 +863,7 @@ def attn_tcgen05_supports(dtype: torch.dtype, head_dim: int, n_q_heads: int, n_k
                           window: int) -> bool:
     """Whether the tcgen05 prompt-attention kernel takes the case (csrc/attn_tcgen05.cu)."""
     g = n_q_heads // max(n_kv_heads, 1)
-    return (dtype == torch.bfloat16 and head_dim == 128 and n_q_heads % n_kv_heads == 0
+    return (dtype == torch.bfloat16 and head_dim in (64, 128) and n_q_heads % n_kv_heads == 0
             and 1 <= g <= 16 and page_size in (8, 16, 32, 64, 128))      # any mask (`window`) is taken
 
 

@@ -42,8 +42,8 @@ class Attention(Part):
         self.use_mma = ops.attn_mma_supports(ctx.dtype, self.d)
         if self.use_mma:
             self.kernels = ("rope_kv", "attn_mma", "gemm_simt", "linear_skinny")
-            if self.d == 128:
-                self.kernels += ("attn_tcgen05", "attn_decode_tcgen05")
+            if self.d in (64, 128):
+                self.kernels += ("attn_tcgen05",) + (("attn_decode_tcgen05",) if self.d == 128 else ())
         self.w_qkv = self.w_o = self.q_norm = self.k_norm = None
 
     # -------------------------------------------------------------------- weights
@@ -88,7 +88,7 @@ class Attention(Part):
 
     def tile_classes(self, page_size: int):
         """Entries of several tokens: tiles of the mma.sync (or CUDA-core) kernel, and for portions that fill
-        a 128-row tile of the tcgen05 kernel (head size 128, bfloat16, any mask) tiles of that one."""
+        a 128-row tile of the tcgen05 kernel (head size 128 or 64, bfloat16, any mask) tiles of that one."""
         small = (ops.attn_mma_tokens_per_tile if self.use_mma else ops.attn_simt_tokens_per_tile)(self.hq, self.hkv)
         if ops.attn_tcgen05_supports(self.ctx.dtype, self.d, self.hq, self.hkv, page_size, self.window):
             big = ops.attn_tcgen05_tokens_per_tile(self.hq, self.hkv)

@@ -116,7 +116,7 @@ class GeneralAttention(Part):
                 ("talk_prepare" if self.talking else "head_prepare",)
         # Which attention kernel: once queries and keys are prepared, a mixer with one softmax map, no cap and
         # values shaped like its keys IS the plain grouped-query attention, and goes the way of that mixer (the
-        # tcgen05 kernels for heads of 128, mma.sync for 16/32/64, in bfloat16).  Every other bfloat16 mixer with
+        # tcgen05 kernels for heads of 128 and of 64 (prompts), mma.sync for 16/32 and decoded heads of 64, in bfloat16).  Every other bfloat16 mixer with
         # sizes in steps of 16 takes the tensor-core kernel compiled for its pair of sizes; the rest, and 32-bit,
         # the CUDA-core kernel.
         # a temperature per head, a bias by distance and a sink are options of both of these
@@ -139,9 +139,9 @@ class GeneralAttention(Part):
         elif ops.attn_general_mma_supports(ctx.dtype, self.dk, self.dv):
             self.general = ops.attn_general_mma_library(self.dk, self.dv)
             self.kernels += (self.general,)
-        # heads of 128 with sigmoid weights, or with a softmax that has a cap, a temperature per head, a bias by distance, a
+        # heads of 128 or 64 with sigmoid weights, or with a softmax that has a cap, a temperature per head, a bias by distance, a
         # sink or kept first tokens: prompt portions that fill a 128-row tile go to the tcgen05 kernel
-        self.big_tiles = (self.general is not None and self.hv == self.hk and self.dv == self.d == 128
+        self.big_tiles = (self.general is not None and self.hv == self.hk and self.dv == self.d and self.d in (64, 128)
                           and spec.twin is None and not (spec.weights == "sigmoid" and (self.extras or spec.score_cap))
                           and self.out_scale == 1.0 and not self.talking)
         # scores mixed across heads: prompt portions on heads of 128 go to the tcgen05 kernel for whole key rows (of one key

@@ -574,6 +574,76 @@ def test_parts_added_up(shape, parts):
             assert torch.equal(ops.BranchSum(plus, ops.PickedRows(rows, pick, coef)).tensor(), coef * rows.float() + d)
 
 
+# ------------------------------------------------------------------------------- heads of 64 on the tcgen05 prompt kernel
+@pytest.mark.parametrize("hq,hk,page", [(4, 1, 16), (16, 1, 8), (6, 2, 64), (3, 3, 128), (10, 2, 32)])
+@pytest.mark.parametrize("option", ["plain", "window", "chunk", "kept, capped", "sigmoid", "shaped"])
+def test_heads_of_64_of_prompts(hq, hk, page, option):
+    """Whole tiles of 128 rows and a part of one (heads that do not divide 128 leave rows over), contexts and ends on and off the edges
+    of key tiles, an output of wider rows; places that no query sees hold NaN, pages before them are missing."""
+    ops = _ops()
+    d, scale, g = 64, 0.2, hq // hk
+    window, keep, mask, cap = (130, 0, 130, 0.0) if option == "window" else (100, 5, 100, 6.0) if option == "kept, capped" else \
+        (0, 0, -192 if option == "chunk" else 0, 0.0)
+    ctx, new = [0, 127, 300, 5], [1, 130, 129, 300]
+    n, widest = len(ctx), -(-max(c + m for c, m in zip(ctx, new)) // page)
+    k_pool, v_pool = (torch.full((n * widest, page, hk, d), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    table = torch.randperm(n * widest, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(n, widest).cuda()
+
+    def first(pos):
+        return max(0, pos - mask + 1) if mask > 0 else pos - pos % -mask if mask < 0 else 0
+    keys, values = [], []
+    for e, (c, m) in enumerate(zip(ctx, new)):
+        k, v = (_rand(c + m, hk, d, seed=10 * i + e, dtype=torch.bfloat16) for i in (1, 2))
+        at = torch.arange(c + m, device="cuda")
+        there = at[(at >= first(c)) | (at < keep)]
+        k_pool[table[e, there // page].long(), there % page] = k[there]
+        v_pool[table[e, there // page].long(), there % page] = v[there]
+        pages = torch.arange(widest, device="cuda")
+        table[e, (pages * page >= keep) & ((pages + 1) * page <= first(c))] = -1
+        keys.append(k.double())
+        values.append(v.double())
+    tokens, per = sum(new), 128 // g
+    q = _rand(tokens, hq * d + 8, seed=9, dtype=torch.bfloat16)
+    out = torch.full((tokens, hq * d + 16), float("nan"), device="cuda", dtype=torch.bfloat16)
+    cu = torch.tensor([0] + new, device="cuda").cumsum(0).to(torch.int32)
+    work = torch.tensor([(e, i) for e in range(n) for i in range(0, new[e], per)], dtype=torch.int32, device="cuda")
+    extra = {}
+    if option == "sigmoid":
+        extra = dict(sigmoid=True, bias=_rand(hq, seed=5))
+    elif option == "shaped":
+        extra = dict(head_scale=1.0 + 0.3 * _rand(hq, seed=5), dist_bias=_rand(hq, 37, seed=6), sink=_rand(hq, seed=7), out_scale=1.5)
+    assert ops.attn_tcgen05_supports(torch.bfloat16, d, hq, hk, page, mask)
+    ops.attn_tcgen05(q, q.stride(0), out[:, 8:8 + hq * d], k_pool, v_pool, table, cu,
+                     torch.tensor(ctx, dtype=torch.int32, device="cuda"), work, work.shape[0], hq, hk, d, scale, window=mask, keep=keep,
+                     score_cap=cap, **extra)
+    ops.check_status()
+    assert bool(out[:, :8].isnan().all()) and bool(out[:, 8 + hq * d:].isnan().all())
+    row = 0
+    for e, (c, m) in enumerate(zip(ctx, new)):
+        pos, at = c + torch.arange(m, device="cuda"), torch.arange(c + m, device="cuda")
+        low = torch.tensor([first(int(x)) for x in pos], device="cuda")
+        hidden = (at[None] > pos[:, None]) | ((at[None] < low[:, None]) & (at[None] >= keep))
+        k, v = (x.repeat_interleave(g, 1) for x in (keys[e], values[e]))
+        score = torch.einsum("thd,jhd->htj", q[row:row + m, :hq * d].view(m, hq, d).double(), k) * scale
+        if option == "shaped":
+            score = score * extra["head_scale"].double()[:, None, None] + \
+                extra["dist_bias"].double()[:, (pos[:, None] - at[None]).clamp(0, 36)]
+        if cap:
+            score = cap * torch.tanh(score / cap)
+        if option == "sigmoid":
+            p = torch.sigmoid(score + extra["bias"].double()[:, None, None]).masked_fill(hidden[None], 0.0)
+        else:
+            score = score.masked_fill(hidden[None], float("-inf"))
+            if option == "shaped":
+                score = torch.cat([score, extra["sink"].double()[:, None, None].expand(-1, m, 1)], 2)
+            p = score.softmax(2)[:, :, :c + m] * extra.get("out_scale", 1.0)
+        want, weight = torch.einsum("htj,jhd->thd", p, v), torch.einsum("htj,jhd->thd", p, v.abs())
+        # the weights and the result are rounded to 16 bits (2^-9 each, a sum of such weights as much again)
+        bound = 1.5 * 2.0 ** -8 * weight + 2.0 ** -8 * want.abs() + 1e-5
+        assert bool(((out[row:row + m, 8:8 + hq * d].view(m, hq, d).double() - want).abs() <= bound).all())
+        row += m
+
+
 # ------------------------------------------------------------------------------- keys of decoded tokens cut evenly
 @pytest.mark.parametrize("hq,hk,splits", [(4, 1, 1), (4, 1, 3), (40, 2, 7), (3, 3, 64)])
 @pytest.mark.parametrize("mask,keep,sigmoid", [(0, 0, False), (100, 5, False), (-128, 0, True)])
