@@ -19,9 +19,8 @@
 //                            n <- keep n + take k, den = max(|n . q|, exp(-m')) + 1e-6,
 //                            w = keep (every channel), k <- take k, r = q, no removal term; n is one more column
 //                            of the state whose value is 1, so n . q is that column's output, and o is divided by
-//                            den when the heads are normed          (jv_memory_gates: a scan over m alone, one warp a
-//                                                                    head, an add and a max a token; then all tokens
-//                                                                    at once)
+//                            den when the heads are normed          (jv_memory_gates: a scan over m alone; then all
+//                                                                    tokens at once)
 //
 // The columns of S evolve independently of one another, so the scan is parallel over (entry, head, value column) and
 // serial over an entry's tokens; a thread keeps its state elements in registers from the entry's first token to its last,
@@ -120,61 +119,87 @@ __global__ void __launch_bounds__(128) gla_prepare_kernel(const T* __restrict__ 
   }
 }
 
-// The gates of the matrix memory in two kernels.  (1) One warp per (entry, head) scans the running maximum: the two
-// log gates of 32 tokens are formed side by side, one per lane, then the chain m' = max(f + m, i), which is all that
-// is serial, runs over the lanes in order (an add and a max a token).  gates: [n, heads, 4] = (keep, take, m', -);
+// The gates of the matrix memory in two kernels.  (1) A block per (entry, head) scans the running maximum.  A run of tokens takes m to
+// max(F + m, I) with numbers F and I of its own, and two runs one behind the other to one: a thread forms those of its GATE_PER
+// tokens, the threads' are put together in a scan over the block, and each thread then goes through its tokens from the m that it starts
+// with.  (The chain token by token, an add and a max each behind two shuffles: 2,048 tokens of 8 heads 58.4 us, 11.2 so.)
+// gates: [n, heads, 4] = (keep, take, m', -);
 // the fourth place receives n . q from the scan.  state_m: [slots][heads], rows `slot_stride` floats apart.
-template <typename T, typename W>
-__global__ void __launch_bounds__(32) gate_scan_kernel(const T* __restrict__ proj, long long stride, int i_off, int f_off,
-                                                       const W* __restrict__ i_bias, const W* __restrict__ f_bias,
-                                                       float cap, float* __restrict__ gates, float* __restrict__ state_m,
-                                                       long long slot_stride, const int* __restrict__ cu_seqlens,
-                                                       const int* __restrict__ slots, int n_slots, int heads,
-                                                       int* __restrict__ status) {
+constexpr int GATE_PER = 4;
+
+template <int WARPS, typename T, typename W>
+__global__ void __launch_bounds__(32 * WARPS) gate_scan_kernel(const T* __restrict__ proj, long long stride, int i_off, int f_off,
+                                                               const W* __restrict__ i_bias, const W* __restrict__ f_bias,
+                                                               float cap, float* __restrict__ gates, float* __restrict__ state_m,
+                                                               long long slot_stride, const int* __restrict__ cu_seqlens,
+                                                               const int* __restrict__ slots, int n_slots, int heads,
+                                                               int* __restrict__ status) {
+  __shared__ float2 runs[2][WARPS];                     // of the warps; a tile of tokens uses one half, the next the other
   pdl_trigger();
   pdl_wait();
-  const int entry = blockIdx.x, h = blockIdx.y, lane = threadIdx.x;
+  const int entry = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int t0 = cu_seqlens[entry], t1 = cu_seqlens[entry + 1];
   const int slot = slots[entry];
   if (slot < 0 || slot >= n_slots) {
-    if (lane == 0) atomicOr(status, JV_STATUS_BAD_ROW);
+    if (tid == 0) atomicOr(status, JV_STATUS_BAD_ROW);
     return;
   }
   float* sm = state_m + (size_t)slot * slot_stride + h;
   float m = *sm;
   const float ib = to_f32(i_bias[h]), fb = to_f32(f_bias[h]);
-  auto fetch = [&](int t, float& zi, float& zf) {
-    if (t < t1) {
-      const T* row = proj + (size_t)t * stride;
-      zi = to_f32(row[i_off + h]);
-      zf = to_f32(row[f_off + h]);
+  T zi[GATE_PER], zf[GATE_PER];
+  auto fetch = [&](int base) {
+#pragma unroll
+    for (int j = 0; j < GATE_PER; ++j) {
+      const T* row = proj + (size_t)min(base + tid * GATE_PER + j, max(t0, t1 - 1)) * stride;
+      zi[j] = row[i_off + h];
+      zf[j] = row[f_off + h];
     }
   };
-  float zi_n = 0.f, zf_n = 0.f;
-  fetch(t0 + lane, zi_n, zf_n);
-  for (int base = t0; base < t1; base += 32) {
-    const int t = base + lane;
-    const float zi = zi_n, zf = zf_n;
-    fetch(t + 32, zi_n, zf_n);                          // the next group's loads fly while this one is computed
-    // a lane without a token leaves the maximum as it is: f = 0, i = -inf
-    const float gi = t < t1 ? cap * tanhf((zi + ib) / cap) : -INFINITY;
-    const float gf = t < t1 ? log_sigmoid(cap * tanhf((zf + fb) / cap)) : 0.f;
-    float before = 0.f, after = 0.f;
+  if (t0 < t1) fetch(t0);
+  int half = 0;
+  for (int base = t0; base < t1; base += 32 * WARPS * GATE_PER, half ^= 1) {
+    const int t = base + tid * GATE_PER;
+    float gi[GATE_PER], gf[GATE_PER], F = 0.f, I = -INFINITY;
 #pragma unroll
-    for (int l = 0; l < 32; ++l) {
-      const float f = __shfl_sync(0xffffffffu, gf, l), i = __shfl_sync(0xffffffffu, gi, l);
-      const float m_new = fmaxf(f + m, i);
-      if (lane == l) { before = m; after = m_new; }
-      m = m_new;
+    for (int j = 0; j < GATE_PER; ++j) {                // a token that is not there leaves the maximum as it is: f = 0, i = -inf
+      gi[j] = t + j < t1 ? cap * tanhf((to_f32(zi[j]) + ib) / cap) : -INFINITY;
+      gf[j] = t + j < t1 ? log_sigmoid(cap * tanhf((to_f32(zf[j]) + fb) / cap)) : 0.f;
+      F += gf[j];
+      I = fmaxf(I + gf[j], gi[j]);
     }
-    if (t < t1) {
-      float* out = gates + ((size_t)t * heads + h) * 4;
-      out[0] = expf(gf + before - after);
-      out[1] = expf(gi - after);
+    if (base + 32 * WARPS * GATE_PER < t1) fetch(base + 32 * WARPS * GATE_PER);     // the next tile's loads fly meanwhile
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {                  // runs up to and including this lane's
+      const float Fb = __shfl_up_sync(0xffffffffu, F, o), Ib = __shfl_up_sync(0xffffffffu, I, o);
+      if (lane >= o) {
+        I = fmaxf(Ib + F, I);
+        F += Fb;
+      }
+    }
+    if (lane == 31) runs[half][warp] = make_float2(F, I);
+    __syncthreads();
+    float before = m;                                   // behind the warps before this one
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      const float2 r = runs[half][w];
+      if (w < warp) before = fmaxf(r.x + before, r.y);
+      m = fmaxf(r.x + m, r.y);
+    }
+    const float Fb = __shfl_up_sync(0xffffffffu, F, 1), Ib = __shfl_up_sync(0xffffffffu, I, 1);
+    if (lane > 0) before = fmaxf(Fb + before, Ib);
+#pragma unroll
+    for (int j = 0; j < GATE_PER; ++j) {
+      if (t + j >= t1) break;
+      const float after = fmaxf(gf[j] + before, gi[j]);
+      float* out = gates + ((size_t)(t + j) * heads + h) * 4;
+      out[0] = expf(gf[j] + before - after);
+      out[1] = expf(gi[j] - after);
       out[2] = after;
+      before = after;
     }
   }
-  if (lane == 0) *sm = m;
+  if (tid == 0) *sm = m;
 }
 
 // (2) Per token and head, all at once: packed [n, heads, 3, D] = (q * q_scale, take * k, keep in every channel).
@@ -962,7 +987,9 @@ JV_EXPORT int jv_memory_gates(const void* proj, int dtype, long long stride, int
                               int* status, cudaStream_t stream) {
   if (entries == 0 || n == 0) return JV_OK;
   JV_DISPATCH_DTYPE(dtype, T, JV_DISPATCH_DTYPE(w_dtype, W, {
-    const int rc = jv_launch(gate_scan_kernel<T, W>, dim3(entries, heads), dim3(32), 0, stream, (const T*)proj, stride,
+    // one warp where every entry has one token (whose gates are the same either way)
+    auto kern = n <= entries ? gate_scan_kernel<1, T, W> : gate_scan_kernel<4, T, W>;
+    const int rc = jv_launch(kern, dim3(entries, heads), dim3(n <= entries ? 32 : 128), 0, stream, (const T*)proj, stride,
                              i_off, f_off, (const W*)i_bias, (const W*)f_bias, cap, gates, state_m, slot_stride,
                              cu_seqlens, slots, n_slots, heads, status);
     if (rc != JV_OK || packed == nullptr || (work != nullptr && n_work == 0)) return rc;

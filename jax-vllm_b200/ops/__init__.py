@@ -1967,44 +1967,42 @@ def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
     return out
 
 
-# `chunk_scan` goes through a portion's tokens in order, so it is taken where portions are long and where its two-warp blocks, one
-# per portion, head and 32 value columns, keep the device busy for as long as the longest portion takes: tokens * heads * strips /
-# longest of them are at work on average.  With fewer the scan in segments is faster, the more so the fewer key channels a state has
-# (chunks take the same time for up to 64).  A layer, chunks / segments in us, by keys and blocks at work:
-#   up to 32   2,048 tokens 128 blocks 379 / 330; 300 tokens 86 / 88
-#   64         2,000 and 5 tokens 64 blocks 342 / 252; 1,500 and 600 90 blocks 272 / 234; 2,048 100 blocks 469 / 430; 48 and 82 102
-#              blocks 49 / 84, 555 and 945 186 / 193, 1,517 and 2,579 461 / 412; 803, 1,365 and 1,928 136 blocks 373 / 414
-#   128        2,000 and 5 64 blocks 432 / 395; 1,500 and 600 90 blocks 346 / 395; 2,048 92 blocks 463 / 582
+# `chunk_scan` is three launches whose work lies side by side, so portions of any number of tokens and heads keep the device busy; below
+# CHUNK_SCAN_MIN_TOKENS a portion the token-by-token scan's one launch is as fast (a layer of 32 heads of 64 x 64, 100 tokens: 43 us,
+# of which the chunks are 20; memories of 4 heads of 64 x 128, 1,000 tokens: 45, in segments 96).
 CHUNK_SCAN_MIN_TOKENS = 64
+CHUNK_SCAN_MAX_KEY = 256
+CHUNK_SCAN_TOKENS = 128           # of a chunk (csrc/chunk_scan.cu)
+
+
+def chunk_scan_takes(row: torch.Tensor, offsets, n_entries: int, dim: int, columns: int, n_tokens: int | None = None) -> bool:
+    """Whether `chunk_scan` takes these sizes and is the better choice for `n_entries` portions of `n_tokens` tokens (all rows if
+    not given): 16-bit rows whose heads start on 16-byte boundaries, keys of up to 256 and values in steps of 8, enough
+    tokens a portion."""
+    tokens = row.shape[0] if n_tokens is None else n_tokens
+    return (n_entries >= 1 and row.dtype == torch.bfloat16 and tokens >= CHUNK_SCAN_MIN_TOKENS * n_entries
+            and 8 <= dim <= CHUNK_SCAN_MAX_KEY and dim % 8 == 0 and columns % 8 == 0 and row.stride(1) == 1
+            and row.stride(0) % 8 == 0 and all((row.data_ptr() + 2 * o) % 16 == 0 for o in offsets))
 
 
 def chunk_scan_min_blocks(dim: int) -> int:
     return 160 if dim <= 32 else 101 if dim <= 64 else 80
 
 
-CHUNK_SCAN_MAX_KEY = 128
-
-
 def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, dim: int, columns: int,
                         n_tokens: int | None = None, longest: int = 0) -> bool:
-    """Whether `chunk_scan` takes these sizes and is the better choice for `n_entries` portions of `n_tokens` tokens (all rows if
-    not given), the longest of `longest` (0: all alike): 16-bit rows whose heads start on 16-byte boundaries, keys of up to 128 in
-    steps of 8, values in steps of 8, enough tokens a portion and enough blocks at work."""
-    if n_entries < 1:
-        return False
+    """`chunk_scan_takes`, and blocks of 32 value columns that go through the portions side by side, the longest of `longest` tokens
+    (0: all alike), would keep `chunk_scan_min_blocks` multiprocessors at work."""
     tokens = row.shape[0] if n_tokens is None else n_tokens
-    longest = longest or -(-tokens // n_entries)
-    return (row.dtype == torch.bfloat16 and tokens >= CHUNK_SCAN_MIN_TOKENS * n_entries and 8 <= dim <= CHUNK_SCAN_MAX_KEY
-            and tokens * heads * -(-columns // 32) >= chunk_scan_min_blocks(dim) * longest
-            and dim % 8 == 0 and columns % 8 == 0 and row.stride(1) == 1 and row.stride(0) % 8 == 0
-            and all((row.data_ptr() + 2 * o) % 16 == 0 for o in offsets))
+    return (chunk_scan_takes(row, offsets, n_entries, dim, columns, n_tokens) and dim <= 128
+            and tokens * heads * -(-columns // 32) >= chunk_scan_min_blocks(dim) * (longest or -(-tokens // n_entries)))
 
 
 def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor, cu_seqlens: torch.Tensor,
                slots: torch.Tensor, n_entries: int, heads: int, groups: int, dim: int, columns: int, scale: float = 1.0,
                gates: torch.Tensor | None = None, state_n: torch.Tensor | None = None, dt_raw: torch.Tensor | None = None,
                dt_bias: torch.Tensor | None = None, a_log: torch.Tensor | None = None, portions: int = 0) -> torch.Tensor:
-    """S <- a S + g k v^T and o = scale * S^T q with one decay a and one step g a head and token, 32 tokens at a time
+    """S <- a S + g k v^T and o = scale * S^T q with one decay a and one step g a head and token, 128 tokens at a time
     (csrc/chunk_scan.cu): the mixers' scan (`mamba_prepare` or the second half of `memory_gates`, then `state_scan`) for portions
     of many tokens.  `row` [n, ..] bfloat16 holds q and k (`groups` of `dim`, shared by heads // groups heads each) and v (`heads` of
     `columns`).  Either `gates` [n, heads, 4] (keep, take, ..) with `state_n` as for `state_scan`, or the raw step sizes `dt_raw`
@@ -2035,14 +2033,19 @@ def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: tor
             raise KernelError("chunk_scan: the step sizes do not fit")
         w_code = _code(dt_bias, "dt_bias")
     out = torch.empty((n, heads * columns), dtype=torch.float32, device=row.device)
+    taken = portions or n_entries
+    n_taken = n - (n_entries - taken)                    # tokens of the portions: the others have one each
+    scratch = torch.empty((n_taken // CHUNK_SCAN_TOKENS + taken) * heads * (dim * columns + dim + 1), dtype=torch.float32, device=row.device)
     f = _fn("chunk_scan", "jv_chunk_scan", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_float, c_void_p,
                                             c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
-                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                            c_void_p])
     base = row.data_ptr()
     _check(f(base + 2 * q_off, row.stride(0), base + 2 * k_off, row.stride(0), base + 2 * v_off, row.stride(0), heads // groups,
              float(scale), _ptr(gates), _ptr(dt_raw), 0 if dt_raw is None else dt_raw.stride(0), _ptr(dt_bias), _ptr(a_log), w_code,
              out.data_ptr(), state.data_ptr(), state.stride(0), _ptr(state_n), cu_seqlens.data_ptr(), slots.data_ptr(),
-             state.shape[0], n_entries, heads, dim, columns, portions, _status_ptr(row.device), _stream()), "chunk_scan")
+             state.shape[0], n_entries, heads, dim, columns, portions, n_taken, scratch.data_ptr(), _status_ptr(row.device),
+             _stream()), "chunk_scan", launches=3)
     return out
 
 

@@ -156,8 +156,8 @@ class MatrixMemory(_StateMixer):
         mats = hd * self.dv
         where, state_n = (state, step.cu_seqlens, step.state_slots), state[:, mats:mats + hd]
         work, singles = step.decode_work
-        chunks = ops.chunk_scan_supports(row, (0, hd, 2 * hd), step.n_entries - singles, h, self.d, self.dv,
-                                         n_tokens=step.n_tokens - singles, longest=max(step.host_q_lens, default=0))
+        chunks = ops.chunk_scan_takes(row, (0, hd, 2 * hd), step.n_entries - singles, self.d, self.dv,
+                                      n_tokens=step.n_tokens - singles)
         packed, gates = ops.memory_gates(row, 0, hd, 2 * hd + 2 * hv, 2 * hd + 2 * hv + h, self.i_bias, self.f_bias,
                                          self.spec.gate_cap, self.d ** -0.5, state[:, mats + hd:], step.cu_seqlens,
                                          step.state_slots, step.n_entries, h, self.d, gates_only=chunks and not singles,

@@ -94,8 +94,7 @@ class StateSpace(Part):
         dt_raw = row[:, 2 * inner + 2 * gn:2 * inner + 2 * gn + self.h]
         where, (work, singles) = (state, step.cu_seqlens, step.state_slots), step.decode_work
         prepare = (xbc, inner, inner + gn, dt_raw, self.dt_bias, self.a_log, self.h, self.g, self.n)
-        if ops.chunk_scan_supports(xbc, (0, inner, inner + gn), step.n_entries - singles, self.h, self.n, self.e,
-                                   n_tokens=step.n_tokens - singles, longest=max(step.host_q_lens, default=0)):
+        if ops.chunk_scan_takes(xbc, (0, inner, inner + gn), step.n_entries - singles, self.n, self.e, n_tokens=step.n_tokens - singles):
             o = ops.chunk_scan(xbc, inner + gn, inner, 0, *where, step.n_entries, self.h, self.g, self.n, self.e, dt_raw=dt_raw,
                                dt_bias=self.dt_bias, a_log=self.a_log, portions=step.n_entries - singles if singles else 0)
             if singles:                     # decoded tokens beside the portions

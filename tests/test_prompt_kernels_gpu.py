@@ -220,6 +220,46 @@ def test_chunked_states_later_infinity_stays_out_of_earlier_outputs():
     assert left[:, [3, 6]].all() and left.sum() == 2 * dim
 
 
+@pytest.mark.parametrize("heads,dim,columns", [(3, 8, 72), (2, 24, 8), (2, 64, 64), (1, 136, 128), (2, 256, 520)])
+def test_chunked_states_over_several_chunks(heads, dim, columns):
+    """Portions that end at, before and after the edges of chunks, some passed by; a value that is no number stays in its
+    column and out of earlier outputs, over the chunks that follow too."""
+    ops, lengths = _ops(), [128, 1, 129, 300, 1, 256, 15]
+    cu, slots, n_slots = _entries(lengths)
+    n, hd, hv, portions = sum(lengths), heads * dim, heads * columns, sum(m > 1 for m in lengths)
+    row = _rand(n, 2 * hd + hv, seed=1, dtype=torch.bfloat16)
+    gates = 0.5 + 0.5 * torch.rand(n, heads, 4, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    rows = _rand(n_slots, hd * columns + hd, seed=3)
+    bad = int(cu[3]) + 140                               # in the second chunk of 300 tokens
+    row[bad, 2 * hd + 5] = float("inf")
+    runs = []
+    for chunked in (True, False):
+        st, g = rows.clone(), gates.clone()
+        if chunked:
+            o = ops.chunk_scan(row, 0, hd, 2 * hd, st, cu, slots, len(lengths), heads, heads, dim, columns, scale=dim ** -0.5, gates=g,
+                               state_n=st[:, hd * columns:], portions=portions)
+            ops.check_status()
+        else:
+            q, k = (row[:, i * hd:(i + 1) * hd].float().view(n, heads, dim) for i in range(2))
+            packed = torch.stack([q * dim ** -0.5, g[:, :, 1:2] * k, g[:, :, :1].expand(n, heads, dim)], 2).contiguous()
+            o = ops.state_scan(packed, row, 2 * hd, st, cu, slots, len(lengths), columns, state_n=st[:, hd * columns:], gates=g, segment=0)
+        runs.append((o, st, g[:, :, 3]))
+    taken = torch.cat([torch.full((m,), m > 1, device="cuda") for m in lengths])
+    (o, st, nq), (o_want, st_want, nq_want) = runs
+    for e, m in enumerate(lengths):
+        s = int(slots[e])
+        if m == 1:
+            assert torch.equal(st[s], rows[s])
+            st[s] = st_want[s]
+    finite = torch.isfinite(o_want)
+    assert torch.equal(torch.isfinite(o)[taken], finite[taken]) and not finite[bad:int(cu[4]), 5].any() and finite[:bad].all()
+    left = torch.isfinite(st_want)
+    assert torch.equal(torch.isfinite(st), left)
+    for got, want in ((o[taken & finite.all(1)], o_want[taken & finite.all(1)]), (st[left], st_want[left]), (nq[taken], nq_want[taken])):
+        # two 32-bit sums of up to 300 + 256 terms
+        assert (got.double() - want.double()).norm() <= 3e-6 * want.double().norm()
+
+
 # ------------------------------------------------------- convolution and finish of the state-space mixer
 @pytest.mark.parametrize("taps", [2, 3, 4])
 @pytest.mark.parametrize("channels,off", [(8192, 0), (8196, 4), (8192, 2), (512, 0)])
