@@ -17,7 +17,7 @@
 // (group, head), fully parallel, and group_scan_kernel reads them through a ring of bulk copies.
 //
 // What bounds it is that chain's latency (0.5 us a group whatever the number of heads up to two blocks a multiprocessor).
-// 2,048 tokens of 32 heads of 64: prepare 40 and scan 258 us, where the token-by-token kernels took 69 and 815; 64 heads: 77 and 258.
+// 2,048 tokens of 32 heads of 64: prepare 40 and scan 201 us, where the token-by-token kernels took 69 and 815; 64 heads: 77 and 258.
 #include "mbarrier.cuh"
 #include "scan.cuh"
 
@@ -169,27 +169,30 @@ struct GroupScanParams {
   int* status;
 };
 
-// A block takes 16 value columns of one (entry, head), a warp eight of them; eight lanes share a pair of columns, lane kl the
-// channels 32 i + 4 kl .. + 3 (i < KPT / 4), so that a 16-byte read of eight lanes is a run of 128 bytes.  Two columns a thread:
+// LANES lanes share a pair of value columns, lane kl the channels 4 LANES i + 4 kl .. + 3 (i < KPT / 4), so that a 16-byte read of eight
+// lanes is a run of 128 bytes; a warp takes 64 / LANES columns of one (entry, head), a block twice as many.  Two columns a thread:
 // shared memory hands out 128 bytes a clock and each number read should serve more than one multiply-add.
+// Eight lanes; 16, which halves what a warp has to do in a group for one more step of every sum over the lanes, where the blocks of eight
+// would leave multiprocessors without one and keys have 64 channels or more (32 heads of 64, 2,048 tokens: 258 us with eight, 201 with 16).
 // RING_: the stages of the ring.  Six (about 100 KB, two blocks a multiprocessor) carry a block through the latency of its copies;
 // where there are more blocks than two a multiprocessor, others do that, and two stages leave room for more of them (32 heads of 64:
 // 2,048 tokens in one entry 430 us a layer with six, 598 with two; five entries of 400 313 and 281, eight of 8 tokens 51 and 45).
-template <int KPT, int RING_> struct GroupScanShape {
-  static constexpr int DP = 8 * KPT;
+template <int LANES, int KPT, int RING_> struct GroupScanShape {
+  static constexpr int DP = LANES * KPT;
   static constexpr int FLOATS = VECS * DP + COEF;                       // of a group
-  static constexpr int GROUPS = KPT <= 8 ? 4 : KPT <= 16 ? 2 : 1;       // groups of a stage
-  static constexpr int RING = RING_, COLS = 16, THREADS = 64;
+  static constexpr int GROUPS = DP <= 64 ? 4 : DP <= 128 ? 2 : 1;       // groups of a stage
+  static constexpr int RING = RING_, THREADS = 64, COLS = 2 * 64 / LANES;
   static constexpr int VLD = GROUPS * T4 + 4;                           // values of a column in a stage, padded
   static constexpr int STAGE = GROUPS * FLOATS;
   static constexpr int SMEM = (int)sizeof(float) * (RING * STAGE + 2 * COLS * VLD);
 };
 
-template <int KPT, int RING_, typename T>
+template <int LANES, int KPT, int RING_, typename T>
 __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p) {
-  using Shape = GroupScanShape<KPT, RING_>;
+  using Shape = GroupScanShape<LANES, KPT, RING_>;
   constexpr int DP = Shape::DP, FLOATS = Shape::FLOATS, GROUPS = Shape::GROUPS, RING = Shape::RING, COLS = Shape::COLS;
-  constexpr int VLD = Shape::VLD, TOK = GROUPS * T4, Q = KPT / 4, THREADS = Shape::THREADS;
+  constexpr int VLD = Shape::VLD, TOK = GROUPS * T4, Q = KPT / 4, THREADS = Shape::THREADS, RUN = 4 * LANES, WARP_COLS = 64 / LANES;
+  constexpr int FINE = LANES / 8;                      // lanes that finish the same output
   // keys of up to 64: a group's vectors are asked for before the group before is finished (there are registers for it)
   constexpr bool AHEAD = Q <= 2;
   extern __shared__ __align__(16) float smem[];
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
   const int entry = entry_of(blockIdx.x, p.portions, p.cu_seqlens, p.n_entries);
   if (entry < 0) return;
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int kl = lane & 7, lcol = warp * 8 + (lane >> 3) * 2, base = blockIdx.z * COLS, col = base + lcol;
+  const int kl = lane % LANES, lcol = warp * WARP_COLS + lane / LANES * 2, base = blockIdx.z * COLS, col = base + lcol;
   const int D = p.D, V = p.V;
   const int t0 = p.cu_seqlens[entry], t1 = p.cu_seqlens[entry + 1];
   const int slot = p.slots[entry];
@@ -217,7 +220,7 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
     return;
   }
   float* S_g = p.state + (size_t)slot * p.slot_stride + (size_t)h * D * V;
-  auto channel = [&](int i) { return (i / 4) * 32 + kl * 4 + (i & 3); };
+  auto channel = [&](int i) { return (i / 4) * RUN + kl * 4 + (i & 3); };
   const size_t group_stride = (size_t)p.heads * FLOATS;
   const float* src = p.packed + ((size_t)g0 * p.heads + h) * FLOATS;
   // one thread asks for a stage: a bulk copy a group (copies by all threads held up the reads of shared memory behind them)
@@ -258,18 +261,18 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
       S[c][i] = pack2(col + c < V && c0 < D ? S_g[(size_t)c0 * V + col + c] : 0.f,
                       col + c < V && c1 < D ? S_g[(size_t)c1 * V + col + c] : 0.f);
     }
-  const int jo = kl >> 1, co = kl & 1;                 // the token of a group and the column whose output this lane finishes
+  const int jo = kl / FINE >> 1, co = kl / FINE & 1;   // the token of a group and the column whose output this lane finishes
   const size_t orow = (size_t)p.heads * V;
   float* o_next = p.out + (size_t)t0 * orow + (size_t)h * V + col + co + jo * orow;
-  const bool live = col + co < V;
+  const bool live = col + co < V && kl % FINE == 0;
   ulonglong2 U[T4][Q], R[T4][Q];
   auto load_ur = [&](const float* vec) {
 #pragma unroll
     for (int j = 0; j < T4; ++j)
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        U[j][q] = *reinterpret_cast<const ulonglong2*>(vec + j * DP + q * 32);
-        R[j][q] = *reinterpret_cast<const ulonglong2*>(vec + (T4 + j) * DP + q * 32);
+        U[j][q] = *reinterpret_cast<const ulonglong2*>(vec + j * DP + q * RUN);
+        R[j][q] = *reinterpret_cast<const ulonglong2*>(vec + (T4 + j) * DP + q * RUN);
       }
   };
   auto dot = [&](const ulonglong2 (&x)[Q], const uint64_t (&s)[KPT / 2]) {
@@ -321,6 +324,7 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
 #pragma unroll
           for (int c = 0; c < 2; ++c) dp[c][j] += __shfl_xor_sync(0xffffffffu, dp[c][j], m);
       };
+      if (LANES == 16) exchange(8);
       exchange(4);
       float v[2][T4];
 #pragma unroll
@@ -342,7 +346,7 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
       exchange(2);
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(vec + 4 * T4 * DP + q * 32);
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(vec + 4 * T4 * DP + q * RUN);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           S[c][2 * q] = mul2(w.x, S[c][2 * q]);
@@ -350,7 +354,7 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
         }
 #pragma unroll
         for (int j = 0; j < T4; ++j) {
-          const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(vec + (2 * T4 + j) * DP + q * 32);
+          const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(vec + (2 * T4 + j) * DP + q * RUN);
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const uint64_t vv = pack2(v[c][j], v[c][j]);
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
 #pragma unroll
       for (int j = 0; j < T4; ++j)
 #pragma unroll
-        for (int q = 0; q < Q; ++q) B[j][q] = *reinterpret_cast<const ulonglong2*>(vec + (3 * T4 + j) * DP + q * 32);
+        for (int q = 0; q < Q; ++q) B[j][q] = *reinterpret_cast<const ulonglong2*>(vec + (3 * T4 + j) * DP + q * RUN);
       if (AHEAD && more) load_ur(vec + FLOATS);
       // the p's one after the other
 #pragma unroll
@@ -393,16 +397,17 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
           }
         }
       // the outputs: eight sums over eight lanes, a lane hands on those that it does not finish
-      const bool up = kl & 4, up2 = kl & 2, up1 = kl & 1;
+      const bool up = kl & 4 * FINE, up2 = kl & 2 * FINE, up1 = kl & FINE;
       float e[4], f[2];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {                    // (token i / 2 of a half, column i & 1)
         const float lo = dr[i & 1][i >> 1], hi = dr[i & 1][2 + (i >> 1)];
-        e[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, 4);
+        e[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, 4 * FINE);
       }
 #pragma unroll
-      for (int i = 0; i < 2; ++i) f[i] = (up2 ? e[2 + i] : e[i]) + __shfl_xor_sync(0xffffffffu, up2 ? e[i] : e[2 + i], 2);
-      float o = (up1 ? f[1] : f[0]) + __shfl_xor_sync(0xffffffffu, up1 ? f[0] : f[1], 1);
+      for (int i = 0; i < 2; ++i) f[i] = (up2 ? e[2 + i] : e[i]) + __shfl_xor_sync(0xffffffffu, up2 ? e[i] : e[2 + i], 2 * FINE);
+      float o = (up1 ? f[1] : f[0]) + __shfl_xor_sync(0xffffffffu, up1 ? f[0] : f[1], FINE);
+      if (FINE > 1) o += __shfl_xor_sync(0xffffffffu, o, 1);
       const float4 rk = *reinterpret_cast<const float4*>(cf + 32 + jo * 4), rb = *reinterpret_cast<const float4*>(cf + 48 + jo * 4);
       const float ok[T4] = {rk.x, rk.y, rk.z, rk.w}, ob[T4] = {rb.x, rb.y, rb.z, rb.w};
 #pragma unroll
@@ -433,10 +438,10 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
     }
 }
 
-template <int KPT, int RING, typename T>
+template <int LANES, int KPT, int RING, typename T>
 int launch_ring(const GroupScanParams& p, int entries, cudaStream_t stream) {
-  using Shape = GroupScanShape<KPT, RING>;
-  auto kern = group_scan_kernel<KPT, RING, T>;
+  using Shape = GroupScanShape<LANES, KPT, RING>;
+  auto kern = group_scan_kernel<LANES, KPT, RING, T>;
   static bool done[JV_MAX_DEVICES] = {};
   if (!jv_once_per_device(done, [&] {
         return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM) == cudaSuccess;
@@ -447,9 +452,12 @@ int launch_ring(const GroupScanParams& p, int entries, cudaStream_t stream) {
 
 template <int KPT, typename T>
 int launch_scan(const GroupScanParams& p, int entries, cudaStream_t stream) {
-  constexpr int COLS = GroupScanShape<KPT, 6>::COLS;
+  constexpr int COLS = GroupScanShape<8, KPT, 6>::COLS;
   const long long blocks = (long long)entries * p.heads * ((p.V + COLS - 1) / COLS);
-  return blocks > 2 * jv_multiprocessors() ? launch_ring<KPT, 2, T>(p, entries, stream) : launch_ring<KPT, 6, T>(p, entries, stream);
+  if constexpr (KPT >= 8) {
+    if (blocks <= jv_multiprocessors()) return launch_ring<16, KPT / 2, 6, T>(p, entries, stream);
+  }
+  return blocks > 2 * jv_multiprocessors() ? launch_ring<8, KPT, 2, T>(p, entries, stream) : launch_ring<8, KPT, 6, T>(p, entries, stream);
 }
 
 int padded(int D) { return D <= 32 ? 32 : D <= 64 ? 64 : D <= 128 ? 128 : 256; }
