@@ -132,6 +132,14 @@ template <typename T> __device__ __forceinline__ void store_four(T* p, const flo
   }
 }
 
+// 1 / x to 2^-23 (1 / inf = 0): for results that are rounded to 16 bits right away.  The dozen instructions of a division were what a
+// long portion waited for: 4,096 tokens of 10,240 channels 84 us with it, 54 so.
+__device__ __forceinline__ float approx_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
+  return y;
+}
+
 template <typename TI, typename TO, typename TW, int TAPS>
 __global__ void __launch_bounds__(THREADS) short_conv_vec_kernel(const ConvParams p) {
   constexpr int K = TAPS - 1, RAW = VEC * sizeof(TI) / 4;
@@ -216,7 +224,7 @@ __global__ void __launch_bounds__(THREADS) short_conv_vec_kernel(const ConvParam
         for (int k = 0; k + 1 < K; ++k) win[k][v] = win[k + 1][v];
         win[K - 1][v] = x;
         y[v] = p.residual ? x + acc : acc + bias[v];
-        if (p.act == 1) y[v] = y[v] / (1.f + expf(-y[v]));
+        if (p.act == 1) y[v] = sizeof(TO) == 2 ? y[v] * approx_rcp(1.f + expf(-y[v])) : y[v] / (1.f + expf(-y[v]));
       }
       store_four<TO>(out + (size_t)(i + u) * p.out_stride, y);
     }
