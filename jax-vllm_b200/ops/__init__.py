@@ -1056,17 +1056,18 @@ def attn_rows_decode(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache:
 
 # --------------------------------------------------------------------------- linear
 def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
-    """x [M, K] times weight [N, K] transposed, accumulated in float32 on CUDA cores."""
+    """x [M, K] times weight [N, K] transposed, as exact as in float32 on CUDA cores (csrc/gemm_f32.cu).  The weight is read before
+    the kernels launched before this one have finished: none of them may write it."""
     _cuda(x, "x", contiguous=False); _cuda(weight, "weight")
     if x.dim() != 2 or weight.dim() != 2 or x.shape[1] != weight.shape[1] or x.stride(1) != 1:
         raise KernelError(f"gemm shapes {tuple(x.shape)} x {tuple(weight.shape)}^T do not fit")
     m, k = x.shape
     n = weight.shape[0]
     y = torch.empty((m, n), dtype=out_dtype, device=x.device)
-    f = _fn("gemm_simt", "jv_gemm_tn_simt", [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
-                                             c_int, c_int, c_int, c_void_p])
+    f = _fn("gemm_f32", "jv_gemm_f32", [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
+                                        c_int, c_int, c_int, c_void_p, c_void_p])
     _check(f(x.data_ptr(), _code(x, "x"), x.stride(0), weight.data_ptr(), _code(weight, "weight"), weight.stride(0),
-             y.data_ptr(), _code(y, "out"), y.stride(0), m, n, k, _stream()), "gemm_simt")
+             y.data_ptr(), _code(y, "out"), y.stride(0), m, n, k, _status_ptr(x.device), _stream()), "gemm_f32")
     return y
 
 
@@ -1240,8 +1241,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     """y = x @ weight.T.  With `parts_ok` the result may be a PartialSum (the caller hands it to `rmsnorm`,
     `residual_add` or `swiglu`, which add its parts as they read them).
 
-    float32 weights: the CUDA-core product of this package in true 32-bit (16-bit activations are read as they
-    are and widened inside).  bfloat16 weights and activations: up to STREAM_BEST_ROWS rows (decoding) the
+    float32 weights: the product of this package as exact as 32-bit multiply-adds (csrc/gemm_f32.cu; 16-bit activations
+    are read as they are).  bfloat16 weights and activations: up to STREAM_BEST_ROWS rows (decoding) the
     weight-streaming product on tcgen05 (csrc/linear_stream.cu), which cuts the k of a weight with few strips into
     parts; where the reader wants one tensor and the strips are few, the mma.sync product (csrc/linear_skinny.cu, up
     to SKINNY_MAX_ROWS rows), whose strips are 16 rows; else (prompts) cuBLAS through torch.mm.  All
@@ -1376,7 +1377,7 @@ def gate_heads(o: torch.Tensor, gate: torch.Tensor | None) -> torch.Tensor:
 def bmm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """One product per head: out[h] = a[h] @ w[h].T, a [heads, n, k] (any strides with unit inner stride),
     w [heads, m, k] contiguous, out [heads, n, m] (made contiguous if not given; given, any strides with unit
-    inner stride).  float32 operands: the CUDA-core product of this package (csrc/gemm_simt.cu);
+    inner stride).  float32 operands: the 32-bit product of this package (csrc/gemm_f32.cu);
     bfloat16: the library's batched product (as the prompt products of this package are the library's)."""
     _cuda(a, "a", contiguous=False); _cuda(w, "w", a.dtype)
     heads, n, k = a.shape
@@ -1395,11 +1396,12 @@ def bmm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None)
     _cuda(out, "out", a.dtype, contiguous=False)
     if out.shape != (heads, n, m) or out.stride(2) != 1:
         raise KernelError("out does not fit the batched product")
-    f = _fn("gemm_simt", "jv_gemm_tn_simt_batched", [c_void_p, c_int, c_int, c_longlong, c_void_p, c_int, c_int, c_longlong,
-                                                    c_void_p, c_int, c_int, c_longlong, c_int, c_int, c_int, c_int,
-                                                    c_void_p])
+    f = _fn("gemm_f32", "jv_gemm_f32_batched", [c_void_p, c_int, c_int, c_longlong, c_void_p, c_int, c_int, c_longlong,
+                                                c_void_p, c_int, c_int, c_longlong, c_int, c_int, c_int, c_int,
+                                                c_void_p, c_void_p])
     _check(f(a.data_ptr(), _code(a, "a"), a.stride(1), a.stride(0), w.data_ptr(), _code(w, "w"), w.stride(1), w.stride(0),
-             out.data_ptr(), _code(out, "out"), out.stride(1), out.stride(0), n, m, k, heads, _stream()), "bmm_heads")
+             out.data_ptr(), _code(out, "out"), out.stride(1), out.stride(0), n, m, k, heads, _status_ptr(a.device),
+             _stream()), "bmm_heads")
     return out
 
 

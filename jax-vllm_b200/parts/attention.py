@@ -21,7 +21,7 @@ from .registry import POSITIONS, build, register_mixer
 
 
 class Attention(Part):
-    kernels = ("rope_kv", "attn_simt", "gemm_simt")
+    kernels = ("rope_kv", "attn_simt", "gemm_f32")
 
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx
@@ -41,7 +41,7 @@ class Attention(Part):
         # bfloat16 with a head size the tensor-core kernels are built for; else the CUDA-core kernel
         self.use_mma = ops.attn_mma_supports(ctx.dtype, self.d)
         if self.use_mma:
-            self.kernels = ("rope_kv", "attn_mma", "gemm_simt", "linear_skinny")
+            self.kernels = ("rope_kv", "attn_mma", "gemm_f32", "linear_skinny")
             if self.d in (64, 128):
                 self.kernels += ("attn_tcgen05",) + (("attn_decode_tcgen05",) if self.d == 128 else ())
         self.w_qkv = self.w_o = self.q_norm = self.k_norm = None

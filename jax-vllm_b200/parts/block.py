@@ -61,7 +61,7 @@ class PreNormBlock(Part):
         self.gate_b = [None, None]
         self.packed = [None, None]        # per sublayer: its input matrix with the gate's stacked under it
         if gates is not None:
-            self.kernels = self.kernels + ("dyt", "gemm_simt")
+            self.kernels = self.kernels + ("dyt", "gemm_f32")
 
     def parts(self):
         return tuple(part for part in (self.mixer_norm, self.mixer, self.ffn_norm, self.feed_forward) if part is not None)

@@ -14,7 +14,7 @@ from .registry import register_feed_forward
 
 
 class DenseMLP(Part):
-    kernels = ("activation", "gemm_simt")
+    kernels = ("activation", "gemm_f32")
 
     def __init__(self, spec, prefix, ctx):
         self.poly = spec.activation == "poly_norm"
@@ -22,7 +22,7 @@ class DenseMLP(Part):
             raise ValueError(f"feed-forward: activation {spec.activation!r} is not built "
                              f"({', '.join(ops.UNARY_ACTIVATIONS)} and poly_norm are)")
         if self.poly:
-            self.kernels = ("poly_norm", "gemm_simt")
+            self.kernels = ("poly_norm", "gemm_f32")
         self.spec, self.ctx = spec, ctx
         self.prefix = f"{prefix}.{spec.prefix}" if spec.prefix else prefix
         self.in_rows = self.heads_out = spec.intermediate_size

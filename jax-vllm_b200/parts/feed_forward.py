@@ -16,7 +16,7 @@ from .registry import register_feed_forward
 
 
 class GatedMLP(Part):
-    kernels = ("activation", "gemm_simt")
+    kernels = ("activation", "gemm_f32")
     BLOCK = 128          # gate/up interleaving of the fused product (a tile of it is 256 columns wide)
 
     def __init__(self, spec, prefix, ctx):
@@ -46,7 +46,7 @@ class GatedMLP(Part):
         self.block = None
         if self.ctx.dtype == torch.bfloat16 and g.dtype == torch.bfloat16 and inter % self.BLOCK == 0 and hidden % 8 == 0:
             self.block = self.BLOCK
-            self.kernels = ("activation", "gemm_simt", "gemm_tcgen05", "linear_skinny")
+            self.kernels = ("activation", "gemm_f32", "gemm_tcgen05", "linear_skinny")
             self.w_gate_up = torch.stack([g.reshape(-1, self.BLOCK, hidden), u.reshape(-1, self.BLOCK, hidden)],
                                          dim=1).reshape(2 * inter, hidden).contiguous()
         else:

@@ -62,7 +62,7 @@ def distance_buckets(buckets: int, saturate: int) -> list:
 
 
 class GeneralAttention(Part):
-    kernels = ("attn_prepare", "attn_simt", "attn_finish", "gemm_simt")
+    kernels = ("attn_prepare", "attn_simt", "attn_finish", "gemm_f32")
     FOREVER = 1 << 30
 
     def __init__(self, spec, prefix, ctx):

@@ -34,7 +34,7 @@ from .registry import POSITIONS, build, register_mixer
 
 
 class LatentAttention(Part):
-    kernels = ("latent_prepare", "attn_simt", "gemm_simt")
+    kernels = ("latent_prepare", "attn_simt", "gemm_f32")
 
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx
@@ -59,9 +59,9 @@ class LatentAttention(Part):
         # other row sizes in bfloat16: the tensor-core kernels written for latent rows (key = the row, value = its start)
         self.use_latent_mma = not self.use_mma and ops.attn_latent_mma_supports(ctx.dtype, self.dk, self.dc)
         if self.use_latent_mma:
-            self.kernels = ("latent_prepare", "attn_latent_mma", "attn_latent_tcgen05", "gemm_simt", "linear_skinny")
+            self.kernels = ("latent_prepare", "attn_latent_mma", "attn_latent_tcgen05", "gemm_f32", "linear_skinny")
         if self.use_mma:
-            self.kernels = ("latent_prepare", "attn_mma", "gemm_simt", "linear_skinny")
+            self.kernels = ("latent_prepare", "attn_mma", "gemm_f32", "linear_skinny")
             if self.dk == 128:
                 self.kernels += ("attn_tcgen05", "attn_decode_tcgen05")
         if self.dq is not None:

@@ -18,7 +18,7 @@ from .registry import register_mixer
 
 
 class MinGRU(Part):
-    kernels = ("min_gru", "gemm_simt")
+    kernels = ("min_gru", "gemm_f32")
 
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx

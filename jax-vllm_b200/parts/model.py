@@ -72,7 +72,7 @@ class Model(Part):
         self.lm_head = self.compute_weight(head, self.ctx).contiguous()
 
     def kernels(self):
-        names = {"embed", "norm", "gemm_simt"}
+        names = {"embed", "norm", "gemm_f32"}
         names.update(getattr(self.final_norm, "kernels", ()))
         if self.pass_table is not None or self.spec.pass_vectors is not None:
             names.add("dyt")

@@ -27,7 +27,7 @@ from .registry import register_mixer
 
 
 class _StateMixer(Part):
-    kernels = ("recurrent", "state_step", "gemm_simt")
+    kernels = ("recurrent", "state_step", "gemm_f32")
 
     def _bind_in(self, tensors, keys):
         mats = [self.compute_weight(tensors[self.names[k]], self.ctx) for k in keys]

@@ -33,7 +33,7 @@ from .registry import register_feed_forward
 
 
 class RoutedExperts(Part):
-    kernels = ("moe_route", "moe_gemm_simt", "gemm_simt")
+    kernels = ("moe_route", "moe_gemm_simt", "gemm_f32")
 
     def __init__(self, spec, prefix, ctx):
         if spec.activation not in ("gelu", "clamped_glu", "swiglu"):
@@ -48,7 +48,7 @@ class RoutedExperts(Part):
         if spec.activation == "clamped_glu" and not spec.limit > 0:
             raise ValueError("routed experts: the clamped activation needs a positive limit")
         if self.gated:
-            self.kernels = ("moe_route", "moe_gemm_simt", "gemm_simt", "activation")
+            self.kernels = ("moe_route", "moe_gemm_simt", "gemm_f32", "activation")
         if self.by_table and (spec.correction is not None or spec.identity):
             raise ValueError("routed experts: a table knows no correction and no identity experts")
         # the router's experts: those with tensors, then the identity experts
@@ -100,7 +100,7 @@ class RoutedExperts(Part):
         self.w_up = torch.stack(ups).contiguous()
         self.w_down = torch.stack(downs).contiguous()
         if self._tensor_cores():
-            self.kernels = ("moe_route", "gemm_tcgen05", "linear_stream", "gemm_simt") + (("activation",) if self.gated else ())
+            self.kernels = ("moe_route", "gemm_tcgen05", "linear_stream", "gemm_f32") + (("activation",) if self.gated else ())
         if self.shared is not None:
             self.shared.bind(tensors)
             self.kernels += tuple(k for k in self.shared.kernels if k not in self.kernels)

@@ -24,7 +24,7 @@ from .registry import register_mixer
 
 
 class StateSpace(Part):
-    kernels = ("short_conv", "mamba2", "recurrent", "state_step", "chunk_scan", "gemm_simt")
+    kernels = ("short_conv", "mamba2", "recurrent", "state_step", "chunk_scan", "gemm_f32")
 
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx

@@ -16,7 +16,7 @@ from .registry import register_token_input
 
 
 class TokenInput(Part):
-    kernels = ("token_input", "gemm_simt")
+    kernels = ("token_input", "gemm_f32")
 
     def __init__(self, spec, prefix, ctx):
         self.spec, self.ctx = spec, ctx

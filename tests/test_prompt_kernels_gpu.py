@@ -614,6 +614,35 @@ def test_parts_added_up(shape, parts):
             assert torch.equal(ops.BranchSum(plus, ops.PickedRows(rows, pick, coef)).tensor(), coef * rows.float() + d)
 
 
+# ------------------------------------------------------------------------------- the 32-bit product in parts of 16 bits
+@pytest.mark.parametrize("m,n,k", [(17, 129, 96), (64, 384, 1024), (65, 1024, 640), (128, 2304, 260), (129, 1536, 1056), (257, 1000, 4096)])
+def test_tiles_and_parts_of_the_32bit_product(m, n, k):
+    """Edges of the tiles of rows, strips with and without parts of k, a last part that is shorter."""
+    ops = _ops()
+    x, w = _rand(m, k, seed=m), _rand(n, k, seed=n + k)
+    y, want = ops.gemm_simt(x, w, torch.float32), x.double() @ w.double().T
+    assert ((y.double() - want).abs() <= (k + 2) * EPS32 * (x.double().abs() @ w.double().abs().T)).all()
+    for first, rows in ((0, 1), (m - 16, 16), (m // 2, 1), (3, m - 5)):
+        assert torch.equal(ops.gemm_simt(x[first:first + rows], w, torch.float32), y[first:first + rows])
+
+
+@pytest.mark.parametrize("m", [3, 40])
+def test_product_32bit_of_infinities(m):
+    """An infinity, a NaN and numbers next to the largest give what multiply-adds give, and stay in their rows and columns."""
+    ops, n, k = _ops(), 70, 300
+    x, w = _rand(m, k, seed=1), _rand(n, k, seed=2)
+    x[0, 7], w[5, 11], x[1, 3], w[6, 200], x[2, 290] = float("inf"), float("-inf"), float("nan"), 3.4e38, 3.3e38
+    y, want = ops.gemm_simt(x, w, torch.float32), x.double() @ w.double().T
+    plain = torch.zeros(m, n, device="cuda")
+    for i in range(k):
+        plain = plain + x[:, i:i + 1] * w[:, i]
+    # where two of them meet, a product that overflows by itself need not in a multiply-add
+    y[0, 6] = plain[0, 6] = y[1, 6] = plain[1, 6] = y[2, 5] = plain[2, 5] = y[2, 6] = plain[2, 6] = want[2, 6] = 0.0
+    assert torch.equal(y.isnan(), plain.isnan()) and torch.equal(y.isinf(), plain.isinf()) and torch.equal(y[y.isinf()], plain[plain.isinf()])
+    fine = torch.isfinite(plain) & (want.abs() < 1e30)
+    assert ((y.double() - want)[fine].abs() <= (k + 2) * EPS32 * (x.double().abs() @ w.double().abs().T)[fine]).all()
+
+
 # ------------------------------------------------------------------------------- heads of 64 on the tcgen05 prompt kernel
 @pytest.mark.parametrize("hq,hk,page", [(4, 1, 16), (16, 1, 8), (6, 2, 64), (3, 3, 128), (10, 2, 32)])
 @pytest.mark.parametrize("option", ["plain", "window", "chunk", "kept, capped", "sigmoid", "shaped"])
