@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_decode_tcgen05_kernel(const _
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- mma issuer
-    if (lane == 0) {
+    if (elect_one()) {
       auto issue_qk = [&](int t, const Cursor& c) -> bool {      // S^T[t % 2] = K_t Q^T
         const int s = t % STAGES, sp = c.seg & 1;
         if ((t == 0 || c.j == 0) && !mbar_wait(&sh->q_full[sp], (c.seg >> 1) & 1)) return false;
@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_decode_tcgen05_kernel(const _
   if (sh->failed) {
     // a wait ran out: products already issued may still write tensor memory and copies already asked for still land
     // in this block's shared memory; both get a bounded time to finish before tensor memory is freed and the block ends
-    if (warp == 1 && lane == 0) drain_products_after_failure(&sh->drain);
+    if (warp == 1 && elect_one()) drain_products_after_failure(&sh->drain);
     if ((warp == 0 || warp == 6) && lane == 0) {
       const int which = warp == 6;
       for (int s = 0; s < STAGES; ++s)

@@ -45,13 +45,6 @@ constexpr int MAX_LISTED = 16;                  // rounds whose item a block loo
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr uint32_t IDESC_PV0 = IDESC_PV & ~(0x3Fu << 17);      // without the number of columns
 
-// One thread of a converged warp.  The compiler sees that a branch on it leaves a single thread.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t one;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-  return one != 0;
-}
-
 struct Params {
   __nv_bfloat16* out; int out_stride;
   const int* block_table; int table_width;
@@ -522,7 +515,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_latent_tcgen05_kernel(const _
   if (sh->failed) {
     // a wait ran out: products already issued may still write tensor memory and copies already asked for still land in this
     // block's shared memory; both get a bounded time to finish before tensor memory is freed and the block ends
-    if (warp == 1 && lane == 0) drain_products_after_failure(&sh->drain);
+    if (warp == 1 && elect_one()) drain_products_after_failure(&sh->drain);
     if (warp == 0 && lane == 0) {
       if (sh->armed_q >= 0) drain_copies_after_failure(&sh->q_full, sh->armed_q);
       for (int s = 0; s < stages; ++s)

@@ -277,52 +277,50 @@ __global__ void __launch_bounds__(THREADS, 1) attn_rows_tcgen05_kernel(const __g
     if (!ok && lane == 0) { atomicOr(p.status, JV_STATUS_WAIT_EXPIRED); sh->failed = 1; }
   } else if (warp == 1) {
     // -------------------------------------------------------------- mma issuer
-    // The whole warp walks through the tiles; lane 0 takes a tile's stages of keys and issues the products.
+    // The whole warp walks through the tiles; one thread issues the products.
     const uint64_t q_desc = desc_k_major(smem_u32(q_s)), rq_desc = desc_k_major(smem_u32(r_s));
     const uint64_t k_desc = desc_k_major(smem_u32(r_s), GROUP_BYTES);
     const uint64_t v_desc = desc_mn_major(smem_u32(r_s), GROUP_BYTES / 2, GROUP_BYTES);
     int s_at = 0, s_ph = 0;             // the next stage and the parity of its phase
     auto next_stage = [&]() { if (++s_at == STAGES) { s_at = 0; s_ph ^= 1; } };
     auto wait = [&](uint64_t* bar, int parity) -> bool { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); };
-    auto issue_qk_lane = [&](int n, int j, int n_tiles, int gt) -> bool {   // S[gt % 2] = sum_c Q_c K_c^T
-      if (j == 0 && !mbar_wait(&sh->q_full[ONE ? 1 : n % QB], (n / QB) & 1)) return false;
+    auto issue_qk = [&](int n, int j, int n_tiles, int gt) -> bool {   // S[gt % 2] = sum_c Q_c K_c^T
+      if (j == 0 && !wait(&sh->q_full[ONE ? 1 : n % QB], (n / QB) & 1)) return false;
       const uint32_t tmem_s = tmem + (gt & 1) * 128;
       const uint64_t q_item = q_desc + (uint64_t)(((n % QB) * KEPT * TILE_BYTES) >> 4);
 #pragma unroll (NCT > 0 ? NCT : 1)
       for (int cc = 0; cc < NC; ++cc) {
         const int c = cc + 1 == NC ? 0 : cc + 1;
-        if (ONE && j == 0 && c == 0 && !mbar_wait(&sh->q_full[0], n & 1)) return false;
+        if (ONE && j == 0 && c == 0 && !wait(&sh->q_full[0], n & 1)) return false;
         uint64_t q0 = q_item + (uint64_t)((c * TILE_BYTES) >> 4);
         int sq = -1;
         if (NCT == 0 && c >= KEPT) {
           sq = s_at;
-          if (!mbar_wait(&sh->full[sq], s_ph)) return false;
+          if (!wait(&sh->full[sq], s_ph)) return false;
           next_stage();
           q0 = rq_desc + (uint64_t)((sq * TILE_BYTES) >> 4);
         }
         const int s = s_at;
-        if (!mbar_wait(&sh->full[s], s_ph)) return false;
+        if (!wait(&sh->full[s], s_ph)) return false;
         next_stage();
         TC_FENCE_AFTER();
         const uint64_t k0 = k_desc + (uint64_t)((s * TILE_BYTES) >> 4);
         const uint64_t q1 = q0 + (HALF_BYTES >> 4), k1 = k0 + (GROUP_BYTES / 2 >> 4);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) umma(tmem_s, q0 + 2 * kk, k0 + 2 * kk, IDESC_QK, (cc | kk) != 0);
+          for (int kk = 0; kk < 4; ++kk) umma(tmem_s, q0 + 2 * kk, k0 + 2 * kk, IDESC_QK, (cc | kk) != 0);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) umma(tmem_s, q1 + 2 * kk, k1 + 2 * kk, IDESC_QK, 1);
-        if (sq >= 0) umma_commit(&sh->empty[sq]);
-        umma_commit(&sh->empty[s]);
+          for (int kk = 0; kk < 4; ++kk) umma(tmem_s, q1 + 2 * kk, k1 + 2 * kk, IDESC_QK, 1);
+          if (sq >= 0) umma_commit(&sh->empty[sq]);
+          umma_commit(&sh->empty[s]);
+          if (cc + 1 == NC) {
+            if (ONE && j == n_tiles - 1) umma_commit(&sh->q_free[1]);     // the other pieces have been used for the last time
+            umma_commit(&sh->s_full[gt & 1]);
+          }
+        }
+        __syncwarp();
       }
-      if (ONE && j == n_tiles - 1) umma_commit(&sh->q_free[1]);     // the other pieces have been used for the last time
-      umma_commit(&sh->s_full[gt & 1]);
       return true;
-    };
-    auto issue_qk = [&](int n, int j, int n_tiles, int gt) -> bool {
-      bool fine = true;
-      if (lane == 0) fine = issue_qk_lane(n, j, n_tiles, gt);
-      s_at = __shfl_sync(0xffffffffu, s_at, 0);
-      s_ph = __shfl_sync(0xffffffffu, s_ph, 0);
-      return __all_sync(0xffffffffu, fine);
     };
     bool ok = true;
     int r = 0, n = 0, gt = 0;
@@ -360,7 +358,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_rows_tcgen05_kernel(const __g
         if (!wait(&sh->p_full[gt & 1], (gt >> 1) & 1)) { ok = false; break; }
         // an item's first product overwrites the output of the item before it, which its softmax threads must have read
         if (j == 0 && n > 0 && !wait(&sh->o_free, (n - 1) & 1)) { ok = false; break; }
-        if (lane == 0) {
+        if (elect_one()) {
           TC_FENCE_AFTER();
           // O += P V : 8 steps of 16 keys; P from tensor memory (8 columns a step), two 8-row groups down V
           const uint32_t tmem_p = tmem + TMEM_P + (gt & 1) * 64;
@@ -558,7 +556,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_rows_tcgen05_kernel(const __g
   if (sh->failed) {
     // a wait ran out: products already issued may still write tensor memory and copies already asked for still land in this
     // block's shared memory; both get a bounded time to finish before tensor memory is freed and the block ends
-    if (warp == 1 && lane == 0) drain_products_after_failure(&sh->drain);
+    if (warp == 1 && elect_one()) drain_products_after_failure(&sh->drain);
     if (warp == 0 && lane == 0) {
       for (int b = 0; b < 2; ++b)
         if (sh->armed_q[b] >= 0) drain_copies_after_failure(&sh->q_full[b], sh->armed_q[b]);

@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
     if (!ok && lane == 0) { atomicOr(p.status, JV_STATUS_WAIT_EXPIRED); sh->failed = 1; }
   } else if (warp == 1) {
     // -------------------------------------------------------------- mma issuer
-    if (lane == 0) {
+    if (elect_one()) {
       uint64_t q_desc[Q_BUFFERS][2], k_desc[K_STAGES][2], v_desc[V_STAGES];
 #pragma unroll
       for (int b = 0; b < Q_BUFFERS; ++b) {
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
   if (sh->failed) {
     // a wait ran out: products already issued may still write tensor memory and copies already asked for still land
     // in this block's shared memory; both get a bounded time to finish before tensor memory is freed and the block ends
-    if (warp == 1 && lane == 0) drain_products_after_failure(&sh->drain);
+    if (warp == 1 && elect_one()) drain_products_after_failure(&sh->drain);
     if (warp == 0 && lane == 0) {
       for (int b = 0; b < Q_BUFFERS; ++b)
         if (sh->armed_q[b] >= 0) drain_copies_after_failure(&sh->q_full[b], sh->armed_q[b]);

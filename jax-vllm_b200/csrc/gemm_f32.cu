@@ -77,13 +77,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&a)[4],
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n"
                ::"r"(taddr), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]) : "memory");
 }
-__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory"); }
-// True for one thread of a warp that is whole: the compiler then knows that what follows is one thread's work.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t one;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
-  return one != 0;
-}
 // Every thread of every block of the cluster; what they wrote before is seen by all after.
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
@@ -268,7 +261,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     }
   } else if (warp == S::ISSUER) {
     // ------------------------------------------------------------- products
-    // (the whole warp takes every turn and one elected thread issues: behind `lane == 0` a product took 62 clocks to issue)
+    // (the whole warp takes every turn and one elected thread issues)
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(rows16 >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
     const uint64_t a_desc = smem_desc(smem_u32(stages));
     Place<STAGES> at;
@@ -390,7 +383,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   TC_FENCE_BEFORE();
   __syncthreads();
   if (sh->failed) {                                    // products and copies under way get a bounded time to finish
-    if (warp == S::ISSUER && lane == 0) drain_products_after_failure(&sh->drain);
+    if (warp == S::ISSUER && elect_one()) drain_products_after_failure(&sh->drain);
     if (TMA && warp == S::BRINGER && lane == 0)
       for (int c = max(0, brought - RAW); c < brought; ++c) {
         drain_copies_after_failure(&sh->w_full[c % RAW], (c / RAW) & 1);

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tcgen05_kernel(const __grid_c
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- mma issuer
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0, phase = 0, it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_tcgen05_kernel(const __grid_c
   if (sh->failed) {
     // a wait ran out: products already issued may still write tensor memory and copies already asked for still land
     // in this block's shared memory; both get a bounded time to finish before tensor memory is freed and the block ends
-    if (warp == 1 && lane == 0) drain_products_after_failure(&sh->drain);
+    if (warp == 1 && elect_one()) drain_products_after_failure(&sh->drain);
     if (warp == 0 && lane == 0)
       for (int s = 0; s < STAGES; ++s)
         if (sh->armed[s] >= 0) drain_copies_after_failure(&sh->full[s], sh->armed[s]);

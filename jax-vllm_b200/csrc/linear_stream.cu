@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- mma issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // bfloat16 x bfloat16 -> float, both operands K-major, M = 128, N = rows of x rounded up to 16
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.rows16 >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       int s = 0, phase = 0, n = 0;
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_stream_kernel(const __grid_
   if (sh->failed) {
     // a wait ran out: products already issued may still write tensor memory and copies already asked for still land
     // in this block's shared memory; both get a bounded time to finish before tensor memory is freed and the block ends
-    if (warp == 1 && lane == 0) drain_products_after_failure(&sh->drain);
+    if (warp == 1 && elect_one()) drain_products_after_failure(&sh->drain);
     if (warp == 0 && lane == 0)
       for (int s = 0; s < p.stages; ++s)
         if (sh->armed[s] >= 0) drain_copies_after_failure(&sh->full[s], sh->armed[s]);

@@ -46,6 +46,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, int parity, long long c
   return true;
 }
 
+// True for one thread of a converged warp.  The compiler sees that a branch on it leaves a single thread: a tcgen05.mma behind
+// `lane == 0` took 62 clocks to issue, behind this 12, which a product of few rows (some 40 clocks of work) does not hide: the
+// 12 weight-streaming products of a decode step of four layers of width 2,048, eight rows, 67.7 us before and 57.9 so, the grouped ones
+// of one token 17.7 and 13.1, decode attention 68.9 and 66.3.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+  return one != 0;
+}
+
 // Arrives on `bar` once every tcgen05.mma that this thread has issued so far has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
