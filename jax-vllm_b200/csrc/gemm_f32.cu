@@ -221,7 +221,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     mbar_expect_tx(&sh->w_full[s], BM * Eight<TW>::ROW_BYTES);
     tma_load_3d(raw + s * S::RAW_STAGE, &w_map, k0 + c * CHUNK, n0, blockIdx.y, &sh->w_full[s]);
   };
-  if (warp == S::BRINGER && lane == 0) {
+  if (warp == S::BRINGER && elect_one()) {
     for (int s = 0; s < RAW; ++s) { mbar_init(&sh->w_full[s], 1); mbar_init(&sh->a_full[s], 1); mbar_init(&sh->raw_empty[s], GROUP); }
     for (int s = 0; s < STAGES; ++s) { mbar_init(&sh->full[s], GROUP); mbar_init(&sh->empty[s], 1); }
     for (int b = 0; b < ACCS; ++b) { mbar_init(&sh->acc_full[b], 1); mbar_init(&sh->acc_empty[b], S::ADDERS); }
@@ -239,12 +239,12 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   TC_FENCE_AFTER();
   pdl_trigger();                                       // not before this block has its tensor memory
   const uint32_t tmem = __shfl_sync(0xffffffffu, sh->tmem_base, 0), tmem_w = tmem + ACCS * NB;
-  int brought = 0;                                     // chunks that have been asked for, by the thread that does it
+  int brought = 0;                                     // chunks that have been asked for, in the thread that does it
   bool ok = true;
 
   if (warp == S::BRINGER) {
     // ------------------------------------------------------------- rows as they are: zeros past K, N and M
-    if (TMA && lane == 0) {
+    if (TMA && elect_one()) {
       auto bring_a = [&](int c, int s) {
         mbar_expect_tx(&sh->a_full[s], p.row_tile * Eight<TA>::ROW_BYTES);
         tma_load_3d(raw + s * S::RAW_STAGE + S::W_RAW, &a_map, k0 + c * CHUNK, m0, blockIdx.y, &sh->a_full[s]);
@@ -384,7 +384,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   __syncthreads();
   if (sh->failed) {                                    // products and copies under way get a bounded time to finish
     if (warp == S::ISSUER && elect_one()) drain_products_after_failure(&sh->drain);
-    if (TMA && warp == S::BRINGER && lane == 0)
+    if (TMA && warp == S::BRINGER && brought > 0)
       for (int c = max(0, brought - RAW); c < brought; ++c) {
         drain_copies_after_failure(&sh->w_full[c % RAW], (c / RAW) & 1);
         drain_copies_after_failure(&sh->a_full[c % RAW], (c / RAW) & 1);
