@@ -24,10 +24,10 @@
 // in the tensor core: 3.4e-7 relative for 128 channels, this way 0.8e-7, as token by token).  L is summed in 64-bit and kept as two
 // floats: L_t - L_s keeps its digits behind a large decay.  The normaliser's sums are made on the CUDA cores.
 //
-// What bounds it: the two kernels on the tensor cores, their rate of mma.sync (one a 2.2 clocks and multiprocessor at best; 4.7 and 6.1
-// here), the middle one its bytes.  4,096 tokens in three entries, 128 heads of 128 x 64: 115, 55 and 286 us; chunks of 32 that a
-// block went through in order took 620.  2,048 tokens of 8 heads of 128 x 256 with a normaliser: 19, 9 and 41, where a scan token by token
-// in segments took 276; 2,000 tokens of 8 heads of 256 x 512: 58, 18 and 149 (888).  1,200 tokens of 64 heads of 128 x 64: 84 (172).
+// What bounds it: the two kernels on the tensor cores, their rate of mma.sync (one a 2.2 clocks and multiprocessor at best; 4.7 and 5.5
+// here), the middle one its bytes.  4,096 tokens in three entries, 128 heads of 128 x 64: 115, 55 and 259 us; chunks of 32 that a
+// block went through in order took 620.  2,048 tokens of 8 heads of 128 x 256 with a normaliser: 19, 9 and 39, where a scan token by token
+// in segments took 276; 2,000 tokens of 8 heads of 256 x 512: 58, 18 and 150 (888).  1,200 tokens of 64 heads of 128 x 64: 81 (172).
 #include "scan.cuh"
 #include <math.h>
 
@@ -340,22 +340,25 @@ __global__ void __launch_bounds__(START_THREADS) chunk_start_kernel(const ChunkP
 constexpr int OUT_THREADS = 256;           // a warp 16 of the chunk's tokens
 
 template <int DP> struct OutShape {
-  static constexpr int LD = DP + 8, DB = DP / 2;       // S_0 passes by in two blocks of channels, where k lay
-  static constexpr int SMEM = (2 * CT * LD + CT * LV) * 2 + (int)sizeof(Weights) + VT * 4;
-  static_assert(3 * DB * LV <= CT * LD, "a block of S_0 in three parts has to fit k's place");
+  static constexpr int LD = DP + 8, DB = DP / 2;       // S_0 passes by in two blocks of channels
+  static constexpr bool KEEP = DP <= 128;              // a warp's queries stay in registers, and S_0 passes by where they lay
+  static constexpr int ROWS = 2 * CT * LD + CT * LV + (KEEP ? 0 : 3 * DB * LV);
+  static constexpr int SMEM = ROWS * 2 + (int)sizeof(Weights) + VT * 4;
+  static_assert(!KEEP || 3 * DB * LV <= CT * LD, "a block of S_0 in three parts has to fit q's place");
 };
 
 template <int DP>
 __global__ void __launch_bounds__(OUT_THREADS, DP <= 128 ? 2 : 1) chunk_output_kernel(const ChunkParams p) {
   using Shape = OutShape<DP>;
   constexpr int LD = Shape::LD, DB = Shape::DB, KT = DP / 16;
-  constexpr bool KEEP = DP <= 128;                     // a warp's queries stay in registers while it goes through the scores
+  constexpr bool KEEP = Shape::KEEP;
   extern __shared__ __align__(16) unsigned char raw[];
   Weights& w = *reinterpret_cast<Weights*>(raw);
   bf16* qs = reinterpret_cast<bf16*>(raw + sizeof(Weights));           // [CT][LD]
-  bf16* ks = qs + CT * LD;                                              // [CT][LD], then [3][DB][LV] of S_0
+  bf16* ks = qs + CT * LD;                                              // [CT][LD]
   bf16* xs = ks + CT * LD;                                              // [CT][LV]
-  int* bad = reinterpret_cast<int*>(xs + CT * LV);
+  bf16* ss = KEEP ? qs : xs + CT * LV;                                  // [3][DB][LV]: a block of S_0
+  int* bad = reinterpret_cast<int*>(qs + Shape::ROWS);
   pdl_trigger();
   pdl_wait();
   Chunk c;
@@ -394,13 +397,80 @@ __global__ void __launch_bounds__(OUT_THREADS, DP <= 128 ? 2 : 1) chunk_output_k
   for (int j = 0; j < 8; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e) O[j][e] = 0.f;
-  if (at_work) {
-    // what the chunk's own tokens give
-    uint32_t qa[KEEP ? KT : 1][4];
-    if (KEEP) {
+  const float fa = w.from_start[ta], fb = w.from_start[tb];
+  uint32_t qa[KEEP ? KT : 1][4];
+  if (KEEP) {
 #pragma unroll
-      for (int kk = 0; kk < KT; ++kk) ldsm(qa[KEEP ? kk : 0], qs + (tm + lr + (lm & 1) * 8) * LD + kk * 16 + (lm >> 1) * 8);
+    for (int kk = 0; kk < KT; ++kk) ldsm(qa[KEEP ? kk : 0], qs + (tm + lr + (lm & 1) * 8) * LD + kk * 16 + (lm >> 1) * 8);
+  }
+  const bool counts = p.state_n != nullptr && e0 == 0 && at_work;
+  if (counts) {
+    // the normaliser: q . n_0 here, the sums of the weighted scores further down
+    float na = 0.f, nb = 0.f;
+    const float* n0 = p.starts_n + at * p.D;
+    for (int d = gq * 2; d < p.D; d += 8) {
+      const float2 n = *reinterpret_cast<const float2*>(n0 + d);
+      const uint32_t a = *reinterpret_cast<const uint32_t*>(qs + ta * LD + d), b = *reinterpret_cast<const uint32_t*>(qs + tb * LD + d);
+      na = fmaf(__uint_as_float(a << 16), n.x, fmaf(__uint_as_float(a & 0xffff0000u), n.y, na));
+      nb = fmaf(__uint_as_float(b << 16), n.x, fmaf(__uint_as_float(b & 0xffff0000u), n.y, nb));
     }
+    sum_a = fa * na;
+    sum_b = fb * nb;
+  }
+  // What the state before the chunk gives: exp(L_t) q S_0.  First, since all warps have as much of it: behind what the chunk's own tokens
+  // give, of which the last warp has eight times the first one's, its barriers made every warp wait for the last (286 us where this order takes 259).
+#pragma unroll (KEEP ? 2 : 1)
+  for (int first = 0; first < DP; first += DB) {
+    if (first >= p.D) break;
+    if (KEEP || first > 0) __syncthreads();            // the queries (or the block before) have been read
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int j = tid + i * OUT_THREADS, d = j / (VT / 4), e = j % (VT / 4) * 4;
+      if (j < DB * (VT / 4)) {
+        uint2 part[3];
+        cut3(s0[i].x, s0[i].y, part[0].x, part[1].x, part[2].x);
+        cut3(s0[i].z, s0[i].w, part[0].y, part[1].y, part[2].y);
+#pragma unroll
+        for (int z = 0; z < 3; ++z) *reinterpret_cast<uint2*>(ss + (z * DB + d) * LV + e) = part[z];
+      }
+    }
+    if (first + DB < p.D) fetch(first + DB);
+    __syncthreads();
+    if (at_work) {
+#pragma unroll
+      for (int kk = 0; kk < DB / 16; ++kk) {
+        uint32_t a[4];
+        if (KEEP) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a[i] = qa[KEEP ? first / 16 + kk : 0][i];
+        } else {
+          ldsm(a, qs + (tm + lr + (lm & 1) * 8) * LD + first + kk * 16 + (lm >> 1) * 8);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j += 4) {
+          float f[4][4];
+#pragma unroll
+          for (int z = 2; z >= 0; --z) {
+            uint32_t b[2][4];
+#pragma unroll
+            for (int v = 0; v < 2; ++v) ldsm_t(b[v], ss + (z * DB + kk * 16 + lr + (lm & 1) * 8) * LV + (j + 2 * v) * 8 + (lm >> 1) * 8);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              if (z == 2) mma<true>(f[u], a, b[u >> 1][2 * (u & 1)], b[u >> 1][2 * (u & 1) + 1]);
+              else mma<false>(f[u], a, b[u >> 1][2 * (u & 1)], b[u >> 1][2 * (u & 1) + 1]);
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) add(O[j + u], f[u]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) { O[j][0] *= fa; O[j][1] *= fa; O[j][2] *= fb; O[j][3] *= fb; }
+  if (!at_work) return;
+  // what the chunk's own tokens give
+  {
     const float2 La = w.L[ta], Lb = w.L[tb];
 #pragma unroll 1
     for (int sn = 0; sn <= tm; sn += 16) {
@@ -433,34 +503,23 @@ __global__ void __launch_bounds__(OUT_THREADS, DP <= 128 ? 2 : 1) chunk_output_k
         cut3(b0, b1, m[0][2 * j + 1], m[1][2 * j + 1], m[2][2 * j + 1]);
       }
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        uint32_t b[4];
-        ldsm_t(b, xs + (sn + lr + (lm & 1) * 8) * LV + j * 8 + (lm >> 1) * 8);
-        float f[2][4];
+      for (int j = 0; j < 8; j += 4) {
+        uint32_t b[2][4];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) mma<true>(f[u], m[2], b[2 * u], b[2 * u + 1]);
+        for (int v = 0; v < 2; ++v) ldsm_t(b[v], xs + (sn + lr + (lm & 1) * 8) * LV + (j + 2 * v) * 8 + (lm >> 1) * 8);
+        float f[4][4];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) mma<false>(f[u], m[1], b[2 * u], b[2 * u + 1]);
+        for (int u = 0; u < 4; ++u) mma<true>(f[u], m[2], b[u >> 1][2 * (u & 1)], b[u >> 1][2 * (u & 1) + 1]);
 #pragma unroll
-        for (int u = 0; u < 2; ++u) mma<false>(f[u], m[0], b[2 * u], b[2 * u + 1]);
-        add(O[j], f[0]);
-        add(O[j + 1], f[1]);
+        for (int u = 0; u < 4; ++u) mma<false>(f[u], m[1], b[u >> 1][2 * (u & 1)], b[u >> 1][2 * (u & 1) + 1]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mma<false>(f[u], m[0], b[u >> 1][2 * (u & 1)], b[u >> 1][2 * (u & 1) + 1]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) add(O[j + u], f[u]);
       }
     }
   }
-  const float fa = w.from_start[ta], fb = w.from_start[tb];
-  if (p.state_n != nullptr && e0 == 0 && at_work) {
-    // the normaliser: the sums of the weighted scores, and q . n_0
-    float qa = 0.f, qb = 0.f;
-    const float* n0 = p.starts_n + at * p.D;
-    for (int d = gq * 2; d < p.D; d += 8) {
-      const float2 n = *reinterpret_cast<const float2*>(n0 + d);
-      const uint32_t a = *reinterpret_cast<const uint32_t*>(qs + ta * LD + d), b = *reinterpret_cast<const uint32_t*>(qs + tb * LD + d);
-      qa = fmaf(__uint_as_float(a << 16), n.x, fmaf(__uint_as_float(a & 0xffff0000u), n.y, qa));
-      qb = fmaf(__uint_as_float(b << 16), n.x, fmaf(__uint_as_float(b & 0xffff0000u), n.y, qb));
-    }
-    sum_a = fmaf(fa, qa, sum_a);
-    sum_b = fmaf(fb, qb, sum_b);
+  if (counts) {
 #pragma unroll
     for (int o = 1; o < 4; o <<= 1) {
       sum_a += __shfl_xor_sync(0xffffffffu, sum_a, o);
@@ -471,53 +530,6 @@ __global__ void __launch_bounds__(OUT_THREADS, DP <= 128 ? 2 : 1) chunk_output_k
       if (tb < c.here) p.nq[((size_t)(c.t0 + tb) * p.heads + h) * 4] = sum_b * p.scale;
     }
   }
-  // what the state before the chunk gives: q S_0, then exp(L_t)
-  float P[8][4];
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) P[j][e] = 0.f;
-#pragma unroll 1
-  for (int first = 0; first < p.D; first += DB) {
-    __syncthreads();                                   // k (or the block before) has been read
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int j = tid + i * OUT_THREADS, d = j / (VT / 4), e = j % (VT / 4) * 4;
-      if (j < DB * (VT / 4)) {
-        uint2 part[3];
-        cut3(s0[i].x, s0[i].y, part[0].x, part[1].x, part[2].x);
-        cut3(s0[i].z, s0[i].w, part[0].y, part[1].y, part[2].y);
-#pragma unroll
-        for (int z = 0; z < 3; ++z) *reinterpret_cast<uint2*>(ks + (z * DB + d) * LV + e) = part[z];
-      }
-    }
-    if (first + DB < p.D) fetch(first + DB);
-    __syncthreads();
-    if (at_work) {
-#pragma unroll 1
-      for (int kk = 0; kk < DB / 16; ++kk) {
-        uint32_t a[4];
-        ldsm(a, qs + (tm + lr + (lm & 1) * 8) * LD + first + kk * 16 + (lm >> 1) * 8);
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          float f[2][4];
-#pragma unroll
-          for (int z = 2; z >= 0; --z) {
-            uint32_t b[4];
-            ldsm_t(b, ks + (z * DB + kk * 16 + lr + (lm & 1) * 8) * LV + j * 8 + (lm >> 1) * 8);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              if (z == 2) mma<true>(f[u], a, b[2 * u], b[2 * u + 1]);
-              else mma<false>(f[u], a, b[2 * u], b[2 * u + 1]);
-            }
-          }
-          add(P[j], f[0]);
-          add(P[j + 1], f[1]);
-        }
-      }
-    }
-  }
-  if (!at_work) return;
   const size_t orow = (size_t)p.heads * p.V;
   float* o = p.out + (size_t)c.t0 * orow + (size_t)h * p.V + e0;
 #pragma unroll
@@ -526,11 +538,11 @@ __global__ void __launch_bounds__(OUT_THREADS, DP <= 128 ? 2 : 1) chunk_output_k
     if (e0 + lc >= p.V) continue;
     const int bad0 = bad[lc], bad1 = bad[lc + 1];
     if (ta < c.here)
-      *reinterpret_cast<float2*>(o + ta * orow + lc) = make_float2(bad0 <= ta ? NAN : fmaf(fa, P[j][0], O[j][0]) * p.scale,
-                                                                    bad1 <= ta ? NAN : fmaf(fa, P[j][1], O[j][1]) * p.scale);
+      *reinterpret_cast<float2*>(o + ta * orow + lc) = make_float2(bad0 <= ta ? NAN : O[j][0] * p.scale,
+                                                                    bad1 <= ta ? NAN : O[j][1] * p.scale);
     if (tb < c.here)
-      *reinterpret_cast<float2*>(o + tb * orow + lc) = make_float2(bad0 <= tb ? NAN : fmaf(fb, P[j][2], O[j][2]) * p.scale,
-                                                                    bad1 <= tb ? NAN : fmaf(fb, P[j][3], O[j][3]) * p.scale);
+      *reinterpret_cast<float2*>(o + tb * orow + lc) = make_float2(bad0 <= tb ? NAN : O[j][2] * p.scale,
+                                                                    bad1 <= tb ? NAN : O[j][3] * p.scale);
   }
 }
 
