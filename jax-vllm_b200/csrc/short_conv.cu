@@ -9,16 +9,15 @@
 // state[slot, j, c], j < taps - 1, holds the input at the sequence's position (tokens so far) - (taps - 1) + j; a
 // fresh slot is zero, which is the zero padding.  All arithmetic is 32-bit, whatever the types of in and out.
 //
-// A thread owns one channel of one segment of SEG tokens of one entry and slides a window of taps - 1 registers over
-// it (SEG is at least taps - 1).  Segments are counted per entry, so only an entry's first segment reads the state; the thread of that segment
+// A thread owns one channel of one segment of 8 to 32 tokens of one entry and slides a window of taps - 1 registers over
+// it (segments are at least taps - 1 long).  Segments are counted per entry, so only an entry's first segment reads the state; the thread of that segment
 // is also the ONE writer of the entry's state for its channel: it has the old state in its window before it writes
 // the new one (the entry's last taps - 1 inputs, or old state shifted where the entry is shorter), so no other
 // thread reads what it overwrites.  Blocks find their (entry, segment) from cu_seqlens; the grid is an upper bound,
-// n / SEG + entries, and blocks beyond the last segment leave.
+// n / (tokens of a segment) + entries, and blocks beyond the last segment leave.
 #include "common.cuh"
 
 namespace {
-constexpr int SEG = 32;
 constexpr int THREADS = 128;
 constexpr int BATCH = 8;       // inputs a thread asks for before it uses the first
 
@@ -29,6 +28,7 @@ struct ConvParams {
   float* state; long long state_stride;      // elements between slots
   const int* cu_seqlens; const int* slots;
   int n_entries, n_slots, channels, act, residual;
+  int seg_log2;                              // tokens of a segment (a shift: every block goes through the entries)
   int* status;
 };
 
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(THREADS) short_conv_kernel(const ConvParams p)
   int entry = -1, seg = 0, before = 0;
   for (int e = 0; e < p.n_entries; ++e) {
     const int q = p.cu_seqlens[e + 1] - p.cu_seqlens[e];
-    const int segs = (q + SEG - 1) / SEG;
+    const int segs = (q + (1 << p.seg_log2) - 1) >> p.seg_log2;
     if ((int)blockIdx.x < before + segs) { entry = e; seg = blockIdx.x - before; break; }
     before += segs;
   }
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(THREADS) short_conv_kernel(const ConvParams p)
   const int c = blockIdx.y * THREADS + threadIdx.x;
   if (c >= p.channels) return;
   const int t_begin = p.cu_seqlens[entry], q = p.cu_seqlens[entry + 1] - t_begin;
-  const int i0 = seg * SEG, i1 = min(q, i0 + SEG);
+  const int i0 = seg << p.seg_log2, i1 = min(q, i0 + (1 << p.seg_log2));
   constexpr int K = TAPS - 1;
   const int slot = K > 0 ? p.slots[entry] : 0;        // one tap keeps nothing
   if (K > 0 && (slot < 0 || slot >= p.n_slots)) {
@@ -142,14 +142,14 @@ __device__ __forceinline__ float approx_rcp(float x) {
 
 template <typename TI, typename TO, typename TW, int TAPS>
 __global__ void __launch_bounds__(THREADS) short_conv_vec_kernel(const ConvParams p) {
-  constexpr int K = TAPS - 1, RAW = VEC * sizeof(TI) / 4;
+  constexpr int K = TAPS - 1, RAW = VEC * sizeof(TI) / 4, WRAW = VEC * sizeof(TW) / 4;
   static_assert(K > 0, "one tap keeps no state");
   pdl_trigger();
   pdl_wait();
   int entry = -1, seg = 0, before = 0;
   for (int e = 0; e < p.n_entries; ++e) {
     const int q = p.cu_seqlens[e + 1] - p.cu_seqlens[e];
-    const int segs = (q + SEG - 1) / SEG;
+    const int segs = (q + (1 << p.seg_log2) - 1) >> p.seg_log2;
     if ((int)blockIdx.x < before + segs) { entry = e; seg = blockIdx.x - before; break; }
     before += segs;
   }
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(THREADS) short_conv_vec_kernel(const ConvParam
   const int c = (blockIdx.y * THREADS + threadIdx.x) * VEC;
   if (c >= p.channels) return;
   const int t_begin = p.cu_seqlens[entry], q = p.cu_seqlens[entry + 1] - t_begin;
-  const int i0 = seg * SEG, i1 = min(q, i0 + SEG);
+  const int i0 = seg << p.seg_log2, i1 = min(q, i0 + (1 << p.seg_log2));
   const int slot = p.slots[entry];
   if (slot < 0 || slot >= p.n_slots) {
     if (threadIdx.x == 0) atomicOr(p.status, JV_STATUS_BAD_ROW);
@@ -172,18 +172,32 @@ __global__ void __launch_bounds__(THREADS) short_conv_vec_kernel(const ConvParam
     for (int u = 0; u < BATCH; ++u) load_raw<TI>(ahead[u], in + (size_t)min(i + u, i1 - 1) * p.in_stride);
   };
   fetch(i0);
-  float wt[TAPS][VEC], bias[VEC], win[K][VEC];
+  float wt[TAPS][VEC], bias[VEC] = {}, win[K][VEC];
+  {
+    uint32_t raw[TAPS][WRAW];                          // TAPS weights of VEC channels, one after another
 #pragma unroll
-  for (int v = 0; v < VEC; ++v) {
+    for (int j = 0; j < TAPS; ++j) load_raw<TW>(raw[j], (const TW*)p.w + (size_t)c * TAPS + j * VEC);
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j) wt[j][v] = to_f32(((const TW*)p.w)[(size_t)(c + v) * TAPS + j]);
-    bias[v] = p.bias != nullptr ? to_f32(((const TW*)p.bias)[c + v]) : 0.f;
+    for (int e = 0; e < TAPS * VEC; ++e) wt[e % TAPS][e / TAPS] = raw_at<TW>(raw[e / VEC], e % VEC);
+    if (p.bias != nullptr) {
+      uint32_t rb[WRAW];
+      load_raw<TW>(rb, (const TW*)p.bias + c);
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) bias[v] = raw_at<TW>(rb, v);
+    }
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const int i = i0 - K + k;
+    if (i >= 0) {
+      uint32_t raw[RAW];
+      load_raw<TI>(raw, in + (size_t)i * p.in_stride);
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) win[k][v] = i >= 0 ? to_f32(in[(size_t)i * p.in_stride + v]) : st[(size_t)(K + i) * p.channels + v];
+      for (int v = 0; v < VEC; ++v) win[k][v] = raw_at<TI>(raw, v);
+    } else {
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) win[k][v] = st[(size_t)(K + i) * p.channels + v];
+    }
   }
   if (seg == 0) {
     // the state after this step: the last K inputs of (old state, this entry's tokens)
@@ -272,15 +286,19 @@ JV_EXPORT int jv_short_conv(const void* in, int in_dtype, long long in_stride, v
   p.in = in; p.in_stride = in_stride; p.out = out; p.out_stride = out_stride; p.w = w; p.bias = residual ? nullptr : bias;
   p.state = state; p.state_stride = state_stride; p.cu_seqlens = cu_seqlens; p.slots = slots; p.n_entries = n_entries;
   p.n_slots = n_slots; p.channels = channels; p.act = act; p.residual = residual ? 1 : 0; p.status = status;
-  const dim3 grid(n_tokens / SEG + n_entries, (channels + THREADS - 1) / THREADS);
-  // Four channels a thread from 8 M elements on, for two to four taps and rows on four-element boundaries: 4,096 tokens of 10,240
-  // channels in 84 us against 108 one by one, 2,048 of 4,352 in 20 against 24; with fewer tokens or channels the threads of one
-  // channel each are needed to fill the device (2,048 of 2,304 channels: 16.3 against 15.1).
+  // Four channels a thread where entries have some tokens (or there are 8 M elements), for two to four taps and rows on four-element
+  // boundaries; segments as long as the device still fills, since each reads the weights and the taps - 1 inputs before it.  10,240
+  // channels, one entry of 130, 700, 4,096 tokens: 4.9, 10.5, 45 us, against 9.5, 19.5, 108 a channel a thread (segments of 32
+  // throughout: 7.4, 14, 45; of 8: 4.9, 11, 53).  Entries of one token each a channel a thread: 32 of 2,176 channels 5.4 against 7.1.
   auto fours = [](const void* q, long long stride, int dtype) {
     return ((uintptr_t)q & (dtype == 0 ? 15 : 7)) == 0 && stride % VEC == 0;
   };
-  const bool vec = (long long)n_tokens * channels >= (8LL << 20) && taps >= 2 && taps <= 4 && channels % VEC == 0 &&
-                   fours(in, in_stride, in_dtype) && fours(out, out_stride, out_dtype);
+  const long long size = (long long)n_tokens * channels;
+  const bool vec = (size >= (8LL << 20) || (size >= (1LL << 16) && n_tokens >= 8LL * n_entries)) && taps >= 2 && taps <= 4 && channels % VEC == 0 &&
+                   fours(in, in_stride, in_dtype) && fours(out, out_stride, out_dtype) && fours(w, 0, w_dtype) &&
+                   (bias == nullptr || fours(bias, 0, w_dtype));
+  p.seg_log2 = vec && size < (5LL << 20) ? 3 : vec && size < (16LL << 20) ? 4 : 5;
+  const dim3 grid((n_tokens >> p.seg_log2) + n_entries, (channels + THREADS - 1) / THREADS);
   JV_DISPATCH_DTYPE(in_dtype, TI, JV_DISPATCH_DTYPE(out_dtype, TO, JV_DISPATCH_DTYPE(w_dtype, TW,
       return launch_taps<TI, TO, TW>(p, taps, vec, grid, stream))));
   return JV_ERR_UNSUPPORTED;
