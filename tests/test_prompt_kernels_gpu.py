@@ -643,6 +643,45 @@ def test_product_32bit_of_infinities(m):
     assert ((y.double() - want)[fine].abs() <= (k + 2) * EPS32 * (x.double().abs() @ w.double().abs().T)[fine]).all()
 
 
+# ------------------------------------------------------------------------------- 32-bit attention, rows in vectors
+@pytest.mark.parametrize("hq,hk,d,dv,page", [(4, 2, 32, 32, 16), (16, 4, 64, 64, 8), (6, 1, 36, 128, 4), (2, 1, 256, 256, 32), (20, 1, 288, 512, 16)])
+@pytest.mark.parametrize("option", ["plain", "window, kept, sink", "capped, shaped", "sigmoid"])
+@pytest.mark.parametrize("split", [0, 40])
+def test_rows_of_32_bit_attention(hq, hk, d, dv, page, option, split):
+    """Rows on 16-byte boundaries against rows off them, which the general form takes; a page that is not there is reported by both."""
+    ops, g = _ops(), torch.Generator().manual_seed(5)
+    lengths, starts = ([1, 1, 1], [0, 39, 130]) if split else ([9, 33, 1], [0, 35, 77])
+    n, pages = sum(lengths), [-(-(a + b) // page) for a, b in zip(lengths, starts)]
+    table = torch.full((3, max(pages)), -1, dtype=torch.int32)
+    order = torch.randperm(sum(pages) + 3, generator=g)
+    for e in range(3):
+        table[e, :pages[e]] = order[sum(pages[:e]):sum(pages[:e + 1])]
+    caches = [torch.full((sum(pages) + 3, page, hk, size), float("nan"), device="cuda") for size in (d, dv)]
+    for e in range(3):
+        at = torch.arange(lengths[e] + starts[e])
+        for cache in caches:
+            cache[table[e, at // page].long(), at % page] = _rand(len(at), hk, cache.shape[3], seed=e + cache.shape[3])
+    kw = {"plain": {}, "window, kept, sink": dict(sink=_rand(hq, seed=8), keep=5), "capped, shaped": dict(
+        score_cap=3.0, head_scale=1 + 0.1 * _rand(hq, seed=6), dist_bias=_rand(hq, 20, seed=7)), "sigmoid": dict(sigmoid=True, bias=_rand(hq, seed=9))}[option]
+    cu = torch.tensor([0] + list(torch.tensor(lengths).cumsum(0)), dtype=torch.int32, device="cuda")
+    step = 1 if split else ops.attn_simt_tokens_per_tile(hq, hk)
+    work = torch.tensor([[e, t] for e in range(3) for t in range(0, lengths[e], step)], dtype=torch.int32, device="cuda")
+    room, outs = _rand(n, hq * d + 4, seed=1), []
+    room[:, 1:1 + hq * d] = room[:, :hq * d].clone()
+    first = room[:, :hq * d].clone()
+    for q in (first, room[:, 1:1 + hq * d].copy_(first)):
+        out = torch.zeros(n, hq * dv, device="cuda")
+        ops.attn_simt(q, q.stride(0), out, *caches, table.cuda(), cu, torch.tensor(starts, dtype=torch.int32, device="cuda"), work, len(work), hq, hk,
+                      d, 20 if "window" in option else 0, d ** -0.5, split_size=split, n_splits=4 if split else 0, **kw)
+        ops.check_status()
+        outs.append(out)
+    # scores of d terms, weights that move by twice a score's error, sums of up to 131 weights of at most one each (131 in all for sigmoid)
+    size = float((first.view(n, hq, d).abs().sum(-1).max() * torch.nan_to_num(caches[0]).abs().max()) * d ** -0.5) + 4
+    bound = (2 * (d + 8) * size + 140) * EPS32 * float(torch.nan_to_num(caches[1]).abs().max()) * (131 if option == "sigmoid" else 2)
+    assert torch.isfinite(outs[0]).all() and (outs[0] - outs[1]).abs().max() <= bound
+    assert (outs[0] - outs[1]).norm() <= 2e-6 * outs[1].norm()       # (random rows: a few roundings' root mean square)
+
+
 # ------------------------------------------------------------------------------- heads of 64 on the tcgen05 prompt kernel
 @pytest.mark.parametrize("hq,hk,page", [(4, 1, 16), (16, 1, 8), (6, 2, 64), (3, 3, 128), (10, 2, 32)])
 @pytest.mark.parametrize("option", ["plain", "window", "chunk", "kept, capped", "sigmoid", "shaped"])
