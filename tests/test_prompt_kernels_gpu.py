@@ -643,6 +643,47 @@ def test_product_32bit_of_infinities(m):
     assert ((y.double() - want)[fine].abs() <= (k + 2) * EPS32 * (x.double().abs() @ w.double().abs().T)[fine]).all()
 
 
+# ------------------------------------------------------------------------------- routing and order
+@pytest.mark.parametrize("n", [1, 33])
+@pytest.mark.parametrize("experts,top,groups,keep,identity", [(8, 2, 1, 1, 0), (36, 4, 1, 1, 4), (64, 6, 8, 3, 0), (160, 40, 1, 1, 0), (256, 8, 32, 5, 0),
+                                                              (257, 3, 1, 1, 1)])
+@pytest.mark.parametrize("scoring,mode", [("softmax", "max"), ("sigmoid", "top2_sum")])
+def test_route_and_order(n, experts, top, groups, keep, identity, scoring, mode):
+    """Ties go to the lowest index; a score that is no number, or minus infinity after the correction, is not chosen."""
+    ops, tile, routed = _ops(), 16, experts - identity
+    z = (_rand(n, experts + 3, seed=n + experts) * 8).round()[:, :experts] / 8        # many ties, and rows off 16-byte boundaries
+    correction = (_rand(experts, seed=3) * 8).round() / 64
+    correction[1], correction[2] = float("-inf"), -0.0
+    ids, weights, *own = ops.moe_route(z, top, groups, keep, True, scoring, mode, 1e-20, 2.5, correction=correction, identity=identity)
+    sorted_token, pos_of, tile_expert, used = ops.moe_align(ids, routed, tile, identity)
+    s = z.softmax(1) if scoring == "softmax" else z.sigmoid()
+    if identity:
+        torch.testing.assert_close(own[0], torch.where(ids >= routed, weights, 0.0).sum(1), rtol=1e-6, atol=1e-6)
+    picked = s.gather(1, ids.long())
+    torch.testing.assert_close(weights, 2.5 * picked / picked.sum(1, keepdim=True), rtol=1e-5, atol=1e-6)
+    c = (s + correction).double()
+    c = torch.where(c > float("-inf"), (c * 2 ** 18).round(), c)        # scores a few roundings apart are the same here
+    if groups > 1:
+        best = c.view(n, groups, -1).topk(2, 2).values
+        g = best.sum(2) if mode == "top2_sum" else best[:, :, 0]
+        kept = torch.zeros(n, groups, dtype=torch.bool, device="cuda").scatter_(1, ids.long() // (experts // groups), True)
+        assert (kept.sum(1) <= keep).all() and torch.where(kept, g, float("inf")).amin(1).ge(g.sort(1, descending=True).values[:, keep - 1]).all()
+    else:
+        assert torch.equal(c.gather(1, ids.long()), c.sort(1, descending=True).values[:, :top])
+    taken = c.gather(1, ids.long())
+    same = (taken[:, 1:] == taken[:, :-1]) & (weights[:, 1:] == weights[:, :-1])
+    assert (ids[:, 1:] > ids[:, :-1])[same & (correction[ids[:, 1:].long()] == correction[ids[:, :-1].long()])].all()
+    assert not (ids == 1).any() and all(len(set(row)) == top for row in ids.tolist())
+    # the order: every pair of a routed expert has a row of its own in a tile of its expert, with its token
+    flat, at = ids.flatten().long(), pos_of.flatten().long()
+    assert torch.equal(at < 0, flat >= routed) and len(set(at[at >= 0].tolist())) == int((at >= 0).sum())
+    there = at >= 0
+    assert torch.equal(sorted_token[at[there]].long(), torch.arange(n, device="cuda").repeat_interleave(top)[there])
+    assert torch.equal(tile_expert[at[there] // tile].long(), flat[there]) and int((sorted_token >= 0).sum()) == int(there.sum())
+    tiles = int(sum(-(-int((flat == e).sum()) // tile) for e in range(routed)))
+    assert int(used) == tiles and (tile_expert[tiles:] == -1).all()
+
+
 # ------------------------------------------------------------------------------- 32-bit attention, rows in vectors
 @pytest.mark.parametrize("hq,hk,d,dv,page", [(4, 2, 32, 32, 16), (16, 4, 64, 64, 8), (6, 1, 36, 128, 4), (2, 1, 256, 256, 32), (20, 1, 288, 512, 16)])
 @pytest.mark.parametrize("option", ["plain", "window, kept, sink", "capped, shaped", "sigmoid"])
