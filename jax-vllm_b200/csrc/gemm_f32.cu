@@ -1,5 +1,5 @@
 // C[M, N] = A[M, K] * W[N, K]^T in 32-bit on the 5th-generation tensor cores: the matrix product of the 32-bit path, also used where a
-// result must leave in 32-bit (logits) from 16-bit operands.
+// result must leave in 32-bit (logits) from 16-bit operands; batched, and grouped for routed experts.
 //
 // A 32-bit number is the sum of three 16-bit ones (x = hi + mid + lo, each the nearest to what is left; exactly), and a product of two
 // is hi hi + (hi mid + mid hi) + (hi lo + mid mid + lo hi) but for 2^-25 of it: six products of 16-bit numbers, each exact in the tensor
@@ -34,6 +34,8 @@
 // the CUDA cores and 0.147 so (400 tokens 0.277), the head (one row, 32,000 columns) 26 and 29.6 us.  A product of one to three rows is
 // 1 to 2 us slower than multiply-adds were (K = 1,024: 5 us; four rows the same, 16 rows 12 against 5), which a sum that
 // is the same whatever M is has to bear.
+// Grouped, 16 experts of 2,048 x 1,024 and 1,024 x 512, both products: 4 tokens of two choices 224 us on the CUDA cores and 37 so,
+// 200 tokens 280 and 105.
 #include "tcgen05.cuh"
 
 namespace {
@@ -41,6 +43,7 @@ constexpr int BM = 128, CHUNK = 32, MAX_ROWS = 128;     // rows of A of a block
 constexpr int CUTTERS = 8, GROUP = CUTTERS / 2;        // warps that cut, of a group of them
 constexpr int GROUP_BYTES = 8 * CHUNK * 2;             // eight rows of a chunk in one 16-bit part: four blocks of 8 rows x 16 bytes
 constexpr int LEAST_PART = 64, MAX_PARTS = 6;          // k's of a part; the parts of a tile are one cluster
+constexpr int GROUPED_AT_ONCE = 4;                     // tiles of experts that k's parts are cut for (how many there are, hangs on the tokens)
 constexpr int MAX_RAW = 6, MAX_STAGES = 4, MAX_ACCS = 4;
 
 struct Params {
@@ -50,6 +53,9 @@ struct Params {
   int a_vec, w_vec;                                    // four elements a load along k
   int strips, parts, part_k, row_tile;                 // row_tile: rows of A of a block, a multiple of 16
   int* status;
+  // grouped (routed experts): the expert of every tile of rows of A (-1: nothing to do), the token of every row (-1: nobody's, left alone)
+  const int *tile_expert, *row_token;
+  int gelu;
 };
 
 struct Shared {
@@ -215,11 +221,17 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   const int rows = min(p.row_tile, p.M - m0), rows16 = (rows + 15) / 16 * 16;
   const int k0 = part * p.part_k, k_end = min(p.K, k0 + p.part_k), chunks = (k_end - k0 + CHUNK - 1) / CHUNK;
   const TA* A = (const TA*)p.A + blockIdx.y * p.a_batch + (size_t)m0 * p.lda;
-  const TW* W = (const TW*)p.W + blockIdx.y * p.w_batch + (size_t)n0 * p.ldw;
+  int wb = blockIdx.y;                                 // which of the matrices W
+  if (p.tile_expert != nullptr) {                      // found out by the kernels before this one; the same for the whole cluster
+    pdl_wait();
+    wb = p.tile_expert[m0 / p.row_tile];
+    if (wb < 0) return;
+  }
+  const TW* W = (const TW*)p.W + wb * p.w_batch + (size_t)n0 * p.ldw;
   const int early = TMA ? min(RAW, chunks) : 0;
   auto bring_w = [&](int c, int s) {
     mbar_expect_tx(&sh->w_full[s], BM * Eight<TW>::ROW_BYTES);
-    tma_load_3d(raw + s * S::RAW_STAGE, &w_map, k0 + c * CHUNK, n0, blockIdx.y, &sh->w_full[s]);
+    tma_load_3d(raw + s * S::RAW_STAGE, &w_map, k0 + c * CHUNK, n0, wb, &sh->w_full[s]);
   };
   if (warp == S::BRINGER && elect_one()) {
     for (int s = 0; s < RAW; ++s) { mbar_init(&sh->w_full[s], 1); mbar_init(&sh->a_full[s], 1); mbar_init(&sh->raw_empty[s], GROUP); }
@@ -418,7 +430,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   TC* C = (TC*)p.C + blockIdx.y * p.c_batch + (size_t)m0 * p.ldc + n0;
   for (int e = threadIdx.x; e < n_mine; e += S::THREADS) {
     const int m = (t0 + e) / (BM / 4), n = (t0 + e) % (BM / 4) * 4;
-    if (n0 + n >= p.N) continue;
+    if (n0 + n >= p.N || (p.row_token != nullptr && p.row_token[m0 + m] < 0)) continue;
     float y[4] = {0.f, 0.f, 0.f, 0.f};
     for (int q = 0; q < p.parts; ++q) {
       const float4 v = ours[q * stride + e];
@@ -428,6 +440,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
 #pragma unroll
     for (int i = 0; i < 4; ++i)
       if (n0 + n + i < p.N && !is_number(y[i])) y[i] = plain_sum(A + (size_t)m * p.lda, W + (size_t)(n + i) * p.ldw, p.K);
+    if (p.gelu) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y[i] = 0.5f * y[i] * (1.f + erff(y[i] * 0.70710678118654752f));
+    }
     if constexpr (sizeof(TC) == 4)
       if (vec && n0 + n + 4 <= p.N) {
         *reinterpret_cast<float4*>(dst) = make_float4(y[0], y[1], y[2], y[3]);
@@ -503,15 +519,17 @@ int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const Params& p, 
 }
 
 template <typename TA, typename TW, typename TC>
-int dispatch(Params p, int batch, cudaStream_t stream) {
+int dispatch(Params p, int batch, int matrices, cudaStream_t stream) {
   CUtensorMap w_map = {}, a_map = {};
+  const bool grouped = p.tile_expert != nullptr;
   auto tile_of = [&](int most) {
+    if (grouped) return p.row_tile;
     const int tiles = (p.M + most - 1) / most;
     return ((p.M + tiles - 1) / tiles + 15) / 16 * 16;
   };
   p.row_tile = tile_of(MAX_ROWS);
-  if (p.K < 1 || !addressable<TA>(p.A, p.lda, p.a_batch, batch) || !addressable<TW>(p.W, p.ldw, p.w_batch, batch) ||
-      !make_map<TW>(&w_map, p.W, p.K, p.N, p.ldw, p.w_batch, batch, BM) ||
+  if (p.K < 1 || !addressable<TA>(p.A, p.lda, p.a_batch, batch) || !addressable<TW>(p.W, p.ldw, p.w_batch, matrices) ||
+      !make_map<TW>(&w_map, p.W, p.K, p.N, p.ldw, p.w_batch, matrices, BM) ||
       !make_map<TA>(&a_map, p.A, p.K, p.M, p.lda, p.a_batch, batch, p.row_tile)) {
     p.row_tile = tile_of(64);
     return launch<false, 64, TA, TW, TC>(w_map, a_map, p, batch, stream);
@@ -541,13 +559,13 @@ bool rows_aligned(const void* p, int size, int ld, size_t batch_stride, int batc
 
 int run(const void* A, int a_dtype, int lda, size_t a_batch, const void* W, int w_dtype, int ldw, size_t w_batch, void* C,
         int c_dtype, int ldc, size_t c_batch, int M, int N, int K, int batch, int* status, cudaStream_t stream) {
-  Params p{A, W, C, lda, ldw, ldc, M, N, K, a_batch, w_batch, c_batch, 0, 0, (N + BM - 1) / BM, 1, 0, 0, status};
+  Params p{A, W, C, lda, ldw, ldc, M, N, K, a_batch, w_batch, c_batch, 0, 0, (N + BM - 1) / BM, 1, 0, 0, status, nullptr, nullptr, 0};
   p.part_k = part_of_k(N, K, batch);
   p.parts = K > 0 ? (K + p.part_k - 1) / p.part_k : 1;
   p.a_vec = rows_aligned(A, a_dtype == 0 ? 4 : 2, lda, a_batch, batch);
   p.w_vec = rows_aligned(W, w_dtype == 0 ? 4 : 2, ldw, w_batch, batch);
   JV_DISPATCH_DTYPE(a_dtype, TA, JV_DISPATCH_DTYPE(w_dtype, TW, JV_DISPATCH_DTYPE(c_dtype, TC,
-      return (dispatch<TA, TW, TC>(p, batch, stream)))));
+      return (dispatch<TA, TW, TC>(p, batch, batch, stream)))));
   return JV_ERR_UNSUPPORTED;
 }
 }  // namespace
@@ -557,6 +575,24 @@ JV_EXPORT int jv_gemm_f32(const void* A, int a_dtype, int lda, const void* W, in
                           int M, int N, int K, int* status, cudaStream_t stream) {
   if (M == 0 || N == 0) return JV_OK;
   return run(A, a_dtype, lda, 0, W, w_dtype, ldw, 0, C, c_dtype, ldc, 0, M, N, K, 1, status, stream);
+}
+
+// Routed experts: rows of A and C in tiles of `tile` (16 or 64), tile t of expert tile_expert[t] (-1: nothing to do) with the weight
+// W + expert * w_expert; rows whose row_token is -1 are left alone.  gelu: the exact gelu of the result.
+JV_EXPORT int jv_gemm_f32_grouped(const void* A, int a_dtype, int lda, const void* W, int w_dtype, int ldw, long long w_expert, int experts,
+                                  void* C, int c_dtype, int ldc, int tiles, int tile, const int* tile_expert, const int* row_token,
+                                  int N, int K, int gelu, int* status, cudaStream_t stream) {
+  if (tiles == 0 || N == 0) return JV_OK;
+  if ((tile != 16 && tile != 64) || experts < 1 || tiles > 0x7fffffff / 64) return JV_ERR_UNSUPPORTED;
+  Params p{A, W, C, lda, ldw, ldc, tiles * tile, N, K, 0, (size_t)w_expert, 0, 0, 0, (N + BM - 1) / BM, 1, 0, tile, status,
+           tile_expert, row_token, gelu};
+  p.part_k = part_of_k(N, K, GROUPED_AT_ONCE);
+  p.parts = K > 0 ? (K + p.part_k - 1) / p.part_k : 1;
+  p.a_vec = rows_aligned(A, a_dtype == 0 ? 4 : 2, lda, 0, 1);
+  p.w_vec = rows_aligned(W, w_dtype == 0 ? 4 : 2, ldw, (size_t)w_expert, experts);
+  JV_DISPATCH_DTYPE(a_dtype, TA, JV_DISPATCH_DTYPE(w_dtype, TW, JV_DISPATCH_DTYPE(c_dtype, TC,
+      return (dispatch<TA, TW, TC>(p, 1, experts, stream)))));
+  return JV_ERR_UNSUPPORTED;
 }
 
 // `batch` products of the same sizes in one launch: product b reads A + b*a_batch, W + b*w_batch and writes

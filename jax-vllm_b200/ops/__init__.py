@@ -1474,35 +1474,28 @@ def moe_route_table(tokens: torch.Tensor, table: torch.Tensor, experts: int):
 MOE_ACTS = {None: 0, "gelu": 1}
 
 
-def moe_gemm_simt_tile() -> int:
-    f = _build.load("moe_gemm_simt").jv_moe_gemm_simt_tile
-    f.argtypes, f.restype = [], c_int
-    return int(f())
+def moe_gemm_f32_tile(pairs: int, experts: int) -> int:
+    """The rows of a tile of moe_gemm_f32: a tile costs its expert's weight whatever its rows are, so few rows get a low one."""
+    return 16 if pairs <= 8 * experts else 64
 
 
-def moe_gemm_simt(a: torch.Tensor, gather: torch.Tensor | None, w: torch.Tensor, tile_expert: torch.Tensor,
-                  out_dtype: torch.dtype, act: str | None = None) -> torch.Tensor:
-    """Grouped product on CUDA cores (csrc/moe_gemm_simt.cu): row pos of the result, in a tile of expert e, is
-    act(a[gather[pos]] @ w[e].T) (gather None: a[pos]); w [experts, N, K]; rows of padding are left unwritten."""
-    _cuda(a, "a"); _cuda(w, "w"); _cuda(tile_expert, "tile_expert", torch.int32)
-    tile = moe_gemm_simt_tile()
-    max_tiles = tile_expert.numel()
+def moe_gemm_f32(a: torch.Tensor, w: torch.Tensor, tile: int, tile_expert: torch.Tensor, row_token: torch.Tensor,
+                 out_dtype: torch.dtype, act: str | None = None) -> torch.Tensor:
+    """Grouped product as exact as in 32-bit multiply-adds (csrc/gemm_f32.cu): row pos of the result, in a tile of expert e, is
+    act(a[pos] @ w[e].T); w [experts, N, K]; rows whose token is -1 are left unwritten."""
+    _cuda(a, "a"); _cuda(w, "w"); _cuda(tile_expert, "tile_expert", torch.int32); _cuda(row_token, "row_token", torch.int32)
+    tiles = tile_expert.numel()
     experts, n_out, k = w.shape
     if a.shape[1] != k:
         raise KernelError("grouped product: inner sizes differ")
-    if gather is not None:
-        _cuda(gather, "gather", torch.int32)
-        if gather.numel() != max_tiles * tile:
-            raise KernelError("gather does not fit the tiles")
-    elif a.shape[0] != max_tiles * tile:
+    if a.shape[0] != tiles * tile or row_token.numel() != tiles * tile:
         raise KernelError("rows do not fit the tiles")
-    out = torch.empty((max_tiles * tile, n_out), dtype=out_dtype, device=a.device)
-    f = _fn("moe_gemm_simt", "jv_moe_gemm_simt", [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_longlong, c_int,
-                                                  c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p,
-                                                  c_void_p])
-    _check(f(a.data_ptr(), _code(a, "a"), a.stride(0), _ptr(gather), a.shape[0], w.data_ptr(), _code(w, "w"), w.stride(0),
-             w.stride(1), tile_expert.data_ptr(), max_tiles, out.data_ptr(), _code(out, "out"), out.stride(0), n_out, k,
-             MOE_ACTS[act], _status_ptr(a.device), _stream()), "moe_gemm_simt")
+    out = torch.empty((tiles * tile, n_out), dtype=out_dtype, device=a.device)
+    f = _fn("gemm_f32", "jv_gemm_f32_grouped", [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_longlong, c_int, c_void_p, c_int, c_int,
+                                                c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(f(a.data_ptr(), _code(a, "a"), a.stride(0), w.data_ptr(), _code(w, "w"), w.stride(1), w.stride(0), experts, out.data_ptr(),
+             _code(out, "out"), out.stride(0), tiles, tile, tile_expert.data_ptr(), row_token.data_ptr(), n_out, k, MOE_ACTS[act],
+             _status_ptr(a.device), _stream()), "moe_gemm_f32")
     return out
 
 

@@ -33,7 +33,7 @@ from .registry import register_feed_forward
 
 
 class RoutedExperts(Part):
-    kernels = ("moe_route", "moe_gemm_simt", "gemm_f32")
+    kernels = ("moe_route", "gemm_f32")
 
     def __init__(self, spec, prefix, ctx):
         if spec.activation not in ("gelu", "clamped_glu", "swiglu"):
@@ -48,7 +48,7 @@ class RoutedExperts(Part):
         if spec.activation == "clamped_glu" and not spec.limit > 0:
             raise ValueError("routed experts: the clamped activation needs a positive limit")
         if self.gated:
-            self.kernels = ("moe_route", "moe_gemm_simt", "gemm_f32", "activation")
+            self.kernels = ("moe_route", "gemm_f32", "activation")
         if self.by_table and (spec.correction is not None or spec.identity):
             raise ValueError("routed experts: a table knows no correction and no identity experts")
         # the router's experts: those with tensors, then the identity experts
@@ -107,7 +107,7 @@ class RoutedExperts(Part):
 
     # The grouped tcgen05 product works on 128-row tiles of 256 columns: it is taken for bfloat16 experts whose inner
     # sizes it can address (multiples of 8) and whose matrices are at least this wide; smaller ones, and the 32-bit
-    # path, go to the CUDA-core product with its 32-row tiles.
+    # path, go to the product in 32-bit (csrc/gemm_f32.cu).
     TCGEN05_MIN_SIZE = 128
 
     def _tensor_cores(self) -> bool:
@@ -164,11 +164,13 @@ class RoutedExperts(Part):
             if self.gated:
                 act = self._gate(act, row_token)
             return ops.PickedRows(product(act, self.w_down), pos_of, weights, *own)
-        sorted_token, pos_of, tile_expert, _ = ops.moe_align(ids, s.num_experts, ops.moe_gemm_simt_tile(), s.identity)
-        act = ops.moe_gemm_simt(x, sorted_token, self.w_up, tile_expert, dt, act=first)
+        tile = ops.moe_gemm_f32_tile(ids.numel(), s.num_experts)
+        row_token, pos_of, tile_expert, _ = ops.moe_align(ids, s.num_experts, tile, s.identity)
+        rows = ops.moe_gather_rows(x, pos_of, tile_expert.numel() * tile)
+        act = ops.moe_gemm_f32(rows, self.w_up, tile, tile_expert, row_token, dt, act=first)
         if self.gated:
-            act = self._gate(act)
-        y = ops.moe_gemm_simt(act, None, self.w_down, tile_expert, dt)
+            act = self._gate(act, row_token)
+        y = ops.moe_gemm_f32(act, self.w_down, tile, tile_expert, row_token, dt)
         return ops.PickedRows(y, pos_of, weights, *own)
 
 

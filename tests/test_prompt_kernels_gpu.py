@@ -626,6 +626,32 @@ def test_tiles_and_parts_of_the_32bit_product(m, n, k):
         assert torch.equal(ops.gemm_simt(x[first:first + rows], w, torch.float32), y[first:first + rows])
 
 
+@pytest.mark.parametrize("tile", [16, 64])
+@pytest.mark.parametrize("n,k", [(128, 1024), (300, 2100), (20, 33), (1030, 64)])
+@pytest.mark.parametrize("act", [None, "gelu"])
+def test_experts_32bit_product(tile, n, k, act):
+    """Rows of padding, which may hold anything, are left alone; tiles without an expert too."""
+    ops, experts, chosen = _ops(), 5, [3, -1, 0, 3, 4, -1]
+    rows = len(chosen) * tile
+    for ad, wd, od in ((torch.float32, torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16, torch.bfloat16),
+                       (torch.float32, torch.bfloat16, torch.float32)):
+        a, w = _rand(rows, k, seed=1, dtype=ad), _rand(experts, n, k, seed=2, dtype=wd)
+        token = torch.arange(rows, dtype=torch.int32, device="cuda")
+        token[tile - 3:tile] = -1
+        a[tile - 3:tile] = float("nan")
+        y = ops.moe_gemm_f32(a, w, tile, torch.tensor(chosen, dtype=torch.int32, device="cuda"), token, od, act=act)
+        for t, e in enumerate(chosen):
+            at = slice(t * tile, t * tile + (tile - 3 if t == 0 else tile))
+            if e < 0:
+                continue
+            want = a[at].double() @ w[e].double().T
+            bound = 2 * (k + 4) * EPS32 * (a[at].double().abs() @ w[e].double().abs().T) + 1e-30
+            if act:
+                want, bound = torch.nn.functional.gelu(want), 1.2 * bound + 8 * EPS32 * want.abs()       # (its slope is at most 1.13)
+            assert ((y[at].double() - want).abs() <= bound + (2.0 ** -8 * want.abs() if od == torch.bfloat16 else 0.0)).all()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("m", [3, 40])
 def test_product_32bit_of_infinities(m):
     """An infinity, a NaN and numbers next to the largest give what multiply-adds give, and stay in their rows and columns."""
