@@ -1993,6 +1993,11 @@ def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, 
             and tokens * heads * -(-columns // 32) >= chunk_scan_min_blocks(dim) * (longest or -(-tokens // n_entries)))
 
 
+_CHUNK_SCAN_TYPES = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_float, c_void_p, c_void_p, c_longlong, c_void_p,
+                     c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                     c_int, c_void_p, c_void_p, c_void_p]
+
+
 def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor, cu_seqlens: torch.Tensor,
                slots: torch.Tensor, n_entries: int, heads: int, groups: int, dim: int, columns: int, scale: float = 1.0,
                gates: torch.Tensor | None = None, state_n: torch.Tensor | None = None, dt_raw: torch.Tensor | None = None,
@@ -2031,10 +2036,7 @@ def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: tor
     taken = portions or n_entries
     n_taken = n - (n_entries - taken)                    # tokens of the portions: the others have one each
     scratch = torch.empty((n_taken // CHUNK_SCAN_TOKENS + taken) * heads * (dim * columns + dim + 1), dtype=torch.float32, device=row.device)
-    f = _fn("chunk_scan", "jv_chunk_scan", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_float, c_void_p,
-                                            c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p,
-                                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
-                                            c_void_p])
+    f = _fn("chunk_scan", "jv_chunk_scan", _CHUNK_SCAN_TYPES)
     base = row.data_ptr()
     _check(f(base + 2 * q_off, row.stride(0), base + 2 * k_off, row.stride(0), base + 2 * v_off, row.stride(0), heads // groups,
              float(scale), _ptr(gates), _ptr(dt_raw), 0 if dt_raw is None else dt_raw.stride(0), _ptr(dt_bias), _ptr(a_log), w_code,
@@ -2078,6 +2080,10 @@ SHORT_CONV_MAX_TAPS = 8
 SHORT_CONV_ACTS = {None: 0, "silu": 1}
 
 
+_SHORT_CONV_TYPES = [c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_void_p,
+                     c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p]
+
+
 def short_conv(x: torch.Tensor, weight: torch.Tensor, state: torch.Tensor | None, cu_seqlens: torch.Tensor,
                slots: torch.Tensor, n_entries: int, out_dtype: torch.dtype, bias: torch.Tensor | None = None,
                act: str | None = None, residual: bool = False, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -2106,9 +2112,7 @@ def short_conv(x: torch.Tensor, weight: torch.Tensor, state: torch.Tensor | None
     _cuda(out, "out", out_dtype, contiguous=False)
     if out.shape != x.shape or out.stride(1) != 1:
         raise KernelError("short_conv: out has the shape of x")
-    f = _fn("short_conv", "jv_short_conv", [c_void_p, c_int, c_longlong, c_void_p, c_int, c_longlong, c_void_p, c_void_p,
-                                            c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                                            c_int, c_int, c_int, c_void_p, c_void_p])
+    f = _fn("short_conv", "jv_short_conv", _SHORT_CONV_TYPES)
     _check(f(x.data_ptr(), _code(x, "x"), x.stride(0), out.data_ptr(), _code(out, "out"), out.stride(0),
              weight.data_ptr(), _ptr(bias), _code(weight, "weight"), _ptr(state) if taps > 1 else 0, stride,
              cu_seqlens.data_ptr(), slots.data_ptr(), n_entries, n_slots, n, channels, taps, SHORT_CONV_ACTS[act],
@@ -2331,6 +2335,10 @@ def mamba_prepare(xbc: torch.Tensor, b_off: int, c_off: int, dt_raw: torch.Tenso
     return packed
 
 
+_MAMBA_FINISH_TYPES = [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_float,
+                       c_int, c_int, c_int, c_int, c_void_p]
+
+
 def mamba_finish(o: torch.Tensor, x: torch.Tensor, z: torch.Tensor, skip: torch.Tensor, weight: torch.Tensor,
                  out: torch.Tensor, heads: int, value_dim: int, norm_groups: int, eps: float) -> torch.Tensor:
     """y = (o + skip_h * x) * silu(z), divided by the root mean square of each of its `norm_groups` equal parts, times
@@ -2342,11 +2350,60 @@ def mamba_finish(o: torch.Tensor, x: torch.Tensor, z: torch.Tensor, skip: torch.
             out.shape != o.shape or x.stride(1) != 1 or z.stride(1) != 1 or out.stride(1) != 1 or skip.numel() != heads or \
             weight.numel() != inner:
         raise KernelError("mamba_finish: shapes do not fit")
-    f = _fn("mamba2", "jv_mamba_finish", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p,
-                                          c_int, c_void_p, c_longlong, c_float, c_int, c_int, c_int, c_int, c_void_p])
+    f = _fn("mamba2", "jv_mamba_finish", _MAMBA_FINISH_TYPES)
     _check(f(o.data_ptr(), x.data_ptr(), x.stride(0), z.data_ptr(), z.stride(0), _code(x, "x"), skip.data_ptr(),
              weight.data_ptr(), _code(skip, "skip"), out.data_ptr(), out.stride(0), float(eps), n, heads, value_dim,
              norm_groups, _stream()), "mamba_finish")
+    return out
+
+
+def state_space_prompt_takes(row: torch.Tensor, n_entries: int, heads: int, groups: int, dim: int, columns: int, taps: int) -> bool:
+    """`chunk_scan_takes` for the convolution's output, and a convolution with a state."""
+    inner, side = heads * columns, groups * dim
+    return (n_entries >= 1 and row.dtype == torch.bfloat16 and row.shape[0] >= CHUNK_SCAN_MIN_TOKENS * n_entries and taps > 1
+            and 8 <= dim <= CHUNK_SCAN_MAX_KEY and dim % 8 == 0 and columns % 8 == 0 and inner % 8 == 0 and side % 8 == 0)
+
+
+def state_space_prompt(row: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Tensor, state: torch.Tensor, cu_seqlens: torch.Tensor,
+                       slots: torch.Tensor, n_entries: int, heads: int, groups: int, dim: int, columns: int, dt_bias: torch.Tensor,
+                       a_log: torch.Tensor, skip: torch.Tensor, norm: torch.Tensor, norm_groups: int, eps: float,
+                       out: torch.Tensor) -> torch.Tensor:
+    """`short_conv` (with silu), `chunk_scan` and `mamba_finish` of a state-space mixer's portions, one after another without views
+    and a second look at what the first has checked: the launches of a few hundred tokens take the host longer than the device.
+    `row` [n, ..]: z [heads * columns], what is convolved (x, then k and q of the groups), the raw step sizes [heads]; `state`: the
+    matrices of a slot, then the convolution's inputs."""
+    _cuda(row, "row", torch.bfloat16, contiguous=False); _cuda(state, "state", torch.float32, contiguous=False)
+    _cuda(out, "out", torch.bfloat16, contiguous=False)
+    _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
+    _cuda(conv_w, "conv_w"); _cuda(conv_b, "conv_b", conv_w.dtype); _cuda(dt_bias, "dt_bias"); _cuda(a_log, "a_log", dt_bias.dtype)
+    _cuda(skip, "skip"); _cuda(norm, "norm", skip.dtype)
+    (n, width), (n_slots, state_width), taps = row.shape, state.shape, conv_w.shape[1]
+    inner, side = heads * columns, groups * dim
+    channels, matrices = inner + 2 * side, heads * dim * columns
+    row_stride, row_unit = row.stride()
+    state_stride, state_unit = state.stride()
+    out_stride, out_unit = out.stride()
+    if row_unit != 1 or state_unit != 1 or out_unit != 1 or width < inner + channels + heads or out.shape != (n, inner) or heads % groups or \
+            inner % norm_groups or state_width != matrices + (taps - 1) * channels or not 1 < taps <= SHORT_CONV_MAX_TAPS or \
+            conv_w.shape[0] != channels or conv_b.numel() != channels or dt_bias.numel() != heads or a_log.numel() != heads or \
+            skip.numel() != heads or norm.numel() != inner or cu_seqlens.numel() <= n_entries or slots.numel() < n_entries:
+        raise KernelError("state_space_prompt: shapes do not fit")
+    device = row.device
+    conv = torch.empty((n, channels), dtype=torch.bfloat16, device=device)
+    chunks = n // CHUNK_SCAN_TOKENS + n_entries          # the scan's outputs, and its scratch behind them
+    scan = torch.empty(n * inner + chunks * heads * (dim * columns + dim + 1), dtype=torch.float32, device=device)
+    z, x, o = row.data_ptr(), conv.data_ptr(), scan.data_ptr()
+    matrix, cu, slot, status, stream = state.data_ptr(), cu_seqlens.data_ptr(), slots.data_ptr(), _status_ptr(device), _stream()
+    _check(_fn("short_conv", "jv_short_conv", _SHORT_CONV_TYPES)(
+        z + 2 * inner, 1, row_stride, x, 1, channels, conv_w.data_ptr(), conv_b.data_ptr(), _code(conv_w, "conv_w"), matrix + 4 * matrices,
+        state_stride, cu, slot, n_entries, n_slots, n, channels, taps, SHORT_CONV_ACTS["silu"], 0, status, stream), "short_conv")
+    _check(_fn("chunk_scan", "jv_chunk_scan", _CHUNK_SCAN_TYPES)(
+        x + 2 * (inner + side), channels, x + 2 * inner, channels, x, channels, heads // groups, 1.0, 0, z + 2 * (inner + channels), row_stride,
+        dt_bias.data_ptr(), a_log.data_ptr(), _code(dt_bias, "dt_bias"), o, matrix, state_stride, 0, cu, slot, n_slots, n_entries, heads, dim,
+        columns, 0, n, o + 4 * n * inner, status, stream), "chunk_scan", launches=3)
+    _check(_fn("mamba2", "jv_mamba_finish", _MAMBA_FINISH_TYPES)(
+        o, x, channels, z, row_stride, 1, skip.data_ptr(), norm.data_ptr(), _code(skip, "skip"), out.data_ptr(), out_stride, float(eps), n,
+        heads, columns, norm_groups, stream), "mamba_finish")
     return out
 
 

@@ -88,6 +88,11 @@ class StateSpace(Part):
         inner, gn, dt = self.inner, self.g * self.n, self.ctx.dtype
         state = cache.state
         mats = self.h * self.n * self.e
+        if not step.decode_work[1] and ops.state_space_prompt_takes(row, step.n_entries, self.h, self.g, self.n, self.e, self.taps) and \
+                out.dtype == torch.bfloat16:
+            return ops.state_space_prompt(row, self.conv_w, self.conv_b, state, step.cu_seqlens, step.state_slots, step.n_entries, self.h,
+                                          self.g, self.n, self.e, self.dt_bias, self.a_log, self.skip, self.norm, self.ng,
+                                          self.spec.norm_eps, out)
         conv_state = state[:, mats:] if self.taps > 1 else None
         xbc = ops.short_conv(row[:, inner:inner + self.conv_channels], self.conv_w, conv_state, step.cu_seqlens,
                              step.state_slots, step.n_entries, dt, bias=self.conv_b, act="silu")

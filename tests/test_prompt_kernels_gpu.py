@@ -260,6 +260,34 @@ def test_chunked_states_over_several_chunks(heads, dim, columns):
         assert (got.double() - want.double()).norm() <= 3e-6 * want.double().norm()
 
 
+@pytest.mark.parametrize("heads,groups,dim,columns,taps", [(4, 2, 16, 8, 2), (8, 1, 64, 64, 4), (6, 3, 136, 24, 3)])
+@pytest.mark.parametrize("lengths", [[64], [200, 77, 130]])
+def test_portions_of_the_state_space_mixer(heads, groups, dim, columns, taps, lengths):
+    """The three steps in one call against the three calls, from a column range of wider rows into one of a wider result."""
+    ops = _ops()
+    cu, slots, n_slots = _entries(lengths)
+    n, inner, side = sum(lengths), heads * columns, groups * dim
+    channels, width, matrices = inner + 2 * side, 2 * inner + 2 * side + heads, heads * dim * columns
+    row = _rand(n, width + 16, seed=1, dtype=torch.bfloat16)[:, 8:8 + width]
+    weights = [_rand(*shape, seed=2 + i) for i, shape in enumerate(((channels, taps), (channels,), (heads,), (heads,), (heads,), (inner,)))]
+    conv_w, conv_b, dt_bias, a_log, skip, norm = weights
+    states = [_rand(n_slots, matrices + (taps - 1) * channels, seed=9) for _ in range(2)]
+    outs = [torch.zeros(n, inner + 8, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+    assert ops.state_space_prompt_takes(row, len(lengths), heads, groups, dim, columns, taps)
+    ops.state_space_prompt(row, conv_w, conv_b, states[0], cu, slots, len(lengths), heads, groups, dim, columns, dt_bias, a_log, skip, norm,
+                           groups, 1e-5, outs[0][:, :inner])
+    st = states[1]
+    xbc = ops.short_conv(row[:, inner:inner + channels], conv_w, st[:, matrices:], cu, slots, len(lengths), torch.bfloat16, bias=conv_b, act="silu")
+    o = ops.chunk_scan(xbc, inner + side, inner, 0, st, cu, slots, len(lengths), heads, groups, dim, columns,
+                       dt_raw=row[:, inner + channels:], dt_bias=dt_bias, a_log=a_log)
+    ops.mamba_finish(o, xbc[:, :inner], row[:, :inner], skip, norm, outs[1][:, :inner], heads, columns, groups, 1e-5)
+    ops.check_status()
+    assert torch.equal(states[0], states[1]) and torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0].float()).all()
+    with pytest.raises(ops.KernelError):
+        ops.state_space_prompt(row, conv_w, conv_b, states[0][:, 1:], cu, slots, len(lengths), heads, groups, dim, columns, dt_bias, a_log, skip,
+                               norm, groups, 1e-5, outs[0][:, :inner])
+
+
 # ------------------------------------------------------- convolution and finish of the state-space mixer
 @pytest.mark.parametrize("taps", [2, 3, 4])
 @pytest.mark.parametrize("channels,off", [(8192, 0), (8196, 4), (8192, 2), (512, 0)])
