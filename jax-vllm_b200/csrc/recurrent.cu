@@ -77,8 +77,6 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const T* __restrict_
   }
 }
 
-__device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
-
 // packed [n, heads, 3, D] = (q * q_scale, k, exp(logsigmoid(z) / tau)), z = w_up[e, :] . low + bias[e] in 32-bit.  A block
 // takes TOK tokens, so that a row of w_up is read once for all of them; `low` [n, rank] are columns of the projection.
 template <int TOK, typename T, typename W>

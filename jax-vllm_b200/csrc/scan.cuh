@@ -3,6 +3,8 @@
 
 #include "common.cuh"
 
+__device__ __forceinline__ float log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
+
 // A step may hold decoded tokens beside portions of prompts.  The kernels for portions are then launched with their number,
 // `portions`, and pass by the entries of one token, which state_step.cu takes from the step's list of them: neither kind's sums
 // hang on the other's being there.  Without (0) all entries are taken, those of one token too.

@@ -10,7 +10,14 @@
 //
 // 48 requests of 8 heads of 128 x 256 (50 MB of states, read and written): 16.0 us (6.3 TB/s), 38.8 us on the scan for whole entries
 // (which stages vectors and values for many tokens and keeps 16 channels x 4 columns a thread).
-#include "common.cuh"
+//
+// The state-space layers' vectors are formed here (MAMBA) instead of being read: q = C and k = dt B of the head's group, one decay
+// exp(-exp(A_log) dt) in every channel, dt = softplus(dt_raw + dt_bias), as mamba_prepare (mamba2.cu) forms them, which spares single
+// tokens a launch (one token of 32 heads of 64 x 64: 1.7 and 2.75 us in two launches, 3.1 in one); those of gated linear attention (GLA) as
+// gla_prepare (recurrent.cu) forms them (eight tokens of 8 heads of 128 x 256: 2.4 and 5.2, 5.1 in
+// one).
+#include "scan.cuh"
+#include <math.h>
 
 namespace {
 constexpr int THREADS = 256, ROWS = 8;     // state rows a thread
@@ -23,13 +30,24 @@ struct StepParams {
   float* state_n; float* nq; int nq_stride;  // the normaliser's column (value 1) and where its outputs go, or null
   const int* cu_seqlens; const int* slots;
   int n_slots, heads, D, V;
+  const void *b, *c, *dt_raw; long long bc_stride, dt_stride;      // MAMBA: rows of B, C and the raw step sizes, instead of packed
+  const void *dt_bias, *a_log; int w_dtype, per_group;
+  // GLA: q and k in b and c, the low-rank numbers in dt_raw; their matrix [heads * D, rank] and bias [heads * D] in dt_bias and a_log
+  int rank; float inv_tau, q_scale;
   const int* work; int compact;            // pairs (entry, -), or null: every entry; a row of packed for every pair, not every token
   int* status;
 };
 
 // RG: row groups (D <= ROWS * RG); a thread's rows are rg, rg + RG, ...
-template <int RG, int VEC, bool REMOVAL, typename T>
+enum : int { PLAIN, REMOVAL_TERM, MAMBA, GLA };
+
+__device__ __forceinline__ float weight_at(const void* w, int dtype, size_t i) {
+  return dtype == 0 ? ((const float*)w)[i] : to_f32(((const __nv_bfloat16*)w)[i]);
+}
+
+template <int RG, int VEC, int KIND, typename T>
 __global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p) {
+  constexpr bool REMOVAL = KIND == REMOVAL_TERM;
   constexpr int CQ = THREADS / RG, COLS = CQ * VEC, NV = REMOVAL ? 5 : 3;
   __shared__ float vec[NV * ROWS * RG];
   __shared__ __align__(16) float part[RG * COLS];
@@ -72,7 +90,32 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p)
     const T* vsrc = (const T*)p.v + (size_t)t * p.v_stride + p.v_off + (size_t)h * V + (live ? col : 0);
 #pragma unroll
     for (int c = 0; c < VEC; ++c) vv[c] = to_f32(vsrc[c]);
-    for (int i = tid; i < NV * D; i += THREADS) vec[(i / D) * (ROWS * RG) + i % D] = src[i];
+    if constexpr (KIND == MAMBA) {
+      if (tid < D) {
+        const size_t at = (size_t)t * p.bc_stride + (size_t)(h / p.per_group) * D + tid;
+        const float B = to_f32(((const T*)p.b)[at]), C = to_f32(((const T*)p.c)[at]);
+        const float bias = weight_at(p.dt_bias, p.w_dtype, h), rate = weight_at(p.a_log, p.w_dtype, h);
+        const float z = to_f32(((const T*)p.dt_raw)[(size_t)t * p.dt_stride + h]) + bias;
+        const float dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));             // softplus, no clamp
+        vec[tid] = C;
+        vec[ROWS * RG + tid] = dt * B;
+        vec[2 * ROWS * RG + tid] = expf(-expf(rate) * dt);
+      }
+    } else if constexpr (KIND == GLA) {
+      if (tid < D) {
+        const size_t e = (size_t)h * D + tid, at = (size_t)t * p.bc_stride + e;
+        const float q = to_f32(((const T*)p.b)[at]), k = to_f32(((const T*)p.c)[at]), bias = weight_at(p.a_log, p.w_dtype, e);
+        const T* low = (const T*)p.dt_raw + (size_t)t * p.dt_stride;
+        float z = 0.f;
+#pragma unroll 8
+        for (int r = 0; r < p.rank; ++r) z = fmaf(weight_at(p.dt_bias, p.w_dtype, e * p.rank + r), to_f32(low[r]), z);
+        vec[tid] = q * p.q_scale;
+        vec[ROWS * RG + tid] = k;
+        vec[2 * ROWS * RG + tid] = expf(log_sigmoid(z + bias) * p.inv_tau);
+      }
+    } else {
+      for (int i = tid; i < NV * D; i += THREADS) vec[(i / D) * (ROWS * RG) + i % D] = src[i];
+    }
     __syncthreads();
     float dot[VEC];
     if constexpr (REMOVAL) {
@@ -146,14 +189,25 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p)
 }
 
 template <int RG, typename T>
-int dispatch(const StepParams& p, bool removal, bool vec, int entries, cudaStream_t stream) {
+int dispatch(const StepParams& p, int kind, bool vec, int entries, cudaStream_t stream) {
   const int cols = THREADS / RG * (vec ? 4 : 1);
   const dim3 grid(entries, p.heads, (p.V + cols - 1) / cols);
   if (vec)
-    return removal ? jv_launch(state_step_kernel<RG, 4, true, T>, grid, dim3(THREADS), 0, stream, p)
-                   : jv_launch(state_step_kernel<RG, 4, false, T>, grid, dim3(THREADS), 0, stream, p);
-  return removal ? jv_launch(state_step_kernel<RG, 1, true, T>, grid, dim3(THREADS), 0, stream, p)
-                 : jv_launch(state_step_kernel<RG, 1, false, T>, grid, dim3(THREADS), 0, stream, p);
+    return kind == REMOVAL_TERM ? jv_launch(state_step_kernel<RG, 4, REMOVAL_TERM, T>, grid, dim3(THREADS), 0, stream, p)
+           : kind == MAMBA      ? jv_launch(state_step_kernel<RG, 4, MAMBA, T>, grid, dim3(THREADS), 0, stream, p)
+           : kind == GLA        ? jv_launch(state_step_kernel<RG, 4, GLA, T>, grid, dim3(THREADS), 0, stream, p)
+                                : jv_launch(state_step_kernel<RG, 4, PLAIN, T>, grid, dim3(THREADS), 0, stream, p);
+  return kind == REMOVAL_TERM ? jv_launch(state_step_kernel<RG, 1, REMOVAL_TERM, T>, grid, dim3(THREADS), 0, stream, p)
+         : kind == MAMBA      ? jv_launch(state_step_kernel<RG, 1, MAMBA, T>, grid, dim3(THREADS), 0, stream, p)
+         : kind == GLA        ? jv_launch(state_step_kernel<RG, 1, GLA, T>, grid, dim3(THREADS), 0, stream, p)
+                              : jv_launch(state_step_kernel<RG, 1, PLAIN, T>, grid, dim3(THREADS), 0, stream, p);
+}
+
+template <typename T> int by_size(const StepParams& p, int kind, int entries, cudaStream_t stream) {
+  const bool vec = p.V % 4 == 0 && ((uintptr_t)p.state & 15) == 0 && p.slot_stride % 4 == 0;
+  if (p.D <= 64) return dispatch<8, T>(p, kind, vec, entries, stream);
+  if (p.D <= 128) return dispatch<16, T>(p, kind, vec, entries, stream);
+  return dispatch<32, T>(p, kind, vec, entries, stream);
 }
 }  // namespace
 
@@ -166,12 +220,41 @@ JV_EXPORT int jv_state_step(const float* packed, int removal, const void* v, int
   if (entries == 0) return JV_OK;
   if ((compact && work == nullptr) || heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || (removal && state_n != nullptr)) return JV_ERR_UNSUPPORTED;
   StepParams p{packed, v, v_stride, v_off, out, state, slot_stride, state_n, nq, nq_stride, cu_seqlens, slots, n_slots, heads, D, V,
-               work, compact, status};
-  const bool vec = V % 4 == 0 && ((uintptr_t)state & 15) == 0 && slot_stride % 4 == 0;
-  JV_DISPATCH_DTYPE(v_dtype, T, {
-    if (D <= 64) return dispatch<8, T>(p, removal != 0, vec, entries, stream);
-    if (D <= 128) return dispatch<16, T>(p, removal != 0, vec, entries, stream);
-    return dispatch<32, T>(p, removal != 0, vec, entries, stream);
-  });
+               nullptr, nullptr, nullptr, 0, 0, nullptr, nullptr, 0, 1, 0, 0.f, 0.f, work, compact, status};
+  JV_DISPATCH_DTYPE(v_dtype, T, return by_size<T>(p, removal != 0 ? REMOVAL_TERM : PLAIN, entries, stream));
+  return JV_ERR_UNSUPPORTED;
+}
+
+// The same for a state-space layer, from the convolved rows [x | .. ] of `dtype` (B at b_off, C at c_off, [groups][D] each; x first)
+// and the raw step sizes; dt_bias, a_log: [heads] of w_dtype.
+JV_EXPORT int jv_mamba_step(const void* xbc, int dtype, long long xbc_stride, int b_off, int c_off, const void* dt_raw, long long dt_stride,
+                            const void* dt_bias, const void* a_log, int w_dtype, float* out, float* state, long long slot_stride,
+                            const int* cu_seqlens, const int* slots, int n_slots, int entries, int heads, int groups, int D, int V,
+                            const int* work, int* status, cudaStream_t stream) {
+  if (entries == 0) return JV_OK;
+  if (heads < 1 || groups < 1 || heads % groups || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || w_dtype < 0 || w_dtype > 1)
+    return JV_ERR_UNSUPPORTED;
+  const size_t size = dtype == 0 ? 4 : 2;
+  StepParams p{nullptr, xbc, xbc_stride, 0, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
+               (const char*)xbc + b_off * size, (const char*)xbc + c_off * size, dt_raw, xbc_stride, dt_stride, dt_bias, a_log, w_dtype,
+               heads / groups, 0, 0.f, 0.f, work, 0, status};
+  JV_DISPATCH_DTYPE(dtype, T, return by_size<T>(p, MAMBA, entries, stream));
+  return JV_ERR_UNSUPPORTED;
+}
+
+// The same for gated linear attention, from rows of the projection: q, k and v [heads][..] and `rank` low-rank numbers at their columns;
+// w_up: [heads * D, rank], bias: [heads * D] of w_dtype.
+JV_EXPORT int jv_gla_step(const void* proj, int dtype, long long stride, int q_off, int k_off, int v_off, int low_off, int rank, const void* w_up,
+                          const void* bias, int w_dtype, float inv_tau, float q_scale, float* out, float* state, long long slot_stride,
+                          const int* cu_seqlens, const int* slots, int n_slots, int entries, int heads, int D, int V, int* status,
+                          cudaStream_t stream) {
+  if (entries == 0) return JV_OK;
+  if (heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || rank < 1 || w_dtype < 0 || w_dtype > 1) return JV_ERR_UNSUPPORTED;
+  const size_t size = dtype == 0 ? 4 : 2;
+  const char* row = (const char*)proj;
+  StepParams p{nullptr, proj, stride, v_off, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
+               row + q_off * size, row + k_off * size, row + low_off * size, stride, stride, w_up, bias, w_dtype, 1, rank, inv_tau, q_scale,
+               nullptr, 0, status};
+  JV_DISPATCH_DTYPE(dtype, T, return by_size<T>(p, GLA, entries, stream));
   return JV_ERR_UNSUPPORTED;
 }

@@ -1773,6 +1773,19 @@ def state_step(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
     return out
 
 
+# Up to how many blocks a multiprocessor a step of single tokens forms its vectors itself (`mamba_step`, `gla_step`): every block of a head
+# forms them again, which few blocks do while their states arrive.  State-space: 16 tokens of 64 heads of 128 x 64 (7 blocks) 12.8 us
+# against 14.5 in two launches, 32 tokens 28.8 against 27.5; linear attention (16 products a number): 16 tokens of 8 heads of 128 x 256
+# (3.5 blocks) 9.1 against 10.7, 32 tokens 14.7 against 14.2, 8 tokens of 256 x 512 (7 blocks) 22.7 against 21.3.
+MAMBA_STEP_BLOCKS, GLA_STEP_BLOCKS = 8, 4
+
+
+def state_step_blocks(device, n_entries: int, heads: int, dim: int, value_dim: int) -> float:
+    """The blocks that `state_step` has for each multiprocessor (csrc/state_step.cu: 128, 64 or 32 columns a block)."""
+    columns = 128 if dim <= 64 else 64 if dim <= 128 else 32
+    return n_entries * heads * -(-value_dim // columns) / multiprocessors(device)
+
+
 def delta_prepare(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, zw: torch.Tensor, a_bias: torch.Tensor,
                   w_bias: torch.Tensor, heads: int, dim: int, singles: tuple | None = None) -> torch.Tensor:
     """Per token and head the vectors (r, k, w, u, b) of the generalized delta rule as float32 [n, heads, 5, dim]:
@@ -1847,6 +1860,28 @@ def gla_prepare(proj: torch.Tensor, q_off: int, k_off: int, low_off: int, w_up: 
              bias.data_ptr(), _code(w_up, "w_up"), 1.0 / float(tau), float(q_scale), packed.data_ptr(), n, heads, dim,
              _stream()), "gla_prepare")
     return packed
+
+
+def gla_step(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, low_off: int, w_up: torch.Tensor, bias: torch.Tensor, tau: float,
+             q_scale: float, heads: int, dim: int, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, n_entries: int,
+             value_dim: int, out: torch.Tensor) -> torch.Tensor:
+    """`gla_prepare` and `state_step` in one launch, for the first n_entries entries of one token (csrc/state_step.cu)."""
+    _cuda(proj, "proj", contiguous=False); _cuda(w_up, "w_up"); _cuda(bias, "bias", w_up.dtype)
+    _cuda(state, "state", torch.float32, contiguous=False); _cuda(out, "out", torch.float32)
+    _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
+    (n, width), rank = proj.shape, w_up.shape[1]
+    if proj.stride(1) != 1 or w_up.shape[0] != heads * dim or bias.numel() != heads * dim or \
+            max(max(q_off, k_off) + heads * dim, v_off + heads * value_dim, low_off + rank) > width or state.stride(1) != 1 or \
+            state.shape[1] < heads * dim * value_dim or dim > SCAN_MAX_KEY or out.shape != (n, heads * value_dim):
+        raise KernelError("gla_step: shapes do not fit")
+    f = _fn("state_step", "jv_gla_step", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_float,
+                                          c_float, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                          c_void_p, c_void_p])
+    _check(f(proj.data_ptr(), _code(proj, "proj"), proj.stride(0), q_off, k_off, v_off, low_off, rank, w_up.data_ptr(), bias.data_ptr(),
+             _code(w_up, "w_up"), 1.0 / float(tau), float(q_scale), out.data_ptr(), state.data_ptr(), state.stride(0),
+             cu_seqlens.data_ptr(), slots.data_ptr(), state.shape[0], n_entries, heads, dim, value_dim, _status_ptr(proj.device),
+             _stream()), "gla_step")
+    return out
 
 
 def memory_gates(proj: torch.Tensor, q_off: int, k_off: int, i_off: int, f_off: int, i_bias: torch.Tensor,
@@ -2333,6 +2368,34 @@ def mamba_prepare(xbc: torch.Tensor, b_off: int, c_off: int, dt_raw: torch.Tenso
              dt_bias.data_ptr(), a_log.data_ptr(), _code(dt_bias, "dt_bias"), packed.data_ptr(), n, heads, groups, state,
              work, cu, _stream()), "mamba_prepare")
     return packed
+
+
+def mamba_step(xbc: torch.Tensor, b_off: int, c_off: int, dt_raw: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, groups: int,
+               dim: int, state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, work: torch.Tensor | None, n_work: int,
+               value_dim: int, out: torch.Tensor) -> torch.Tensor:
+    """`mamba_prepare` and `state_step` in one launch, for entries of one token (csrc/state_step.cu): `work` [n_work, 2] lists them
+    (None: the first n_work entries).  The values are the first columns of `xbc`.  Writes the entries' rows of `out`."""
+    _cuda(xbc, "xbc", contiguous=False); _cuda(dt_raw, "dt", xbc.dtype, contiguous=False)
+    _cuda(dt_bias, "dt_bias"); _cuda(a_log, "A_log", dt_bias.dtype)
+    _cuda(state, "state", torch.float32, contiguous=False); _cuda(out, "out", torch.float32)
+    _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
+    (n, width), heads = xbc.shape, dt_bias.numel()
+    if xbc.stride(1) != 1 or dt_raw.stride(1) != 1 or dt_raw.shape != (n, heads) or heads % groups or a_log.numel() != heads or \
+            max(max(b_off, c_off) + groups * dim, heads * value_dim) > width or state.stride(1) != 1 or \
+            state.shape[1] < heads * dim * value_dim or dim > SCAN_MAX_KEY or out.shape != (n, heads * value_dim):
+        raise KernelError("mamba_step: shapes do not fit")
+    if work is not None:
+        _cuda(work, "work", torch.int32)
+        if work.shape[0] < n_work or work.shape[1] != 2:
+            raise KernelError("mamba_step: a list of entries is [n_work, 2]")
+    f = _fn("state_step", "jv_mamba_step", [c_void_p, c_int, c_longlong, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p, c_int,
+                                            c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                                            c_void_p, c_void_p, c_void_p])
+    _check(f(xbc.data_ptr(), _code(xbc, "xbc"), xbc.stride(0), b_off, c_off, dt_raw.data_ptr(), dt_raw.stride(0), dt_bias.data_ptr(),
+             a_log.data_ptr(), _code(dt_bias, "dt_bias"), out.data_ptr(), state.data_ptr(), state.stride(0), cu_seqlens.data_ptr(),
+             slots.data_ptr(), state.shape[0], n_work, heads, groups, dim, value_dim, _ptr(work), _status_ptr(xbc.device), _stream()),
+           "mamba_step")
+    return out
 
 
 _MAMBA_FINISH_TYPES = [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_float,

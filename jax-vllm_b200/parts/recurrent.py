@@ -218,10 +218,14 @@ class GatedLinearAttention(_StateMixer):
 
     def from_projection(self, row, step, cache, out):
         hd, hv = self.hd, self.hv
-        packed = ops.gla_prepare(row, 0, hd, 2 * hd + 2 * hv, self.w_up, self.bias, self.spec.tau, self.spec.q_scale, self.h,
-                                 self.d)
-        o = ops.state_scan(packed, row, 2 * hd, cache.state, step.cu_seqlens, step.state_slots, step.n_entries, self.dv,
-                           singles=step.decode_work)
+        low, where = 2 * hd + 2 * hv, (cache.state, step.cu_seqlens, step.state_slots, step.n_entries)
+        if step.decode_work[1] == step.n_entries and \
+                ops.state_step_blocks(row.device, step.n_entries, self.h, self.d, self.dv) <= ops.GLA_STEP_BLOCKS:     # few decoded tokens
+            o = torch.empty((step.n_tokens, hv), dtype=torch.float32, device=row.device)
+            ops.gla_step(row, 0, hd, 2 * hd, low, self.w_up, self.bias, self.spec.tau, self.spec.q_scale, self.h, self.d, *where, self.dv, o)
+        else:
+            packed = ops.gla_prepare(row, 0, hd, low, self.w_up, self.bias, self.spec.tau, self.spec.q_scale, self.h, self.d)
+            o = ops.state_scan(packed, row, 2 * hd, *where, self.dv, singles=step.decode_work)
         return ops.head_norm_gate(o, self.norm, row[:, 2 * hd + hv:2 * hd + 2 * hv], out, self.h, self.dv, self.spec.norm_eps,
                                   gate_act="silu")
 

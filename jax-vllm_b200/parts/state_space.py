@@ -99,12 +99,15 @@ class StateSpace(Part):
         dt_raw = row[:, 2 * inner + 2 * gn:2 * inner + 2 * gn + self.h]
         where, (work, singles) = (state, step.cu_seqlens, step.state_slots), step.decode_work
         prepare = (xbc, inner, inner + gn, dt_raw, self.dt_bias, self.a_log, self.h, self.g, self.n)
+        one = (xbc, inner, inner + gn, dt_raw, self.dt_bias, self.a_log, self.g, self.n)
         if ops.chunk_scan_takes(xbc, (0, inner, inner + gn), step.n_entries - singles, self.n, self.e, n_tokens=step.n_tokens - singles):
             o = ops.chunk_scan(xbc, inner + gn, inner, 0, *where, step.n_entries, self.h, self.g, self.n, self.e, dt_raw=dt_raw,
                                dt_bias=self.dt_bias, a_log=self.a_log, portions=step.n_entries - singles if singles else 0)
             if singles:                     # decoded tokens beside the portions
-                packed = ops.mamba_prepare(*prepare, singles=(work, singles, step.cu_seqlens))
-                ops.state_step(packed, xbc, 0, *where, work, singles, self.e, o)
+                ops.mamba_step(*one, *where, work, singles, self.e, o)
+        elif singles == step.n_entries and ops.state_step_blocks(row.device, singles, self.h, self.n, self.e) <= ops.MAMBA_STEP_BLOCKS:
+            o = torch.empty((step.n_tokens, inner), dtype=torch.float32, device=row.device)
+            ops.mamba_step(*one, *where, None, singles, self.e, o)
         else:
             o = ops.state_scan(ops.mamba_prepare(*prepare), xbc, 0, *where, step.n_entries, self.e, singles=step.decode_work)
         return ops.mamba_finish(o, xbc[:, :inner], row[:, :inner], self.skip, self.norm, out, self.h, self.e, self.ng,

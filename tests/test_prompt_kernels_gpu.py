@@ -288,6 +288,47 @@ def test_portions_of_the_state_space_mixer(heads, groups, dim, columns, taps, le
                                norm, groups, 1e-5, outs[0][:, :inner])
 
 
+@pytest.mark.parametrize("heads,groups,dim,columns", [(4, 2, 16, 8), (6, 3, 65, 7), (8, 1, 128, 64), (2, 2, 256, 130)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("listed", [False, True])
+def test_single_tokens_of_the_state_space_mixer(heads, groups, dim, columns, dtype, listed):
+    """The vectors formed in the step against those read from memory: the same bits."""
+    ops, lengths = _ops(), [1, 3, 1, 1] if listed else [1, 1, 1]
+    cu, slots, n_slots = _entries(lengths)
+    n, inner, side = sum(lengths), heads * columns, groups * dim
+    xbc = _rand(n, inner + 2 * side + 3, seed=1, dtype=dtype)[:, :inner + 2 * side]
+    dt_raw = _rand(n, heads + 2, seed=2, dtype=dtype)[:, 1:1 + heads]
+    dt_bias, a_log = _rand(heads, seed=3), _rand(heads, seed=4)
+    entries = [e for e, m in enumerate(lengths) if m == 1]
+    work = torch.tensor([[e, 0] for e in entries], dtype=torch.int32, device="cuda") if listed else None
+    states = [_rand(n_slots, heads * dim * columns + 5, seed=5) for _ in range(2)]
+    outs = [torch.full((n, inner), 7.0, device="cuda") for _ in range(2)]
+    ops.mamba_step(xbc, inner, inner + side, dt_raw, dt_bias, a_log, groups, dim, states[0], cu, slots, work, len(entries), columns, outs[0])
+    packed = ops.mamba_prepare(xbc, inner, inner + side, dt_raw, dt_bias, a_log, heads, groups, dim)
+    ops.state_step(packed, xbc, 0, states[1], cu, slots, work, len(entries), columns, outs[1])
+    ops.check_status()
+    assert torch.equal(states[0], states[1]) and torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0]).all()
+
+
+@pytest.mark.parametrize("heads,dim,columns,rank", [(4, 16, 8, 3), (6, 65, 7, 16), (3, 128, 64, 16), (2, 256, 130, 33)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_single_tokens_of_linear_attention(heads, dim, columns, rank, dtype):
+    """As above, for the vectors of gated linear attention."""
+    ops = _ops()
+    cu, slots, n_slots = _entries([1, 1, 1, 1, 1])
+    hd, hv = heads * dim, heads * columns
+    row = _rand(5, 2 * hd + 2 * hv + rank + 1, seed=1, dtype=dtype)[:, 1:]
+    for wd in (torch.float32, torch.bfloat16):
+        w_up, bias = _rand(hd, rank, seed=2, dtype=wd), _rand(hd, seed=3, dtype=wd)
+        states = [_rand(n_slots, heads * dim * columns, seed=5) for _ in range(2)]
+        outs = [torch.zeros(5, hv, device="cuda") for _ in range(2)]
+        ops.gla_step(row, 0, hd, 2 * hd, 2 * hd + 2 * hv, w_up, bias, 16.0, 0.3, heads, dim, states[0], cu, slots, 5, columns, outs[0])
+        packed = ops.gla_prepare(row, 0, hd, 2 * hd + 2 * hv, w_up, bias, 16.0, 0.3, heads, dim)
+        ops.state_step(packed, row, 2 * hd, states[1], cu, slots, None, 5, columns, outs[1])
+        ops.check_status()
+        assert torch.equal(states[0], states[1]) and torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0]).all()
+
+
 # ------------------------------------------------------- convolution and finish of the state-space mixer
 @pytest.mark.parametrize("taps", [2, 3, 4])
 @pytest.mark.parametrize("channels,off", [(8192, 0), (8196, 4), (8192, 2), (512, 0)])
