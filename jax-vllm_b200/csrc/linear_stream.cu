@@ -19,7 +19,7 @@
 // The grouped form (routed experts, few tokens) takes a stack of weights and x in row tiles of one expert each: a unit is a strip of
 // the expert's weight with the rows of one tile, which leaves the strips of experts that nobody chose unread; it writes bfloat16, after
 // the exact gelu if asked.  8 tokens of 4 choices among 32 experts, up and down products of
-// 3 x 2,048 x 1,024 (252 MB of the 20 experts chosen): 52 us, 74 on 128-row tiles of x (gemm_tcgen05.cu); 64 tokens 79 against 90.
+// 3 x 2,048 x 1,024 (252 MB of the 20 experts chosen): 48 us, 74 on 128-row tiles of x (gemm_tcgen05.cu); 64 tokens 76 against 90.
 // Weights are asked for before the wait on the kernel that produces x (nobody writes them; in the grouped form which ones is known
 // only after it).  Every wait on an
 // mbarrier is bounded by a clock deadline; a wait that runs out sets a bit in the status word and the block
