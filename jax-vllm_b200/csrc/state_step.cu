@@ -15,7 +15,8 @@
 // exp(-exp(A_log) dt) in every channel, dt = softplus(dt_raw + dt_bias), as mamba_prepare (mamba2.cu) forms them, which spares single
 // tokens a launch (one token of 32 heads of 64 x 64: 1.7 and 2.75 us in two launches, 3.1 in one); those of gated linear attention (GLA) as
 // gla_prepare (recurrent.cu) forms them (eight tokens of 8 heads of 128 x 256: 2.4 and 5.2, 5.1 in
-// one).
+// one), those of the delta rule (DELTA) as delta_prepare does (16 tokens of
+// 32 heads of 64 x 64: 2.8 and 7.3, 8.0 in one).
 #include "scan.cuh"
 #include <math.h>
 
@@ -34,12 +35,14 @@ struct StepParams {
   const void *dt_bias, *a_log; int w_dtype, per_group;
   // GLA: q and k in b and c, the low-rank numbers in dt_raw; their matrix [heads * D, rank] and bias [heads * D] in dt_bias and a_log
   int rank; float inv_tau, q_scale;
+  // DELTA: r and k in c and b, z_a in dt_raw, their biases a_bias and w_bias [heads * D] in dt_bias and a_log, zw rows of its own
+  const void* zw; long long zw_stride;
   const int* work; int compact;            // pairs (entry, -), or null: every entry; a row of packed for every pair, not every token
   int* status;
 };
 
 // RG: row groups (D <= ROWS * RG); a thread's rows are rg, rg + RG, ...
-enum : int { PLAIN, REMOVAL_TERM, MAMBA, GLA };
+enum : int { PLAIN, REMOVAL_TERM, MAMBA, GLA, DELTA };
 
 __device__ __forceinline__ float weight_at(const void* w, int dtype, size_t i) {
   return dtype == 0 ? ((const float*)w)[i] : to_f32(((const __nv_bfloat16*)w)[i]);
@@ -47,7 +50,7 @@ __device__ __forceinline__ float weight_at(const void* w, int dtype, size_t i) {
 
 template <int RG, int VEC, int KIND, typename T>
 __global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p) {
-  constexpr bool REMOVAL = KIND == REMOVAL_TERM;
+  constexpr bool REMOVAL = KIND == REMOVAL_TERM || KIND == DELTA;
   constexpr int CQ = THREADS / RG, COLS = CQ * VEC, NV = REMOVAL ? 5 : 3;
   __shared__ float vec[NV * ROWS * RG];
   __shared__ __align__(16) float part[RG * COLS];
@@ -112,6 +115,32 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p)
         vec[tid] = q * p.q_scale;
         vec[ROWS * RG + tid] = k;
         vec[2 * ROWS * RG + tid] = expf(log_sigmoid(z + bias) * p.inv_tau);
+      }
+    } else if constexpr (KIND == DELTA) {
+      const T* row = (const T*)p.b + (size_t)t * p.bc_stride + (size_t)h * D;
+      const int half = D > 64 ? 128 : 64;                // the sum of squares in the order of delta_prepare's block
+      const size_t e = (size_t)h * D + tid;
+      float ss = 0.f, k = 0.f, r = 0.f, za = 0.f, zd = 0.f;
+      if (tid < D) {
+        k = to_f32(row[tid]);
+        r = to_f32(((const T*)p.c)[(size_t)t * p.bc_stride + e]);
+        za = to_f32(((const T*)p.dt_raw)[(size_t)t * p.dt_stride + e]) + weight_at(p.dt_bias, p.w_dtype, e);
+        zd = to_f32(((const T*)p.zw)[(size_t)t * p.zw_stride + e]) + weight_at(p.a_log, p.w_dtype, e);
+      }
+      if (tid < half)
+        for (int d = tid; d < D; d += half) {
+          const float x = to_f32(row[d]);
+          ss = fmaf(x, x, ss);
+        }
+      ss = block_sum(ss, scratch);
+      const float inv = 1.f / sqrtf(ss + 1e-6f), c = 0.60653065971263342f;      // e^(-1/2)
+      if (tid < D) {
+        const float a = 1.f / (1.f + expf(-za)), u = k * inv;
+        vec[tid] = r;
+        vec[ROWS * RG + tid] = k;
+        vec[2 * ROWS * RG + tid] = expf(-c / (1.f + expf(-zd)));
+        vec[3 * ROWS * RG + tid] = u;
+        vec[4 * ROWS * RG + tid] = a * u;
       }
     } else {
       for (int i = tid; i < NV * D; i += THREADS) vec[(i / D) * (ROWS * RG) + i % D] = src[i];
@@ -196,10 +225,12 @@ int dispatch(const StepParams& p, int kind, bool vec, int entries, cudaStream_t 
     return kind == REMOVAL_TERM ? jv_launch(state_step_kernel<RG, 4, REMOVAL_TERM, T>, grid, dim3(THREADS), 0, stream, p)
            : kind == MAMBA      ? jv_launch(state_step_kernel<RG, 4, MAMBA, T>, grid, dim3(THREADS), 0, stream, p)
            : kind == GLA        ? jv_launch(state_step_kernel<RG, 4, GLA, T>, grid, dim3(THREADS), 0, stream, p)
+           : kind == DELTA      ? jv_launch(state_step_kernel<RG, 4, DELTA, T>, grid, dim3(THREADS), 0, stream, p)
                                 : jv_launch(state_step_kernel<RG, 4, PLAIN, T>, grid, dim3(THREADS), 0, stream, p);
   return kind == REMOVAL_TERM ? jv_launch(state_step_kernel<RG, 1, REMOVAL_TERM, T>, grid, dim3(THREADS), 0, stream, p)
          : kind == MAMBA      ? jv_launch(state_step_kernel<RG, 1, MAMBA, T>, grid, dim3(THREADS), 0, stream, p)
          : kind == GLA        ? jv_launch(state_step_kernel<RG, 1, GLA, T>, grid, dim3(THREADS), 0, stream, p)
+         : kind == DELTA      ? jv_launch(state_step_kernel<RG, 1, DELTA, T>, grid, dim3(THREADS), 0, stream, p)
                               : jv_launch(state_step_kernel<RG, 1, PLAIN, T>, grid, dim3(THREADS), 0, stream, p);
 }
 
@@ -220,7 +251,7 @@ JV_EXPORT int jv_state_step(const float* packed, int removal, const void* v, int
   if (entries == 0) return JV_OK;
   if ((compact && work == nullptr) || heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || (removal && state_n != nullptr)) return JV_ERR_UNSUPPORTED;
   StepParams p{packed, v, v_stride, v_off, out, state, slot_stride, state_n, nq, nq_stride, cu_seqlens, slots, n_slots, heads, D, V,
-               nullptr, nullptr, nullptr, 0, 0, nullptr, nullptr, 0, 1, 0, 0.f, 0.f, work, compact, status};
+               nullptr, nullptr, nullptr, 0, 0, nullptr, nullptr, 0, 1, 0, 0.f, 0.f, nullptr, 0, work, compact, status};
   JV_DISPATCH_DTYPE(v_dtype, T, return by_size<T>(p, removal != 0 ? REMOVAL_TERM : PLAIN, entries, stream));
   return JV_ERR_UNSUPPORTED;
 }
@@ -237,7 +268,7 @@ JV_EXPORT int jv_mamba_step(const void* xbc, int dtype, long long xbc_stride, in
   const size_t size = dtype == 0 ? 4 : 2;
   StepParams p{nullptr, xbc, xbc_stride, 0, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
                (const char*)xbc + b_off * size, (const char*)xbc + c_off * size, dt_raw, xbc_stride, dt_stride, dt_bias, a_log, w_dtype,
-               heads / groups, 0, 0.f, 0.f, work, 0, status};
+               heads / groups, 0, 0.f, 0.f, nullptr, 0, work, 0, status};
   JV_DISPATCH_DTYPE(dtype, T, return by_size<T>(p, MAMBA, entries, stream));
   return JV_ERR_UNSUPPORTED;
 }
@@ -254,7 +285,24 @@ JV_EXPORT int jv_gla_step(const void* proj, int dtype, long long stride, int q_o
   const char* row = (const char*)proj;
   StepParams p{nullptr, proj, stride, v_off, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
                row + q_off * size, row + k_off * size, row + low_off * size, stride, stride, w_up, bias, w_dtype, 1, rank, inv_tau, q_scale,
-               nullptr, 0, status};
+               nullptr, 0, nullptr, 0, status};
   JV_DISPATCH_DTYPE(dtype, T, return by_size<T>(p, GLA, entries, stream));
+  return JV_ERR_UNSUPPORTED;
+}
+
+// The same for the delta rule, from rows of the projection (r, k, v and z_a [heads][D] each at their columns) and of zw; a_bias, w_bias:
+// [heads * D] of w_dtype.
+JV_EXPORT int jv_delta_step(const void* proj, int dtype, long long stride, int r_off, int k_off, int v_off, int a_off, const void* zw,
+                            long long zw_stride, const void* a_bias, const void* w_bias, int w_dtype, float* out, float* state,
+                            long long slot_stride, const int* cu_seqlens, const int* slots, int n_slots, int entries, int heads, int D, int V,
+                            const int* work, int* status, cudaStream_t stream) {
+  if (entries == 0) return JV_OK;
+  if (heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || w_dtype < 0 || w_dtype > 1) return JV_ERR_UNSUPPORTED;
+  const size_t size = dtype == 0 ? 4 : 2;
+  const char* row = (const char*)proj;
+  StepParams p{nullptr, proj, stride, v_off, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
+               row + k_off * size, row + r_off * size, row + a_off * size, stride, stride, a_bias, w_bias, w_dtype, 1, 0, 0.f, 0.f,
+               zw, zw_stride, work, 0, status};
+  JV_DISPATCH_DTYPE(dtype, T, return by_size<T>(p, DELTA, entries, stream));
   return JV_ERR_UNSUPPORTED;
 }

@@ -1773,11 +1773,12 @@ def state_step(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
     return out
 
 
-# Up to how many blocks a multiprocessor a step of single tokens forms its vectors itself (`mamba_step`, `gla_step`): every block of a head
+# Up to how many blocks a multiprocessor a step of single tokens forms its vectors itself (`mamba_step`, `gla_step`, `delta_step`): every block of a head
 # forms them again, which few blocks do while their states arrive.  State-space: 16 tokens of 64 heads of 128 x 64 (7 blocks) 12.8 us
 # against 14.5 in two launches, 32 tokens 28.8 against 27.5; linear attention (16 products a number): 16 tokens of 8 heads of 128 x 256
-# (3.5 blocks) 9.1 against 10.7, 32 tokens 14.7 against 14.2, 8 tokens of 256 x 512 (7 blocks) 22.7 against 21.3.
-MAMBA_STEP_BLOCKS, GLA_STEP_BLOCKS = 8, 4
+# (3.5 blocks) 9.1 against 10.7, 32 tokens 14.7 against 14.2, 8 tokens of 256 x 512 (7 blocks) 22.7 against 21.3; delta rule: 16 tokens of 32
+# heads of 64 x 64 8.0 against 10.1, 32 of 64 heads (14 blocks) 26.7 against 27.1, 64 of 64 heads 51.4 against 51.3.
+MAMBA_STEP_BLOCKS, GLA_STEP_BLOCKS, DELTA_STEP_BLOCKS = 8, 4, 16
 
 
 def state_step_blocks(device, n_entries: int, heads: int, dim: int, value_dim: int) -> float:
@@ -1807,6 +1808,33 @@ def delta_prepare(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, zw: to
              a_bias.data_ptr(), w_bias.data_ptr(), _code(a_bias, "a_bias"), packed.data_ptr(), n, heads, dim, work, cu, _stream()),
            "delta_prepare")
     return packed
+
+
+def delta_step(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, v_off: int, zw: torch.Tensor, a_bias: torch.Tensor, w_bias: torch.Tensor,
+               state: torch.Tensor, cu_seqlens: torch.Tensor, slots: torch.Tensor, work: torch.Tensor | None, n_work: int, heads: int, dim: int,
+               columns: int, out: torch.Tensor) -> torch.Tensor:
+    """`delta_prepare` and `state_step` in one launch, for entries of one token (csrc/state_step.cu): `work` [n_work, 2] lists them
+    (None: the first n_work entries).  Writes the entries' rows of `out`."""
+    _cuda(proj, "proj", contiguous=False); _cuda(zw, "zw", proj.dtype, contiguous=False)
+    _cuda(a_bias, "a_bias"); _cuda(w_bias, "w_bias", a_bias.dtype)
+    _cuda(state, "state", torch.float32, contiguous=False); _cuda(out, "out", torch.float32)
+    _cuda(cu_seqlens, "cu_seqlens", torch.int32); _cuda(slots, "slots", torch.int32)
+    (n, width), wide = proj.shape, heads * dim
+    if proj.stride(1) != 1 or zw.stride(1) != 1 or zw.shape != (n, wide) or a_bias.numel() != wide or w_bias.numel() != wide or \
+            max(max(r_off, k_off, a_off) + wide, v_off + heads * columns) > width or state.stride(1) != 1 or \
+            state.shape[1] < wide * columns or dim > SCAN_MAX_KEY or out.shape != (n, heads * columns):
+        raise KernelError("delta_step: shapes do not fit")
+    if work is not None:
+        _cuda(work, "work", torch.int32)
+        if work.shape[0] < n_work or work.shape[1] != 2:
+            raise KernelError("delta_step: a list of entries is [n_work, 2]")
+    f = _fn("state_step", "jv_delta_step", [c_void_p, c_int, c_longlong, c_int, c_int, c_int, c_int, c_void_p, c_longlong, c_void_p, c_void_p,
+                                            c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                            c_void_p, c_void_p, c_void_p])
+    _check(f(proj.data_ptr(), _code(proj, "proj"), proj.stride(0), r_off, k_off, v_off, a_off, zw.data_ptr(), zw.stride(0), a_bias.data_ptr(),
+             w_bias.data_ptr(), _code(a_bias, "a_bias"), out.data_ptr(), state.data_ptr(), state.stride(0), cu_seqlens.data_ptr(),
+             slots.data_ptr(), state.shape[0], n_work, heads, dim, columns, _ptr(work), _status_ptr(proj.device), _stream()), "delta_step")
+    return out
 
 
 def delta_scan(proj: torch.Tensor, r_off: int, k_off: int, a_off: int, v_off: int, zw: torch.Tensor, a_bias: torch.Tensor,

@@ -100,7 +100,10 @@ class DeltaRule(_StateMixer):
         o = torch.empty((step.n_tokens, hd), dtype=torch.float32, device=row.device)
         where, (work, singles) = (cache.state, step.cu_seqlens, step.state_slots), step.decode_work
         mixed = 0 < singles < step.n_entries
-        if singles:                         # decoded tokens
+        if singles and ops.state_step_blocks(row.device, singles, self.h, self.d, self.d) <= ops.DELTA_STEP_BLOCKS:     # few decoded tokens
+            ops.delta_step(row, 0, hd, 4 * hd, 2 * hd, zw, self.a_bias, self.w_bias, *where, work if mixed else None, singles, self.h,
+                           self.d, self.d, o)
+        elif singles:                       # decoded tokens
             packed = ops.delta_prepare(row, 0, hd, 4 * hd, zw, self.a_bias, self.w_bias, self.h, self.d,
                                        singles=(work, singles, step.cu_seqlens) if mixed else None)
             ops.state_step(packed, row, 2 * hd, *where, work if mixed else None, singles, self.d, o)

@@ -329,6 +329,28 @@ def test_single_tokens_of_linear_attention(heads, dim, columns, rank, dtype):
         assert torch.equal(states[0], states[1]) and torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0]).all()
 
 
+@pytest.mark.parametrize("heads,dim,columns", [(4, 16, 8), (6, 65, 7), (3, 64, 64), (2, 128, 130), (2, 200, 40), (1, 256, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("listed", [False, True])
+def test_single_tokens_of_the_delta_rule(heads, dim, columns, dtype, listed):
+    """As above, for the delta rule: the sum of squares behind a key's norm in the same order too."""
+    ops, lengths = _ops(), [1, 2, 1, 1] if listed else [1, 1, 1]
+    cu, slots, n_slots = _entries(lengths)
+    n, hd, hv = sum(lengths), heads * dim, heads * columns
+    row, zw = _rand(n, 3 * hd + hv + 1, seed=1, dtype=dtype)[:, 1:], _rand(n, hd + 2, seed=2, dtype=dtype)[:, :hd]
+    entries = [e for e, m in enumerate(lengths) if m == 1]
+    work = torch.tensor([[e, 0] for e in entries], dtype=torch.int32, device="cuda") if listed else None
+    for wd in (torch.float32, torch.bfloat16):
+        a_bias, w_bias = _rand(hd, seed=3, dtype=wd), _rand(hd, seed=4, dtype=wd)
+        states = [_rand(n_slots, heads * dim * columns, seed=5) for _ in range(2)]
+        outs = [torch.full((n, hv), 7.0, device="cuda") for _ in range(2)]
+        ops.delta_step(row, 0, hd, 2 * hd, 3 * hd, zw, a_bias, w_bias, states[0], cu, slots, work, len(entries), heads, dim, columns, outs[0])
+        packed = ops.delta_prepare(row, 0, hd, 2 * hd, zw, a_bias, w_bias, heads, dim)
+        ops.state_step(packed, row, 3 * hd, states[1], cu, slots, work, len(entries), columns, outs[1])
+        ops.check_status()
+        assert torch.equal(states[0], states[1]) and torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0]).all()
+
+
 # ------------------------------------------------------- convolution and finish of the state-space mixer
 @pytest.mark.parametrize("taps", [2, 3, 4])
 @pytest.mark.parametrize("channels,off", [(8192, 0), (8196, 4), (8192, 2), (512, 0)])
