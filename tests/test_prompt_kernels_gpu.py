@@ -378,6 +378,22 @@ def test_short_conv_many_tokens(taps, channels, off):
             at += length
 
 
+@pytest.mark.parametrize("channels,lengths", [(512, [300, 40]), (2176, [1, 1, 1]), (77, [70, 3])])
+def test_short_conv_16_bit_results_are_the_32_bit_ones_rounded(channels, lengths):
+    """No digit is lost before the rounding to 16 bits, near its boundaries, far out on either side, at zero and next to it."""
+    ops = _ops()
+    cu, slots, n_slots = _entries(lengths)
+    w, b, before = _rand(channels, 4, seed=2), _rand(channels, seed=3), _rand(n_slots, 3 * channels, seed=4)
+    for scale, dtype in ((1.0, torch.bfloat16), (1.0, torch.float32), (40.0, torch.float32), (1e-33, torch.float32), (1e-39, torch.float32),
+                         (float("inf"), torch.float32)):
+        x = _rand(sum(lengths), channels, seed=1, dtype=dtype, scale=scale)
+        x[::7] = 0.0
+        small = scale if scale < 1 else 1.0
+        got = [ops.short_conv(x, w, before * small, cu, slots, len(lengths), od, bias=b * small, act="silu") for od in (torch.bfloat16, torch.float32)]
+        want = got[1].to(torch.bfloat16)
+        assert torch.equal(got[0].isnan(), want.isnan()) and torch.equal(got[0].nan_to_num(), want.nan_to_num())
+
+
 @pytest.mark.parametrize("n", [63, 64])
 @pytest.mark.parametrize("heads,value_dim,groups,off", [(2, 8, 2, 0), (3, 24, 1, 0), (16, 64, 8, 8), (16, 64, 1, 1), (5, 7, 1, 0), (96, 128, 1, 0)])
 def test_mamba_finish_vectors(n, heads, value_dim, groups, off):
