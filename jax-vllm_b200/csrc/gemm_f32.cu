@@ -52,6 +52,7 @@ struct Params {
   size_t a_batch, w_batch, c_batch;                    // independent products: grid.y of them, operands this far apart
   int a_vec, w_vec;                                    // four elements a load along k
   int strips, parts, part_k, row_tile;                 // row_tile: rows of A of a block, a multiple of 16
+  int w_fixed;                                         // no kernel before this one writes W: it is asked for before they have finished
   int* status;
   // grouped (routed experts): the expert of every tile of rows of A (-1: nothing to do), the token of every row (-1: nobody's, left alone)
   const int *tile_expert, *row_token;
@@ -240,8 +241,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     mbar_init(&sh->drain, 1);
     sh->failed = 0;
     mbar_fence_init();
-    for (int c = 0; c < early; ++c) bring_w(c, c);     // weights: nobody writes them, so they are requested before the kernels that
-  }                                                    // produce A have finished
+    if (p.w_fixed)
+      for (int c = 0; c < early; ++c) bring_w(c, c);
+  }
   if (warp == S::ISSUER) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sh->tmem_base)), "n"(S::TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
@@ -262,7 +264,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         tma_load_3d(raw + s * S::RAW_STAGE + S::W_RAW, &a_map, k0 + c * CHUNK, m0, blockIdx.y, &sh->a_full[s]);
       };
       pdl_wait();
-      for (int c = 0; c < early; ++c) bring_a(c, c);
+      for (int c = 0; c < early; ++c) {
+        if (!p.w_fixed) bring_w(c, c);
+        bring_a(c, c);
+      }
       brought = early;
       Place<RAW> to;
       for (; brought < chunks; ++brought, to.next()) {
@@ -558,8 +563,8 @@ bool rows_aligned(const void* p, int size, int ld, size_t batch_stride, int batc
 }
 
 int run(const void* A, int a_dtype, int lda, size_t a_batch, const void* W, int w_dtype, int ldw, size_t w_batch, void* C,
-        int c_dtype, int ldc, size_t c_batch, int M, int N, int K, int batch, int* status, cudaStream_t stream) {
-  Params p{A, W, C, lda, ldw, ldc, M, N, K, a_batch, w_batch, c_batch, 0, 0, (N + BM - 1) / BM, 1, 0, 0, status, nullptr, nullptr, 0};
+        int c_dtype, int ldc, size_t c_batch, int M, int N, int K, int batch, int w_fixed, int* status, cudaStream_t stream) {
+  Params p{A, W, C, lda, ldw, ldc, M, N, K, a_batch, w_batch, c_batch, 0, 0, (N + BM - 1) / BM, 1, 0, 0, w_fixed, status, nullptr, nullptr, 0};
   p.part_k = part_of_k(N, K, batch);
   p.parts = K > 0 ? (K + p.part_k - 1) / p.part_k : 1;
   p.a_vec = rows_aligned(A, a_dtype == 0 ? 4 : 2, lda, a_batch, batch);
@@ -570,11 +575,12 @@ int run(const void* A, int a_dtype, int lda, size_t a_batch, const void* W, int 
 }
 }  // namespace
 
-// A: [M, K] rows of lda elements; W: [N, K] rows of ldw elements; C: [M, N] rows of ldc.
+// A: [M, K] rows of lda elements; W: [N, K] rows of ldw elements; C: [M, N] rows of ldc.  w_fixed: none of the kernels launched before
+// this one writes W, which is then read before they have finished.
 JV_EXPORT int jv_gemm_f32(const void* A, int a_dtype, int lda, const void* W, int w_dtype, int ldw, void* C, int c_dtype, int ldc,
-                          int M, int N, int K, int* status, cudaStream_t stream) {
+                          int M, int N, int K, int w_fixed, int* status, cudaStream_t stream) {
   if (M == 0 || N == 0) return JV_OK;
-  return run(A, a_dtype, lda, 0, W, w_dtype, ldw, 0, C, c_dtype, ldc, 0, M, N, K, 1, status, stream);
+  return run(A, a_dtype, lda, 0, W, w_dtype, ldw, 0, C, c_dtype, ldc, 0, M, N, K, 1, w_fixed, status, stream);
 }
 
 // Routed experts: rows of A and C in tiles of `tile` (16 or 64), tile t of expert tile_expert[t] (-1: nothing to do) with the weight
@@ -584,7 +590,7 @@ JV_EXPORT int jv_gemm_f32_grouped(const void* A, int a_dtype, int lda, const voi
                                   int N, int K, int gelu, int* status, cudaStream_t stream) {
   if (tiles == 0 || N == 0) return JV_OK;
   if ((tile != 16 && tile != 64) || experts < 1 || tiles > 0x7fffffff / 64) return JV_ERR_UNSUPPORTED;
-  Params p{A, W, C, lda, ldw, ldc, tiles * tile, N, K, 0, (size_t)w_expert, 0, 0, 0, (N + BM - 1) / BM, 1, 0, tile, status,
+  Params p{A, W, C, lda, ldw, ldc, tiles * tile, N, K, 0, (size_t)w_expert, 0, 0, 0, (N + BM - 1) / BM, 1, 0, tile, 0, status,
            tile_expert, row_token, gelu};
   p.part_k = part_of_k(N, K, GROUPED_AT_ONCE);
   p.parts = K > 0 ? (K + p.part_k - 1) / p.part_k : 1;
@@ -599,9 +605,9 @@ JV_EXPORT int jv_gemm_f32_grouped(const void* A, int a_dtype, int lda, const voi
 // C + b*c_batch (strides in elements; rows of one product may lie between rows of another).
 JV_EXPORT int jv_gemm_f32_batched(const void* A, int a_dtype, int lda, long long a_batch, const void* W, int w_dtype, int ldw,
                                   long long w_batch, void* C, int c_dtype, int ldc, long long c_batch, int M, int N, int K,
-                                  int batch, int* status, cudaStream_t stream) {
+                                  int batch, int w_fixed, int* status, cudaStream_t stream) {
   if (M == 0 || N == 0 || batch == 0) return JV_OK;
   if (batch > 65535) return JV_ERR_UNSUPPORTED;
   return run(A, a_dtype, lda, (size_t)a_batch, W, w_dtype, ldw, (size_t)w_batch, C, c_dtype, ldc, (size_t)c_batch, M, N, K, batch,
-             status, stream);
+             w_fixed, status, stream);
 }

@@ -1055,9 +1055,9 @@ def attn_rows_decode(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache:
 
 
 # --------------------------------------------------------------------------- linear
-def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
-    """x [M, K] times weight [N, K] transposed, as exact as in float32 on CUDA cores (csrc/gemm_f32.cu).  The weight is read before
-    the kernels launched before this one have finished: none of them may write it."""
+def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype, fixed_weight: bool = False) -> torch.Tensor:
+    """x [M, K] times weight [N, K] transposed, as exact as in float32 on CUDA cores (csrc/gemm_f32.cu).  `fixed_weight`: none of the
+    kernels launched before this one writes the weight, which is then read before they have finished."""
     _cuda(x, "x", contiguous=False); _cuda(weight, "weight")
     if x.dim() != 2 or weight.dim() != 2 or x.shape[1] != weight.shape[1] or x.stride(1) != 1:
         raise KernelError(f"gemm shapes {tuple(x.shape)} x {tuple(weight.shape)}^T do not fit")
@@ -1065,9 +1065,9 @@ def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype) -> 
     n = weight.shape[0]
     y = torch.empty((m, n), dtype=out_dtype, device=x.device)
     f = _fn("gemm_f32", "jv_gemm_f32", [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
-                                        c_int, c_int, c_int, c_void_p, c_void_p])
+                                        c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(f(x.data_ptr(), _code(x, "x"), x.stride(0), weight.data_ptr(), _code(weight, "weight"), weight.stride(0),
-             y.data_ptr(), _code(y, "out"), y.stride(0), m, n, k, _status_ptr(x.device), _stream()), "gemm_f32")
+             y.data_ptr(), _code(y, "out"), y.stride(0), m, n, k, 1 if fixed_weight else 0, _status_ptr(x.device), _stream()), "gemm_f32")
     return y
 
 
@@ -1241,6 +1241,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     """y = x @ weight.T.  With `parts_ok` the result may be a PartialSum (the caller hands it to `rmsnorm`,
     `residual_add` or `swiglu`, which add its parts as they read them).
 
+    The weight is one that stays: the products of this package read it before the kernels launched before them have finished.
     float32 weights: the product of this package as exact as 32-bit multiply-adds (csrc/gemm_f32.cu; 16-bit activations
     are read as they are).  bfloat16 weights and activations: up to STREAM_BEST_ROWS rows (decoding) the
     weight-streaming product on tcgen05 (csrc/linear_stream.cu), which cuts the k of a weight with few strips into
@@ -1249,7 +1250,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype | None 
     accumulate in 32-bit and give the result in `out_dtype` (bfloat16 by default, float32 for logits)."""
     out_dtype = out_dtype or x.dtype
     if weight.dtype == torch.float32 or x.dtype == torch.float32:
-        return gemm_simt(x, weight, out_dtype)
+        return gemm_simt(x, weight, out_dtype, fixed_weight=True)
     _cuda(x, "x", torch.bfloat16, contiguous=False); _cuda(weight, "weight", torch.bfloat16)
     if _stream_ok(x, weight) and x.shape[0] <= STREAM_BEST_ROWS and out_dtype in (torch.bfloat16, torch.float32) and \
             (parts_ok or _strips_fill_the_device(x.device, weight.shape[0])):
@@ -1374,10 +1375,10 @@ def gate_heads(o: torch.Tensor, gate: torch.Tensor | None) -> torch.Tensor:
     return out
 
 
-def bmm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+def bmm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, fixed_weight: bool = False) -> torch.Tensor:
     """One product per head: out[h] = a[h] @ w[h].T, a [heads, n, k] (any strides with unit inner stride),
     w [heads, m, k] contiguous, out [heads, n, m] (made contiguous if not given; given, any strides with unit
-    inner stride).  float32 operands: the 32-bit product of this package (csrc/gemm_f32.cu);
+    inner stride).  float32 operands: the 32-bit product of this package (csrc/gemm_f32.cu), `fixed_weight` as in `gemm_simt`;
     bfloat16: the library's batched product (as the prompt products of this package are the library's)."""
     _cuda(a, "a", contiguous=False); _cuda(w, "w", a.dtype)
     heads, n, k = a.shape
@@ -1398,9 +1399,9 @@ def bmm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None)
         raise KernelError("out does not fit the batched product")
     f = _fn("gemm_f32", "jv_gemm_f32_batched", [c_void_p, c_int, c_int, c_longlong, c_void_p, c_int, c_int, c_longlong,
                                                 c_void_p, c_int, c_int, c_longlong, c_int, c_int, c_int, c_int,
-                                                c_void_p, c_void_p])
+                                                c_int, c_void_p, c_void_p])
     _check(f(a.data_ptr(), _code(a, "a"), a.stride(1), a.stride(0), w.data_ptr(), _code(w, "w"), w.stride(1), w.stride(0),
-             out.data_ptr(), _code(out, "out"), out.stride(1), out.stride(0), n, m, k, heads, _status_ptr(a.device),
+             out.data_ptr(), _code(out, "out"), out.stride(1), out.stride(0), n, m, k, heads, 1 if fixed_weight else 0, _status_ptr(a.device),
              _stream()), "bmm_heads")
     return out
 

@@ -169,7 +169,7 @@ class LatentAttention(Part):
         q = torch.empty((n, H * self.dk), dtype=dt, device=x.device)
         # the batched product writes the latent part of every query head in place
         ops.bmm_heads(q_plain, self.w_uk.to(dt) if wide else self.w_uk,
-                      out=q.view(n, H, self.dk)[:, :, :self.dc].transpose(0, 1))
+                      out=q.view(n, H, self.dk)[:, :, :self.dc].transpose(0, 1), fixed_weight=not wide)
         ops.latent_prepare(row, 0, self.kv_off, None, q, step.positions, step.token_entry, table,
                            self.position.table() if self.position is not None else None,
                            self.latent_norm, self.spec.latent_norm_eps, cache.k if writes else None,
@@ -178,9 +178,10 @@ class LatentAttention(Part):
         w_uv = self.w_uv.to(dt) if wide else self.w_uv
         if self.g_off < 0:                                              # no gate: the product writes the rows in place
             o = torch.empty((n, H * self.dv), dtype=o_lat.dtype, device=x.device)
-            ops.bmm_heads(o_lat[:, :, :self.dc].transpose(0, 1), w_uv, out=o.view(n, H, self.dv).transpose(0, 1))
+            ops.bmm_heads(o_lat[:, :, :self.dc].transpose(0, 1), w_uv, out=o.view(n, H, self.dv).transpose(0, 1),
+                          fixed_weight=not wide)
         else:
-            o = ops.bmm_heads(o_lat[:, :, :self.dc].transpose(0, 1), w_uv)
+            o = ops.bmm_heads(o_lat[:, :, :self.dc].transpose(0, 1), w_uv, fixed_weight=not wide)
             o = ops.gate_heads(o, (row if kv_row is None else kv_row)[:, self.g_off:self.g_off + H * self.dv])
         return ops.linear(o, self.w_o, dt, parts_ok=True)
 

@@ -733,6 +733,23 @@ def test_tiles_and_parts_of_the_32bit_product(m, n, k):
         assert torch.equal(ops.gemm_simt(x[first:first + rows], w, torch.float32), y[first:first + rows])
 
 
+@pytest.mark.parametrize("k", [64, 1024])
+def test_a_weight_of_the_kernel_before_is_waited_for(k):
+    """A weight that the kernel launched right before makes, in a buffer that held another: the product of the new one."""
+    ops, n = _ops(), 2048
+    x, gates = _rand(3, k, seed=1), [_rand(n, 2 * k, seed=s) for s in range(4)]
+    w, plain, batched = torch.zeros(n, k, device="cuda"), [], []
+    for g in gates:
+        ops.swiglu(g, out=w)
+        plain.append(ops.gemm_simt(x, w, torch.float32))
+    for g in gates:
+        ops.swiglu(g, out=w)
+        batched.append(ops.bmm_heads(x[None], w[None])[0])
+    for i, g in enumerate(gates):
+        want = ops.gemm_simt(x, ops.swiglu(g).clone(), torch.float32)
+        assert torch.equal(plain[i], want) and torch.equal(batched[i], want)
+
+
 @pytest.mark.parametrize("tile", [16, 64])
 @pytest.mark.parametrize("n,k", [(128, 1024), (300, 2100), (20, 33), (1030, 64)])
 @pytest.mark.parametrize("act", [None, "gelu"])
