@@ -396,7 +396,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     for (int i = 0; i < HALF; ++i)
       if (i < mine) sums[(first + i) * BM + quad * 32 + lane] = acc[i];
   }
-  if (!ok && lane == 0) { atomicOr(p.status, JV_STATUS_WAIT_EXPIRED); sh->failed = 1; }
+  // (a wait that one elected thread made alone counts too, whichever it is)
+  if (__any_sync(0xffffffffu, !ok) && lane == 0) { atomicOr(p.status, JV_STATUS_WAIT_EXPIRED); sh->failed = 1; }
   TC_FENCE_BEFORE();
   __syncthreads();
   if (sh->failed) {                                    // products and copies under way get a bounded time to finish
