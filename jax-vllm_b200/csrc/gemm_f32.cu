@@ -520,7 +520,7 @@ int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const Params& p, 
       }))
     return JV_ERR_UNSUPPORTED;
   const long long blocks = (long long)p.strips * p.parts * ((p.M + p.row_tile - 1) / p.row_tile);
-  if (blocks > 0x7fffffff || (long long)p.M * ((p.N + 3) / 4) > 0x7fffffff) return JV_ERR_UNSUPPORTED;
+  if (blocks > 0x7fffffff) return JV_ERR_UNSUPPORTED;
   return launch_clusters(kern, dim3((unsigned)blocks, batch), dim3(Shape<TMA, NB, TA, TW>::THREADS), smem, p.parts, stream, w_map, a_map, p);
 }
 

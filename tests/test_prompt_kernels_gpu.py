@@ -733,6 +733,16 @@ def test_tiles_and_parts_of_the_32bit_product(m, n, k):
         assert torch.equal(ops.gemm_simt(x[first:first + rows], w, torch.float32), y[first:first + rows])
 
 
+def test_product_32bit_of_more_than_2_to_the_33_numbers():
+    ops, m, n, k = _ops(), 1 << 20, 8200, 8
+    x, w = _rand(m, k, seed=1, dtype=torch.bfloat16), _rand(n, k, seed=2, dtype=torch.bfloat16)
+    y = ops.gemm_simt(x, w, torch.bfloat16)              # 17 GB
+    for first in (0, m // 2 - 3, m - 5):
+        want = x[first:first + 5].double() @ w.double().T
+        assert bool(((y[first:first + 5].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all())
+    ops.check_status()
+
+
 @pytest.mark.parametrize("k", [64, 1024])
 def test_a_weight_of_the_kernel_before_is_waited_for(k):
     """A weight that the kernel launched right before makes, in a buffer that held another: the product of the new one."""
