@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(1024) mamba_finish_vec_kernel(const float* __r
   const bool live = i < group_size;
   float y[8] = {}, wv[8] = {}, D = 0.f;
   float ss = 0.f;
-  if (EARLY && live) {                                 // weights: nobody writes them
+  if (EARLY && live) {
     D = to_f32(skip[at / value_dim]);
 #pragma unroll
     for (int e = 0; e < 8; ++e) wv[e] = to_f32(w[at + e]);
@@ -185,10 +185,11 @@ JV_EXPORT int jv_mamba_prepare(const void* xbc, int dtype, long long xbc_stride,
 }
 
 // o: float [n, inner] (the scan's output); x, z: rows of `dtype`, [inner] used; skip: [heads] and w: [inner] of
-// w_dtype; out: rows of `dtype`.  inner = heads * value_dim = norm_groups * group_size.
+// w_dtype; out: rows of `dtype`.  inner = heads * value_dim = norm_groups * group_size.  w_fixed: none of the kernels launched before this
+// one writes skip or w, which may then be read before they have finished.
 JV_EXPORT int jv_mamba_finish(const float* o, const void* x, long long x_stride, const void* z, long long z_stride,
                               int dtype, const void* skip, const void* w, int w_dtype, void* out, long long out_stride,
-                              float eps, int n, int heads, int value_dim, int norm_groups, cudaStream_t stream) {
+                              float eps, int n, int heads, int value_dim, int norm_groups, int w_fixed, cudaStream_t stream) {
   if (n == 0) return JV_OK;
   const int inner = heads * value_dim;
   if (heads < 1 || value_dim < 1 || norm_groups < 1 || inner % norm_groups) return JV_ERR_UNSUPPORTED;
@@ -199,7 +200,7 @@ JV_EXPORT int jv_mamba_finish(const float* o, const void* x, long long x_stride,
   if (value_dim % 8 == 0 && group_size % 8 == 0 && group_size <= 8192 && eights(o, inner, 4) && eights(x, x_stride, size) &&
       eights(z, z_stride, size) && eights(out, out_stride, size)) {
     const int threads = (group_size / 8 + 31) / 32 * 32;
-    const bool early = (long long)n * norm_groups * threads <= 2048LL * jv_multiprocessors();
+    const bool early = w_fixed && (long long)n * norm_groups * threads <= 2048LL * jv_multiprocessors();
     JV_DISPATCH_DTYPE(dtype, T, JV_DISPATCH_DTYPE(w_dtype, TW,
         return jv_launch(early ? mamba_finish_vec_kernel<true, T, TW> : mamba_finish_vec_kernel<false, T, TW>, dim3(n, norm_groups), dim3(threads), 0, stream, o, (const T*)x, x_stride,
                          (const T*)z, z_stride, (const TW*)skip, (const TW*)w, (T*)out, out_stride, eps, value_dim, group_size,

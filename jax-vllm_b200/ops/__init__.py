@@ -2428,13 +2428,15 @@ def mamba_step(xbc: torch.Tensor, b_off: int, c_off: int, dt_raw: torch.Tensor, 
 
 
 _MAMBA_FINISH_TYPES = [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_int, c_void_p, c_longlong, c_float,
-                       c_int, c_int, c_int, c_int, c_void_p]
+                       c_int, c_int, c_int, c_int, c_int, c_void_p]
 
 
 def mamba_finish(o: torch.Tensor, x: torch.Tensor, z: torch.Tensor, skip: torch.Tensor, weight: torch.Tensor,
-                 out: torch.Tensor, heads: int, value_dim: int, norm_groups: int, eps: float) -> torch.Tensor:
+                 out: torch.Tensor, heads: int, value_dim: int, norm_groups: int, eps: float,
+                 fixed_weights: bool = False) -> torch.Tensor:
     """y = (o + skip_h * x) * silu(z), divided by the root mean square of each of its `norm_groups` equal parts, times
-    `weight`; o float32 [n, heads * value_dim], x and z column ranges of rows in the compute type; written to `out`."""
+    `weight`; o float32 [n, heads * value_dim], x and z column ranges of rows in the compute type; written to `out`.
+    `fixed_weights`: none of the kernels launched before this one writes skip or weight, which may then be read before they have finished."""
     _cuda(o, "o", torch.float32); _cuda(x, "x", contiguous=False); _cuda(z, "z", x.dtype, contiguous=False)
     _cuda(skip, "skip"); _cuda(weight, "weight", skip.dtype); _cuda(out, "out", x.dtype, contiguous=False)
     n, inner = o.shape
@@ -2445,7 +2447,7 @@ def mamba_finish(o: torch.Tensor, x: torch.Tensor, z: torch.Tensor, skip: torch.
     f = _fn("mamba2", "jv_mamba_finish", _MAMBA_FINISH_TYPES)
     _check(f(o.data_ptr(), x.data_ptr(), x.stride(0), z.data_ptr(), z.stride(0), _code(x, "x"), skip.data_ptr(),
              weight.data_ptr(), _code(skip, "skip"), out.data_ptr(), out.stride(0), float(eps), n, heads, value_dim,
-             norm_groups, _stream()), "mamba_finish")
+             norm_groups, 1 if fixed_weights else 0, _stream()), "mamba_finish")
     return out
 
 
@@ -2461,7 +2463,8 @@ def state_space_prompt(row: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Te
                        a_log: torch.Tensor, skip: torch.Tensor, norm: torch.Tensor, norm_groups: int, eps: float,
                        out: torch.Tensor) -> torch.Tensor:
     """`short_conv` (with silu), `chunk_scan` and `mamba_finish` of a state-space mixer's portions, one after another without views
-    and a second look at what the first has checked: the launches of a few hundred tokens take the host longer than the device.
+    and a second look at what the first has checked: the launches of a few hundred tokens take the host longer than the device.  The
+    weights are ones that stay (`fixed_weights` of `mamba_finish`).
     `row` [n, ..]: z [heads * columns], what is convolved (x, then k and q of the groups), the raw step sizes [heads]; `state`: the
     matrices of a slot, then the convolution's inputs."""
     _cuda(row, "row", torch.bfloat16, contiguous=False); _cuda(state, "state", torch.float32, contiguous=False)
@@ -2495,7 +2498,7 @@ def state_space_prompt(row: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Te
         columns, 0, n, o + 4 * n * inner, status, stream), "chunk_scan", launches=3)
     _check(_fn("mamba2", "jv_mamba_finish", _MAMBA_FINISH_TYPES)(
         o, x, channels, z, row_stride, 1, skip.data_ptr(), norm.data_ptr(), _code(skip, "skip"), out.data_ptr(), out_stride, float(eps), n,
-        heads, columns, norm_groups, stream), "mamba_finish")
+        heads, columns, norm_groups, 1, stream), "mamba_finish")
     return out
 
 

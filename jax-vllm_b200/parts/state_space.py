@@ -111,7 +111,7 @@ class StateSpace(Part):
         else:
             o = ops.state_scan(ops.mamba_prepare(*prepare), xbc, 0, *where, step.n_entries, self.e, singles=step.decode_work)
         return ops.mamba_finish(o, xbc[:, :inner], row[:, :inner], self.skip, self.norm, out, self.h, self.e, self.ng,
-                                self.spec.norm_eps)
+                                self.spec.norm_eps, fixed_weights=True)
 
 
 register_mixer("state_space", StateSpace)

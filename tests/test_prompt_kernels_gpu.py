@@ -410,6 +410,23 @@ def test_mamba_finish_vectors(n, heads, value_dim, groups, off):
         assert ((out.double() - y).abs() <= (2.0 ** -8 if dtype == torch.bfloat16 else 4e-6) * y.abs() + 1e-6).all()
 
 
+def test_mamba_finish_waits_for_weights_of_the_kernel_before():
+    """Weights that the kernel launched right before makes, in buffers that held others."""
+    ops, n, heads, value_dim = _ops(), 2, 32, 64
+    inner = heads * value_dim
+    o, x, z = (_rand(n, inner, seed=i) for i in range(3))
+    made, skip = torch.zeros(1, inner, device="cuda"), torch.zeros(1, heads, device="cuda")
+    gates, got = [(_rand(1, 2 * heads, seed=s), _rand(1, 2 * inner, seed=s + 10)) for s in range(5, 9)], []
+    for a, b in gates:
+        out = torch.empty(n, inner, device="cuda")
+        ops.swiglu(a, out=skip)
+        ops.swiglu(b, out=made)
+        got.append(ops.mamba_finish(o, x, z, skip[0], made[0], out, heads, value_dim, 1, 1e-5))
+    for (a, b), y in zip(gates, got):
+        skip, made = ops.swiglu(a).clone(), ops.swiglu(b).clone()
+        assert torch.equal(y, ops.mamba_finish(o, x, z, skip[0], made[0], torch.empty_like(o), heads, value_dim, 1, 1e-5))
+
+
 # --------------------------------------------------------------------- experts of few tokens, picked rows
 @pytest.mark.parametrize("tokens,top,experts,n,k", [(1, 1, 1, 128, 128), (3, 2, 5, 136, 200), (16, 4, 8, 256, 1024), (17, 6, 64, 384, 128),
                                                     (64, 8, 8, 2048, 136)])
