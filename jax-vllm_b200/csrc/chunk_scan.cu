@@ -48,6 +48,7 @@ struct ChunkParams {
   float* state; long long slot_stride;     // S of (slot, head) at state + slot * slot_stride + head * D * V
   float* state_n;                          // the normaliser's state [slots][heads * D], rows slot_stride apart (or null)
   float* nq;                               // its outputs, every fourth float (the gates' last place)
+  int h0;                                  // a launch takes as many heads from here on as its grid has rows, the scratch's [heads]
   float* starts;                           // [chunks][heads][D][V]: D of a chunk, then S_0
   float* starts_n;                         // [chunks][heads][D]: the same of the normaliser
   float* whole;                            // [chunks][heads]: exp(L_T)
@@ -211,7 +212,7 @@ __global__ void __launch_bounds__(DELTA_THREADS) chunk_delta_kernel(const ChunkP
   pdl_wait();
   Chunk c;
   if (!find_chunk(p, blockIdx.x, c)) return;
-  const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = p.h0 + blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gr = lane >> 2, gq = lane & 3, lr = lane & 7, lm = lane >> 3;
   const int d_parts = (p.D + DS - 1) / DS, d0 = blockIdx.z % d_parts * DS, e0 = blockIdx.z / d_parts * VT;
   if (tid < VT) bad[tid] = CT;
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(DELTA_THREADS) chunk_delta_kernel(const ChunkP
   __syncthreads();
   take_out<DELTA_THREADS>(xs, bad);
   __syncthreads();
-  const size_t at = (size_t)blockIdx.x * p.heads + h;
+  const size_t at = (size_t)blockIdx.x * gridDim.y + blockIdx.y;
   float acc[MT][2][4];
 #pragma unroll
   for (int i = 0; i < MT; ++i)
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(START_THREADS) chunk_start_kernel(const ChunkP
   pdl_wait();
   const int entry = entry_of(blockIdx.z, p.portions, p.cu_seqlens, p.n_entries);
   if (entry < 0) return;
-  const int h = blockIdx.y, matrix = p.D * p.V / 4, i = blockIdx.x * START_THREADS + threadIdx.x;
+  const int h = p.h0 + blockIdx.y, matrix = p.D * p.V / 4, i = blockIdx.x * START_THREADS + threadIdx.x;
   const bool normaliser = i >= matrix;
   if (i >= matrix + (p.state_n != nullptr ? p.D / 4 : 0)) return;
   const int len = p.cu_seqlens[entry + 1] - p.cu_seqlens[entry];
@@ -313,9 +314,9 @@ __global__ void __launch_bounds__(START_THREADS) chunk_start_kernel(const ChunkP
   }
   const int size = normaliser ? p.D : p.D * p.V, e = 4 * (normaliser ? i - matrix : i);
   float* state = (normaliser ? p.state_n : p.state) + (size_t)slot * p.slot_stride + (size_t)h * size + e;
-  float* at = (normaliser ? p.starts_n : p.starts) + ((size_t)g0 * p.heads + h) * size + e;
-  const float* whole = p.whole + (size_t)g0 * p.heads + h;
-  const size_t step = (size_t)p.heads * size;
+  float* at = (normaliser ? p.starts_n : p.starts) + ((size_t)g0 * gridDim.y + blockIdx.y) * size + e;
+  const float* whole = p.whole + (size_t)g0 * gridDim.y + blockIdx.y;
+  const size_t step = (size_t)gridDim.y * size;
   float4 S = make_float4(state[0], state[1], state[2], state[3]);
   for (int c0 = 0; c0 < chunks; c0 += START_AHEAD) {
     float4 d[START_AHEAD];
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(START_THREADS) chunk_start_kernel(const ChunkP
     for (int j = 0; j < START_AHEAD; ++j) {
       const int c = min(c0 + j, chunks - 1);
       d[j] = *reinterpret_cast<const float4*>(at + c * step);
-      a[j] = whole[(size_t)c * p.heads];
+      a[j] = whole[(size_t)c * gridDim.y];
     }
 #pragma unroll
     for (int j = 0; j < START_AHEAD; ++j) {
@@ -363,10 +364,10 @@ __global__ void __launch_bounds__(OUT_THREADS, DP <= 128 ? 2 : 1) chunk_output_k
   pdl_wait();
   Chunk c;
   if (!find_chunk(p, blockIdx.x, c)) return;
-  const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = p.h0 + blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gr = lane >> 2, gq = lane & 3, lr = lane & 7, lm = lane >> 3;
   const int e0 = blockIdx.z * VT;
-  const size_t at = (size_t)blockIdx.x * p.heads + h;
+  const size_t at = (size_t)blockIdx.x * gridDim.y + blockIdx.y;
   if (tid < VT) bad[tid] = CT;
   copy_rows<DP, LD, OUT_THREADS>(qs, p.q + c.t0 * p.q_stride + (h / p.per_group) * p.D, p.q_stride, c.here, p.D);
   copy_rows<DP, LD, OUT_THREADS>(ks, p.k + c.t0 * p.k_stride + (h / p.per_group) * p.D, p.k_stride, c.here, p.D);
@@ -547,7 +548,7 @@ __global__ void __launch_bounds__(OUT_THREADS, DP <= 128 ? 2 : 1) chunk_output_k
 }
 
 template <int DP>
-int launch(const ChunkParams& p, int entries, cudaStream_t stream) {
+int launch(ChunkParams p, int entries, int at_once, cudaStream_t stream) {
   static bool done[JV_MAX_DEVICES] = {};
   if (!jv_once_per_device(done, [&] {
         return cudaFuncSetAttribute(chunk_delta_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DeltaShape<DP>::SMEM) == cudaSuccess &&
@@ -557,11 +558,16 @@ int launch(const ChunkParams& p, int entries, cudaStream_t stream) {
   const int v_parts = (p.V + VT - 1) / VT, d_parts = (p.D + DeltaShape<DP>::DS - 1) / DeltaShape<DP>::DS;
   const int fours = p.D * p.V / 4 + (p.state_n != nullptr ? p.D / 4 : 0);
   if (v_parts * d_parts > 65535 || entries > 65535) return JV_ERR_UNSUPPORTED;
-  int rc = jv_launch(chunk_delta_kernel<DP>, dim3(p.max_chunks, p.heads, v_parts * d_parts), dim3(DELTA_THREADS), DeltaShape<DP>::SMEM, stream, p);
-  if (rc != JV_OK) return rc;
-  rc = jv_launch(chunk_start_kernel, dim3((fours + START_THREADS - 1) / START_THREADS, p.heads, entries), dim3(START_THREADS), 0, stream, p);
-  if (rc != JV_OK) return rc;
-  return jv_launch(chunk_output_kernel<DP>, dim3(p.max_chunks, p.heads, v_parts), dim3(OUT_THREADS), OutShape<DP>::SMEM, stream, p);
+  for (p.h0 = 0; p.h0 < p.heads; p.h0 += at_once) {
+    const int heads = p.heads - p.h0 < at_once ? p.heads - p.h0 : at_once;
+    int rc = jv_launch(chunk_delta_kernel<DP>, dim3(p.max_chunks, heads, v_parts * d_parts), dim3(DELTA_THREADS), DeltaShape<DP>::SMEM, stream, p);
+    if (rc != JV_OK) return rc;
+    rc = jv_launch(chunk_start_kernel, dim3((fours + START_THREADS - 1) / START_THREADS, heads, entries), dim3(START_THREADS), 0, stream, p);
+    if (rc != JV_OK) return rc;
+    rc = jv_launch(chunk_output_kernel<DP>, dim3(p.max_chunks, heads, v_parts), dim3(OUT_THREADS), OutShape<DP>::SMEM, stream, p);
+    if (rc != JV_OK) return rc;
+  }
+  return JV_OK;
 }
 
 bool rows_of_16_bytes(const void* p, long long stride) { return ((uintptr_t)p & 15) == 0 && stride % 8 == 0; }
@@ -570,27 +576,28 @@ bool rows_of_16_bytes(const void* p, long long stride) { return ((uintptr_t)p & 
 // q, k, v: the first head's columns in rows of `.._stride` 16-bit elements (head h reads q and k at (h / per_group) * D, v at h * V);
 // gates [n, heads, 4] float with nq = gates + 3 and state_n, or null with dt_raw (rows of dt_stride elements, [heads] used),
 // dt_bias, a_log [heads] of w_dtype; out [n, heads * V]; state as for jv_state_scan; portions > 0: entries of one token
-// are passed by, which leaves this many, with n tokens; scratch: (n / 128 + portions) * heads * (D * V + D + 1)
-// floats, 16-byte aligned.  Taken for D up to 256
+// are passed by, which leaves this many, with n tokens; scratch: (n / 128 + portions) * at_once * (D * V + D + 1)
+// floats, 16-byte aligned, for at_once heads, which are gone through so many at a time.  Taken for D up to 256
 // and V, both in steps of 8, with rows on 16-byte boundaries.
 JV_EXPORT int jv_chunk_scan(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
                             int per_group, float scale, float* gates, const void* dt_raw, long long dt_stride, const void* dt_bias,
                             const void* a_log, int w_dtype, float* out, float* state, long long slot_stride, float* state_n,
                             const int* cu_seqlens, const int* slots, int n_slots, int entries, int heads, int D, int V, int portions,
-                            int n, float* scratch, int* status, cudaStream_t stream) {
+                            int n, float* scratch, int at_once, int* status, cudaStream_t stream) {
   if (entries == 0 || n == 0) return JV_OK;
   if (D < 8 || D > 256 || D % 8 || V < 8 || V % 8 || per_group < 1 || heads % per_group || heads > 65535 || entries < 0 || n < 0 ||
-      !rows_of_16_bytes(q, q_stride) || !rows_of_16_bytes(k, k_stride) || !rows_of_16_bytes(v, v_stride) || w_dtype < 0 || w_dtype > 1 ||
+      !rows_of_16_bytes(q, q_stride) || !rows_of_16_bytes(k, k_stride) || !rows_of_16_bytes(v, v_stride) || w_dtype < 0 || w_dtype > 1 || at_once < 1 ||
       (gates == nullptr && (dt_raw == nullptr || state_n != nullptr)) || ((uintptr_t)gates & 7) || ((uintptr_t)scratch & 15))
     return JV_ERR_UNSUPPORTED;
+  if (at_once > heads) at_once = heads;
   const int taken = portions > 0 ? portions : entries, max_chunks = n / CT + taken;
-  float* starts_n = scratch + (size_t)max_chunks * heads * D * V;
+  float* starts_n = scratch + (size_t)max_chunks * at_once * D * V;
   ChunkParams p{(const bf16*)q, (const bf16*)k, (const bf16*)v, q_stride, k_stride, v_stride, per_group, scale, gates,
                 (const bf16*)dt_raw, dt_stride, dt_bias, a_log, w_dtype, out, state, slot_stride, state_n,
-                gates == nullptr ? nullptr : gates + 3, scratch, starts_n, starts_n + (size_t)max_chunks * heads * D,
+                gates == nullptr ? nullptr : gates + 3, 0, scratch, starts_n, starts_n + (size_t)max_chunks * at_once * D,
                 cu_seqlens, slots, n_slots, heads, D, V, portions, entries, max_chunks, status};
-  if (D <= 32) return launch<32>(p, taken, stream);
-  if (D <= 64) return launch<64>(p, taken, stream);
-  if (D <= 128) return launch<128>(p, taken, stream);
-  return launch<256>(p, taken, stream);
+  if (D <= 32) return launch<32>(p, taken, at_once, stream);
+  if (D <= 64) return launch<64>(p, taken, at_once, stream);
+  if (D <= 128) return launch<128>(p, taken, at_once, stream);
+  return launch<256>(p, taken, at_once, stream);
 }

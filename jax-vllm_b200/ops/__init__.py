@@ -2032,6 +2032,16 @@ def state_scan(packed: torch.Tensor, v: torch.Tensor, v_off: int, state: torch.T
 CHUNK_SCAN_MIN_TOKENS = 64
 CHUNK_SCAN_MAX_KEY = 256
 CHUNK_SCAN_TOKENS = 128           # of a chunk (csrc/chunk_scan.cu)
+# Floats of scratch (256 MB): a longer step's heads are gone through some at a time, so that what a layer call needs beside its rows does
+# not grow with the step.  (4,096 tokens of 128 heads of 128 x 64 take 150 MB.)
+CHUNK_SCAN_SCRATCH = 1 << 26
+
+
+def _chunk_scan_scratch(chunks: int, heads: int, dim: int, columns: int) -> tuple:
+    """(heads at a time, floats of scratch)"""
+    a_head = chunks * (dim * columns + dim + 1)
+    at_once = max(1, min(heads, CHUNK_SCAN_SCRATCH // a_head))
+    return at_once, at_once * a_head
 
 
 def chunk_scan_takes(row: torch.Tensor, offsets, n_entries: int, dim: int, columns: int, n_tokens: int | None = None) -> bool:
@@ -2059,7 +2069,7 @@ def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, 
 
 _CHUNK_SCAN_TYPES = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_float, c_void_p, c_void_p, c_longlong, c_void_p,
                      c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
-                     c_int, c_void_p, c_void_p, c_void_p]
+                     c_int, c_void_p, c_int, c_void_p, c_void_p]
 
 
 def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: torch.Tensor, cu_seqlens: torch.Tensor,
@@ -2099,14 +2109,15 @@ def chunk_scan(row: torch.Tensor, q_off: int, k_off: int, v_off: int, state: tor
     out = torch.empty((n, heads * columns), dtype=torch.float32, device=row.device)
     taken = portions or n_entries
     n_taken = n - (n_entries - taken)                    # tokens of the portions: the others have one each
-    scratch = torch.empty((n_taken // CHUNK_SCAN_TOKENS + taken) * heads * (dim * columns + dim + 1), dtype=torch.float32, device=row.device)
+    at_once, floats = _chunk_scan_scratch(n_taken // CHUNK_SCAN_TOKENS + taken, heads, dim, columns)
+    scratch = torch.empty(floats, dtype=torch.float32, device=row.device)
     f = _fn("chunk_scan", "jv_chunk_scan", _CHUNK_SCAN_TYPES)
     base = row.data_ptr()
     _check(f(base + 2 * q_off, row.stride(0), base + 2 * k_off, row.stride(0), base + 2 * v_off, row.stride(0), heads // groups,
              float(scale), _ptr(gates), _ptr(dt_raw), 0 if dt_raw is None else dt_raw.stride(0), _ptr(dt_bias), _ptr(a_log), w_code,
              out.data_ptr(), state.data_ptr(), state.stride(0), _ptr(state_n), cu_seqlens.data_ptr(), slots.data_ptr(),
-             state.shape[0], n_entries, heads, dim, columns, portions, n_taken, scratch.data_ptr(), _status_ptr(row.device),
-             _stream()), "chunk_scan", launches=3)
+             state.shape[0], n_entries, heads, dim, columns, portions, n_taken, scratch.data_ptr(), at_once, _status_ptr(row.device),
+             _stream()), "chunk_scan", launches=3 * -(-heads // at_once))
     return out
 
 
@@ -2485,8 +2496,8 @@ def state_space_prompt(row: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Te
         raise KernelError("state_space_prompt: shapes do not fit")
     device = row.device
     conv = torch.empty((n, channels), dtype=torch.bfloat16, device=device)
-    chunks = n // CHUNK_SCAN_TOKENS + n_entries          # the scan's outputs, and its scratch behind them
-    scan = torch.empty(n * inner + chunks * heads * (dim * columns + dim + 1), dtype=torch.float32, device=device)
+    at_once, floats = _chunk_scan_scratch(n // CHUNK_SCAN_TOKENS + n_entries, heads, dim, columns)
+    scan = torch.empty(n * inner + floats, dtype=torch.float32, device=device)       # the scan's outputs, and its scratch behind them
     z, x, o = row.data_ptr(), conv.data_ptr(), scan.data_ptr()
     matrix, cu, slot, status, stream = state.data_ptr(), cu_seqlens.data_ptr(), slots.data_ptr(), _status_ptr(device), _stream()
     _check(_fn("short_conv", "jv_short_conv", _SHORT_CONV_TYPES)(
@@ -2495,7 +2506,7 @@ def state_space_prompt(row: torch.Tensor, conv_w: torch.Tensor, conv_b: torch.Te
     _check(_fn("chunk_scan", "jv_chunk_scan", _CHUNK_SCAN_TYPES)(
         x + 2 * (inner + side), channels, x + 2 * inner, channels, x, channels, heads // groups, 1.0, 0, z + 2 * (inner + channels), row_stride,
         dt_bias.data_ptr(), a_log.data_ptr(), _code(dt_bias, "dt_bias"), o, matrix, state_stride, 0, cu, slot, n_slots, n_entries, heads, dim,
-        columns, 0, n, o + 4 * n * inner, status, stream), "chunk_scan", launches=3)
+        columns, 0, n, o + 4 * n * inner, at_once, status, stream), "chunk_scan", launches=3 * -(-heads // at_once))
     _check(_fn("mamba2", "jv_mamba_finish", _MAMBA_FINISH_TYPES)(
         o, x, channels, z, row_stride, 1, skip.data_ptr(), norm.data_ptr(), _code(skip, "skip"), out.data_ptr(), out_stride, float(eps), n,
         heads, columns, norm_groups, 1, stream), "mamba_finish")

@@ -260,6 +260,33 @@ def test_chunked_states_over_several_chunks(heads, dim, columns):
         assert (got.double() - want.double()).norm() <= 3e-6 * want.double().norm()
 
 
+@pytest.mark.parametrize("heads,groups,dim,columns,at_once", [(5, 1, 64, 64, 1), (6, 2, 136, 24, 4), (8, 8, 16, 72, 3)])
+def test_chunked_states_some_heads_at_a_time(heads, groups, dim, columns, at_once, monkeypatch):
+    """Scratch for a few heads: no more memory than that, the same bits."""
+    ops, lengths = _ops(), [128, 1, 300, 77]
+    cu, slots, n_slots = _entries(lengths)
+    n, gn, hv, portions = sum(lengths), groups * dim, heads * columns, 3
+    row = _rand(n, hv + 2 * gn, seed=1, dtype=torch.bfloat16)
+    dt_raw, dt_bias, a_log = _rand(n, heads, seed=3, dtype=torch.bfloat16), _rand(heads, seed=4), _rand(heads, seed=5)
+    rows = _rand(n_slots, hv * dim + heads * dim, seed=3)
+    limit = at_once * (n // 128 + portions) * (dim * columns + dim + 1)
+    for with_gates in ([False, True] if groups == heads else [False]):
+        gates, runs = torch.rand(n, heads, 4, device="cuda"), []
+        for floats in (1 << 26, limit):
+            monkeypatch.setattr(ops, "CHUNK_SCAN_SCRATCH", floats, raising=False)
+            st, g = rows.clone(), gates.clone()
+            more = dict(gates=g, state_n=st[:, hv * dim:]) if with_gates else dict(dt_raw=dt_raw, dt_bias=dt_bias, a_log=a_log)
+            torch.cuda.reset_peak_memory_stats()
+            before = torch.cuda.memory_allocated()
+            o = ops.chunk_scan(row, hv + gn, hv, 0, st, cu, slots, len(lengths), heads, groups, dim, columns, portions=portions, **more)
+            if floats == limit:                          # beside the result; the allocator rounds up to 512 bytes
+                assert torch.cuda.max_memory_allocated() - before <= 4 * (n * hv + limit) + 1024
+            o[128] = 0.0                                 # the entry of one token is passed by
+            runs.append((o, st, g[:, :, 3]))
+        ops.check_status()
+        assert all(torch.equal(a, b) for a, b in zip(*runs)) and bool(torch.isfinite(runs[0][0]).all())
+
+
 @pytest.mark.parametrize("heads,groups,dim,columns,taps", [(4, 2, 16, 8, 2), (8, 1, 64, 64, 4), (6, 3, 136, 24, 3)])
 @pytest.mark.parametrize("lengths", [[64], [200, 77, 130]])
 def test_portions_of_the_state_space_mixer(heads, groups, dim, columns, taps, lengths):
