@@ -2054,19 +2054,6 @@ def chunk_scan_takes(row: torch.Tensor, offsets, n_entries: int, dim: int, colum
             and row.stride(0) % 8 == 0 and all((row.data_ptr() + 2 * o) % 16 == 0 for o in offsets))
 
 
-def chunk_scan_min_blocks(dim: int) -> int:
-    return 160 if dim <= 32 else 101 if dim <= 64 else 80
-
-
-def chunk_scan_supports(row: torch.Tensor, offsets, n_entries: int, heads: int, dim: int, columns: int,
-                        n_tokens: int | None = None, longest: int = 0) -> bool:
-    """`chunk_scan_takes`, and blocks of 32 value columns that go through the portions side by side, the longest of `longest` tokens
-    (0: all alike), would keep `chunk_scan_min_blocks` multiprocessors at work."""
-    tokens = row.shape[0] if n_tokens is None else n_tokens
-    return (chunk_scan_takes(row, offsets, n_entries, dim, columns, n_tokens) and dim <= 128
-            and tokens * heads * -(-columns // 32) >= chunk_scan_min_blocks(dim) * (longest or -(-tokens // n_entries)))
-
-
 _CHUNK_SCAN_TYPES = [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_float, c_void_p, c_void_p, c_longlong, c_void_p,
                      c_void_p, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                      c_int, c_void_p, c_int, c_void_p, c_void_p]

@@ -25,17 +25,24 @@ def test_latent_splits_under_a_window_do_not_grow_with_the_longest_sequence_ther
     assert ops.latent_splits(32768, 0, 1, 148, 256)[1] > 100        # without one all keys count
 
 
-def test_chunks_are_chosen_by_the_blocks_that_are_at_work():
-    """Portions of a few tokens beside a long one keep no multiprocessor busy: they change nothing."""
-    def taken(lengths, heads, dim, columns):
-        row = torch.empty((sum(lengths), 3 * 64), dtype=torch.bfloat16)
-        return ops.chunk_scan_supports(row, (0, 64, 128), len(lengths), heads, dim, columns, longest=max(lengths))
-    for heads, dim, columns in ((32, 64, 64), (8, 128, 256), (64, 64, 64), (64, 128, 64), (64, 32, 64), (96, 32, 64)):
-        for few in ([5], [5, 7, 3]):
-            assert taken([2000] + few, heads, dim, columns) == taken([2000], heads, dim, columns)
-    assert not taken([2000], 32, 64, 64) and taken([1000, 1000], 32, 64, 64)
-    assert not taken([2000], 64, 32, 64) and taken([2000], 64, 64, 64)
-    assert not taken([63], 64, 64, 64) and taken([64], 64, 64, 64)           # too short
-    row = torch.empty((256, 192), dtype=torch.bfloat16)
-    assert not ops.chunk_scan_supports(row, (0, 64, 128), 0, 64, 64, 64)     # no portions
-    assert ops.chunk_scan_supports(row, (0, 64, 128), 1, 64, 64, 64) and not ops.chunk_scan_supports(row.float(), (0, 64, 128), 1, 64, 64, 64)
+def test_chunks_are_chosen_by_the_tokens_of_a_portion():
+    def taken(tokens, portions, dim, columns, offsets=(0, 64, 128), dtype=torch.bfloat16, singles=0, row=None):
+        row = torch.empty((tokens + singles, 192), dtype=dtype) if row is None else row
+        return ops.chunk_scan_takes(row, offsets, portions, dim, columns, n_tokens=tokens)
+
+    def prompt(tokens, portions, dim, columns, taps=4, dtype=torch.bfloat16):
+        return ops.state_space_prompt_takes(torch.empty((tokens, 192), dtype=dtype), portions, 2, 1, dim, columns, taps)
+    for rule in (taken, prompt):
+        assert not rule(63, 1, 64, 64) and rule(64, 1, 64, 64)
+        assert not rule(191, 3, 64, 64) and rule(192, 3, 64, 64)             # of a portion, on average
+        assert not rule(256, 0, 64, 64) and not rule(256, 1, 64, 64, dtype=torch.float32)
+        for dim in (8, 64, 128, 136, 256):
+            assert rule(256, 1, dim, 64)
+        for dim, columns in ((4, 64), (12, 64), (264, 64), (64, 12)):
+            assert not rule(256, 1, dim, columns)
+    assert not taken(63, 1, 64, 64, singles=40) and taken(64, 1, 64, 64, singles=40)      # decoded tokens beside the portions do not count
+    assert not taken(256, 1, 64, 64, offsets=(0, 64, 132))                   # heads that start off 16-byte boundaries
+    wide = torch.empty((256, 200), dtype=torch.bfloat16)
+    assert taken(256, 1, 64, 64, row=wide[:, 8:]) and not taken(256, 1, 64, 64, row=wide[:, 4:])
+    assert not taken(256, 1, 64, 64, row=torch.empty((256, 196), dtype=torch.bfloat16)[:, :192])
+    assert not prompt(256, 1, 64, 64, taps=1)                                # a convolution without a state
