@@ -37,7 +37,7 @@ class EngineConfig:
                                           # that is free when the driver is made (never more than the worst case)
     max_tokens_per_step: int = 2048       # token budget of one step (decoded tokens + prompt portions)
     prefix_cache: bool = True
-    decode_split_size: int = 256          # key positions per split of a decoded token's attention (kernels that cut evenly do without)
+    decode_split_size: int = 256          # key positions per split of a decoded token's attention (up to twice as many where all are cut evenly)
     cuda_graphs: bool = True              # replay decode-only steps from captured graphs
     device: str = "cuda:0"
 

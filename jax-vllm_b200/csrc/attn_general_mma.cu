@@ -63,7 +63,8 @@ struct Params {
   int n_v_heads, n_k_heads;
   float out_scale;
   int tokens_per_tile, heads_per_tile, n_head_groups;
-  int split_size, n_splits;    // keys of a split; 0: each token's keys are cut evenly into (up to) n_splits
+  int split_size, n_splits;    // keys of a split; 0: each token's keys are cut evenly into (up to) n_splits, of `least` keys or more
+  int least;
   int* status;
   int* counters;               // decode: one per (work item, kv head, head group), zero between launches
 };
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(THREADS) attn_decode_general_kernel(const Para
   const int pos_q = p.start_pos[entry];
   const KeyRun run(first_visible(pos_q, p.window), p.keep);
   const int n_vis = run.places(pos_q + 1);             // all of them visible; the splits share the places of the run
-  const int split_size = p.split_size > 0 ? p.split_size : even_split(n_vis, p.n_splits);
+  const int split_size = p.split_size > 0 ? p.split_size : max(even_split(n_vis, p.n_splits), p.least);
   const int n_lo = blockIdx.z * split_size;
   const int n_hi = min(n_vis, n_lo + split_size);
   if (n_lo >= n_hi) return;
@@ -719,28 +720,46 @@ JV_EXPORT int jv_attn_general_tokens_per_tile(int n_q_heads, int n_kv_heads) {
   return ROWS_PREFILL / (G < 16 ? G : 16);
 }
 
-// Into how many even splits (split_size 0) to cut the keys of n_work single tokens that see up to `most` of them: the number with
-// which the last wave of blocks ends first, if a block takes as long as its keys and OVERHEAD more for its first copies and
-// the merge.  (Splits of 256 keys, the last as short as it falls: 24 requests of 4 key heads and 1,028 visible keys were 480 blocks on 296
-// places, 96 of them of four keys, and the kernel took 29.7 us; in three splits of 352 it takes 21.9.)
-JV_EXPORT int jv_attn_general_even_splits(int n_work, int n_q_heads, int n_kv_heads, int most) {
-  if (n_work < 1 || n_kv_heads < 1 || n_q_heads < n_kv_heads || most < 1) return 1;
-  constexpr int OVERHEAD = 64, MOST_SPLITS = 64;
-  const int groups = (n_q_heads / n_kv_heads + 15) / 16;
-  const long long places = (long long)jv_multiprocessors() * max(1, (int)((227 * 1024) / (decode_smem() + 4 * 1024)));
-  const long long blocks = (long long)n_work * n_kv_heads * groups;
-  int best = 1;
-  long long least = 0;
-  for (int n = 1; n <= MOST_SPLITS && (n == 1 || (long long)(n - 1) * BN < most); ++n) {
-    const long long cost = (blocks * n + places - 1) / places * (even_split(most, n) + OVERHEAD);
-    if (n == 1 || cost < least) { best = n; least = cost; }
+static long long decode_places() { return (long long)jv_multiprocessors() * max(1, (int)((227 * 1024) / (decode_smem() + 4 * 1024))); }
+static long long decode_blocks(int n_work, int n_q_heads, int n_kv_heads) {
+  return (long long)n_work * n_kv_heads * ((n_q_heads / n_kv_heads + 15) / 16);
+}
+
+// The keys of the smallest even split of n_work single tokens that see up to `most` keys: with it the blocks of all tokens just run at
+// once, but no more than `usual`, since most tokens may see far fewer keys than the longest.
+JV_EXPORT int jv_attn_general_least_split(int n_work, int n_q_heads, int n_kv_heads, int most, int usual) {
+  if (n_work < 1 || n_kv_heads < 1 || n_q_heads < n_kv_heads || most < 1 || usual < 1) return BN;
+  const long long fit = decode_places() / decode_blocks(n_work, n_q_heads, n_kv_heads);
+  const int least = even_split(most, (int)(fit > 1 ? fit : 1));
+  return least < usual ? least : usual > BN ? usual : BN;
+}
+
+// Into how many even splits (split_size <= 0) to cut their keys: the number with which the last wave of blocks ends first, if a block takes
+// as long as its keys and OVERHEAD more for its first copies and the merge.  (Splits of 256 keys, the last as short as it
+// falls: 24 requests of 4 key heads and 1,028 visible keys were 480 blocks on 296 places, 96 of them of four keys, and the kernel took 29.7 us;
+// in three splits of 352 it takes 21.9.)  No split has more than twice the usual keys, however many tokens there are: the longest of a
+// ragged step is walked by the blocks of one token, and the step waits for them.  (73 tokens of 500 keys beside one of
+// 32,768, four key heads: 1,187 us uncut, 144 in splits of 256, 115 so.)
+JV_EXPORT int jv_attn_general_even_splits(int n_work, int n_q_heads, int n_kv_heads, int most, int usual) {
+  if (n_work < 1 || n_kv_heads < 1 || n_q_heads < n_kv_heads || most < 1 || usual < 1) return 1;
+  constexpr int OVERHEAD = 64, TRIED = 64;
+  const long long places = decode_places(), blocks = decode_blocks(n_work, n_q_heads, n_kv_heads);
+  const int least = jv_attn_general_least_split(n_work, n_q_heads, n_kv_heads, most, usual);
+  const int longest = 2 * usual > least ? 2 * usual : least;
+  const int first = (most + longest - 1) / longest, last = (most + least - 1) / least;
+  int best = first;
+  long long shortest = 0;
+  for (int n = first; n <= last && n < first + TRIED; ++n) {
+    const int even = even_split(most, n), keys = even > least ? even : least;
+    const long long cost = (blocks * n + places - 1) / places * (keys + OVERHEAD);
+    if (n == first || cost < shortest) { best = n; shortest = cost; }
   }
   return best;
 }
 
 // Arguments as for jv_attn_simt_ex (csrc/attn_simt.cu), bfloat16 only, for the key and value sizes of this library.
 // k_cache: [num_pages, page_size, n_k_heads, KD], v_cache: [num_pages, page_size, n_v_heads, VD].  n_splits == 0: prompt portions, work = (entry, first token of the
-// tile).  n_splits > 0: single tokens (split_size 0: their keys cut evenly), part_o [n_work*Hq*n_splits*VD] and part_ml [n_work*Hq*n_splits*2] floats of
+// tile).  n_splits > 0: single tokens (split_size <= 0: their keys cut evenly, -split_size or more a split), part_o [n_work*Hq*n_splits*VD] and part_ml [n_work*Hq*n_splits*2] floats of
 // scratch, and `counters`, n_work * n_kv_heads * ceil(G/16) ints that are zero before the launch (the kernel leaves
 // them zero).
 JV_EXPORT int jv_attn_general_mma(const void* q, int q_stride, void* out, int out_stride, int out_f32, float* part_o,
@@ -775,6 +794,7 @@ JV_EXPORT int jv_attn_general_mma(const void* q, int q_stride, void* out, int ou
   p.n_head_groups = (G + p.heads_per_tile - 1) / p.heads_per_tile;
   p.tokens_per_tile = n_splits > 0 ? 1 : ROWS_PREFILL / p.heads_per_tile;
   p.split_size = split_size > 0 ? split_size : 0;
+  p.least = split_size < 0 ? -split_size : 0;
   p.n_splits = n_splits;
   return launch(p, n_work, n_splits > 0, stream);
 }

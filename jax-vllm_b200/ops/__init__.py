@@ -556,10 +556,19 @@ def attn_general_mma_tokens_per_tile(n_q_heads: int, n_kv_heads: int) -> int:
     return 64 // min(n_q_heads // n_kv_heads, 16)
 
 
-def attn_general_mma_splits(n_work: int, n_q_heads: int, n_kv_heads: int, key_dim: int, value_dim: int, most: int) -> int:
-    """Into how many even splits `attn_general_mma` best cuts the keys, up to `most`, of each of `n_work` single tokens."""
-    f = _fn(attn_general_mma_library(key_dim, value_dim), "jv_attn_general_even_splits", [c_int] * 4)
-    return f(n_work, n_q_heads, n_kv_heads, most)
+def attn_general_mma_splits(n_work: int, n_q_heads: int, n_kv_heads: int, key_dim: int, value_dim: int, most: int,
+                            usual: int = 256) -> int:
+    """Into how many even splits `attn_general_mma` best cuts the keys, up to `most`, of each of `n_work` single tokens, none of more
+    than 2 `usual` keys."""
+    f = _fn(attn_general_mma_library(key_dim, value_dim), "jv_attn_general_even_splits", [c_int] * 5)
+    return f(n_work, n_q_heads, n_kv_heads, most, usual)
+
+
+def attn_general_mma_least(n_work: int, n_q_heads: int, n_kv_heads: int, key_dim: int, value_dim: int, most: int,
+                           usual: int = 256) -> int:
+    """The keys that such a split should hold at least, of a token that sees fewer than `most`."""
+    f = _fn(attn_general_mma_library(key_dim, value_dim), "jv_attn_general_least_split", [c_int] * 5)
+    return f(n_work, n_q_heads, n_kv_heads, most, usual)
 
 
 def attn_general_mma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
@@ -571,7 +580,8 @@ def attn_general_mma(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache:
     """Paged causal attention on the tensor cores with the options of `attn_simt`: the key size and the key heads are the
     key cache's, the value size and the value heads the value cache's; bfloat16 in, bfloat16 or float32 out.
     `window`: the mask as one number (`mask_code`).  Single tokens (`n_splits` > 0): splits of `split_size` keys, or with
-    `split_size` 0 every token's keys cut evenly into up to `n_splits` (`attn_general_mma_splits`)."""
+    `split_size` 0 or less every token's keys cut evenly into up to `n_splits` of at least -`split_size` keys
+    (`attn_general_mma_splits`, `attn_general_mma_least`)."""
     n_dist = _score_extras("attn_general_mma", n_q_heads, head_scale, dist_bias, sink)
     for t, nm in ((q, "q"), (k_cache, "k_cache"), (v_cache, "v_cache")):
         _cuda(t, nm, torch.bfloat16, contiguous=(nm != "q"))

@@ -386,11 +386,11 @@ class GeneralAttention(Part):
         elif n_dec:
             # the splits share what a query sees: at most its window with the kept tokens, or its chunk
             most = min(step.max_seq_len, s.window + self.keep if s.window else s.chunk or step.max_seq_len)
+            split = self.ctx.decode_split_size
             if self.general is not None:
-                kernel(dwork, n_dec, split_size=0,
-                       n_splits=ops.attn_general_mma_splits(n_dec, self.hq, self.hk, self.dk, self.dv, most))
+                sizes = (n_dec, self.hq, self.hk, self.dk, self.dv, most, split)
+                kernel(dwork, n_dec, split_size=-ops.attn_general_mma_least(*sizes), n_splits=ops.attn_general_mma_splits(*sizes))
             else:
-                split = self.ctx.decode_split_size
                 kernel(dwork, n_dec, split_size=split, n_splits=max(1, -(-most // split)))
 
 

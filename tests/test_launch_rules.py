@@ -25,6 +25,24 @@ def test_latent_splits_under_a_window_do_not_grow_with_the_longest_sequence_ther
     assert ops.latent_splits(32768, 0, 1, 148, 256)[1] > 100        # without one all keys count
 
 
+def test_even_splits_of_decoded_keys_are_bounded():
+    """However many tokens share a step, the longest is not left to a few blocks; and a short one is not cut finer than its step needs."""
+    rng = random.Random(2)
+    for _ in range(3000):
+        n, kv, most, usual = rng.randint(1, 300), rng.choice((1, 2, 4, 8)), rng.randint(1, 200000), rng.choice((16, 64, 256, 1000))
+        sizes = (n, 4 * kv, kv, 64, 64, most, usual)
+        splits, least = ops.attn_general_mma_splits(*sizes), ops.attn_general_mma_least(*sizes)
+        assert 64 <= least <= max(64, usual) and splits >= 1
+        keys = max(64, least, -(-(-(-most // splits)) // 16) * 16)
+        assert keys <= max(2 * usual, 64) + 15 and splits * keys >= most
+    # 74 requests on four key heads, one of them long: as many blocks as splits of 512 keys make
+    assert ops.attn_general_mma_splits(74, 16, 4, 64, 64, 32768) >= 64
+    assert ops.attn_general_mma_splits(1, 1, 1, 64, 64, 131072) >= 256
+    # 24 requests of four key heads that see 1,028 keys: three splits run at once on 148 multiprocessors
+    if not torch.cuda.is_available() or ops.multiprocessors("cuda:0") == 148:
+        assert ops.attn_general_mma_splits(24, 16, 4, 128, 128, 1028) == 3
+
+
 def test_chunks_are_chosen_by_the_tokens_of_a_portion():
     def taken(tokens, portions, dim, columns, offsets=(0, 64, 128), dtype=torch.bfloat16, singles=0, row=None):
         row = torch.empty((tokens + singles, 192), dtype=dtype) if row is None else row

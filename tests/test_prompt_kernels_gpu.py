@@ -1020,3 +1020,23 @@ def test_even_splits_of_decoded_tokens(hq, hk, splits, mask, keep, sigmoid):
     # the weights of a split are rounded to 16 bits against its own maximum
     assert float((got[0] - got[1]).abs().max()) <= 2.0 ** -7 * float(got[1].abs().max())
     assert 1 <= ops.attn_general_mma_splits(n, hq, hk, d, d, 1000) <= 64
+
+
+@pytest.mark.parametrize("least", [1, 100, 256, 5000])
+def test_even_splits_of_no_fewer_keys_than(least):
+    """Tokens with fewer keys than the least, as many, and several times as many, in a launch with room for more splits than they take."""
+    ops = _ops()
+    hq, hk, d, page, lengths = 8, 2, 64, 16, [1, 99, 100, 255, 256, 257, 1000]
+    n, widest = len(lengths), 64
+    k, v = (_rand(n * widest, page, hk, d, seed=i, dtype=torch.bfloat16) for i in (1, 2))
+    table = torch.randperm(n * widest, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(n, widest).cuda()
+    cu, start = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (list(range(n + 1)), [m - 1 for m in lengths]))
+    work = torch.tensor([(e, 0) for e in range(n)], dtype=torch.int32, device="cuda")
+    q, got = _rand(n, hq * d, seed=3, dtype=torch.bfloat16), []
+    for size, count in ((-least, 16), (64, 16)):
+        out = torch.full((n, hq * d), float("nan"), device="cuda")
+        ops.attn_general_mma(q, q.stride(0), out, k, v, table, cu, start, work, n, hq, hk, 0.2, split_size=size, n_splits=count)
+        ops.check_status()
+        got.append(out.double())
+    # the weights of a split are rounded to 16 bits against its own maximum
+    assert float((got[0] - got[1]).abs().max()) <= 2.0 ** -7 * float(got[1].abs().max())
