@@ -174,6 +174,7 @@ struct GroupScanParams {
 // shared memory hands out 128 bytes a clock and each number read should serve more than one multiply-add.
 // Eight lanes; 16, which halves what a warp has to do in a group for one more step of every sum over the lanes, where the blocks of eight
 // would leave multiprocessors without one and keys have 64 channels or more (32 heads of 64, 2,048 tokens: 258 us with eight, 201 with 16).
+// Which of the two hangs on the portions of the step, a portion's sums do not: both add the same numbers in the same order.
 // RING_: the stages of the ring.  Six (about 100 KB, two blocks a multiprocessor) carry a block through the latency of its copies;
 // where there are more blocks than two a multiprocessor, others do that, and two stages leave room for more of them (32 heads of 64:
 // 2,048 tokens in one entry 430 us a layer with six, 598 with two; five entries of 400 313 and 281, eight of 8 tokens 51 and 45).
@@ -187,8 +188,9 @@ template <int LANES, int KPT, int RING_> struct GroupScanShape {
   static constexpr int SMEM = (int)sizeof(float) * (RING * STAGE + 2 * COLS * VLD);
 };
 
+// (The blocks that its shared memory lets a multiprocessor hold: left to itself the compiler kept to 128 registers and spilled some.)
 template <int LANES, int KPT, int RING_, typename T>
-__global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p) {
+__global__ void __launch_bounds__(64, RING_ == 6 ? 2 : LANES * KPT == 32 ? 8 : 4) group_scan_kernel(const GroupScanParams p) {
   using Shape = GroupScanShape<LANES, KPT, RING_>;
   constexpr int DP = Shape::DP, FLOATS = Shape::FLOATS, GROUPS = Shape::GROUPS, RING = Shape::RING, COLS = Shape::COLS;
   constexpr int VLD = Shape::VLD, TOK = GROUPS * T4, Q = KPT / 4, THREADS = Shape::THREADS, RUN = 4 * LANES, WARP_COLS = 64 / LANES;
@@ -275,16 +277,20 @@ __global__ void __launch_bounds__(64) group_scan_kernel(const GroupScanParams p)
         R[j][q] = *reinterpret_cast<const ulonglong2*>(vec + (T4 + j) * DP + q * RUN);
       }
   };
+  // A lane of eight holds the channels of two of the 16: they are summed up apart, and then together, as two of the 16 do it.
+  constexpr int HELD = LANES == 8 && Q >= 2 ? 2 : 1;
   auto dot = [&](const ulonglong2 (&x)[Q], const uint64_t (&s)[KPT / 2]) {
-    uint64_t a = 0, b = 0;
+    float sum[HELD];
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      a = fma2(x[q].x, s[2 * q], a);
-      b = fma2(x[q].y, s[2 * q + 1], b);
+    for (int k = 0; k < HELD; ++k) {
+      uint64_t a = 0;
+#pragma unroll
+      for (int q = k; q < Q; q += HELD) a = fma2(x[q].y, s[2 * q + 1], fma2(x[q].x, s[2 * q], a));
+      float lo, hi;
+      unpack2(a, lo, hi);
+      sum[k] = lo + hi;
     }
-    float lo, hi;
-    unpack2(add2(a, b), lo, hi);
-    return lo + hi;
+    return HELD == 2 ? sum[0] + sum[HELD - 1] : sum[0];
   };
   for (int s = 0; s < n_stages; ++s) {
     float* vbuf = vals + (s & 1) * COLS * VLD;

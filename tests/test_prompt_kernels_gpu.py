@@ -88,6 +88,38 @@ def test_delta_four_tokens_at_a_time(dim, columns, dtype):
         assert torch.equal(state[s], before[s])
 
 
+@pytest.mark.parametrize("heads,dim,columns", [(32, 64, 64), (9, 65, 256), (20, 128, 112), (7, 256, 256), (8, 130, 250)])
+def test_delta_portions_hang_on_their_request_alone(heads, dim, columns):
+    """One portion leaves multiprocessors without a block (16 lanes share a column), two and three do not (eight lanes, the deep and the
+    shallow ring): the same bits, and those of 64-bit sums but for their rounding."""
+    from tests.plain.nufapel_plain import delta_decay, delta_scan
+    ops, length = _ops(), 39
+    blocks, places = heads * -(-columns // 16), torch.cuda.get_device_properties(0).multi_processor_count
+    assert places != 148 or blocks <= places < 2 * blocks <= 2 * places < 3 * blocks
+    hd, hv = heads * dim, heads * columns
+    proj, zw = _rand(3 * length, 3 * hd + hv, seed=dim), _rand(3 * length, hd, seed=3)
+    ab, wb = _rand(hd, seed=4), _rand(hd, seed=5)
+    before = _rand(3, hd * columns, seed=6)
+    outs, states = [], []
+    for n in (1, 2, 3):
+        cu = torch.arange(n + 1, dtype=torch.int32, device="cuda") * length
+        state = before.clone()
+        outs.append(ops.delta_scan(proj[:n * length], 0, hd, 2 * hd, 3 * hd, zw[:n * length], ab, wb, state, cu,
+                                   torch.arange(n, dtype=torch.int32, device="cuda"), n, heads, dim, columns))
+        states.append(state)
+    ops.check_status()
+    for n in (1, 2):
+        assert torch.equal(outs[n][:length], outs[0]) and torch.equal(states[n][0], states[0][0])
+    assert torch.equal(outs[2][:2 * length], outs[1]) and torch.equal(states[2][1], states[1][1])
+    r, k, za = (proj[:length, i * hd:(i + 1) * hd].double().cpu().view(length, heads, dim) for i in range(3))
+    w = delta_decay(zw[:length].double().cpu() + wb.double().cpu()).view(length, heads, dim)
+    a = torch.sigmoid(za + ab.double().cpu().view(heads, dim))
+    v = proj[:length, 3 * hd:].double().cpu().view(length, heads, columns)
+    o, S = delta_scan(r, k, v, w, a, before[0].double().cpu().view(heads, dim, columns))
+    for got, want in ((outs[0].cpu().view(length, heads, columns), o), (states[0][0].cpu().view_as(S), S)):
+        assert (got.double() - want).norm() <= 4e-6 * want.norm()
+
+
 def test_delta_later_infinity_stays_out_of_earlier_outputs():
     ops, heads, dim, n = _ops(), 1, 16, 8
     cu, slots, n_slots = _entries([n])
