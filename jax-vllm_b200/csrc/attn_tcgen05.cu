@@ -27,8 +27,11 @@
 // Masks: causal, a window, chunks; under a window the first `keep` positions of a sequence may stay visible: an item's
 // tiles are then those of the kept positions (as far as they lie before the window's) followed by the window's.
 //
-// Heads of 64 (a tile of keys is 16 KB then, and twice as many are in flight) were the mma.sync kernel's before: 2,999 tokens in three
-// entries behind 77, 16 heads on 4, a window of 512 that keeps 4, capped scores: 67.6 us there, 47.3 here.
+// Heads of 64 (a tile of keys is 16 KB then, and twice as many are in flight): the weights of a softmax meet the values twice, rounded and
+// what the rounding took off, as for latent rows.  The mma.sync kernel that took these heads before rounds against the true maximum, which
+// leaves the largest weight as it is; against one that follows lazily the error against 64 bits was 1 % larger.  2,999 tokens in three
+// entries behind 77, 16 heads on 4, a window of 512 that keeps 4, capped scores: error 4.64e-3 and 67.6 us there, 4.68e-3 and 47.3 us with
+// weights rounded once, 4.44e-3 and 49.4 us so.
 //
 // Restrictions (the caller falls back to the mma.sync kernel otherwise): bfloat16, head size 128 or 64, HPT up to 16, page size a power of two from 8 to 128.
 #include "tcgen05.cuh"
@@ -304,6 +307,8 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
       };
       auto issue_qk = [&](const At& a, int gt) -> bool {          // S[gt % 2] = Q K^T for tile gt of the sequence
         const int qb = a.n % Q_BUFFERS, s = gt % K_STAGES;
+        // the scores go where the rest of the weights of the tile before last lies: its product has to be complete
+        if (D == 64 && !p.sigmoid && gt >= 2 && !mbar_wait(&sh->o_done[gt & 1], ((gt - 2) >> 1) & 1)) return false;
         if (a.j == 0 && !mbar_wait(&sh->q_full[qb], (a.n / Q_BUFFERS) & 1)) return false;
         if (!mbar_wait(&sh->k_full[s], (gt / K_STAGES) & 1)) return false;
         TC_FENCE_AFTER();
@@ -335,6 +340,12 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)   // 16 keys further: 8 columns of P, 16 rows (2048 bytes) down V
           umma_a_tmem(tmem_o, tmem_p + kk * 8, v_desc[s] + kk * (16 * 128 / 16), Shape<D>::PV, (cur.j | kk) != 0);
+        if (D == 64 && !p.sigmoid) {     // and what the rounding of P took off, where the scores were (the second 64 keys from column 64 on)
+          const uint32_t tmem_r = tmem + (gt & 1) * 128;
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            umma_a_tmem(tmem_o, tmem_r + (kk >> 2) * 64 + (kk & 3) * 8, v_desc[s] + kk * (16 * 128 / 16), Shape<D>::PV, 1);
+        }
         umma_commit(&sh->v_empty[s]);
         umma_commit(&sh->o_done[gt & 1]);
         cur = nxt;
@@ -507,7 +518,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
         } else {
           const uint64_t scale2 = pack2(sc, sc), neg_m2 = pack2(-m_scaled, -m_scaled);
           uint64_t sum2[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
-          uint32_t pw[32];
+          uint32_t pw[32], rest[32];
 #pragma unroll
           for (int c = 0; c < 2; ++c)
 #pragma unroll
@@ -518,11 +529,17 @@ __global__ void __launch_bounds__(THREADS, 1) attn_tcgen05_kernel(const __grid_c
               const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
               sum2[(i >> 1) & 1] = add2(sum2[(i >> 1) & 1], pack2(p0, p1));
               const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-              pw[c * 16 + (i >> 1)] = *reinterpret_cast<const uint32_t*>(&h);
+              const uint32_t bits = *reinterpret_cast<const uint32_t*>(&h);
+              pw[c * 16 + (i >> 1)] = bits;
+              if (D == 64) {
+                const __nv_bfloat162 r = __floats2bfloat162_rn(p0 - __uint_as_float(bits << 16), p1 - __uint_as_float(bits & 0xffff0000u));
+                rest[c * 16 + (i >> 1)] = *reinterpret_cast<const uint32_t*>(&r);
+              }
             }
           unpack2(sum2[0], sum[0], sum[1]);
           unpack2(sum2[1], sum[2], sum[3]);
           tmem_st32_bits(tmem + lane_addr + TMEM_P + (gt & 1) * 64 + half * 32, pw);
+          if (D == 64) tmem_st32_bits(s_addr, rest);             // over this thread's own scores
         }
         l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
         // ---- in an item's last tile the value rows past the end become zero (they may hold anything), and so do those

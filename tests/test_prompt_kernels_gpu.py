@@ -1029,6 +1029,29 @@ def test_heads_of_64_of_prompts(hq, hk, page, option):
         row += m
 
 
+@pytest.mark.parametrize("cap", [0.0, 40.0])
+def test_heads_of_64_round_no_weight(cap):
+    """Keys that all score zero, and behind the first tile one that scores up to 2^7.8 times as much and alone has a value: the result is
+    that value times a number that 16 bits need not hold, rounded once."""
+    ops, ctx, new, hq, d, page, at = _ops(), 256, 32, 4, 64, 16, 200
+    k, v = (torch.zeros(ctx + new, 1, d, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    k[at, 0, 0], v[at, 0] = 1.0, _rand(d, seed=1, dtype=torch.bfloat16)
+    q = torch.zeros(new, hq, d, device="cuda", dtype=torch.bfloat16)
+    q[:, :, 0] = torch.linspace(2.0, 21.6, new * hq, device="cuda").view(new, hq).to(torch.bfloat16)
+    out = torch.empty(new, hq * d, device="cuda", dtype=torch.bfloat16)
+    table = torch.arange((ctx + new) // page, dtype=torch.int32, device="cuda")[None]
+    cu, start, work = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, new], [ctx], [[0, 0]]))
+    ops.attn_tcgen05(q.view(new, -1), hq * d, out, k.view(-1, page, 1, d), v.view(-1, page, 1, d), table, cu, start, work, 1, hq, 1, d, 0.25,
+                     score_cap=cap)
+    ops.check_status()
+    score = q[:, :, 0].double() * 0.25
+    score = (cap * torch.tanh(score / cap) if cap else score)[:, :, None]
+    others = (ctx + torch.arange(new, device="cuda").double())[:, None, None]
+    want = v[at, 0].double() * score.exp() / (score.exp() + others)
+    # half a unit of 16 bits; 2^-16 of a weight, and what is left of 32-bit exponentials and sums
+    assert bool(((out.view(new, hq, d).double() - want).abs() <= (2.0 ** -8 + 2.0 ** -15) * want.abs()).all())
+
+
 # ------------------------------------------------------------------------------- keys of decoded tokens cut evenly
 @pytest.mark.parametrize("hq,hk,splits", [(4, 1, 1), (4, 1, 3), (40, 2, 7), (3, 3, 64)])
 @pytest.mark.parametrize("mask,keep,sigmoid", [(0, 0, False), (100, 5, False), (-128, 0, True)])
