@@ -10,7 +10,7 @@
 // 16-bit operands are one part.
 //
 // The rows of W are the 128-row operand (a strip of 128 columns of C), the rows of A the narrow one, up to 128 of them: few rows
-// waste nothing, and an element's sum is the same whatever M is.  (k is cut into up to eight parts by N and K alone, so that strips times
+// waste nothing, and an element's sum is the same whatever M is.  (k is cut into up to six parts by N and K alone, so that strips times
 // parts about fill the device.  Every part is summed with k ascending; the blocks of a tile's parts are a cluster, leave their sums in
 // shared memory and add up each some of the tile, in ascending order.  By a kernel of their own, from memory, that took 5 us a product of 203 rows, 2.2 of one.)
 //
