@@ -12,13 +12,14 @@
 // The rows of W are the 128-row operand (a strip of 128 columns of C), the rows of A the narrow one, up to 128 of them: few rows
 // waste nothing, and an element's sum is the same whatever M is.  (k is cut into up to six parts by N and K alone, so that strips times
 // parts about fill the device.  Every part is summed with k ascending; the blocks of a tile's parts are a cluster, leave their sums in
-// shared memory and add up each some of the tile, in ascending order.  By a kernel of their own, from memory, that took 5 us a product of 203 rows, 2.2 of one.)
+// shared memory and add up each some of the tile, in ascending order.  By a kernel of their own, from memory, that took 5 us a product of 203 rows, 2.2 of one.
+// With up to 16 rows, which wait for latency alone, a block pushes its sums to those that add them up, without a barrier between.)
 //
 // A block is one (strip, tile of rows, part), a pipeline of warps.  One brings 32 k's of the operands' rows with TMA, RAW chunks ahead.
 // Two groups of four cut them, a chunk each in turn.  The parts of W go to tensor memory, a thread a row: through shared memory their
 // stores and the tensor cores' reading them for each part of A again were half of a chunk's traffic for few rows.  The parts of A go to
-// shared memory in 8 x 16 byte blocks as the tensor cores read them without a swizzle (eight rows of a block follow one another, so
-// that a warp's stores are 512 bytes in a row).  One warp issues the products into one of the accumulators, and eight more (four where
+// shared memory (up to 16 rows: two warps of their own cut them) in 8 x 16 byte blocks as the tensor cores read them without a swizzle
+// (eight rows of a block follow one another, so that a warp's stores are 512 bytes in a row).  One warp issues the products into one of the accumulators, and eight more (four where
 // the rows of A are few) add another to their registers, a thread a row of W and half of the rows of A.  What each warp does of a chunk
 // is a chain of latencies longer than the products, so every role is a warp of its own (128 columns of
 // 148 multiprocessors each, clocks a chunk: 128 rows 2,030 with eight warps that brought, cut and eight that issued and added, 1,260 so;
@@ -31,9 +32,9 @@
 // the CUDA cores.
 //
 // Measured, model of width 1,024, two layers, 32-bit: 203 tokens, eight products 0.68 ms with 8 x 8 outputs a thread in multiply-adds on
-// the CUDA cores and 0.147 so (400 tokens 0.277), the head (one row, 32,000 columns) 26 and 29.6 us.  A product of one to three rows is
-// 1 to 2 us slower than multiply-adds were (K = 1,024: 5 us; four rows the same, 16 rows 12 against 5), which a sum that
-// is the same whatever M is has to bear.
+// the CUDA cores and 0.147 so (400 tokens 0.277), the head (one row, 32,000 columns) 26 and 29.6 us.  A product of one row takes
+// 0.5 to 2 us longer than multiply-adds did (N = 1,024 4.8 us against 4.3, 4,256 7.9 against 5.8; 16 rows 5.3 against 13.0 and 8.6 against 13.8),
+// which a sum that is the same whatever M is has to bear; it was 1.5 to 3 us before few rows had their A cut and their sums pushed as above.
 // Grouped, 16 experts of 2,048 x 1,024 and 1,024 x 512, both products: 4 tokens of two choices 224 us on the CUDA cores and 37 so,
 // 200 tokens 280 and 105.
 #include "tcgen05.cuh"
@@ -62,6 +63,7 @@ struct Params {
 struct Shared {
   uint64_t w_full[MAX_RAW], a_full[MAX_RAW], raw_empty[MAX_RAW];      // chunks as they are in memory: rows of W, of A, free places
   uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[MAX_ACCS], acc_empty[MAX_ACCS];       // chunks in parts; their sums
+  uint64_t pushed;                                     // what the blocks of the cluster add up of this block's share (few rows)
   uint64_t drain;                                      // used only after a wait ran out
   uint32_t tmem_base;
   int failed;
@@ -98,6 +100,24 @@ __device__ __forceinline__ float4 cluster_load(uint32_t addr, int rank) {
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
   return v;
 }
+// x into block `rank` of the cluster, at its address of what this block has at `addr`; its barrier at `bar` counts the four bytes.
+__device__ __forceinline__ void cluster_push(uint32_t addr, uint64_t* bar, float x, int rank) {
+  asm volatile("{\n.reg .b32 a, b;\nmapa.shared::cluster.u32 a, %0, %3;\nmapa.shared::cluster.u32 b, %1, %3;\n"
+               "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [a], %2, [b];\n}\n"
+               ::"r"(addr), "r"(smem_u32(bar)), "r"(__float_as_uint(x)), "r"(rank) : "memory");
+}
+// As mbar_wait, for what the other blocks have pushed.
+__device__ __forceinline__ bool wait_pushed(uint64_t* bar) {
+  const long long deadline = clock64() + JV_WAIT_CYCLES;
+  uint32_t done;
+  do {
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(smem_u32(bar)) : "memory");
+  } while (!done && clock64() < deadline);
+  return done != 0;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrived() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
   return *reinterpret_cast<const uint32_t*>(&h);
@@ -183,13 +203,18 @@ __device__ __forceinline__ bool is_number(float x) { return fabsf(x) <= 3.402823
 
 template <bool TMA, int NB, typename TA, typename TW> struct Shape {
   static constexpr int PA = Eight<TA>::PARTS, PW = Eight<TW>::PARTS;
-  static constexpr int ADDERS = NB <= 16 ? 4 : 8, ISSUER = CUTTERS + ADDERS, BRINGER = ISSUER + 1, THREADS = 32 * (BRINGER + 1);
+  static constexpr int ADDERS = NB <= 16 ? 4 : 8, A_CUTTERS = TMA && NB <= 16 ? NB / 8 : 0;      // (few rows: warps of their own cut A)
+  static constexpr int ISSUER = CUTTERS + ADDERS + A_CUTTERS, BRINGER = ISSUER + 1, THREADS = 32 * (BRINGER + 1);
   static constexpr int ACCS = NB <= 64 ? 4 : 2, STAGES = 4;       // accumulators, chunks in parts
   static constexpr int A_PART = NB / 8 * GROUP_BYTES, STAGE = PA * A_PART;
   static constexpr int W_RAW = BM * Eight<TW>::ROW_BYTES, A_RAW = (NB * Eight<TA>::ROW_BYTES + 1023) / 1024 * 1024;
   static constexpr int RAW = !TMA ? 1 : NB <= 16 ? 5 : NB <= 64 ? 6 : 4, RAW_STAGE = W_RAW + A_RAW;
+  // Few rows: the parts' sums of the columns that a block adds up are pushed to it, behind the ring, which it may still be using.
+  static constexpr bool PUSH = TMA && NB <= 16;
   static constexpr int RING = (TMA ? RAW * RAW_STAGE : 0) + STAGES * STAGE, SUMS = 2 * NB * BM * 4 + MAX_PARTS * 16;     // the block's sums, and of all parts those that it adds up, lie over the ring
-  static constexpr int SMEM = (RING > SUMS ? RING : SUMS) + (int)sizeof(Shared) + 1024;
+  static constexpr int HERE = PUSH ? (BM / 4 + MAX_PARTS - 1) * NB * 16 : 0;
+  static constexpr int SMEM = (PUSH ? RING + HERE : RING > SUMS ? RING : SUMS) + (int)sizeof(Shared) + 1024;
+  static_assert(!PUSH || 2 * (SMEM + 1024) <= 228 * 1024, "two blocks a multiprocessor");
   static constexpr int A_GROUPS = (NB / 8 + GROUP - 1) / GROUP;   // of eight rows that a warp cuts
   // tensor memory: accumulators of NB columns, then stages of 16 columns (two k's each) a part of W
   static constexpr int TMEM_COLS = NB <= 16 ? 256 : 512, W_COLS = 16 * PW;
@@ -214,13 +239,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   unsigned char* raw = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);     // [RAW][W rows, A rows]
   unsigned char* stages = raw + (TMA ? RAW * S::RAW_STAGE : 0);
   float* sums = reinterpret_cast<float*>(raw);         // [row of A][row of W], once all is summed
-  Shared* sh = reinterpret_cast<Shared*>(raw + (S::RING > S::SUMS ? S::RING : S::SUMS));
+  Shared* sh = reinterpret_cast<Shared*>(raw + (S::PUSH ? S::RING + S::HERE : S::RING > S::SUMS ? S::RING : S::SUMS));
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // the parts of one tile are a cluster
   const int m_tiles = (p.M + p.row_tile - 1) / p.row_tile;
   const int part = blockIdx.x % p.parts, m0 = blockIdx.x / p.parts % m_tiles * p.row_tile, n0 = blockIdx.x / p.parts / m_tiles * BM;
   const int rows = min(p.row_tile, p.M - m0), rows16 = (rows + 15) / 16 * 16;
   const int k0 = part * p.part_k, k_end = min(p.K, k0 + p.part_k), chunks = (k_end - k0 + CHUNK - 1) / CHUNK;
+  // PUSH: this block adds up `quads` fours of the tile's columns (the last block fewer), from `quad0` on; its room is [part][row][quads]
+  const int quads = (BM / 4 + p.parts - 1) / p.parts, quad0 = part * quads, my_quads = max(0, min(quads, BM / 4 - quad0));
+  float* here = reinterpret_cast<float*>(raw + S::RING);
   const TA* A = (const TA*)p.A + blockIdx.y * p.a_batch + (size_t)m0 * p.lda;
   int wb = blockIdx.y;                                 // which of the matrices W
   if (p.tile_expert != nullptr) {                      // found out by the kernels before this one; the same for the whole cluster
@@ -234,15 +262,25 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     mbar_expect_tx(&sh->w_full[s], BM * Eight<TW>::ROW_BYTES);
     tma_load_3d(raw + s * S::RAW_STAGE, &w_map, k0 + c * CHUNK, n0, wb, &sh->w_full[s]);
   };
-  if (warp == S::BRINGER && elect_one()) {
-    for (int s = 0; s < RAW; ++s) { mbar_init(&sh->w_full[s], 1); mbar_init(&sh->a_full[s], 1); mbar_init(&sh->raw_empty[s], GROUP); }
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&sh->full[s], GROUP); mbar_init(&sh->empty[s], 1); }
-    for (int b = 0; b < ACCS; ++b) { mbar_init(&sh->acc_full[b], 1); mbar_init(&sh->acc_empty[b], S::ADDERS); }
-    mbar_init(&sh->drain, 1);
-    sh->failed = 0;
+  if (warp == S::BRINGER) {
+    constexpr int CUT = GROUP + S::A_CUTTERS;          // warps that cut a chunk
+    for (int i = lane; i < MAX_RAW; i += 32) { mbar_init(&sh->w_full[i], 1); mbar_init(&sh->a_full[i], 1); mbar_init(&sh->raw_empty[i], CUT); }
+    for (int i = lane - MAX_RAW; i >= 0 && i < MAX_STAGES; i += 32) { mbar_init(&sh->full[i], CUT); mbar_init(&sh->empty[i], 1); }
+    for (int i = lane - MAX_RAW - MAX_STAGES; i >= 0 && i < MAX_ACCS; i += 32) { mbar_init(&sh->acc_full[i], 1); mbar_init(&sh->acc_empty[i], S::ADDERS); }
+    if (lane == 31) {
+      mbar_init(&sh->drain, 1);
+      sh->failed = 0;
+      if (S::PUSH) {
+        mbar_init(&sh->pushed, 1);
+        mbar_fence_init();
+        if (p.parts > 1) mbar_expect_tx(&sh->pushed, p.parts * rows * my_quads * 16);
+      }
+    }
     mbar_fence_init();
-    if (p.w_fixed)
+    __syncwarp();
+    if (p.w_fixed && elect_one())
       for (int c = 0; c < early; ++c) bring_w(c, c);
+    __syncwarp();
   }
   if (warp == S::ISSUER) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&sh->tmem_base)), "n"(S::TMEM_COLS) : "memory");
@@ -251,6 +289,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
   TC_FENCE_BEFORE();
   __syncthreads();
   TC_FENCE_AFTER();
+  if (S::PUSH && p.parts > 1) cluster_arrive();        // the others may push
   pdl_trigger();                                       // not before this block has its tensor memory
   const uint32_t tmem = __shfl_sync(0xffffffffu, sh->tmem_base, 0), tmem_w = tmem + ACCS * NB;
   int brought = 0;                                     // chunks that have been asked for, in the thread that does it
@@ -340,10 +379,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
 #pragma unroll
         for (int x = 0; x < PW; ++x) tmem_st8(to_w + 16 * x + 8 * half, part[0][x], part[1][x]);
       }
-      if (TMA && !(ok = __all_sync(0xffffffffu, mbar_wait(&sh->a_full[from.i], from.phase)))) break;
+      if (TMA && S::A_CUTTERS == 0 && !(ok = __all_sync(0xffffffffu, mbar_wait(&sh->a_full[from.i], from.phase)))) break;
       unsigned char* dst = stages + to.i * S::STAGE + kb * 128 + r * 16;
 #pragma unroll
-      for (int i = 0; i < S::A_GROUPS; ++i) {          // A: eight rows at a time, 32 bytes a lane (16 of 16-bit numbers)
+      for (int i = 0; i < (S::A_CUTTERS == 0 ? S::A_GROUPS : 0); ++i) {          // A: eight rows at a time, 32 bytes a lane (16 of 16-bit numbers)
         const int g = quad + i * GROUP, row = g * 8 + r;
         if (g * 8 >= rows16) break;
         Eight<TA> v;
@@ -365,6 +404,31 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
       }
       to.next(); to.next();
       from.next(); from.next();
+    }
+  } else if (warp >= CUTTERS + S::ADDERS) {
+    // ------------------------------------------------------------- few rows of A into parts, eight a warp
+    const int g = warp - CUTTERS - S::ADDERS, r = lane & 7, kb = lane >> 3;
+    Place<STAGES> to;
+    Place<RAW> from;
+    for (int c = 0; c < chunks; ++c, to.next(), from.next()) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&sh->empty[to.i], to.phase ^ 1) && mbar_wait(&sh->a_full[from.i], from.phase));
+      if (!ok) break;
+      if (g * 8 < rows16) {
+        Eight<TA> v;
+        uint32_t part[PA][4];
+        v.read(raw + from.i * S::RAW_STAGE + S::W_RAW, g * 8 + r, kb);
+        v.cut(part);
+#pragma unroll
+        for (int x = 0; x < PA; ++x)
+          *reinterpret_cast<uint4*>(stages + to.i * S::STAGE + kb * 128 + r * 16 + g * GROUP_BYTES + x * S::A_PART) =
+              make_uint4(part[x][0], part[x][1], part[x][2], part[x][3]);
+      }
+      PROXY_FENCE();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&sh->full[to.i]);
+        mbar_arrive(&sh->raw_empty[from.i]);
+      }
     }
   } else {
     // ------------------------------------------------------------- sums
@@ -391,10 +455,26 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
       TC_FENCE_BEFORE();
       warp_arrive(&sh->acc_empty[out.i], lane);
     }
-    // every product of this block is done, and with them every read of the ring
+    if constexpr (S::PUSH) {
+      const int n = quad * 32 + lane, to = (n >> 2) / quads;
+      const uint32_t addr = smem_u32(here + ((part * rows) * quads + (n >> 2) - to * quads) * 4 + (n & 3));
+      if (p.parts > 1) cluster_arrived();
 #pragma unroll
-    for (int i = 0; i < HALF; ++i)
-      if (i < mine) sums[(first + i) * BM + quad * 32 + lane] = acc[i];
+      for (int i = 0; i < HALF; ++i) {
+        if (i >= rows) break;
+        if (p.parts > 1) cluster_push(addr + i * quads * 16, &sh->pushed, acc[i], to);
+        else here[i * quads * 4 + n] = acc[i];
+      }
+    } else {
+      // every product of this block is done, and with them every read of the ring
+#pragma unroll
+      for (int i = 0; i < HALF; ++i)
+        if (i < mine) sums[(first + i) * BM + quad * 32 + lane] = acc[i];
+    }
+  }
+  if (S::PUSH && p.parts > 1 && (warp < CUTTERS || warp >= CUTTERS + S::ADDERS)) {
+    __syncwarp();
+    cluster_arrived();
   }
   // (a wait that one elected thread made alone counts too, whichever it is)
   if (__any_sync(0xffffffffu, !ok) && lane == 0) { atomicOr(p.status, JV_STATUS_WAIT_EXPIRED); sh->failed = 1; }
@@ -414,32 +494,44 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(S::TMEM_COLS) : "memory");
   }
   // ------------------------------------------------------------- the parts' sums, added up in their order: each block some of the tile
-  const int share = (rows * (BM / 4) + p.parts - 1) / p.parts, t0 = part * share, n_mine = min(share, rows * (BM / 4) - t0);     // of four numbers
-  const float4* ours = reinterpret_cast<const float4*>(sums) + t0;
-  int stride = 0;
-  if (p.parts > 1) {
+  const int share = (rows * (BM / 4) + p.parts - 1) / p.parts, t0 = part * share;     // of four numbers
+  const int n_mine = S::PUSH ? rows * my_quads : min(share, rows * (BM / 4) - t0);
+  const float4* ours = S::PUSH ? reinterpret_cast<const float4*>(here) : reinterpret_cast<const float4*>(sums) + t0;
+  int stride = S::PUSH ? rows * quads : 0;
+  if (S::PUSH && p.parts > 1) {
+    // (Read from the others behind a barrier of the cluster they took 1,800 clocks.)
+    if (!__syncthreads_and(wait_pushed(&sh->pushed))) {
+      if (threadIdx.x == 0) atomicOr(p.status, JV_STATUS_WAIT_EXPIRED);
+      cluster_sync();                                  // what others have pushed, or may yet push, finds this block there
+    }
+  } else if (!S::PUSH && p.parts > 1) {
     __syncwarp();
     cluster_sync();
     // they come here first, each block's from its own part on: read in their order, by all blocks alike, they took 4,600 clocks of 112 rows
-    float4* here = reinterpret_cast<float4*>(sums) + NB * (BM / 4);
+    float4* all = reinterpret_cast<float4*>(sums) + NB * (BM / 4);
     for (int u = threadIdx.x; u < p.parts * share; u += S::THREADS) {
       const int turn = u / share, e = u - turn * share, q = turn + part < p.parts ? turn + part : turn + part - p.parts;
-      if (e < n_mine) here[q * share + e] = cluster_load(smem_u32(ours + e), q);
+      if (e < n_mine) all[q * share + e] = cluster_load(smem_u32(ours + e), q);
     }
     __syncthreads();
     cluster_leave();
-    ours = here;
+    ours = all;
     stride = share;
   }
   pdl_wait();                                          // nothing is written before the kernels before this one are done
   const bool vec = sizeof(TC) == 4 && (((uintptr_t)p.C | (p.ldc * sizeof(TC)) | (p.c_batch * sizeof(TC))) & 15) == 0;
   TC* C = (TC*)p.C + blockIdx.y * p.c_batch + (size_t)m0 * p.ldc + n0;
   for (int e = threadIdx.x; e < n_mine; e += S::THREADS) {
-    const int m = (t0 + e) / (BM / 4), n = (t0 + e) % (BM / 4) * 4;
+    int m = (t0 + e) / (BM / 4), n = (t0 + e) % (BM / 4) * 4, at = e;
+    if (S::PUSH) {
+      m = e / my_quads;
+      n = (quad0 + e - m * my_quads) * 4;
+      at = m * quads + e - m * my_quads;
+    }
     if (n0 + n >= p.N || (p.row_token != nullptr && p.row_token[m0 + m] < 0)) continue;
     float y[4] = {0.f, 0.f, 0.f, 0.f};
     for (int q = 0; q < p.parts; ++q) {
-      const float4 v = ours[q * stride + e];
+      const float4 v = ours[q * stride + at];
       y[0] += v.x; y[1] += v.y; y[2] += v.z; y[3] += v.w;
     }
     TC* dst = C + (size_t)m * p.ldc + n;
@@ -459,7 +551,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     for (int i = 0; i < 4; ++i)
       if (n0 + n + i < p.N) dst[i] = from_f32<TC>(y[i]);
   }
-  if (p.parts > 1) {                                   // the others may still read this block's sums
+  if (!S::PUSH && p.parts > 1) {                       // the others may still read this block's sums
     __syncwarp();
     cluster_left();
   }

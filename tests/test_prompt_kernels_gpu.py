@@ -809,6 +809,19 @@ def test_tiles_and_parts_of_the_32bit_product(m, n, k):
         assert torch.equal(ops.gemm_simt(x[first:first + rows], w, torch.float32), y[first:first + rows])
 
 
+@pytest.mark.parametrize("n,k", [(128, 64), (200, 96), (1600, 1024), (2000, 320), (3600, 1056), (4260, 1024), (7000, 260), (9000, 128)])
+@pytest.mark.parametrize("wide", [torch.float32, torch.bfloat16])
+def test_few_rows_of_the_32bit_product(n, k, wide):
+    """One to six parts of k, whose sums are pushed to the block that adds them up: the bits of many rows, for which they are read."""
+    ops = _ops()
+    x, w = _rand(40, k, seed=1, dtype=wide), _rand(n, k, seed=2)
+    y, want = ops.gemm_simt(x, w, torch.float32), x.double() @ w.double().T
+    assert (y.double() - want).norm() <= 4e-7 * want.norm()
+    for first, rows in ((0, 1), (3, 2), (0, 7), (20, 8), (5, 9), (24, 16)):
+        assert torch.equal(ops.gemm_simt(x[first:first + rows], w, torch.float32), y[first:first + rows])
+    ops.check_status()
+
+
 def test_product_32bit_of_more_than_2_to_the_33_numbers():
     ops, m, n, k = _ops(), 1 << 20, 8200, 8
     x, w = _rand(m, k, seed=1, dtype=torch.bfloat16), _rand(n, k, seed=2, dtype=torch.bfloat16)
