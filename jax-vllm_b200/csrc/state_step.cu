@@ -19,6 +19,7 @@
 // 32 heads of 64 x 64: 2.8 and 7.3, 8.0 in one).
 #include "scan.cuh"
 #include <math.h>
+#include <type_traits>
 
 namespace {
 constexpr int THREADS = 256, ROWS = 8;     // state rows a thread
@@ -31,25 +32,29 @@ struct StepParams {
   float* state_n; float* nq; int nq_stride;  // the normaliser's column (value 1) and where its outputs go, or null
   const int* cu_seqlens; const int* slots;
   int n_slots, heads, D, V;
-  const void *b, *c, *dt_raw; long long bc_stride, dt_stride;      // MAMBA: rows of B, C and the raw step sizes, instead of packed
+  const int* work; int compact;            // pairs (entry, -), or null: every entry; a row of packed for every pair, not every token
+  int* status;
+};
+// What the kinds that form their vectors are given besides, instead of packed.
+struct FormParams : StepParams {
+  const void *b, *c, *dt_raw; long long bc_stride, dt_stride;      // MAMBA: rows of B, C and the raw step sizes
   const void *dt_bias, *a_log; int w_dtype, per_group;
   // GLA: q and k in b and c, the low-rank numbers in dt_raw; their matrix [heads * D, rank] and bias [heads * D] in dt_bias and a_log
   int rank; float inv_tau, q_scale;
   // DELTA: r and k in c and b, z_a in dt_raw, their biases a_bias and w_bias [heads * D] in dt_bias and a_log, zw rows of its own
   const void* zw; long long zw_stride;
-  const int* work; int compact;            // pairs (entry, -), or null: every entry; a row of packed for every pair, not every token
-  int* status;
 };
 
 // RG: row groups (D <= ROWS * RG); a thread's rows are rg, rg + RG, ...
 enum : int { PLAIN, REMOVAL_TERM, MAMBA, GLA, DELTA };
+template <int KIND> using ParamsOf = std::conditional_t<KIND == PLAIN || KIND == REMOVAL_TERM, StepParams, FormParams>;
 
 __device__ __forceinline__ float weight_at(const void* w, int dtype, size_t i) {
   return dtype == 0 ? ((const float*)w)[i] : to_f32(((const __nv_bfloat16*)w)[i]);
 }
 
 template <int RG, int VEC, int KIND, typename T>
-__global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p) {
+__global__ void __launch_bounds__(THREADS) state_step_kernel(const ParamsOf<KIND> p) {
   constexpr bool REMOVAL = KIND == REMOVAL_TERM || KIND == DELTA;
   constexpr int CQ = THREADS / RG, COLS = CQ * VEC, NV = REMOVAL ? 5 : 3;
   __shared__ float vec[NV * ROWS * RG];
@@ -217,28 +222,19 @@ __global__ void __launch_bounds__(THREADS) state_step_kernel(const StepParams p)
   if (n_g != nullptr) *n_g = n_state;
 }
 
-template <int RG, typename T>
-int dispatch(const StepParams& p, int kind, bool vec, int entries, cudaStream_t stream) {
+template <int RG, int KIND, typename T>
+int launch(const ParamsOf<KIND>& p, bool vec, int entries, cudaStream_t stream) {
   const int cols = THREADS / RG * (vec ? 4 : 1);
   const dim3 grid(entries, p.heads, (p.V + cols - 1) / cols);
-  if (vec)
-    return kind == REMOVAL_TERM ? jv_launch(state_step_kernel<RG, 4, REMOVAL_TERM, T>, grid, dim3(THREADS), 0, stream, p)
-           : kind == MAMBA      ? jv_launch(state_step_kernel<RG, 4, MAMBA, T>, grid, dim3(THREADS), 0, stream, p)
-           : kind == GLA        ? jv_launch(state_step_kernel<RG, 4, GLA, T>, grid, dim3(THREADS), 0, stream, p)
-           : kind == DELTA      ? jv_launch(state_step_kernel<RG, 4, DELTA, T>, grid, dim3(THREADS), 0, stream, p)
-                                : jv_launch(state_step_kernel<RG, 4, PLAIN, T>, grid, dim3(THREADS), 0, stream, p);
-  return kind == REMOVAL_TERM ? jv_launch(state_step_kernel<RG, 1, REMOVAL_TERM, T>, grid, dim3(THREADS), 0, stream, p)
-         : kind == MAMBA      ? jv_launch(state_step_kernel<RG, 1, MAMBA, T>, grid, dim3(THREADS), 0, stream, p)
-         : kind == GLA        ? jv_launch(state_step_kernel<RG, 1, GLA, T>, grid, dim3(THREADS), 0, stream, p)
-         : kind == DELTA      ? jv_launch(state_step_kernel<RG, 1, DELTA, T>, grid, dim3(THREADS), 0, stream, p)
-                              : jv_launch(state_step_kernel<RG, 1, PLAIN, T>, grid, dim3(THREADS), 0, stream, p);
+  return vec ? jv_launch(state_step_kernel<RG, 4, KIND, T>, grid, dim3(THREADS), 0, stream, p)
+             : jv_launch(state_step_kernel<RG, 1, KIND, T>, grid, dim3(THREADS), 0, stream, p);
 }
 
-template <typename T> int by_size(const StepParams& p, int kind, int entries, cudaStream_t stream) {
+template <int KIND, typename T> int by_size(const ParamsOf<KIND>& p, int entries, cudaStream_t stream) {
   const bool vec = p.V % 4 == 0 && ((uintptr_t)p.state & 15) == 0 && p.slot_stride % 4 == 0;
-  if (p.D <= 64) return dispatch<8, T>(p, kind, vec, entries, stream);
-  if (p.D <= 128) return dispatch<16, T>(p, kind, vec, entries, stream);
-  return dispatch<32, T>(p, kind, vec, entries, stream);
+  if (p.D <= 64) return launch<8, KIND, T>(p, vec, entries, stream);
+  if (p.D <= 128) return launch<16, KIND, T>(p, vec, entries, stream);
+  return launch<32, KIND, T>(p, vec, entries, stream);
 }
 }  // namespace
 
@@ -250,9 +246,9 @@ JV_EXPORT int jv_state_step(const float* packed, int removal, const void* v, int
                             int* status, cudaStream_t stream) {
   if (entries == 0) return JV_OK;
   if ((compact && work == nullptr) || heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || (removal && state_n != nullptr)) return JV_ERR_UNSUPPORTED;
-  StepParams p{packed, v, v_stride, v_off, out, state, slot_stride, state_n, nq, nq_stride, cu_seqlens, slots, n_slots, heads, D, V,
-               nullptr, nullptr, nullptr, 0, 0, nullptr, nullptr, 0, 1, 0, 0.f, 0.f, nullptr, 0, work, compact, status};
-  JV_DISPATCH_DTYPE(v_dtype, T, return by_size<T>(p, removal != 0 ? REMOVAL_TERM : PLAIN, entries, stream));
+  const StepParams p{packed, v, v_stride, v_off, out, state, slot_stride, state_n, nq, nq_stride, cu_seqlens, slots, n_slots, heads, D, V,
+                     work, compact, status};
+  JV_DISPATCH_DTYPE(v_dtype, T, return removal != 0 ? by_size<REMOVAL_TERM, T>(p, entries, stream) : by_size<PLAIN, T>(p, entries, stream));
   return JV_ERR_UNSUPPORTED;
 }
 
@@ -266,10 +262,11 @@ JV_EXPORT int jv_mamba_step(const void* xbc, int dtype, long long xbc_stride, in
   if (heads < 1 || groups < 1 || heads % groups || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || w_dtype < 0 || w_dtype > 1)
     return JV_ERR_UNSUPPORTED;
   const size_t size = dtype == 0 ? 4 : 2;
-  StepParams p{nullptr, xbc, xbc_stride, 0, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
-               (const char*)xbc + b_off * size, (const char*)xbc + c_off * size, dt_raw, xbc_stride, dt_stride, dt_bias, a_log, w_dtype,
-               heads / groups, 0, 0.f, 0.f, nullptr, 0, work, 0, status};
-  JV_DISPATCH_DTYPE(dtype, T, return by_size<T>(p, MAMBA, entries, stream));
+  const FormParams p{{nullptr, xbc, xbc_stride, 0, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
+                      work, 0, status},
+                     (const char*)xbc + b_off * size, (const char*)xbc + c_off * size, dt_raw, xbc_stride, dt_stride, dt_bias, a_log, w_dtype,
+                     heads / groups, 0, 0.f, 0.f, nullptr, 0};
+  JV_DISPATCH_DTYPE(dtype, T, return (by_size<MAMBA, T>(p, entries, stream)));
   return JV_ERR_UNSUPPORTED;
 }
 
@@ -283,10 +280,11 @@ JV_EXPORT int jv_gla_step(const void* proj, int dtype, long long stride, int q_o
   if (heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || rank < 1 || w_dtype < 0 || w_dtype > 1) return JV_ERR_UNSUPPORTED;
   const size_t size = dtype == 0 ? 4 : 2;
   const char* row = (const char*)proj;
-  StepParams p{nullptr, proj, stride, v_off, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
-               row + q_off * size, row + k_off * size, row + low_off * size, stride, stride, w_up, bias, w_dtype, 1, rank, inv_tau, q_scale,
-               nullptr, 0, nullptr, 0, status};
-  JV_DISPATCH_DTYPE(dtype, T, return by_size<T>(p, GLA, entries, stream));
+  const FormParams p{{nullptr, proj, stride, v_off, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
+                      nullptr, 0, status},
+                     row + q_off * size, row + k_off * size, row + low_off * size, stride, stride, w_up, bias, w_dtype, 1, rank, inv_tau,
+                     q_scale, nullptr, 0};
+  JV_DISPATCH_DTYPE(dtype, T, return (by_size<GLA, T>(p, entries, stream)));
   return JV_ERR_UNSUPPORTED;
 }
 
@@ -300,9 +298,10 @@ JV_EXPORT int jv_delta_step(const void* proj, int dtype, long long stride, int r
   if (heads < 1 || D < 1 || D > ROWS * 32 || V < 1 || heads > 65535 || w_dtype < 0 || w_dtype > 1) return JV_ERR_UNSUPPORTED;
   const size_t size = dtype == 0 ? 4 : 2;
   const char* row = (const char*)proj;
-  StepParams p{nullptr, proj, stride, v_off, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
-               row + k_off * size, row + r_off * size, row + a_off * size, stride, stride, a_bias, w_bias, w_dtype, 1, 0, 0.f, 0.f,
-               zw, zw_stride, work, 0, status};
-  JV_DISPATCH_DTYPE(dtype, T, return by_size<T>(p, DELTA, entries, stream));
+  const FormParams p{{nullptr, proj, stride, v_off, out, state, slot_stride, nullptr, nullptr, 0, cu_seqlens, slots, n_slots, heads, D, V,
+                      work, 0, status},
+                     row + k_off * size, row + r_off * size, row + a_off * size, stride, stride, a_bias, w_bias, w_dtype, 1, 0, 0.f, 0.f,
+                     zw, zw_stride};
+  JV_DISPATCH_DTYPE(dtype, T, return (by_size<DELTA, T>(p, entries, stream)));
   return JV_ERR_UNSUPPORTED;
 }
