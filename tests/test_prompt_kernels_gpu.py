@@ -822,6 +822,16 @@ def test_few_rows_of_the_32bit_product(n, k, wide):
     ops.check_status()
 
 
+@pytest.mark.parametrize("m", [3, 40])
+@pytest.mark.parametrize("exponent,limit", [(-105, 4e-7), (-110, 4e-7), (-115, 4e-6)])
+def test_product_32bit_of_small_numbers(m, exponent, limit):
+    """Down to 2^-110 the parts hold a number exactly; below, what is smaller than bfloat16's smallest (2^-133) is lost."""
+    ops = _ops()
+    for small, other in ((_rand(m, 512, seed=1, scale=2.0 ** exponent), _rand(200, 512, seed=2)), (_rand(m, 512, seed=1), _rand(200, 512, seed=2, scale=2.0 ** exponent))):
+        y, want = ops.gemm_simt(small, other, torch.float32), small.double() @ other.double().T
+        assert (y.double() - want).norm() <= limit * want.norm()
+
+
 def test_product_32bit_of_more_than_2_to_the_33_numbers():
     ops, m, n, k = _ops(), 1 << 20, 8200, 8
     x, w = _rand(m, k, seed=1, dtype=torch.bfloat16), _rand(n, k, seed=2, dtype=torch.bfloat16)
