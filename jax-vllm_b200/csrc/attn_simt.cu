@@ -527,7 +527,7 @@ int vec_stages(int D, int DV) {
 bool vec_takes(const AttnParams& p, int dtype) {
   const auto whole = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
   return dtype == 0 && p.head_dim % 4 == 0 && (p.v_dim == 32 || p.v_dim == 64 || p.v_dim == 128 || p.v_dim == 256 || p.v_dim == 512) &&
-         p.v_row % 4 == 0 && p.q_stride % 4 == 0 && whole(p.q) && whole(p.k_cache) && whole(p.v_cache) &&
+         p.v_row % 4 == 0 && p.q_stride % 4 == 0 && whole(p.q) && whole(p.k_cache) && whole(p.v_cache) && whole(p.part_o) &&
          vec_smem(p.head_dim, p.v_dim, 2) <= MAX_SMEM - 2048;
 }
 

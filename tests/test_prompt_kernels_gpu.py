@@ -982,6 +982,32 @@ def test_rows_of_32_bit_attention(hq, hk, d, dv, page, option, split):
     assert (outs[0] - outs[1]).norm() <= 2e-6 * outs[1].norm()       # (random rows: a few roundings' root mean square)
 
 
+def _off_boundaries(monkeypatch, ops, taken):
+    """torch.empty gives float tensors one number off a 16-byte boundary where `taken(shape)` (a caller's own scratch may lie there)."""
+    empty = torch.empty
+
+    def off(*shape, **kw):
+        if kw.get("dtype") is not torch.float32 or not taken(shape[0]):
+            return empty(*shape, **kw)
+        size = torch.Size(shape[0] if isinstance(shape[0], tuple) else shape)
+        return empty(size.numel() + 4, **kw)[1:1 + size.numel()].view(size)
+    monkeypatch.setattr(ops.torch, "empty", off)
+
+
+def test_32_bit_attention_with_scratch_off_boundaries(monkeypatch):
+    ops, hq, hk, d, page, length = _ops(), 4, 2, 64, 16, 100
+    k, v = (_rand(7, page, hk, d, seed=i) for i in (1, 2))
+    table = torch.arange(7, dtype=torch.int32, device="cuda")[None]
+    cu, start, work = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, 1], [length - 1], [[0, 0]]))
+    q, outs = _rand(1, hq * d, seed=3), [torch.zeros(1, hq * d, device="cuda") for _ in range(2)]
+    for out in outs:
+        ops.attn_simt(q, q.stride(0), out, k, v, table, cu, start, work, 1, hq, hk, d, 0, 0.1, split_size=32, n_splits=4)
+        _off_boundaries(monkeypatch, ops, lambda shape: isinstance(shape, int))
+    ops.check_status()
+    # two orders of sums of 100 weights
+    assert (outs[0] - outs[1]).abs().max() <= 200 * EPS32 * float(v.abs().max())
+
+
 # ------------------------------------------------------------------------------- heads of 64 on the tcgen05 prompt kernel
 @pytest.mark.parametrize("hq,hk,page", [(4, 1, 16), (16, 1, 8), (6, 2, 64), (3, 3, 128), (10, 2, 32)])
 @pytest.mark.parametrize("option", ["plain", "window", "chunk", "kept, capped", "sigmoid", "shaped"])
