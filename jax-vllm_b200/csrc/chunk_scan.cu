@@ -533,17 +533,22 @@ __global__ void __launch_bounds__(OUT_THREADS, DP <= 128 ? 2 : 1) chunk_output_k
   }
   const size_t orow = (size_t)p.heads * p.V;
   float* o = p.out + (size_t)c.t0 * orow + (size_t)h * p.V + e0;
+  const bool pairs = ((uintptr_t)o & 7) == 0;          // a caller's result may start on any number
+  auto put = [&](float* dst, float x, float y) {
+    if (pairs) {
+      *reinterpret_cast<float2*>(dst) = make_float2(x, y);
+    } else {
+      dst[0] = x;
+      dst[1] = y;
+    }
+  };
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int lc = j * 8 + gq * 2;
     if (e0 + lc >= p.V) continue;
     const int bad0 = bad[lc], bad1 = bad[lc + 1];
-    if (ta < c.here)
-      *reinterpret_cast<float2*>(o + ta * orow + lc) = make_float2(bad0 <= ta ? NAN : O[j][0] * p.scale,
-                                                                    bad1 <= ta ? NAN : O[j][1] * p.scale);
-    if (tb < c.here)
-      *reinterpret_cast<float2*>(o + tb * orow + lc) = make_float2(bad0 <= tb ? NAN : O[j][2] * p.scale,
-                                                                    bad1 <= tb ? NAN : O[j][3] * p.scale);
+    if (ta < c.here) put(o + ta * orow + lc, bad0 <= ta ? NAN : O[j][0] * p.scale, bad1 <= ta ? NAN : O[j][1] * p.scale);
+    if (tb < c.here) put(o + tb * orow + lc, bad0 <= tb ? NAN : O[j][2] * p.scale, bad1 <= tb ? NAN : O[j][3] * p.scale);
   }
 }
 

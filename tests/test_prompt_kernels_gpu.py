@@ -25,6 +25,18 @@ def _entries(lengths):
     return cu, slots, len(lengths) + 2
 
 
+def _off_boundaries(monkeypatch, ops, taken):
+    """torch.empty gives float tensors one number off a 16-byte boundary where `taken(shape)` (a caller's own scratch may lie there)."""
+    empty = torch.empty
+
+    def off(*shape, **kw):
+        if kw.get("dtype") is not torch.float32 or not taken(shape[0]):
+            return empty(*shape, **kw)
+        size = torch.Size(shape[0] if isinstance(shape[0], tuple) else shape)
+        return empty(size.numel() + 4, **kw)[1:1 + size.numel()].view(size)
+    monkeypatch.setattr(ops.torch, "empty", off)
+
+
 # ------------------------------------------------------------------------------- the 32-bit product
 @pytest.mark.parametrize("m", [1, 2, 3, 8, 16, 17, 64, 65, 200])
 @pytest.mark.parametrize("n,k", [(1, 1), (31, 5), (33, 127), (64, 128), (65, 129), (100, 260), (700, 1000), (64, 2304)])
@@ -290,6 +302,19 @@ def test_chunked_states_over_several_chunks(heads, dim, columns):
     for got, want in ((o[taken & finite.all(1)], o_want[taken & finite.all(1)]), (st[left], st_want[left]), (nq[taken], nq_want[taken])):
         # two 32-bit sums of up to 300 + 256 terms
         assert (got.double() - want.double()).norm() <= 3e-6 * want.double().norm()
+
+
+def test_chunked_states_into_a_result_off_boundaries(monkeypatch):
+    ops, heads, dim, columns, n = _ops(), 2, 16, 24, 150
+    cu, slots, n_slots = _entries([n])
+    row = _rand(n, heads * columns + 2 * heads * dim, seed=1, dtype=torch.bfloat16)
+    dt_raw, bias, rows, outs = _rand(n, heads, seed=3, dtype=torch.bfloat16), _rand(heads, seed=4), _rand(n_slots, heads * dim * columns, seed=5), []
+    for _ in range(2):
+        outs.append(ops.chunk_scan(row, heads * (columns + dim), heads * columns, 0, rows.clone(), cu, slots, 1, heads, heads, dim, columns,
+                                   dt_raw=dt_raw, dt_bias=bias, a_log=bias))
+        _off_boundaries(monkeypatch, ops, lambda shape: isinstance(shape, tuple))
+    ops.check_status()
+    assert outs[0].data_ptr() % 16 == 0 and outs[1].data_ptr() % 16 == 4 and torch.equal(*outs)
 
 
 @pytest.mark.parametrize("heads,groups,dim,columns,at_once", [(5, 1, 64, 64, 1), (6, 2, 136, 24, 4), (8, 8, 16, 72, 3)])
@@ -980,18 +1005,6 @@ def test_rows_of_32_bit_attention(hq, hk, d, dv, page, option, split):
     bound = (2 * (d + 8) * size + 140) * EPS32 * float(torch.nan_to_num(caches[1]).abs().max()) * (131 if option == "sigmoid" else 2)
     assert torch.isfinite(outs[0]).all() and (outs[0] - outs[1]).abs().max() <= bound
     assert (outs[0] - outs[1]).norm() <= 2e-6 * outs[1].norm()       # (random rows: a few roundings' root mean square)
-
-
-def _off_boundaries(monkeypatch, ops, taken):
-    """torch.empty gives float tensors one number off a 16-byte boundary where `taken(shape)` (a caller's own scratch may lie there)."""
-    empty = torch.empty
-
-    def off(*shape, **kw):
-        if kw.get("dtype") is not torch.float32 or not taken(shape[0]):
-            return empty(*shape, **kw)
-        size = torch.Size(shape[0] if isinstance(shape[0], tuple) else shape)
-        return empty(size.numel() + 4, **kw)[1:1 + size.numel()].view(size)
-    monkeypatch.setattr(ops.torch, "empty", off)
 
 
 def test_32_bit_attention_with_scratch_off_boundaries(monkeypatch):
