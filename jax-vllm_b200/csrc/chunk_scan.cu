@@ -24,7 +24,7 @@
 // in the tensor core: 3.4e-7 relative for 128 channels, this way 0.8e-7, as token by token).  L is summed in 64-bit and kept as two
 // floats: L_t - L_s keeps its digits behind a large decay.  The normaliser's sums are made on the CUDA cores.
 //
-// What bounds it: the two kernels on the tensor cores, their rate of mma.sync (one a 2.2 clocks and multiprocessor at best; 4.7 and 5.5
+// What bounds it: the two kernels on the tensor cores, their rate of mma.sync (one a 2.2 clocks and multiprocessor at best; 4.8 and 5.7
 // here), the middle one its bytes.  4,096 tokens in three entries, 128 heads of 128 x 64: 115, 55 and 259 us; chunks of 32 that a
 // block went through in order took 620.  2,048 tokens of 8 heads of 128 x 256 with a normaliser: 19, 9 and 39, where a scan token by token
 // in segments took 276; 2,000 tokens of 8 heads of 256 x 512: 58, 18 and 150 (888).  1,200 tokens of 64 heads of 128 x 64: 81 (172).

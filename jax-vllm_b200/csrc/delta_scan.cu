@@ -17,7 +17,7 @@
 // (group, head), fully parallel, and group_scan_kernel reads them through a ring of bulk copies.
 //
 // What bounds it is that chain's latency (0.5 us a group whatever the number of heads up to two blocks a multiprocessor).
-// 2,048 tokens of 32 heads of 64: prepare 40 and scan 201 us, where the token-by-token kernels took 69 and 815; 64 heads: 77 and 258.
+// 2,048 tokens of 32 heads of 64: prepare 40 and scan 197 us, where the token-by-token kernels took 69 and 815; 64 heads: 77 and 260.
 #include "mbarrier.cuh"
 #include "scan.cuh"
 
@@ -173,7 +173,7 @@ struct GroupScanParams {
 // lanes is a run of 128 bytes; a warp takes 64 / LANES columns of one (entry, head), a block twice as many.  Two columns a thread:
 // shared memory hands out 128 bytes a clock and each number read should serve more than one multiply-add.
 // Eight lanes; 16, which halves what a warp has to do in a group for one more step of every sum over the lanes, where the blocks of eight
-// would leave multiprocessors without one and keys have 64 channels or more (32 heads of 64, 2,048 tokens: 258 us with eight, 201 with 16).
+// would leave multiprocessors without one and keys have 64 channels or more (32 heads of 64, 2,048 tokens: 258 us with eight, 197 with 16).
 // Which of the two hangs on the portions of the step, a portion's sums do not: both add the same numbers in the same order.
 // RING_: the stages of the ring.  Six (about 100 KB, two blocks a multiprocessor) carry a block through the latency of its copies;
 // where there are more blocks than two a multiprocessor, others do that, and two stages leave room for more of them (32 heads of 64:

@@ -36,7 +36,7 @@ struct ConvParams {
 // are rounded to 16 bits right away are first formed with 1 / d to 2^-23, which makes them exact to 2^-22: the 16-bit numbers are the
 // quotients' unless a boundary of the rounding lies as near as that (2^-21 to either side rounds differently then), or d so large that
 // 1 / d is no normal number.  Those are divided, so that every kernel gives the quotient, rounded.
-// (4,096 tokens of 10,240 channels: 84 us with the division throughout, 63.5 so.)
+// (4,096 tokens of 10,240 channels: 77 us with the division throughout, 56.7 so.)
 template <typename TO, int N> __device__ __forceinline__ void silu(float (&y)[N]) {
   if constexpr (sizeof(TO) == 2) {
     float q[N + 1], least = y[0];
@@ -321,8 +321,9 @@ JV_EXPORT int jv_short_conv(const void* in, int in_dtype, long long in_stride, v
   p.n_slots = n_slots; p.channels = channels; p.act = act; p.residual = residual ? 1 : 0; p.status = status;
   // Four channels a thread where entries have some tokens (or there are 8 M elements), for two to four taps and rows on four-element
   // boundaries; segments as long as the device still fills, since each reads the weights and the taps - 1 inputs before it.  10,240
-  // channels, one entry of 130, 700, 4,096 tokens: 4.9, 10.5, 45 us, against 9.5, 19.5, 108 a channel a thread (segments of 32
-  // throughout: 7.4, 14, 45; of 8: 4.9, 11, 53).  Entries of one token each a channel a thread: 32 of 2,176 channels 5.4 against 7.1.
+  // channels, one entry of 130, 700, 4,096 tokens: 5.7, 13.0, 56.7 us, against 9.5, 19.5, 108 a channel a thread (with a silu by the reciprocal
+  // alone 4.7, 10.2 and 44.4, segments of 32 throughout 7.4, 14, 45; of 8 4.9, 11, 53).  Entries of one token each a channel a thread: 32 of 2,176
+  // channels 5.1 against 7.1.
   auto fours = [](const void* q, long long stride, int dtype) {
     return ((uintptr_t)q & (dtype == 0 ? 15 : 7)) == 0 && stride % VEC == 0;
   };
