@@ -33,14 +33,15 @@ struct ConvParams {
 };
 
 // y <- y * sigmoid(y) = y / d, d = 1 + exp(-y).  The dozen instructions of a division were what a long portion waited for, so results that
-// are rounded to 16 bits right away are first formed with 1 / d to 2^-23, which makes them exact to 2^-22: the 16-bit numbers are the
-// quotients' unless a boundary of the rounding lies as near as that (2^-21 to either side rounds differently then), or d so large that
-// 1 / d is no normal number.  Those are divided, so that every kernel gives the quotient, rounded.
-// (4,096 tokens of 10,240 channels: 77 us with the division throughout, 56.7 so.)
+// are rounded to 16 bits right away are first formed with 1 / d to 2^-23, which leaves them within four units in the last place of the
+// quotient, rounded to 32 bits.  Both round to the same 16-bit number unless a boundary of that rounding (a lower half of 0x8000) is as near;
+// where it is within eight, one result in 4,000, or d so large that 1 / d is no normal number, the four of a thread are divided, so that
+// every kernel gives the quotient, rounded.  (4,096 tokens of 10,240 channels: 77 us with the division throughout, 44.4 with the reciprocal
+// alone, 54.8 so.)
 template <typename TO, int N> __device__ __forceinline__ void silu(float (&y)[N]) {
   if constexpr (sizeof(TO) == 2) {
-    float q[N + 1], least = y[0];
-    uint32_t differ = 0;
+    float q[N], least = y[0];
+    uint32_t nearest = 0xffffffffu;                    // two at a time: how far a lower half lies above eight units below the boundary
 #pragma unroll
     for (int e = 0; e < N; ++e) {
       float r;
@@ -48,18 +49,11 @@ template <typename TO, int N> __device__ __forceinline__ void silu(float (&y)[N]
       q[e] = y[e] * r;
       least = fminf(least, y[e]);
     }
-    q[N] = q[N - 1];
+    // (a borrow of the first moves the second by one unit, which the eight leave room for)
 #pragma unroll
-    for (int e = 0; e < N; e += 2) {
-      constexpr float BIT = 1.f / (1 << 21);
-      const uint64_t pair = pack2(q[e], q[e + 1]);
-      float a, b, c, d;
-      unpack2(mul2(pair, pack2(1.f + BIT, 1.f + BIT)), a, b);
-      unpack2(mul2(pair, pack2(1.f - BIT, 1.f - BIT)), c, d);
-      const __nv_bfloat162 up = __floats2bfloat162_rn(a, b), down = __floats2bfloat162_rn(c, d);
-      differ |= *reinterpret_cast<const uint32_t*>(&up) ^ *reinterpret_cast<const uint32_t*>(&down);
-    }
-    if (differ == 0 && least > -80.f) {
+    for (int e = 0; e < N; e += 2)
+      nearest = __vminu2(nearest, __byte_perm(__float_as_uint(q[e]), __float_as_uint(q[e + 1 < N ? e + 1 : e]), 0x5410) - 0x7ff87ff8u);
+    if ((nearest & 0xffffu) > 16 && nearest >> 16 > 16 && least > -80.f) {
 #pragma unroll
       for (int e = 0; e < N; ++e) y[e] = q[e];
       return;
@@ -321,7 +315,7 @@ JV_EXPORT int jv_short_conv(const void* in, int in_dtype, long long in_stride, v
   p.n_slots = n_slots; p.channels = channels; p.act = act; p.residual = residual ? 1 : 0; p.status = status;
   // Four channels a thread where entries have some tokens (or there are 8 M elements), for two to four taps and rows on four-element
   // boundaries; segments as long as the device still fills, since each reads the weights and the taps - 1 inputs before it.  10,240
-  // channels, one entry of 130, 700, 4,096 tokens: 5.7, 13.0, 56.7 us, against 9.5, 19.5, 108 a channel a thread (with a silu by the reciprocal
+  // channels, one entry of 130, 700, 4,096 tokens: 5.5, 12.8, 54.8 us, against 9.5, 19.5, 108 a channel a thread (with a silu by the reciprocal
   // alone 4.7, 10.2 and 44.4, segments of 32 throughout 7.4, 14, 45; of 8 4.9, 11, 53).  Entries of one token each a channel a thread: 32 of 2,176
   // channels 5.1 against 7.1.
   auto fours = [](const void* q, long long stride, int dtype) {
